@@ -94,8 +94,9 @@ typedef struct og_engine_config {
     uint32_t dump;     /* 1: ignore the bitmap, every candidate survives (parity runs) */
     uint32_t room;     /* survivor records per advance; 0 sizes it from the bitmaps' occupancy:
                           the expected count plus eight standard deviations */
-    uint32_t lanes_per_thread; /* paired: lanes each thread of the search kernel carries, 1 or 2
-                          (0: 1); `lanes` is then a multiple of block x this. Chain: 1 */
+    uint32_t lanes_per_thread; /* paired: lanes each thread of the search kernel takes at a time,
+                          1 or 2, one after the other (0: 1); `lanes` is then a multiple of
+                          block x this. Chain: 1 */
 } og_engine_config;
 
 /* The same engine with an explicit shape (no tuning). `bitmap` may be NULL

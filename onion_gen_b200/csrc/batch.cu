@@ -61,6 +61,7 @@
 namespace og {
 
 const std::vector<uint4>& pair_table(uint32_t half);           // engine.cu
+std::array<FeWords, 3> stride_words(const Pt& w);              // engine.cu
 std::vector<uint4> pow2_table(const Pt& stride, uint32_t nbits);  // engine.cu
 MatchTables match_tables(const std::vector<FilterSet::DeviceBucket>& buckets, const uint64_t* keys,
                          const uint32_t* owners, const uint32_t* patterns,
@@ -87,7 +88,7 @@ constexpr double NEED_STEPS = 2.0;
 constexpr size_t STAGED_BYTES = (size_t)(1u << STAGED_BITMAP_BITS) / 8u;
 
 struct BatchDesc {
-    FeWords wx, wy, wt;      // the search's stride for this step: L (2 half + 1) 8 G, affine
+    FeWords wx, wy, wdt;     // the search's stride for this step: W = L (2 half + 1) 8 G, affine, and d wx wy
     FeWords bx, by, bz, bt;  // centre of window W_done (where new lanes start), extended
     const uint32_t* bitmap;  // prefix bitmap (nullptr: the search has no prefix)
     uint32_t bits;
@@ -133,11 +134,11 @@ struct BatchArgs {
     uint32_t nblocks;
     uint4* lanes;    // ({x,y} * 2 + q) * slots + slot
     // per persistent CTA, a region of cta_scratch uint4 in which thread t's
-    // element e, part w, half q is at ((e * 2 + w) * 2 + q) * BLOCK + t
+    // prefix product m, half q is at (2 m + q) SCRATCH_ROW + t
     uint4* scratch;
     size_t cta_scratch;
     size_t slots;
-    const uint4* table;  // Q_m, m = 1..max half; a search of half h reads the first h
+    PairTable table;  // of Q_m, m = 1..max half; a search of half h reads the first h
     uint32_t rounds;
     HitRec* surv;  // the flight's
     uint32_t surv_cap;
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(BLOCK) batch_init_kernel(const BatchArgs a) {
 // 19.67-19.82 s, the searches' small bitmaps no longer competing with the
 // table Q_m for L1).
 __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_kernel(const BatchArgs a) {
-    const uint4* qtab = a.table;  // read through L1, as the single-search kernel does
+    __shared__ uint4 stage_s[(OG_LB_THREADS / 32) * STAGE_RECORDS * STAGE_WORDS];
     __shared__ uint32_t item_s, staged_s;  // staged_s: the search whose bitmap is in og_bitmap_s
     if (threadIdx.x == 0) staged_s = NONE;
     for (;;) {
@@ -203,13 +204,10 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_
         }
         const uint32_t slot = item * BLOCK + threadIdx.x;
         const Sink sink{d.bitmap, d.bits, a.surv, &a.counters->surv, a.surv_cap, sb.sidx, d.sbitmap, d.sbits, staged};
-        fe x = load_fe(a.lanes + 0 * a.slots + slot, a.slots);
-        fe y = load_fe(a.lanes + 2 * a.slots + slot, a.slots);
-        paired_rounds<false>(x, y, words_fe(d.wx), words_fe(d.wy), words_fe(d.wt), qtab, d.half, a.rounds,
-                      a.scratch + blockIdx.x * a.cta_scratch + threadIdx.x, (size_t)BLOCK,
-                      [&](const fe& v, uint32_t step) { test_emit(sink, v, slot, step); });
-        store_fe(a.lanes + 0 * a.slots + slot, a.slots, x);
-        store_fe(a.lanes + 2 * a.slots + slot, a.slots, y);
+        WarpStage st{stage_s + (threadIdx.x / 32) * STAGE_RECORDS * STAGE_WORDS, 0};
+        paired_rounds<false>(a.lanes + slot, a.slots, d.wx, d.wy, d.wdt, a.table, d.half, a.rounds,
+                             a.scratch + blockIdx.x * a.cta_scratch + threadIdx.x, sink, st, slot);
+        stage_flush(sink, a.table.vs, st.recs, st.n);
     }
 }
 
@@ -439,9 +437,7 @@ const std::array<FeWords, 3>& stride_for(og_batch* b, uint32_t lanes, uint32_t h
     const auto key = std::make_pair(lanes, half);
     auto it = b->strides.find(key);
     if (it != b->strides.end()) return it->second;
-    F51 x, y;
-    pt_affine(base_mult_u64(8ULL * (2ULL * half + 1) * lanes), x, y);
-    std::array<FeWords, 3> w{to_words(x), to_words(y), to_words(f_mul(x, y))};
+    const std::array<FeWords, 3> w = stride_words(base_mult_u64(8ULL * (2ULL * half + 1) * lanes));
     return b->strides.emplace(key, w).first->second;
 }
 
@@ -623,7 +619,7 @@ int launch(og_batch* b, bool& launched, char* err, size_t errlen) {
             BatchDesc& d = b->h_descs[s.sidx];
             d.wx = w[0];
             d.wy = w[1];
-            d.wt = w[2];
+            d.wdt = w[2];
             s.lanes_stride = lanes;
             b->mark(s.sidx);
         }
@@ -884,7 +880,7 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
     // its BLOCK threads, so a CTA's accesses stay within a few pages (config
     // 4's long searches at half 2048 on B200: 2.08e10 against 2.05e10 keys/s
     // with rows across the whole grid)
-    const size_t cta_scratch = (size_t)BLOCK * (2 * (size_t)cfg.max_half + 2) * 4;
+    const size_t cta_scratch = (size_t)SCRATCH_ROW * 2 * cfg.max_half;
     CU(b->scratch.alloc((size_t)b->grid * cta_scratch));
     const std::vector<uint4>& tab = pair_table(cfg.max_half);
     CU(b->table.alloc(tab.size()));
@@ -939,7 +935,7 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
         a.scratch = b->scratch.p;
         a.cta_scratch = cta_scratch;
         a.slots = S;
-        a.table = b->table.p;
+        a.table = PairTable{b->table.p, b->table.p + (size_t)cfg.max_half * 2};
         a.rounds = cfg.rounds;
         a.surv = f.surv.p;
         a.surv_cap = (uint32_t)surv_cap;

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstddef>
@@ -57,8 +58,23 @@ static void batch_affine(const std::vector<Pt>& pts, std::vector<F51>& xs, std::
     }
 }
 
-// The table Q_m = 8m G, m = 1..half, affine (x, y, xy), in the device
-// layout; the same for every search, so built once per half.
+// 1/d and d of the curve, for the paired round's table and strides.
+static const F51& inv_curve_d() {
+    static const F51 v = f_inv(curve_d());
+    return v;
+}
+
+// The stride words of the paired round: x, y and d x y of an affine point.
+std::array<FeWords, 3> stride_words(const Pt& w) {
+    F51 x, y;
+    pt_affine(w, x, y);
+    return {to_words(x), to_words(y), to_words(f_mul(curve_d(), f_mul(x, y)))};
+}
+
+// The paired round's table of Q_m = 8m G, m = 1..half (PairTable: q = 1/(d y^2)
+// of every entry, then v = 1/y and s = x/(1 + x^2) of every entry), in the
+// device layout; the same for every search, so built once per half. y and
+// 1 + x^2 are never 0 for a point of odd order.
 const std::vector<uint4>& pair_table(uint32_t half) {
     static std::mutex mu;
     static std::map<uint32_t, std::unique_ptr<std::vector<uint4>>> cache;
@@ -74,15 +90,27 @@ const std::vector<uint4>& pair_table(uint32_t half) {
     }
     std::vector<F51> xs, ys;
     batch_affine(pts, xs, ys);
-    auto v = std::make_unique<std::vector<uint4>>((size_t)half * 6);
+    // 1 / (y (1 + x^2)) of all entries with one inversion
+    std::vector<F51> prefix(half), den(half);
+    F51 run = f_one();
     for (uint32_t m = 0; m < half; m++) {
-        uint4* d = v->data() + (size_t)m * 6;
-        put_fe(d + 0, 1, xs[m]);
-        put_fe(d + 2, 1, ys[m]);
-        put_fe(d + 4, 1, f_mul(xs[m], ys[m]));
+        den[m] = f_add(f_one(), f_sq(xs[m]));
+        prefix[m] = run;
+        run = f_mul(run, f_mul(ys[m], den[m]));
     }
-    auto& ref = *v;
-    cache[half] = std::move(v);
+    F51 inv = f_inv(run);
+    auto tab = std::make_unique<std::vector<uint4>>((size_t)half * 6);
+    for (uint32_t m = half; m-- > 0;) {
+        const F51 i = f_mul(inv, prefix[m]);
+        inv = f_mul(inv, f_mul(ys[m], den[m]));
+        const F51 v = f_mul(den[m], i);
+        put_fe(tab->data() + (size_t)m * 2, 1, f_mul(f_sq(v), inv_curve_d()));
+        uint4* const vs = tab->data() + (size_t)half * 2 + (size_t)m * 4;
+        put_fe(vs + 0, 1, v);
+        put_fe(vs + 2, 1, f_mul(xs[m], f_mul(ys[m], i)));
+    }
+    auto& ref = *tab;
+    cache[half] = std::move(tab);
     return ref;
 }
 
@@ -248,13 +276,6 @@ size_t room_for(uint64_t batch, bool dump, double occupancy) {
     return (size_t)std::min<double>((double)batch, std::max(4096.0, want));
 }
 
-// Bitmaps that let more than this share of candidates through get the
-// paired kernel that stages survivor records per warp (one atomic per 32
-// records): on B200 the direct append ran 21.0 G keys/s at 1.5e-5 and 19.2
-// at 5.2e-2 of candidates surviving, the staged one a flat 20.4, and they
-// cross near 6e-3.
-constexpr double STAGE_OCCUPANCY = 6e-3;
-
 // Expected survivors of one advance that the default shape allows: 2^26
 // records, 3.2 GB of records per advance in flight.
 constexpr double SURVIVOR_BUDGET = (double)(1u << 26);
@@ -368,7 +389,6 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     e->cfg.room = (uint32_t)std::min<size_t>(e->cap, 0xffffffffu);
     const uint32_t coords = cfg.scheme == OG_SCHEME_CHAIN ? 4 : 2;
     CU(e->lanes.alloc(L * coords * 2));
-    const size_t elems = cfg.scheme == OG_SCHEME_CHAIN ? cfg.half : 2 * (size_t)cfg.half + 2;
     {
         // both kernels are persistent: scratch for the resident CTAs only
         // (the chain kernel's no more CTAs than blocks of lanes)
@@ -377,10 +397,10 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
         if (rc) return rc;
         e->grid = std::max<uint32_t>(1, resident / (cfg.block * lpt));
         if (cfg.scheme == OG_SCHEME_CHAIN) e->grid = std::min<uint32_t>(e->grid, (uint32_t)(L / cfg.block));
-        // one scratch column per lane a thread holds; a chain CTA's rows hold
-        // CHAIN_ROW threads whatever its block
-        const size_t row = cfg.scheme == OG_SCHEME_CHAIN ? CHAIN_ROW : (size_t)cfg.block * lpt;
-        CU(e->scratch.alloc((size_t)e->grid * row * elems * 4));
+        // a CTA's rows hold SCRATCH_ROW (CHAIN_ROW) threads whatever its
+        // block: a prefix product a pair, or a numerator and a denominator a step
+        const size_t col = cfg.scheme == OG_SCHEME_CHAIN ? 4 * CHAIN_ROW : 2 * OG_LB_THREADS;
+        CU(e->scratch.alloc((size_t)e->grid * col * cfg.half));
     }
     for (og_engine::Flight& f : e->fl) {
         CU(f.counts.alloc(4));
@@ -433,16 +453,13 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
         const std::vector<uint4>& tab = pair_table(cfg.half);
         CU(e->table.alloc(tab.size()));
         CU(cudaMemcpyAsync(e->table.p, tab.data(), tab.size() * sizeof(uint4), cudaMemcpyHostToDevice, e->stream));
-        F51 wx, wy;
-        pt_affine(base_mult_u64(8ULL * slots * L), wx, wy);
+        const auto w = stride_words(base_mult_u64(8ULL * slots * L));
         PairedArgs& a = e->pa;
         a.table = e->table.p;
         a.lanes = e->lanes.p;
         a.scratch = e->scratch.p;
         a.work = nullptr;  // the flight's counter, set per launch
-        a.slots_n = e->grid * cfg.block * lpt;
         a.lanes_per_thread = lpt;
-        a.stage_records = (!cfg.dump && lpt == 1 && occupancy > STAGE_OCCUPANCY) ? 1u : 0u;
         a.bitmap = cfg.dump ? nullptr : e->bitmap.p;
         a.bits = bits;
         a.sbitmap = e->sbitmap.p;
@@ -451,9 +468,9 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
         a.counter = nullptr;
         a.cap = (uint32_t)std::min<size_t>(e->cap, 0xffffffffu);
         a.search = 0;
-        a.wx = to_words(wx);
-        a.wy = to_words(wy);
-        a.wt = to_words(f_mul(wx, wy));
+        a.wx = w[0];
+        a.wy = w[1];
+        a.wdt = w[2];
         a.lanes_n = cfg.lanes;
         a.half = cfg.half;
         a.rounds = cfg.rounds;

@@ -7,16 +7,16 @@
 
 // Register budget of the search kernels: at most OG_LB_THREADS threads per
 // block and at least OG_LB_MIN_BLOCKS resident blocks per SM. 128 x 5 caps
-// them at 96 registers (20 warps per SM). With the two-accumulator field
-// multiply this measured fastest on B200: 20.5 G keys/s against 20.0 at
-// 80 registers (24 warps, more spills) and 20.3 at 128 (16 warps). With the
-// lane's centre parked in shared memory (paired_rounds) it spills 4 bytes
-// and runs 20.8; at 80 registers 20.9 at half 2048 but 20.7 at half 1024.
+// them at 96 registers (20 warps per SM).
 #ifndef OG_LB_THREADS
 #define OG_LB_THREADS 128
 #endif
 #ifndef OG_LB_MIN_BLOCKS
 #define OG_LB_MIN_BLOCKS 5
+#endif
+// with two blocks of lanes an item: the blocks per SM of its launches
+#ifndef OG_LB2_MIN_BLOCKS
+#define OG_LB2_MIN_BLOCKS 4
 #endif
 
 namespace og {
@@ -47,80 +47,37 @@ __global__ void __launch_bounds__(128) init_kernel(const InitArgs a) {
     }
 }
 
-// Staged: survivor records collected per warp in shared memory and written
-// 32 at a time (WarpStage), for indexes that let many candidates through.
-template <bool Staged>
-__global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) paired_kernel(const PairedArgs a) {
-    // The table is read through L1, not staged in shared memory: every lane
-    // of a warp loads the same entry, and leaving shared memory unused keeps
-    // large tables from capping occupancy (measured 17.97 vs 13.3 G keys/s
-    // at half 1024, and the same speed at half 256).
-    const uint4* qtab = a.table;
-    // Persistent: each CTA takes the next block of lanes until none is left.
-    // The scratch is indexed by the CTA's slot, not the lane.
+// The paired search, bound by the multiply-add pipe. Persistent: each CTA
+// takes the next PerItem blocks of lanes until none is left; its scratch
+// belongs to the CTA, not the lanes. On B200 at half 2048, 757 760 lanes and
+// one 6-symbol prefix an advance takes 74.1 ms (4.19e10 keys/s); with a
+// denominator for each neighbour (ten multiplications a pair) it took 152.3.
+// The table is read through L1, not staged in shared memory: every lane of a
+// warp loads the same entry.
+template <int PerItem>
+__global__ void __launch_bounds__(OG_LB_THREADS, PerItem == 2 ? OG_LB2_MIN_BLOCKS : OG_LB_MIN_BLOCKS)
+    paired_kernel(const PairedArgs a) {
     __shared__ uint32_t item_s;
-    const size_t L = a.lanes_n, S = a.slots_n;
-    const uint32_t nblocks = a.lanes_n / blockDim.x;
-    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ uint4 stage_s[(OG_LB_THREADS / 32) * STAGE_RECORDS * STAGE_WORDS];
+    const size_t L = a.lanes_n;
+    const uint32_t nitems = a.lanes_n / (blockDim.x * PerItem);
     const Sink sink{a.bitmap, a.bits, a.hits, a.counter, a.cap, a.search, a.sbitmap, a.sbits};
-    __shared__ uint4 stage_s[Staged ? (OG_LB_THREADS / 32) * STAGE_RECORDS * 3 : 1];
-    WarpStage st{stage_s + (Staged ? (threadIdx.x / 32) * STAGE_RECORDS * 3 : 0), 0};
-    for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) item_s = atomicAdd(a.work, 1u);
-        __syncthreads();
-        const uint32_t item = item_s;
-        if (item >= nblocks) break;
-        const uint32_t lane = item * blockDim.x + threadIdx.x;
-        fe x = load_fe(a.lanes + 0 * L + lane, L);
-        fe y = load_fe(a.lanes + 2 * L + lane, L);
-        paired_rounds<true>(x, y, words_fe(a.wx), words_fe(a.wy), words_fe(a.wt), qtab, a.half, a.rounds, a.scratch + slot, S,
-                      [&](const fe& v, uint32_t step) { test_emit<Staged>(sink, v, lane, step, &st); });
-        if (Staged) stage_flush(sink, st);
-        store_fe(a.lanes + 0 * L + lane, L, x);
-        store_fe(a.lanes + 2 * L + lane, L, y);
-    }
-}
-
-// Two lanes per thread (paired_rounds_n): each work item is 2 blocks of
-// lanes, thread t taking lanes item * 2 B + t and item * 2 B + B + t; the
-// scratch has two columns per thread, slot t and slot t + S / 2. Its
-// register bound (128 threads, OG_LB2_MIN_BLOCKS blocks per SM) holds the
-// two lanes' field elements without spills.
-#ifndef OG_LB2_MIN_BLOCKS
-#define OG_LB2_MIN_BLOCKS 4
-#endif
-__global__ void __launch_bounds__(OG_LB_THREADS, OG_LB2_MIN_BLOCKS) paired_kernel2(const PairedArgs a) {
-    const uint4* qtab = a.table;
-    __shared__ uint32_t item_s;
-    const size_t L = a.lanes_n, S = a.slots_n;
-    const uint32_t per_item = 2 * blockDim.x;
-    const uint32_t nitems = a.lanes_n / per_item;
-    const uint32_t half_slots = a.slots_n / 2;
-    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
-    uint4* const scr[2] = {a.scratch + slot, a.scratch + half_slots + slot};
-    const Sink sink{a.bitmap, a.bits, a.hits, a.counter, a.cap, a.search, a.sbitmap, a.sbits};
+    const PairTable tab{a.table, a.table + (size_t)a.half * 2};
+    uint4* const scr = a.scratch + (size_t)blockIdx.x * a.half * (2 * SCRATCH_ROW) + threadIdx.x;
+    WarpStage st{stage_s + (threadIdx.x / 32) * STAGE_RECORDS * STAGE_WORDS, 0};
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) item_s = atomicAdd(a.work, 1u);
         __syncthreads();
         const uint32_t item = item_s;
         if (item >= nitems) break;
-        const uint32_t lane[2] = {item * per_item + threadIdx.x, item * per_item + blockDim.x + threadIdx.x};
-        fe x[2], y[2];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            x[k] = load_fe(a.lanes + 0 * L + lane[k], L);
-            y[k] = load_fe(a.lanes + 2 * L + lane[k], L);
-        }
-        paired_rounds_n<2>(x, y, words_fe(a.wx), words_fe(a.wy), words_fe(a.wt), qtab, a.half, a.rounds, scr, S,
-                           [&](int k, const fe& v, uint32_t step) { test_emit(sink, v, lane[k], step); });
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            store_fe(a.lanes + 0 * L + lane[k], L, x[k]);
-            store_fe(a.lanes + 2 * L + lane[k], L, y[k]);
+#pragma unroll 1
+        for (uint32_t k = 0; k < PerItem; k++) {
+            const uint32_t lane = (item * PerItem + k) * blockDim.x + threadIdx.x;
+            paired_rounds<true>(a.lanes + lane, L, a.wx, a.wy, a.wdt, tab, a.half, a.rounds, scr, sink, st, lane);
         }
     }
+    stage_flush(sink, tab.vs, st.recs, st.n);
 }
 
 // The chain kernel (the config-1 contract) keeps 96 registers: at 80 it
@@ -243,15 +200,13 @@ cudaError_t launch_init(const InitArgs& a, int block, cudaStream_t s) {
 
 cudaError_t launch_paired(const PairedArgs& a, int block, int grid, cudaStream_t s) {
     const uint32_t n = a.lanes_per_thread;
-    if ((n != 1 && n != 2) || block % 32 != 0 || grid <= 0 || a.lanes_n % ((uint32_t)block * n) != 0 ||
-        a.slots_n != (uint32_t)grid * (uint32_t)block * n)
+    if ((n != 1 && n != 2) || block % 32 != 0 || block > (int)SCRATCH_ROW || grid <= 0 ||
+        a.lanes_n % ((uint32_t)block * n) != 0)
         return cudaErrorInvalidValue;
     if (n == 2)
-        paired_kernel2<<<grid, block, 0, s>>>(a);
-    else if (a.stage_records)
-        paired_kernel<true><<<grid, block, 0, s>>>(a);
+        paired_kernel<2><<<grid, block, 0, s>>>(a);
     else
-        paired_kernel<false><<<grid, block, 0, s>>>(a);
+        paired_kernel<1><<<grid, block, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -274,7 +229,7 @@ static cudaError_t info_of(const void* fn, int block, size_t smem, KernelInfo* i
 }
 
 cudaError_t paired_info(int block, uint32_t, uint32_t lanes_per_thread, KernelInfo* info) {
-    return info_of(lanes_per_thread == 2 ? (const void*)paired_kernel2 : (const void*)paired_kernel<true>, block, 0, info);
+    return info_of(lanes_per_thread == 2 ? (const void*)paired_kernel<2> : (const void*)paired_kernel<1>, block, 0, info);
 }
 
 // sized for a staged 16-bit bitmap, the most a chain launch takes

@@ -5,14 +5,11 @@
 //
 //  * paired (the production engine). A lane holds an affine centre P. One
 //    round yields y(P + Q_m) and y(P - Q_m) for the table Q_m = 8m G,
-//    m = 1..half, plus y(P) itself, from the dedicated Edwards formulas
-//        y(P + Q) = (t1 - t2) / (x1 y2 - y1 x2),
-//        y(P - Q) = (t1 + t2) / (x1 y2 + y1 x2),      t = x y,
-//    i.e. two multiplications per pair, and moves P to the next centre
-//    P + W with x(P + W) = (t1 + tW) / (y1 yW - x1 xW) whose two divisions
-//    ride in the same batch. Every denominator of the round is inverted with
-//    one field inversion (Montgomery's trick, numerators folded into the
-//    forward products as in src/pairs.rs:174-224).
+//    m = 1..half, plus y(P) itself, from a formula in which both have the
+//    same denominator (search_common.cuh), and moves P to the next centre
+//    P + W. Every denominator of the round is inverted with one field
+//    inversion (Montgomery's trick): four multiplications and two partial
+//    ones a pair.
 //  * chain (the contract of src/batch.rs): a lane steps its projective point
 //    by +8G (seven multiplications, the addend's Z scaled to one) and
 //    batch-inverts Z over its `n` steps.
@@ -57,11 +54,10 @@ struct FeWords {
 };
 
 struct PairedArgs {
-    const uint4* table;      // Q_m, m = 1..half: ((m-1)*3 + {x,y,t}) * 2 + q
+    const uint4* table;      // PairTable of Q_m, m = 1..half: q (2 uint4 an entry), then v and s (4)
     uint4* lanes;            // affine centres: ({x,y} * 2 + q) * L + lane
-    uint4* scratch;          // ((e * 2 + {num,den}) * 2 + q) * S + slot, e < 2 half + 2
+    uint4* scratch;          // per CTA c, from c half 2 SCRATCH_ROW: (2 m + q) SCRATCH_ROW + thread, m < half
     uint32_t* work;          // next block of lanes to take, zero at launch
-    uint32_t slots_n;        // S: persistent CTAs x block, the scratch slots
     const uint32_t* bitmap;  // prefix bitmap as 32-bit words (nullptr: none)
     uint32_t bits;
     HitRec* hits;
@@ -70,12 +66,11 @@ struct PairedArgs {
     uint32_t search;         // copied into every record
     const uint32_t* sbitmap; // suffix bitmap (nullptr: none); with neither bitmap every candidate survives
     uint32_t sbits;
-    FeWords wx, wy, wt;      // the round stride W = L (2 half + 1) 8 G, affine
+    FeWords wx, wy, wdt;     // the round stride W = L (2 half + 1) 8 G, affine, and d wx wy
     uint32_t lanes_n;        // L, a multiple of the block size times lanes_per_thread
     uint32_t half;
     uint32_t rounds;         // rounds per launch
-    uint32_t lanes_per_thread;  // 1 (paired_kernel) or 2 (paired_kernel2); S = CTAs x block x this
-    uint32_t stage_records;  // 1: survivors staged per warp in shared memory (one lane a thread only)
+    uint32_t lanes_per_thread;  // blocks of lanes a CTA takes at a time, 1 or 2
 };
 
 // Rows of a chain CTA's scratch hold this many threads (the largest block).

@@ -17,6 +17,7 @@
 // to the kernels.
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstring>
 #include <mutex>
 
@@ -25,11 +26,14 @@
 #include "search_common.cuh"
 
 namespace og {
+
+std::array<FeWords, 3> stride_words(const Pt& w);  // engine.cu
+
 namespace {
 
 constexpr size_t SCRATCH_BYTES = OG_NOALLOC_SCRATCH_BYTES;
 constexpr uint32_t NBLOCK = 128;
-static_assert(NBLOCK <= PARK_STRIDE, "paired_rounds parks PARK_STRIDE lanes per block");
+static_assert(NBLOCK == SCRATCH_ROW, "a row of a CTA's scratch holds its threads");
 constexpr uint32_t POW2 = 24;
 constexpr int MAX_DEVICES = 64;
 
@@ -56,7 +60,7 @@ struct NoAllocArgs {
     uint4* scratch;
     FeWords bx, by, bz, bt;  // first centre, extended
     FeWords ex, ey, ez, et;  // 8G, extended (table entry 1)
-    FeWords wx, wy, wt;      // round stride, affine
+    FeWords wx, wy, wdt;     // round stride W, affine, and d wx wy
     const uint32_t* bitmap;
     uint32_t bits;
     HitRec* hits;
@@ -67,9 +71,9 @@ struct NoAllocArgs {
     uint32_t rounds;
 };
 
-// The table Q_m = m * 8G, m = 1..half, affine with x y. Entry m - 1 starts
-// from 8G and adds 2^k * 8G (from `pow8`) for every bit k of m - 1, then is
-// normalised.
+// The paired round's table (PairTable) of Q_m = m * 8G, m = 1..half. Entry
+// m - 1 starts from 8G and adds 2^k * 8G (from `pow8`) for every bit k of
+// m - 1.
 __global__ void __launch_bounds__(NBLOCK) noalloc_table_kernel(const NoAllocArgs a, const Pow2Table pow8) {
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= a.half) return;
@@ -79,12 +83,15 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_table_kernel(const NoAllocArgs
             const uint4* p = pow8.v + (size_t)k * 6;
             add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
         }
-    const fe zi = fe_invert(Z);
-    const fe x = fe_mulv(X, zi), y = fe_mulv(Y, zi);
-    uint4* d = a.table + (size_t)m * 6;
-    store_fe(d + 0, 1, x);
-    store_fe(d + 2, 1, y);
-    store_fe(d + 4, 1, fe_mulv(x, y));
+    // of the affine (x, y): v = 1/y = Z (Z^2 + X^2) i, s = x / (1 + x^2) = X Y Z i and
+    // q = v^2 / d, with i = 1 / (Y (Z^2 + X^2))
+    const fe den = fe_add(fe_sqv(Z), fe_sqv(X));
+    const fe zi = fe_mulv(Z, fe_invert(fe_mulv(Y, den)));
+    const fe v = fe_canon(fe_mulv(den, zi));
+    store_fe(a.table + (size_t)m * 2, 1, fe_canon(fe_mulv(fe_sqv(v), const_inv_d())));
+    uint4* const vs = a.table + (size_t)a.half * 2 + (size_t)m * 4;
+    store_fe(vs + 0, 1, v);
+    store_fe(vs + 2, 1, fe_canon(fe_mulv(fe_mulv(X, Y), zi)));
 }
 
 // Lane l starts on the centre of window l: the first centre plus 2^k times
@@ -107,14 +114,14 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_init_kernel(const NoAllocArgs 
 // The production paired kernel with its scratch in the file-scope array; the
 // table is read through L1 as in the single engine.
 __global__ void __launch_bounds__(NBLOCK, 5) noalloc_paired_kernel(const NoAllocArgs a) {
-    const uint4* qtab = a.table;
+    __shared__ uint4 stage_s[(NBLOCK / 32) * STAGE_RECORDS * STAGE_WORDS];
     const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t L = a.lanes_n;
     const Sink sink{a.bitmap, a.bits, a.hits, a.counter, a.cap, 0, nullptr, 0};
-    fe x = load_fe(a.lanes + 0 * L + lane, L);
-    fe y = load_fe(a.lanes + 2 * L + lane, L);
-    paired_rounds<true>(x, y, words_fe(a.wx), words_fe(a.wy), words_fe(a.wt), qtab, a.half, a.rounds, a.scratch + lane, L,
-                  [&](const fe& v, uint32_t step) { test_emit(sink, v, lane, step); });
+    const PairTable tab{a.table, a.table + (size_t)a.half * 2};
+    WarpStage st{stage_s + (threadIdx.x / 32) * STAGE_RECORDS * STAGE_WORDS, 0};
+    paired_rounds<true>(a.lanes + lane, a.lanes_n, a.wx, a.wy, a.wdt, tab, a.half, a.rounds,
+                        a.scratch + (size_t)blockIdx.x * a.half * (2 * SCRATCH_ROW) + threadIdx.x, sink, st, lane);
+    stage_flush(sink, tab.vs, st.recs, st.n);
 }
 
 // The array's device address, per device, taken on the first call there.
@@ -190,11 +197,10 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
     a.ey = to_words(eight.Y);
     a.ez = to_words(eight.Z);
     a.et = to_words(eight.T);
-    F51 wx, wy;
-    pt_affine(base_mult_u64(8ULL * slots * lanes), wx, wy);
-    a.wx = to_words(wx);
-    a.wy = to_words(wy);
-    a.wt = to_words(f_mul(wx, wy));
+    const auto w = stride_words(base_mult_u64(8ULL * slots * lanes));
+    a.wx = w[0];
+    a.wy = w[1];
+    a.wdt = w[2];
     a.bitmap = d_bitmap;
     a.bits = bits;
     a.hits = reinterpret_cast<HitRec*>(d_hits);

@@ -64,48 +64,26 @@ __device__ __forceinline__ uint32_t suffix_slot(const fe& y, uint32_t sbits) {
     return sbits >= 32 ? w : w & ((1u << sbits) - 1u);
 }
 
-// Survivor records staged per warp in shared memory, for dense indexes: a
-// warp collects up to STAGE_RECORDS records and writes them with one atomic
-// on the counter, where the direct append pays one for every warp-step that
-// carries a survivor (at config 3's 5 % survivors, four warp-steps in five).
-constexpr uint32_t STAGE_RECORDS = 32;
-
-struct WarpStage {
-    uint4* recs;  // this warp's STAGE_RECORDS records, three uint4 each, in shared memory
-    uint32_t n;   // records held; the same in every lane of the warp
-};
-
-// Writes a warp's staged records to the sink (all lanes of the warp call it
-// together). Records past the sink's room are counted, not written, as in
-// test_emit.
-__device__ __forceinline__ void stage_flush(const Sink& k, WarpStage& st) {
-    if (st.n == 0) return;
-    __syncwarp();
-    const unsigned me = threadIdx.x & 31u;
-    uint32_t base = 0;
-    if (me == 0) base = atomicAdd(k.counter, st.n);
-    base = __shfl_sync(FULL, base, 0);
-    if (me < st.n && base + me < k.cap) {
-        uint4* dst = reinterpret_cast<uint4*>(k.hits + base + me);
-        const uint4* src = st.recs + me * 3;
-        dst[0] = src[0];
-        dst[1] = src[1];
-        dst[2] = src[2];
+// Whether the slot of a key whose canonical low limb is `y0` is set in the
+// sink's prefix bitmap: bytes 0..3 of the key, big-endian, are the top of the
+// slot.
+__device__ __forceinline__ bool prefix_hit(const Sink& k, uint32_t y0) {
+    const uint32_t head = __byte_perm(y0, 0, 0x0123);
+    const uint32_t slot = k.bits >= 32 ? head : head >> (32 - k.bits);
+    if (k.staged) {
+        extern __shared__ uint32_t og_bitmap_s[];
+        return (og_bitmap_s[slot >> 5] >> (slot & 31)) & 1u;
     }
-    __syncwarp();
-    st.n = 0;
+    return (__ldg(k.bitmap + (slot >> 5)) >> (slot & 31)) & 1u;
 }
 
-// Canonicalises y, tests its slot in the prefix bitmap and in the suffix
-// bitmap (either lets it through; with neither, every candidate survives)
-// and appends a record for every lane of the warp that hit, with one atomic
-// per warp; with `Staged`, into the warp's stage `st` instead (flushed when
-// full, and by the kernel at the end of each work item). Every lane of the
-// warp must call this together (the kernels keep warps converged: lane
-// counts are whole blocks and loop trip counts are uniform).
-template <bool Staged = false>
+// Tests a candidate's slots in the prefix bitmap and in the suffix bitmap
+// (either lets it through; with neither, every candidate survives) and
+// appends a record for every lane of the warp that hit, canonicalised, with
+// one atomic per warp. Lanes with `valid` false have no candidate. Every
+// lane of the warp calls this together.
 __device__ __forceinline__ void test_emit(const Sink& k, const fe& yraw, uint32_t lane, uint32_t step,
-                                          WarpStage* st = nullptr) {
+                                          bool valid = true) {
     // The canonical limbs the bitmaps read (0, 6 and 7), without the full
     // canonicalisation. Folding bit 255 adds 19 to limb 0; its carry reaches
     // limb 6 only through limbs 1..5 all ones, and the value can be p or
@@ -117,21 +95,11 @@ __device__ __forceinline__ void test_emit(const Sink& k, const fe& yraw, uint32_
     y.v[6] = yraw.v[6];
     y.v[7] = yraw.v[7] & 0x7fffffffu;
     if ((yraw.v[1] & yraw.v[2] & yraw.v[3] & yraw.v[4] & yraw.v[5]) == 0xffffffffu) y = fe_canon(yraw);
-    bool hit = true;
+    bool hit = valid;
     if (k.bitmap || k.sbitmap) {
         hit = false;
-        if (k.bitmap) {
-            // bytes 0..3 of the key, big-endian: the top of the slot
-            const uint32_t head = __byte_perm(y.v[0], 0, 0x0123);
-            const uint32_t slot = k.bits >= 32 ? head : head >> (32 - k.bits);
-            if (k.staged) {
-                extern __shared__ uint32_t og_bitmap_s[];
-                hit = (og_bitmap_s[slot >> 5] >> (slot & 31)) & 1u;
-            } else {
-                hit = (__ldg(k.bitmap + (slot >> 5)) >> (slot & 31)) & 1u;
-            }
-        }
-        if (k.sbitmap) {
+        if (k.bitmap && valid) hit = prefix_hit(k, y.v[0]);
+        if (k.sbitmap && valid) {
             const uint32_t slot = suffix_slot(y, k.sbits);
             hit |= ((__ldg(k.sbitmap + (slot >> 5)) >> (slot & 31)) & 1u) != 0;
         }
@@ -139,20 +107,6 @@ __device__ __forceinline__ void test_emit(const Sink& k, const fe& yraw, uint32_
     const unsigned mask = __ballot_sync(FULL, hit);
     if (mask == 0) return;
     const unsigned me = threadIdx.x & 31u;
-    if constexpr (Staged) {
-        const uint32_t count = (uint32_t)__popc(mask);
-        if (st->n + count > STAGE_RECORDS) stage_flush(k, *st);
-        if (hit) {
-            const uint32_t idx = st->n + (uint32_t)__popc(mask & ((1u << me) - 1u));
-            y = fe_canon(yraw);
-            uint4* rec = st->recs + idx * 3;
-            rec[0] = make_uint4(lane, step, k.search, 0u);
-            rec[1] = make_uint4(y.v[0], y.v[1], y.v[2], y.v[3]);
-            rec[2] = make_uint4(y.v[4], y.v[5], y.v[6], y.v[7]);
-        }
-        st->n += count;
-        return;
-    }
     const unsigned leader = __ffs(mask) - 1;
     uint32_t base = 0;
     if (me == leader) base = atomicAdd(k.counter, (uint32_t)__popc(mask));
@@ -284,202 +238,208 @@ __device__ __forceinline__ void add_cached(fe& X, fe& Y, fe& Z, fe& T, const fe&
     T = fe_mulv(x3, y3);
 }
 
-// A lane's centre x, y and t = x y parked in shared memory for the forward
-// pass: each fe as two 16-byte quarters at park[(k * 2 + q) * PARK_STRIDE],
-// so a warp's loads are conflict-free. Loaded with volatile asm right
-// before each use so that the compiler cannot hoist them back into
-// registers for the whole loop. The 24 registers this frees took the
-// single-search kernel at 96 registers from 72 bytes of spills to 4 and
-// from 20.6 to 20.8 G keys/s on B200. The batched kernel does not park
-// (Park = false): with its staged bitmap the 12 KB a block would leave L1
-// too small for the table Q_m at half 2048, and it ran 6 % slower parked.
-constexpr int PARK_STRIDE = OG_LB_THREADS;
+// ---- the paired round ---------------------------------------------------
+//
+// For a centre P = (x, y) and a table point Q = (x2, y2) of odd order, the
+// curve equation -x^2 + y^2 = 1 + d x^2 y^2 lets the denominators of
+// y(P + Q) and y(P - Q) be one and the same:
+//
+//     y(P +- Q) = (z v +- c s) / (q - X),
+//     X = x^2, z = y (1/d - X), c = (1 + 1/d) x          (the lane's)
+//     q = 1 / (d y2^2), v = 1 / y2, s = x2 / (1 + x2^2)  (the table's)
+//
+// (substitute y^2 = (1 + x^2) / (1 - d x^2) into the addition formula's
+// numerators and 1 -+ d x x2 y y2; the common factors cancel). Its
+// denominator is (1/y2^2 - d x^2) / d, which has no zero because d is not a
+// square, so no centre is exceptional; z is 0 only for the two centres of
+// order four. With one inversion for the round's denominators (Montgomery's
+// trick), the prefix products started from z and e = c / z, a pair costs
+// four multiplications,
+//
+//     P_m = P_(m-1) (q - X),   w = P_(m-1) I  [= z / (q - X)],
+//     I <- I (q - X),          f = e w,
+//
+// and y(P +- Q) = v w +- s f, of which only what the bitmap reads is
+// computed (low_product below): about a third of a multiplication each.
+// Only P_m is kept between the passes, 32 bytes a pair.
 
-__device__ __forceinline__ void park_fe(uint4* park, int k, const fe& v) {
-    park[(k * 2 + 0) * PARK_STRIDE] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
-    park[(k * 2 + 1) * PARK_STRIDE] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
+// The table of one half: q per entry (two uint4), then v and s per entry
+// (four), in one array of 6 half uint4.
+struct PairTable {
+    const uint4* q;
+    const uint4* vs;
+};
+
+__device__ __forceinline__ fe const_inv_d() {  // 1/d
+    return fe{{0xcdc9f843u, 0x25e0f276u, 0x4279542eu, 0x0b5dd698u, 0xcdb9cf66u, 0x2b162114u, 0x14d5ce43u, 0x40907ed2u}};
 }
 
-__device__ __forceinline__ fe unpark_fe(const uint4* park, int k) {
-    fe r;
-    const uint32_t a0 = (uint32_t)__cvta_generic_to_shared(park + (k * 2 + 0) * PARK_STRIDE);
-    const uint32_t a1 = (uint32_t)__cvta_generic_to_shared(park + (k * 2 + 1) * PARK_STRIDE);
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]) : "r"(a0));
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7]) : "r"(a1));
-    return r;
+__device__ __forceinline__ fe const_inv_d_plus_1() {  // 1 + 1/d
+    return fe{{0xcdc9f844u, 0x25e0f276u, 0x4279542eu, 0x0b5dd698u, 0xcdb9cf66u, 0x2b162114u, 0x14d5ce43u, 0x40907ed2u}};
 }
 
-// One lane's `rounds` paired rounds around its affine centre (x, y); see
-// kernels.cuh for the formulas and the candidate numbering. `scr` is the
-// lane's scratch: element e, part w (0 numerator, 1 denominator), half q at
-// scr + ((e * 2 + w) * 2 + q) * stride. `visit(y, step)` receives every
-// candidate's y (not yet canonical) with step = round * (2 half + 1) + index.
-// Park: keep the centre in shared memory during the forward pass (above).
-template <bool Park, class Visit>
-__device__ __forceinline__ void paired_rounds(fe& x, fe& y, const fe& wx, const fe& wy, const fe& wt,
-                                              const uint4* qtab, uint32_t half, uint32_t rounds, uint4* scr,
-                                              size_t stride, Visit&& visit) {
-    const size_t L = stride;
+// What the low limb of a canonical product needs. With T = a b < 2^512 and
+// k = floor(T / p), T mod p = T - k p, and p = -19 (mod 2^32), so its low
+// limb is lo + 19 k with lo = a0 b0 (mod 2^32). T / p is
+// T / 2^255 + 19 T / 2^510 (the next term is below 2^-240), so in units of
+// 2^-31 it is the product's words 7 and 8 plus 38 times its word 15: `acc`
+// holds these from the products of columns 7 and 8 (mod 2^64), the high
+// halves of column 6 and the high half of a7 b7. What is left out: column
+// 6's low halves (below 7), column 5 (below 6) and lower; 38 times the rest
+// of word 15 (below 3.01): the true value is in [acc, acc + 128).
+// About 21 multiply-add slots against 74 for the multiplication.
+struct LowProduct {
+    uint64_t acc;
+    uint32_t lo;
+};
+
+constexpr uint32_t LOW_PRODUCT_ERROR = 128;
+
+__device__ __forceinline__ LowProduct low_product(const fe& a, const fe& b) {
+    uint64_t acc = 0, c6 = 0;
+    uint32_t c8 = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) acc += (uint64_t)a.v[i] * b.v[7 - i];
+#pragma unroll
+    for (int i = 0; i < 7; i++) c6 += __umulhi(a.v[i], b.v[6 - i]);
+#pragma unroll
+    for (int i = 1; i < 8; i++) c8 += a.v[i] * b.v[8 - i];
+    acc += c6 + 38ull * __umulhi(a.v[7], b.v[7]) + ((uint64_t)c8 << 32);
+    return LowProduct{acc, a.v[0] * b.v[0]};
+}
+
+// Whether a key that is the sum (or difference) of two low products may be
+// in the prefix bitmap: its low limb is exact unless the sum's uncertainty
+// (2 LOW_PRODUCT_ERROR above `acc`) reaches the next k, once in 2^23 keys;
+// those count as hits and are decided by the full product.
+__device__ __forceinline__ bool low_may_hit(const Sink& k, uint64_t acc, uint32_t lo) {
+    const uint32_t q = __funnelshift_l((uint32_t)acc, (uint32_t)(acc >> 32), 1);  // acc >> 31
+    const bool unsure = ((uint32_t)acc & 0x7fffffffu) >= 0x80000000u - 2u * LOW_PRODUCT_ERROR;
+    return unsure | prefix_hit(k, lo + 19u * q);
+}
+
+// Candidates that may survive, collected per warp in shared memory: w and f
+// (64 bytes), the candidate's lane and step, and its table entry with the
+// sign (0: the centre, whose y is w). stage_flush computes their keys with
+// 32 lanes at once, tests them exactly and appends the survivors. The search
+// loop itself holds neither the full products nor the record writes, and an
+// index that passes one candidate in a hundred costs it no more than a rare
+// one.
+constexpr uint32_t STAGE_RECORDS = 32;
+constexpr uint32_t STAGE_WORDS = 5;  // uint4 a record
+
+struct WarpStage {
+    uint4* recs;  // this warp's STAGE_RECORDS records in shared memory
+    uint32_t n;   // records held; the same in every lane of the warp
+};
+
+static __device__ __noinline__ void stage_flush(const Sink& k, const uint4* vs, const uint4* recs, uint32_t n) {
+    if (n == 0) return;
+    __syncwarp();
+    const unsigned me = threadIdx.x & 31u;
+    const bool valid = me < n;
+    const uint4* r = recs + (valid ? me : 0) * STAGE_WORDS;
+    const fe w = load_fe(r, 1), f = load_fe(r + 2, 1);
+    const uint4 id = r[4];
+    const uint32_t m = id.z & 0x7fffffffu;
+    const uint4* t = vs + (size_t)(m ? m - 1 : 0) * 4;
+    const fe A = fe_mulv(load_fe(t, 1), w), B = fe_mulv(load_fe(t + 2, 1), f);
+    const fe sum = fe_add(A, B), diff = fe_sub(A, B);
+    const fe y = select_fe(m == 0, w, select_fe(id.z >> 31, diff, sum));
+    test_emit(k, y, id.x, id.y, valid);
+    __syncwarp();
+}
+
+// Adds the candidates of the warp's lanes with `hit` set.
+__device__ __forceinline__ void stage_push(const Sink& k, const uint4* vs, WarpStage& st, bool hit, const fe& w,
+                                           const fe& f, uint32_t lane, uint32_t step, uint32_t entry) {
+    const unsigned mask = __ballot_sync(FULL, hit);
+    if (mask == 0) return;
+    const uint32_t count = (uint32_t)__popc(mask);
+    if (st.n + count > STAGE_RECORDS) {
+        stage_flush(k, vs, st.recs, st.n);
+        st.n = 0;
+    }
+    if (hit) {
+        uint4* r = st.recs + (st.n + (uint32_t)__popc(mask & ((1u << (threadIdx.x & 31u)) - 1u))) * STAGE_WORDS;
+        store_fe(r, 1, w);
+        store_fe(r + 2, 1, f);
+        r[4] = make_uint4(lane, step, entry, 0u);
+    }
+    st.n += count;
+}
+
+// Rows of a CTA's scratch hold this many threads (the largest block).
+constexpr uint32_t SCRATCH_ROW = OG_LB_THREADS;
+
+// One lane's `rounds` paired rounds; see kernels.cuh for the candidate
+// numbering. `centre` points at the lane's affine centre in the lane state
+// (x, then y, 16-byte halves `cstride` apart), which is left on the centre
+// after the last round. `wdt` is d xW yW of the stride W. `scr` is the
+// thread's column of its CTA's scratch: prefix product m, half q at
+// scr + (2 m + q) SCRATCH_ROW. Candidates that may survive go to `st`.
+// OneInversion: one field inversion for the block's lanes (block_invert),
+// else one a lane.
+template <bool OneInversion>
+__device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, const FeWords& wx, const FeWords& wy,
+                                              const FeWords& wdt, const PairTable& tab, uint32_t half, uint32_t rounds,
+                                              uint4* scr, const Sink& sink, WarpStage& st, uint32_t lane) {
     const uint32_t slots = 2 * half + 1;
-    __shared__ uint4 park_s[Park ? 6 * PARK_STRIDE : 1];
-    uint4* const park = park_s + (Park ? threadIdx.x : 0);
-#define SCR(e, w) (scr + ((size_t)(e) * 4 + (w) * 2) * L)
+    const bool approx = sink.bitmap && !sink.sbitmap;
     for (uint32_t r = 0; r < rounds; r++) {
-        const fe t = fe_mulv(x, y);
-        // e = 0: y(P + W) = (t - tW) / (x yW - y xW); e = 1: x(P + W) = (t + tW) / (y yW - x xW)
-        fe run;
+        fe X, e, I;
+        const uint32_t mid = r * slots + half;
         {
-            const fe den0 = fe_sub(fe_mulv(x, wy), fe_mulv(y, wx));
-            store_fe(SCR(0, 0), L, fe_sub(t, wt));
-            store_fe(SCR(0, 1), L, den0);
-            const fe den1 = fe_sub(fe_mulv(y, wy), fe_mulv(x, wx));
-            store_fe(SCR(1, 0), L, fe_mulv(fe_add(t, wt), den0));
-            store_fe(SCR(1, 1), L, den1);
-            run = fe_mulv(den0, den1);
-        }
-        if (Park) {
-            park_fe(park, 0, x);
-            park_fe(park, 1, y);
-            park_fe(park, 2, t);
-        }
-        const auto centre = [&](int k) -> fe { return Park ? unpark_fe(park, k) : k == 0 ? x : k == 1 ? y : t; };
+            const fe x = load_fe(centre, cstride), y = load_fe(centre + 2 * cstride, cstride);
+            X = fe_sqv(x);
+            const fe z = fe_mulv(y, fe_sub(const_inv_d(), X));
+            fe run = z;
 #pragma unroll 1
-        for (uint32_t m = 1; m <= half; m++) {
-            const uint4* q = qtab + (size_t)(m - 1) * 6;
-            const fe A = fe_mulv(centre(0), load_fe(q + 2, 1));
-            const fe B = fe_mulv(centre(1), load_fe(q + 0, 1));
-            const fe d0 = fe_sub(A, B);  // P + Q_m
-            const fe qt = load_fe(q + 4, 1);
-            store_fe(SCR(2 * m, 0), L, fe_mulv(fe_sub(centre(2), qt), run));
-            store_fe(SCR(2 * m, 1), L, d0);
-            run = fe_mulv(run, d0);
-            const fe d1 = fe_add(A, B);  // P - Q_m
-            store_fe(SCR(2 * m + 1, 0), L, fe_mulv(fe_add(centre(2), qt), run));
-            store_fe(SCR(2 * m + 1, 1), L, d1);
-            run = fe_mulv(run, d1);
+            for (uint32_t m = 0; m < half; m++) {
+                store_fe(scr + (size_t)m * (2 * SCRATCH_ROW), SCRATCH_ROW, run);
+                run = fe_mulv(run, fe_sub(load_fe(tab.q + (size_t)m * 2, 1), X));
+            }
+            // the stride by the complete addition: with k = d x y xW yW,
+            // x(P + W) = (x yW + y xW) / (1 + k), y(P + W) = (y yW + x xW) / (1 - k);
+            // 1 - k^2 joins the round's inversion
+            const fe k = fe_mulv(fe_mulv(x, y), words_fe(wdt));
+            const fe E = fe_sub(fe_one(), fe_sqv(k));
+            const fe total = fe_mulv(fe_mulv(run, z), E);  // z^2 E prod(q - X)
+            const fe U = OneInversion ? block_invert(total) : fe_invert(total);
+            const fe a = fe_mulv(U, E);
+            e = fe_mulv(fe_mulv(const_inv_d_plus_1(), x), fe_mulv(a, run));  // c / z
+            I = fe_mulv(fe_sqv(z), a);
+            const fe invE = fe_mulv(run, fe_mulv(z, U));
+            const fe nx = fe_mulv(fe_add(fe_mulv(x, words_fe(wy)), fe_mulv(y, words_fe(wx))),
+                                  fe_mulv(fe_sub(fe_one(), k), invE));
+            const fe ny = fe_mulv(fe_add(fe_mulv(y, words_fe(wy)), fe_mulv(x, words_fe(wx))),
+                                  fe_mulv(fe_add(fe_one(), k), invE));
+            store_fe(centre, cstride, nx);
+            store_fe(centre + 2 * cstride, cstride, ny);
+            // the centre's own key: its low limb is exact with bit 255
+            // folded, unless y is p or more
+            const bool hit = !approx || (y.v[7] & 0x7fffffffu) == 0x7fffffffu ||
+                             prefix_hit(sink, y.v[0] + ((y.v[7] >> 31) ? 19u : 0u));
+            stage_push(sink, tab.vs, st, hit, y, y, lane, mid, 0u);
         }
-        // one inversion for the block's lanes where the centre is parked; the
-        // batched kernel keeps it in registers, which the call would save and
-        // restore (measured 1 % slower there), so it inverts per lane
-        fe acc = Park ? block_invert(run) : fe_invert(run);
-        const uint32_t base_step = r * slots;
-        visit(centre(1), base_step + half);
 #pragma unroll 1
         for (uint32_t m = half; m >= 1; m--) {
-            {
-                const fe v = fe_mulv(load_fe(SCR(2 * m + 1, 0), L), acc);
-                acc = fe_mulv(acc, load_fe(SCR(2 * m + 1, 1), L));
-                visit(v, base_step + half - m);
+            const fe w = fe_mulv(load_fe(scr + (size_t)(m - 1) * (2 * SCRATCH_ROW), SCRATCH_ROW), I);
+            I = fe_mulv(I, fe_sub(load_fe(tab.q + (size_t)(m - 1) * 2, 1), X));
+            const fe f = fe_mulv(e, w);
+            bool plus = true, minus = true;
+            if (approx) {
+                const uint4* t = tab.vs + (size_t)(m - 1) * 4;
+                const LowProduct A = low_product(load_fe(t, 1), w), B = low_product(load_fe(t + 2, 1), f);
+                plus = low_may_hit(sink, A.acc + B.acc, A.lo + B.lo);
+                minus = low_may_hit(sink, A.acc - B.acc - LOW_PRODUCT_ERROR, A.lo - B.lo);
             }
-            {
-                const fe v = fe_mulv(load_fe(SCR(2 * m, 0), L), acc);
-                acc = fe_mulv(acc, load_fe(SCR(2 * m, 1), L));
-                visit(v, base_step + half + m);
+            if (__any_sync(FULL, plus | minus)) {
+                stage_push(sink, tab.vs, st, plus, w, f, lane, mid + m, m);
+                stage_push(sink, tab.vs, st, minus, w, f, lane, mid - m, m | 0x80000000u);
             }
-        }
-        const fe xn = fe_mulv(load_fe(SCR(1, 0), L), acc);
-        acc = fe_mulv(acc, load_fe(SCR(1, 1), L));
-        y = fe_mulv(load_fe(SCR(0, 0), L), acc);
-        x = xn;
-    }
-#undef SCR
-}
-
-// N lanes per thread (N = 2): the rounds of paired_rounds for the lanes
-// (x[k], y[k]), k < N, whose scratch columns start at scr[k] (element e,
-// part w, half q at scr[k] + ((e * 2 + w) * 2 + q) * stride). The lanes'
-// passes are written step by step side by side, so that the scheduler can
-// issue one lane's products while the other lane's carry chains settle, and
-// the lanes of a thread share the table loads and one inversion per round
-// (Montgomery's trick over their N final products: 1 inversion and 3
-// multiplications instead of 2 inversions). `visit(k, y, step)` receives
-// lane k's candidates with the numbering of paired_rounds. Centres are
-// parked in shared memory as there (3 N field elements a thread).
-template <int N, class Visit>
-__device__ __forceinline__ void paired_rounds_n(fe (&x)[N], fe (&y)[N], const fe& wx, const fe& wy, const fe& wt,
-                                                const uint4* qtab, uint32_t half, uint32_t rounds,
-                                                uint4* const (&scr)[N], size_t stride, Visit&& visit) {
-    static_assert(N == 2, "paired_rounds covers one lane a thread; this function two");
-    const size_t L = stride;
-    const uint32_t slots = 2 * half + 1;
-    __shared__ uint4 park_s[N * 6 * PARK_STRIDE];
-    uint4* const park = park_s + threadIdx.x;
-#define SCRN(k, e, w) (scr[k] + ((size_t)(e) * 4 + (w) * 2) * L)
-    for (uint32_t r = 0; r < rounds; r++) {
-        fe run[N];
-#pragma unroll
-        for (int k = 0; k < N; k++) {
-            const fe t = fe_mulv(x[k], y[k]);
-            const fe den0 = fe_sub(fe_mulv(x[k], wy), fe_mulv(y[k], wx));
-            store_fe(SCRN(k, 0, 0), L, fe_sub(t, wt));
-            store_fe(SCRN(k, 0, 1), L, den0);
-            const fe den1 = fe_sub(fe_mulv(y[k], wy), fe_mulv(x[k], wx));
-            store_fe(SCRN(k, 1, 0), L, fe_mulv(fe_add(t, wt), den0));
-            store_fe(SCRN(k, 1, 1), L, den1);
-            run[k] = fe_mulv(den0, den1);
-            park_fe(park, 3 * k + 0, x[k]);
-            park_fe(park, 3 * k + 1, y[k]);
-            park_fe(park, 3 * k + 2, t);
-        }
-#pragma unroll 1
-        for (uint32_t m = 1; m <= half; m++) {
-            const uint4* q = qtab + (size_t)(m - 1) * 6;
-            fe A[N], B[N];
-#pragma unroll
-            for (int k = 0; k < N; k++) {
-                A[k] = fe_mulv(unpark_fe(park, 3 * k + 0), load_fe(q + 2, 1));
-                B[k] = fe_mulv(unpark_fe(park, 3 * k + 1), load_fe(q + 0, 1));
-            }
-            const fe qt = load_fe(q + 4, 1);
-#pragma unroll
-            for (int k = 0; k < N; k++) {
-                const fe d0 = fe_sub(A[k], B[k]);  // P + Q_m
-                const fe tk = unpark_fe(park, 3 * k + 2);
-                store_fe(SCRN(k, 2 * m, 0), L, fe_mulv(fe_sub(tk, qt), run[k]));
-                store_fe(SCRN(k, 2 * m, 1), L, d0);
-                run[k] = fe_mulv(run[k], d0);
-                const fe d1 = fe_add(A[k], B[k]);  // P - Q_m
-                store_fe(SCRN(k, 2 * m + 1, 0), L, fe_mulv(fe_add(tk, qt), run[k]));
-                store_fe(SCRN(k, 2 * m + 1, 1), L, d1);
-                run[k] = fe_mulv(run[k], d1);
-            }
-        }
-        fe acc[N];
-        {
-            const fe inv = fe_invert(fe_mulv(run[0], run[1]));
-            acc[0] = fe_mulv(inv, run[1]);
-            acc[1] = fe_mulv(inv, run[0]);
-        }
-        const uint32_t base_step = r * slots;
-#pragma unroll
-        for (int k = 0; k < N; k++) visit(k, unpark_fe(park, 3 * k + 1), base_step + half);
-#pragma unroll 1
-        for (uint32_t m = half; m >= 1; m--) {
-            fe v[N];
-#pragma unroll
-            for (int k = 0; k < N; k++) {
-                v[k] = fe_mulv(load_fe(SCRN(k, 2 * m + 1, 0), L), acc[k]);
-                acc[k] = fe_mulv(acc[k], load_fe(SCRN(k, 2 * m + 1, 1), L));
-            }
-#pragma unroll
-            for (int k = 0; k < N; k++) visit(k, v[k], base_step + half - m);
-#pragma unroll
-            for (int k = 0; k < N; k++) {
-                v[k] = fe_mulv(load_fe(SCRN(k, 2 * m, 0), L), acc[k]);
-                acc[k] = fe_mulv(acc[k], load_fe(SCRN(k, 2 * m, 1), L));
-            }
-#pragma unroll
-            for (int k = 0; k < N; k++) visit(k, v[k], base_step + half + m);
-        }
-#pragma unroll
-        for (int k = 0; k < N; k++) {
-            const fe xn = fe_mulv(load_fe(SCRN(k, 1, 0), L), acc[k]);
-            acc[k] = fe_mulv(acc[k], load_fe(SCRN(k, 1, 1), L));
-            y[k] = fe_mulv(load_fe(SCRN(k, 0, 0), L), acc[k]);
-            x[k] = xn;
         }
     }
-#undef SCRN
 }
 
 }  // namespace og
