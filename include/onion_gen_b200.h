@@ -397,8 +397,8 @@ void og_serve_free(og_serve* s);
  * beyond that the call fails with OG_E_CAPACITY before touching the device.
  * Work is enqueued on `stream` (a cudaStream_t; NULL for the legacy default
  * stream) and the call returns without waiting for it: it enqueues one
- * memset of `*d_count` and three kernels, whose constants travel as launch
- * parameters, and copies nothing from host memory.
+ * memset of `*d_count` and three or four kernels, whose constants travel as
+ * launch parameters, and copies nothing from host memory.
  *
  * The first call on a device looks up the array's device address
  * (cudaGetSymbolAddress); make that first call before any stream capture.

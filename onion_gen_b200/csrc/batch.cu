@@ -55,12 +55,12 @@
 #define OG_LB_THREADS 128
 #endif
 #ifndef OG_LB_MIN_BLOCKS
-#define OG_LB_MIN_BLOCKS 5
+#define OG_LB_MIN_BLOCKS 4
 #endif
 
 namespace og {
 
-const std::vector<uint4>& pair_table(uint32_t half);           // engine.cu
+cudaError_t make_pair_table(DevBuf<uint4>& table, uint32_t half, cudaStream_t s);  // engine.cu
 std::array<FeWords, 3> stride_words(const Pt& w);              // engine.cu
 std::vector<uint4> pow2_table(const Pt& stride, uint32_t nbits);  // engine.cu
 MatchTables match_tables(const std::vector<FilterSet::DeviceBucket>& buckets, const uint64_t* keys,
@@ -123,7 +123,8 @@ struct Counters {
     uint32_t surv;        // bitmap survivors written
     uint32_t hits;        // exact hits written
     uint32_t mismatch;    // suffix survivors whose recomputed key differed
-    uint32_t pad[3];
+    uint32_t failed;      // a wait of the search kernel ran out
+    uint32_t pad[2];
 };
 
 struct BatchArgs {
@@ -133,8 +134,7 @@ struct BatchArgs {
     Counters* counters;  // the flight's
     uint32_t nblocks;
     uint4* lanes;    // ({x,y} * 2 + q) * slots + slot
-    // per persistent CTA, a region of cta_scratch uint4 in which thread t's
-    // prefix product m, half q is at (2 m + q) SCRATCH_ROW + t
+    // per persistent CTA, cta_scratch uint4 (cta_scratch_uint4 of the largest half)
     uint4* scratch;
     size_t cta_scratch;
     size_t slots;
@@ -179,9 +179,11 @@ __global__ void __launch_bounds__(BLOCK) batch_init_kernel(const BatchArgs a) {
 // 19.67-19.82 s, the searches' small bitmaps no longer competing with the
 // table Q_m for L1).
 __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_kernel(const BatchArgs a) {
-    __shared__ uint4 stage_s[(OG_LB_THREADS / 32) * STAGE_RECORDS * STAGE_WORDS];
+    __shared__ __align__(128) RoundShared sh;
     __shared__ uint32_t item_s, staged_s;  // staged_s: the search whose bitmap is in og_bitmap_s
     if (threadIdx.x == 0) staged_s = NONE;
+    MatrixUnit mu;
+    matrix_open(sh);
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) item_s = atomicAdd(&a.counters->work, 1u);
@@ -203,12 +205,17 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_
             if (threadIdx.x == 0) staged_s = sb.sidx;
         }
         const uint32_t slot = item * BLOCK + threadIdx.x;
-        const Sink sink{d.bitmap, d.bits, a.surv, &a.counters->surv, a.surv_cap, sb.sidx, d.sbitmap, d.sbits, staged};
-        WarpStage st{stage_s + (threadIdx.x / 32) * STAGE_RECORDS * STAGE_WORDS, 0};
-        paired_rounds<false>(a.lanes + slot, a.slots, d.wx, d.wy, d.wdt, a.table, d.half, a.rounds,
-                             a.scratch + blockIdx.x * a.cta_scratch + threadIdx.x, sink, st, slot);
-        stage_flush(sink, a.table.vs, st.recs, st.n);
+        const Sink sink{d.bitmap, d.bits, a.surv, &a.counters->surv, a.surv_cap, sb.sidx, d.sbitmap, d.sbits, staged,
+                        &a.counters->failed};
+        uint4* const scr = a.scratch + blockIdx.x * a.cta_scratch + threadIdx.x;
+        if (sink_is_narrow(d.bitmap != nullptr, d.bits, d.sbitmap != nullptr))
+            paired_rounds<false>(a.lanes + slot, a.slots, d.wx, d.wy, d.wdt, a.table, d.half, a.rounds, scr, sink, sh,
+                                 mu, slot, true);
+        else
+            paired_rounds_full<false>(a.lanes + slot, a.slots, d.wx, d.wy, d.wdt, a.table, d.half, a.rounds, scr, sink,
+                                      slot, true);
     }
+    matrix_close(sh);
 }
 
 // Exact match of the bitmap survivors: per distinct filter length, a binary
@@ -560,7 +567,7 @@ void rebalance(og_batch* b, std::vector<uint32_t>& init) {
 
 int enqueue_step(og_batch* b, const BatchArgs& a, char* err, size_t errlen) {
     CU(cudaMemsetAsync(a.counters, 0, offsetof(Counters, init_count), b->stream));
-    CU(cudaMemsetAsync(&a.counters->surv, 0, 3 * sizeof(uint32_t), b->stream));  // surv, hits, mismatch
+    CU(cudaMemsetAsync(&a.counters->surv, 0, 4 * sizeof(uint32_t), b->stream));  // surv, hits, mismatch, failed
     batch_init_kernel<<<b->nblocks, BLOCK, 0, b->stream>>>(a);
     CU(cudaGetLastError());
     batch_search_kernel<<<b->grid, BLOCK, STAGED_BYTES, b->stream>>>(a);
@@ -681,6 +688,7 @@ int collect(og_batch* b, og_batch_hit* out, size_t cap, size_t* n, char* err, si
     cudaEventElapsedTime(&b->last_ms, f.ev0, f.ev1);
     b->last_launches = 3;
     const Counters c = *f.h_counters.p;
+    if (c.failed) return fail(err, errlen, OG_E_TIMEOUT, "a wait of the search kernel ran out");
     if (c.surv > f.args.surv_cap || c.hits > f.args.hit_cap)
         return fail(err, errlen, OG_E_OVERFLOW, "a step produced %u survivors (room %u) and %u hits (room %u)", c.surv,
                     f.args.surv_cap, c.hits, f.args.hit_cap);
@@ -840,12 +848,16 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
     if (!b) return fail(err, errlen, OG_E_NOMEM, "host memory");
     b->device = ordinal;
     int per_sm = 0, sms = 0;
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_search_kernel, BLOCK, STAGED_BYTES));
+    // with the staged bitmap a block's shared memory passes 48 KB
+    CU(cudaFuncSetAttribute(batch_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STAGED_BYTES));
+    CU(matrix_blocks_per_sm((const void*)batch_search_kernel, STAGED_BYTES, &per_sm));
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ordinal));
     const uint32_t fit = (uint32_t)std::max(1, per_sm);
     cfg.grid = cfg.grid == 0 ? fit : std::min(cfg.grid, fit);
     b->grid = cfg.grid * (uint32_t)sms;
-    if (cfg.slots == 0) cfg.slots = 2 * b->grid * BLOCK;
+    // two waves of five blocks per SM, whatever number is resident: the default
+    // pool does not move with the kernel's resources
+    if (cfg.slots == 0) cfg.slots = 2 * 5 * (uint32_t)sms * BLOCK;
     cfg.slots = (cfg.slots + BLOCK - 1) / BLOCK * BLOCK;
     b->slots = cfg.slots;
     b->nblocks = cfg.slots / BLOCK;
@@ -880,11 +892,10 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
     // its BLOCK threads, so a CTA's accesses stay within a few pages (config
     // 4's long searches at half 2048 on B200: 2.08e10 against 2.05e10 keys/s
     // with rows across the whole grid)
-    const size_t cta_scratch = (size_t)SCRATCH_ROW * 2 * cfg.max_half;
+    const size_t cta_scratch = cta_scratch_uint4(cfg.max_half);
     CU(b->scratch.alloc((size_t)b->grid * cta_scratch));
-    const std::vector<uint4>& tab = pair_table(cfg.max_half);
-    CU(b->table.alloc(tab.size()));
-    CU(cudaMemcpy(b->table.p, tab.data(), tab.size() * sizeof(uint4), cudaMemcpyHostToDevice));
+    CU(make_pair_table(b->table, cfg.max_half, b->stream));
+    CU(cudaStreamSynchronize(b->stream));
     for (uint32_t h = cfg.half; h <= cfg.max_half; h *= 2) {
         std::vector<uint4> pw = pow2_table(base_mult_u64(8ULL * (2ULL * h + 1)), POW2_BITS);
         DevBuf<uint4>& d = b->pow2[h];
@@ -935,7 +946,7 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
         a.scratch = b->scratch.p;
         a.cta_scratch = cta_scratch;
         a.slots = S;
-        a.table = PairTable{b->table.p, b->table.p + (size_t)cfg.max_half * 2};
+        a.table = pair_table_at<const uint4>(b->table.p, cfg.max_half);
         a.rounds = cfg.rounds;
         a.surv = f.surv.p;
         a.surv_cap = (uint32_t)surv_cap;
@@ -1196,7 +1207,9 @@ int og_batch_tune(int ordinal, uint32_t searches, float max_step_ms, og_batch_co
     if (ordinal < 0 || ordinal >= count) return fail(err, errlen, OG_E_ARG, "device %d of %d", ordinal, count);
     CU(cudaSetDevice(ordinal));
     int per_sm = 0, sms = 0;
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_search_kernel, BLOCK, STAGED_BYTES));
+    // with the staged bitmap a block's shared memory passes 48 KB
+    CU(cudaFuncSetAttribute(batch_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STAGED_BYTES));
+    CU(matrix_blocks_per_sm((const void*)batch_search_kernel, STAGED_BYTES, &per_sm));
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ordinal));
     const uint32_t fit = (uint32_t)std::max(1, per_sm);
     // a mix that never finishes: each search one ten-symbol prefix (50 bits)

@@ -71,47 +71,59 @@ std::array<FeWords, 3> stride_words(const Pt& w) {
     return {to_words(x), to_words(y), to_words(f_mul(curve_d(), f_mul(x, y)))};
 }
 
-// The paired round's table of Q_m = 8m G, m = 1..half (PairTable: q = 1/(d y^2)
-// of every entry, then v = 1/y and s = x/(1 + x^2) of every entry), in the
-// device layout; the same for every search, so built once per half. y and
-// 1 + x^2 are never 0 for a point of odd order.
-const std::vector<uint4>& pair_table(uint32_t half) {
+// The per-entry part of the PairTable of Q_m = 8m G for half `half` (q =
+// 1/(d y^2) of every entry, then v = 1/y and s = x/(1 + x^2) of every entry;
+// whole groups, so up to two entries past `half`), in the device layout; the
+// same for every search, so built once per half. y and 1 + x^2 are never 0
+// for a point of odd order.
+static const std::vector<uint4>& pair_entries(uint32_t half) {
     static std::mutex mu;
     static std::map<uint32_t, std::unique_ptr<std::vector<uint4>>> cache;
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(half);
     if (it != cache.end()) return *it->second;
-    std::vector<Pt> pts(half);
+    const uint32_t n = groups_of(half) * GROUP;
+    std::vector<Pt> pts(n);
     const Pt eight = base_mult_u64(8);
     Pt p = eight;
-    for (uint32_t m = 0; m < half; m++) {
+    for (uint32_t m = 0; m < n; m++) {
         pts[m] = p;
         p = pt_add(p, eight);
     }
     std::vector<F51> xs, ys;
     batch_affine(pts, xs, ys);
     // 1 / (y (1 + x^2)) of all entries with one inversion
-    std::vector<F51> prefix(half), den(half);
+    std::vector<F51> prefix(n), den(n);
     F51 run = f_one();
-    for (uint32_t m = 0; m < half; m++) {
+    for (uint32_t m = 0; m < n; m++) {
         den[m] = f_add(f_one(), f_sq(xs[m]));
         prefix[m] = run;
         run = f_mul(run, f_mul(ys[m], den[m]));
     }
     F51 inv = f_inv(run);
-    auto tab = std::make_unique<std::vector<uint4>>((size_t)half * 6);
-    for (uint32_t m = half; m-- > 0;) {
+    auto tab = std::make_unique<std::vector<uint4>>((size_t)n * 6);
+    for (uint32_t m = n; m-- > 0;) {
         const F51 i = f_mul(inv, prefix[m]);
         inv = f_mul(inv, f_mul(ys[m], den[m]));
         const F51 v = f_mul(den[m], i);
         put_fe(tab->data() + (size_t)m * 2, 1, f_mul(f_sq(v), inv_curve_d()));
-        uint4* const vs = tab->data() + (size_t)half * 2 + (size_t)m * 4;
+        uint4* const vs = tab->data() + (size_t)n * 2 + (size_t)m * 4;
         put_fe(vs + 0, 1, v);
         put_fe(vs + 2, 1, f_mul(xs[m], f_mul(ys[m], i)));
     }
     auto& ref = *tab;
     cache[half] = std::move(tab);
     return ref;
+}
+
+// A device PairTable for half `half`, its entries copied and its groups
+// computed on `s`.
+cudaError_t make_pair_table(DevBuf<uint4>& table, uint32_t half, cudaStream_t s) {
+    cudaError_t e = table.alloc(pair_table_uint4(half));
+    if (e != cudaSuccess) return e;
+    const std::vector<uint4>& tab = pair_entries(half);
+    e = cudaMemcpyAsync(table.p, tab.data(), tab.size() * sizeof(uint4), cudaMemcpyHostToDevice, s);
+    return e == cudaSuccess ? launch_group_table(table.p, half, s) : e;
 }
 
 // 2^k * stride for k < nbits in cached form (y+x, y-x, 2dxy), device layout.
@@ -170,6 +182,10 @@ uint64_t words_hash(const uint64_t* w, size_t n) {
 
 }  // namespace og
 
+namespace {
+constexpr size_t COUNTS = 5;  // words an advance's counters take
+}
+
 struct og_engine {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -188,7 +204,7 @@ struct og_engine {
     // advance's results while the next one runs; the lanes and the scratch
     // are shared, the launches being ordered on one stream.
     struct Flight {
-        DevBuf<uint32_t> counts;  // survivors, matches, mismatched suffix keys
+        DevBuf<uint32_t> counts;  // survivors, matches, mismatched suffix keys, blocks taken, a wait that ran out
         DevBuf<HitRec> hits;
         DevBuf<MatchRec> matches;
         HostBuf<uint32_t> h_counts;
@@ -247,18 +263,42 @@ namespace {
                         "%s: %s", #call, cuda_text(_e).c_str());                              \
     } while (0)
 
-// Lanes one wave of the search kernel holds: resident CTAs x block x lanes
-// per thread.
-int resident_lanes(int device, uint32_t scheme, uint32_t half, uint32_t block, uint32_t* out, char* err,
-                   size_t errlen, uint32_t lanes_per_thread = 1) {
+// The lanes that shapes are counted in waves of. For the paired scheme these
+// are the blocks an SM held while its kernel had 96 registers a thread (21
+// warps, and at most 11 blocks; 16 and 8 with two lanes per thread): a fixed
+// count, so that a default shape, and with it what one advance covers, does
+// not move with the kernel's resources. The chain kernel's are its resident
+// blocks.
+int resident_lanes(int device, uint32_t scheme, uint32_t block, uint32_t* out, char* err, size_t errlen,
+                   uint32_t lanes_per_thread = 1) {
+    uint32_t blocks = 0;
+    if (scheme == OG_SCHEME_CHAIN) {
+        KernelInfo info{};
+        const cudaError_t e = chain_info((int)block, &info);
+        if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "kernel attributes: %s", cuda_text(e).c_str());
+        blocks = (uint32_t)std::max(0, info.blocks_per_sm);
+    } else if (block <= OG_LB_THREADS) {
+        blocks = lanes_per_thread == 2 ? std::min(8u, 16u / (block / 32)) : std::min(11u, 21u / (block / 32));
+    }
+    int sms = 0;
+    const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "device attributes: %s", cuda_text(e).c_str());
+    *out = std::max(1u, blocks) * (uint32_t)sms * block * lanes_per_thread;
+    return OG_OK;
+}
+
+// The persistent CTAs a search of `lanes` lanes runs on: as many as are
+// resident, but no more than it has blocks of lanes.
+int search_grid(int device, const og_engine_config& cfg, bool narrow, uint32_t* out, char* err, size_t errlen) {
     KernelInfo info{};
-    cudaError_t e = scheme == OG_SCHEME_CHAIN ? chain_info((int)block, &info)
-                                              : paired_info((int)block, half, lanes_per_thread, &info);
+    const bool chain = cfg.scheme == OG_SCHEME_CHAIN;
+    cudaError_t e = chain ? chain_info((int)cfg.block, &info) : paired_info(narrow, cfg.lanes_per_thread, &info);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "kernel attributes: %s", cuda_text(e).c_str());
     int sms = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "device attributes: %s", cuda_text(e).c_str());
-    *out = (uint32_t)std::max(1, info.blocks_per_sm) * (uint32_t)sms * block * lanes_per_thread;
+    const uint32_t per_item = chain ? cfg.block : OG_LB_THREADS * cfg.lanes_per_thread;
+    *out = std::min((uint32_t)std::max(1, info.blocks_per_sm) * (uint32_t)sms, (cfg.lanes + per_item - 1) / per_item);
     return OG_OK;
 }
 
@@ -328,7 +368,7 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     }
     if (cfg.lanes == 0) {
         uint32_t resident = 0;
-        int rc = resident_lanes(ordinal, cfg.scheme, cfg.half, cfg.block, &resident, err, errlen, lpt);
+        int rc = resident_lanes(ordinal, cfg.scheme, cfg.block, &resident, err, errlen, lpt);
         if (rc) return rc;
         if (cfg.scheme == OG_SCHEME_PAIRED) {
             // the persistent kernel takes lanes a block at a time: eight
@@ -391,21 +431,16 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     CU(e->lanes.alloc(L * coords * 2));
     {
         // both kernels are persistent: scratch for the resident CTAs only
-        // (the chain kernel's no more CTAs than blocks of lanes)
-        uint32_t resident = 0;
-        int rc = resident_lanes(ordinal, cfg.scheme, cfg.half, cfg.block, &resident, err, errlen, lpt);
+        const bool narrow = sink_is_narrow(!cfg.dump && bitmap, bits, suffixed);
+        int rc = search_grid(ordinal, cfg, narrow, &e->grid, err, errlen);
         if (rc) return rc;
-        e->grid = std::max<uint32_t>(1, resident / (cfg.block * lpt));
-        if (cfg.scheme == OG_SCHEME_CHAIN) e->grid = std::min<uint32_t>(e->grid, (uint32_t)(L / cfg.block));
-        // a CTA's rows hold SCRATCH_ROW (CHAIN_ROW) threads whatever its
-        // block: a prefix product a pair, or a numerator and a denominator a step
-        const size_t col = cfg.scheme == OG_SCHEME_CHAIN ? 4 * CHAIN_ROW : 2 * OG_LB_THREADS;
-        CU(e->scratch.alloc((size_t)e->grid * col * cfg.half));
+        const size_t cta = cfg.scheme == OG_SCHEME_CHAIN ? (size_t)4 * CHAIN_ROW * cfg.half : cta_scratch_uint4(cfg.half);
+        CU(e->scratch.alloc((size_t)e->grid * cta));
     }
     for (og_engine::Flight& f : e->fl) {
-        CU(f.counts.alloc(4));
+        CU(f.counts.alloc(COUNTS));
         CU(f.hits.alloc(e->cap));
-        CU(f.h_counts.alloc(4));
+        CU(f.h_counts.alloc(COUNTS));
     }
     CU(e->h_recs.alloc(e->cap));
     if (!cfg.dump && bitmap) {
@@ -450,9 +485,7 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     CU(launch_init(ia, 128, e->stream));
 
     if (cfg.scheme == OG_SCHEME_PAIRED) {
-        const std::vector<uint4>& tab = pair_table(cfg.half);
-        CU(e->table.alloc(tab.size()));
-        CU(cudaMemcpyAsync(e->table.p, tab.data(), tab.size() * sizeof(uint4), cudaMemcpyHostToDevice, e->stream));
+        CU(make_pair_table(e->table, cfg.half, e->stream));
         const auto w = stride_words(base_mult_u64(8ULL * slots * L));
         PairedArgs& a = e->pa;
         a.table = e->table.p;
@@ -603,17 +636,18 @@ int enable_matching(og_engine* e, const og_filters* f, char* err, size_t errlen)
 // search kernel, optionally the device match, and the copy of the counters.
 int enqueue_advance(og_engine* e, bool match, char* err, size_t errlen) {
     if (!e) return fail(err, errlen, OG_E_ARG, "null argument");
-    if (e->overflowed) return fail(err, errlen, OG_E_STATE, "an earlier advance overflowed; the engine is closed");
+    if (e->overflowed) return fail(err, errlen, OG_E_STATE, "an earlier advance failed; the engine is closed");
     if (e->inflight == 2) return fail(err, errlen, OG_E_STATE, "two advances are in flight: collect one first");
     og_engine::Flight& f = e->fl[(e->head + e->inflight) & 1];
     CU(cudaSetDevice(e->device));
-    CU(cudaMemsetAsync(f.counts.p, 0, 4 * sizeof(uint32_t), e->stream));
+    CU(cudaMemsetAsync(f.counts.p, 0, COUNTS * sizeof(uint32_t), e->stream));
     CU(cudaEventRecord(f.ev0, e->stream));
     if (e->cfg.scheme == OG_SCHEME_PAIRED) {
         e->pa.hits = f.hits.p;
         e->pa.counter = f.counts.p;
         e->pa.work = f.counts.p + 3;
-        CU(launch_paired(e->pa, (int)e->cfg.block, (int)e->grid, e->stream));
+        e->pa.failed = f.counts.p + 4;
+        CU(launch_paired(e->pa, (int)e->grid, e->stream));
     } else {
         e->ca.hits = f.hits.p;
         e->ca.counter = f.counts.p;
@@ -633,7 +667,7 @@ int enqueue_advance(og_engine* e, bool match, char* err, size_t errlen) {
         CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
         CU(launch_match(m, std::max(sms, 1) * 4, e->stream));
     }
-    CU(cudaMemcpyAsync(f.h_counts.p, f.counts.p, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream));
+    CU(cudaMemcpyAsync(f.h_counts.p, f.counts.p, COUNTS * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream));
     CU(cudaEventRecord(f.done, e->stream));
     f.launch = e->launches++;
     f.match = match;
@@ -663,6 +697,10 @@ int collect_flight(og_engine* e, bool match, uint32_t* count, uint64_t* launch, 
     CU(cudaEventSynchronize(f.done));
     cudaEventElapsedTime(&e->last_ms, f.ev0, f.ev1);
     *launch = f.launch;
+    if (f.h_counts.p[4]) {
+        e->overflowed = true;
+        return fail(err, errlen, OG_E_TIMEOUT, "a wait of the search kernel ran out; the engine is closed");
+    }
     const uint32_t found = f.h_counts.p[0];
     if (found > e->cap) {
         e->overflowed = true;
@@ -791,7 +829,7 @@ int og_engine_resident_lanes(int ordinal, uint32_t scheme, uint32_t block, uint3
     if (block % 32 != 0 || block > 1024) return fail(err, errlen, OG_E_ARG, "block %u: a multiple of 32 up to 1024", block);
     cudaError_t e = cudaSetDevice(ordinal);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "device %d: %s", ordinal, cuda_text(e).c_str());
-    return resident_lanes(ordinal, scheme, 0, block, lanes, err, errlen);
+    return resident_lanes(ordinal, scheme, block, lanes, err, errlen);
 }
 
 int og_engine_new_config(int ordinal, const uint8_t start[128], const og_engine_config* cfg, const uint64_t* bitmap,
@@ -850,7 +888,7 @@ int og_engine_new(int ordinal, const uint8_t start[128], uint32_t threads, const
     for (uint32_t lpt : {1u, 2u})
     for (uint32_t half : {512u, 1024u, 2048u}) {
         uint32_t resident = 0;
-        if (resident_lanes(ordinal, OG_SCHEME_PAIRED, half, 128, &resident, err, errlen, lpt) != OG_OK) continue;
+        if (resident_lanes(ordinal, OG_SCHEME_PAIRED, 128, &resident, err, errlen, lpt) != OG_OK) continue;
         for (uint32_t mult : {2u, 4u, 8u}) {
             og_engine_config c{};
             c.scheme = OG_SCHEME_PAIRED;

@@ -1,18 +1,21 @@
 // Key-search kernels for sm_100a. See kernels.cuh for the schemes and the
 // candidate numbering; field.cuh for the arithmetic.
+#include <algorithm>
+
 #include "field.cuh"
 #include "kernels.cuh"
 #include "search_common.cuh"
 #include "suffix_match.cuh"
 
 // Register budget of the search kernels: at most OG_LB_THREADS threads per
-// block and at least OG_LB_MIN_BLOCKS resident blocks per SM. 128 x 5 caps
-// them at 96 registers (20 warps per SM).
+// block and at least OG_LB_MIN_BLOCKS resident blocks per SM. 128 x 4 gives
+// them 128 registers (16 warps per SM); the paired kernel ran 52.6 ms a launch
+// of 3.1e9 candidates so, 54.3 at 96 registers (20 warps), 56.0 at 168.
 #ifndef OG_LB_THREADS
 #define OG_LB_THREADS 128
 #endif
 #ifndef OG_LB_MIN_BLOCKS
-#define OG_LB_MIN_BLOCKS 5
+#define OG_LB_MIN_BLOCKS 4
 #endif
 // with two blocks of lanes an item: the blocks per SM of its launches
 #ifndef OG_LB2_MIN_BLOCKS
@@ -50,21 +53,26 @@ __global__ void __launch_bounds__(128) init_kernel(const InitArgs a) {
 // The paired search, bound by the multiply-add pipe. Persistent: each CTA
 // takes the next PerItem blocks of lanes until none is left; its scratch
 // belongs to the CTA, not the lanes. On B200 at half 2048, 757 760 lanes and
-// one 6-symbol prefix an advance takes 74.1 ms (4.19e10 keys/s); with a
-// denominator for each neighbour (ten multiplications a pair) it took 152.3.
-// The table is read through L1, not staged in shared memory: every lane of a
-// warp loads the same entry.
-template <int PerItem>
+// one 6-symbol prefix a launch takes 52.6 ms (5.9e10 keys/s); ten
+// multiplications a pair took 147.
+// Narrow: a prefix bitmap of at most 24 bits (sink_is_narrow).
+template <int PerItem, bool Narrow>
 __global__ void __launch_bounds__(OG_LB_THREADS, PerItem == 2 ? OG_LB2_MIN_BLOCKS : OG_LB_MIN_BLOCKS)
     paired_kernel(const PairedArgs a) {
     __shared__ uint32_t item_s;
-    __shared__ uint4 stage_s[(OG_LB_THREADS / 32) * STAGE_RECORDS * STAGE_WORDS];
     const size_t L = a.lanes_n;
-    const uint32_t nitems = a.lanes_n / (blockDim.x * PerItem);
-    const Sink sink{a.bitmap, a.bits, a.hits, a.counter, a.cap, a.search, a.sbitmap, a.sbits};
-    const PairTable tab{a.table, a.table + (size_t)a.half * 2};
-    uint4* const scr = a.scratch + (size_t)blockIdx.x * a.half * (2 * SCRATCH_ROW) + threadIdx.x;
-    WarpStage st{stage_s + (threadIdx.x / 32) * STAGE_RECORDS * STAGE_WORDS, 0};
+    constexpr uint32_t per_item = OG_LB_THREADS * PerItem;
+    const uint32_t nitems = (a.lanes_n + per_item - 1) / per_item;
+    const Sink sink{a.bitmap, a.bits, a.hits, a.counter, a.cap, a.search, a.sbitmap, a.sbits, false, a.failed};
+    const PairTable tab = pair_table_at(a.table, a.half);
+    uint4* const scr = a.scratch + (size_t)blockIdx.x * cta_scratch_uint4(a.half) + threadIdx.x;
+    MatrixUnit mu;
+    RoundShared* sh = nullptr;
+    if constexpr (Narrow) {
+        __shared__ __align__(128) RoundShared shared;
+        sh = &shared;
+        matrix_open(*sh);
+    }
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) item_s = atomicAdd(a.work, 1u);
@@ -73,11 +81,21 @@ __global__ void __launch_bounds__(OG_LB_THREADS, PerItem == 2 ? OG_LB2_MIN_BLOCK
         if (item >= nitems) break;
 #pragma unroll 1
         for (uint32_t k = 0; k < PerItem; k++) {
-            const uint32_t lane = (item * PerItem + k) * blockDim.x + threadIdx.x;
-            paired_rounds<true>(a.lanes + lane, L, a.wx, a.wy, a.wdt, tab, a.half, a.rounds, scr, sink, st, lane);
+            const uint32_t lane = item * per_item + k * OG_LB_THREADS + threadIdx.x;
+            const bool active = lane < a.lanes_n;
+            uint4* const centre = a.lanes + (active ? lane : 0);
+            if constexpr (Narrow)
+                paired_rounds<true>(centre, L, a.wx, a.wy, a.wdt, tab, a.half, a.rounds, scr, sink, *sh, mu, lane, active);
+            else
+                paired_rounds_full<true>(centre, L, a.wx, a.wy, a.wdt, tab, a.half, a.rounds, scr, sink, lane, active);
         }
     }
-    stage_flush(sink, tab.vs, st.recs, st.n);
+    if constexpr (Narrow) matrix_close(*sh);
+}
+
+// The per-group part of a PairTable whose q, v and s are in place.
+__global__ void __launch_bounds__(128) group_table_kernel(uint4* table, uint32_t half) {
+    fill_group_table(pair_table_at(table, half), groups_of(half), blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // The chain kernel (the config-1 contract) keeps 96 registers: at 80 it
@@ -198,15 +216,24 @@ cudaError_t launch_init(const InitArgs& a, int block, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_paired(const PairedArgs& a, int block, int grid, cudaStream_t s) {
+cudaError_t launch_paired(const PairedArgs& a, int grid, cudaStream_t s) {
     const uint32_t n = a.lanes_per_thread;
-    if ((n != 1 && n != 2) || block % 32 != 0 || block > (int)SCRATCH_ROW || grid <= 0 ||
-        a.lanes_n % ((uint32_t)block * n) != 0)
-        return cudaErrorInvalidValue;
-    if (n == 2)
-        paired_kernel<2><<<grid, block, 0, s>>>(a);
+    constexpr int block = OG_LB_THREADS;
+    if ((n != 1 && n != 2) || grid <= 0) return cudaErrorInvalidValue;
+    const bool narrow = sink_is_narrow(a.bitmap != nullptr, a.bits, a.sbitmap != nullptr);
+    if (n == 2 && narrow)
+        paired_kernel<2, true><<<grid, block, 0, s>>>(a);
+    else if (n == 2)
+        paired_kernel<2, false><<<grid, block, 0, s>>>(a);
+    else if (narrow)
+        paired_kernel<1, true><<<grid, block, 0, s>>>(a);
     else
-        paired_kernel<1><<<grid, block, 0, s>>>(a);
+        paired_kernel<1, false><<<grid, block, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_group_table(uint4* table, uint32_t half, cudaStream_t s) {
+    group_table_kernel<<<(groups_of(half) * 48 + 127) / 128, 128, 0, s>>>(table, half);
     return cudaGetLastError();
 }
 
@@ -228,8 +255,28 @@ static cudaError_t info_of(const void* fn, int block, size_t smem, KernelInfo* i
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&info->blocks_per_sm, fn, block, smem);
 }
 
-cudaError_t paired_info(int block, uint32_t, uint32_t lanes_per_thread, KernelInfo* info) {
-    return info_of(lanes_per_thread == 2 ? (const void*)paired_kernel<2> : (const void*)paired_kernel<1>, block, 0, info);
+cudaError_t matrix_blocks_per_sm(const void* fn, size_t smem, int* blocks) {
+    cudaFuncAttributes attr;
+    int device = 0, regs = 0, shared = 0, reserved = 0;
+    cudaError_t e = cudaFuncGetAttributes(&attr, fn);
+    if (e == cudaSuccess) e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&regs, cudaDevAttrMaxRegistersPerMultiprocessor, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device);
+    if (e != cudaSuccess) return e;
+    const int warp_regs = (attr.numRegs * 32 + 255) / 256 * 256;  // allocated 256 at a time
+    const size_t block_shared = (attr.sharedSizeBytes + smem + reserved + 127) / 128 * 128;
+    *blocks = std::min({regs / (warp_regs * (OG_LB_THREADS / 32)), (int)(shared / block_shared),
+                        (int)(512 / TMEM_COLUMNS)});
+    return cudaSuccess;
+}
+
+cudaError_t paired_info(bool narrow, uint32_t lanes_per_thread, KernelInfo* info) {
+    const void* const fn[2][2] = {{(const void*)paired_kernel<1, false>, (const void*)paired_kernel<1, true>},
+                                  {(const void*)paired_kernel<2, false>, (const void*)paired_kernel<2, true>}};
+    const void* const f = fn[lanes_per_thread == 2][narrow];
+    const cudaError_t e = info_of(f, OG_LB_THREADS, 0, info);
+    return e == cudaSuccess && narrow ? matrix_blocks_per_sm(f, 0, &info->blocks_per_sm) : e;
 }
 
 // sized for a staged 16-bit bitmap, the most a chain launch takes

@@ -8,8 +8,7 @@
 //    m = 1..half, plus y(P) itself, from a formula in which both have the
 //    same denominator (search_common.cuh), and moves P to the next centre
 //    P + W. Every denominator of the round is inverted with one field
-//    inversion (Montgomery's trick): four multiplications and two partial
-//    ones a pair.
+//    inversion (Montgomery's trick): nine multiplications for three pairs.
 //  * chain (the contract of src/batch.rs): a lane steps its projective point
 //    by +8G (seven multiplications, the addend's Z scaled to one) and
 //    batch-inverts Z over its `n` steps.
@@ -24,6 +23,10 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+
+#ifndef OG_LB_THREADS
+#define OG_LB_THREADS 128  // the most threads a block of the search kernels has
+#endif
 
 namespace og {
 
@@ -53,10 +56,48 @@ struct FeWords {
     uint32_t v[8];
 };
 
+// Rows of a CTA's scratch hold this many threads (the largest block).
+constexpr uint32_t SCRATCH_ROW = OG_LB_THREADS;
+
+// The tables of one half, for G = ceil(half / 3) groups. Per entry (3 G of
+// them) q (two uint4) and v, s (four), for the full products; per group s1,
+// s2 = the sums of products, e0 = s3 - s1 s2 (six uint4) and the constants of
+// its matrix product.
+struct PairTable {
+    const uint4* q;
+    const uint4* vs;
+    const uint4* cubic;
+    const uint4* constants;
+};
+
+constexpr uint32_t GROUP = 3;                     // pairs per group
+constexpr uint32_t GROUP_CONSTANTS = 12 * 48;     // uint4 a group
+
+__host__ __device__ constexpr uint32_t groups_of(uint32_t half) { return (half + GROUP - 1) / GROUP; }
+// uint4 of a PairTable in one array: q, vs, cubic, constants.
+__host__ __device__ constexpr size_t pair_table_uint4(uint32_t half) {
+    return (size_t)groups_of(half) * (GROUP * 6 + 6 + GROUP_CONSTANTS);
+}
+template <class T>
+__host__ __device__ PairTable pair_table_at(T* base, uint32_t half) {
+    const size_t g = groups_of(half);
+    return PairTable{base, base + g * GROUP * 2, base + g * GROUP * 6, base + g * (GROUP * 6 + 6)};
+}
+// uint4 of a CTA's scratch: per group a prefix product and E, per thread; or
+// per pair a prefix product (paired_rounds_full).
+__host__ __device__ constexpr size_t cta_scratch_uint4(uint32_t half) {
+    return (size_t)groups_of(half) * GROUP * 2 * SCRATCH_ROW;
+}
+
+// Whether paired_rounds can serve a sink.
+__host__ __device__ inline bool sink_is_narrow(bool prefix_bitmap, uint32_t bits, bool suffix_bitmap) {
+    return prefix_bitmap && bits <= 24 && !suffix_bitmap;
+}
+
 struct PairedArgs {
-    const uint4* table;      // PairTable of Q_m, m = 1..half: q (2 uint4 an entry), then v and s (4)
+    const uint4* table;      // PairTable of Q_m, m = 1..half (pair_table_at)
     uint4* lanes;            // affine centres: ({x,y} * 2 + q) * L + lane
-    uint4* scratch;          // per CTA c, from c half 2 SCRATCH_ROW: (2 m + q) SCRATCH_ROW + thread, m < half
+    uint4* scratch;          // cta_scratch_uint4(half) per CTA
     uint32_t* work;          // next block of lanes to take, zero at launch
     const uint32_t* bitmap;  // prefix bitmap as 32-bit words (nullptr: none)
     uint32_t bits;
@@ -71,6 +112,7 @@ struct PairedArgs {
     uint32_t half;
     uint32_t rounds;         // rounds per launch
     uint32_t lanes_per_thread;  // blocks of lanes a CTA takes at a time, 1 or 2
+    uint32_t* failed;        // set to 1 when a wait of the kernel ran out
 };
 
 // Rows of a chain CTA's scratch hold this many threads (the largest block).
@@ -163,11 +205,13 @@ struct MatchArgs {
 
 cudaError_t launch_init(const InitArgs& a, int block, cudaStream_t s);
 cudaError_t launch_match(const MatchArgs& a, int grid, cudaStream_t s);
-// The paired kernel is persistent: `grid` CTAs (the resident ones) take the
-// lanes a block at a time (two blocks with two lanes per thread) from
-// `work`, so the scratch covers only the lanes in flight and no SM idles in
-// a tail wave.
-cudaError_t launch_paired(const PairedArgs& a, int block, int grid, cudaStream_t s);
+// The paired kernel is persistent: `grid` CTAs of OG_LB_THREADS (the resident
+// ones) take the lanes a block at a time (two blocks with two lanes per
+// thread) from `work`, so the scratch covers only the lanes in flight and no
+// SM idles in a tail wave.
+cudaError_t launch_paired(const PairedArgs& a, int grid, cudaStream_t s);
+// Completes a PairTable whose per-entry part is on the device.
+cudaError_t launch_group_table(uint4* table, uint32_t half, cudaStream_t s);
 cudaError_t launch_chain(const ChainArgs& a, int block, int grid, cudaStream_t s);
 
 // Register and shared-memory footprint of the search kernels, for the shape
@@ -178,7 +222,11 @@ struct KernelInfo {
     size_t local_bytes;
     int blocks_per_sm;
 };
-cudaError_t paired_info(int block, uint32_t half, uint32_t lanes_per_thread, KernelInfo* info);
+// Resident blocks per SM of a kernel that allocates tensor memory, from its
+// registers, shared memory and tensor memory: the occupancy calculator counts
+// one block per SM for such a kernel.
+cudaError_t matrix_blocks_per_sm(const void* fn, size_t dynamic_shared, int* blocks);
+cudaError_t paired_info(bool narrow, uint32_t lanes_per_thread, KernelInfo* info);
 cudaError_t chain_info(int block, KernelInfo* info);
 
 }  // namespace og

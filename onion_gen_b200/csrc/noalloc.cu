@@ -39,12 +39,20 @@ constexpr int MAX_DEVICES = 64;
 
 static __device__ __align__(256) uint4 og_noalloc_scratch[SCRATCH_BYTES / sizeof(uint4)];
 
-// Layout inside the array, in uint4 units: the table Q_m (half * 6), the
-// lane centres (lanes * 4) and the Montgomery scratch
-// (lanes * (2 half + 2) * 4).
+// The limit callers are told, in uint4 units: lanes * (2 half + 3) * 64 +
+// half * 96 bytes. Inside it lie the PairTable, the lane centres (lanes * 4)
+// and the CTAs' scratch: 600 g + lanes * (4 + 6 g) for g = groups_of(half),
+// which is less for every half and at least one block of lanes.
 size_t need_uint4(uint32_t lanes, uint32_t half) {
     return (size_t)half * 6 + (size_t)lanes * 4 + (size_t)lanes * (2 * (size_t)half + 2) * 4;
 }
+constexpr bool layout_fits(uint32_t half) {
+    return pair_table_uint4(half) + NBLOCK * 4 + cta_scratch_uint4(half) <=
+               half * 6 + NBLOCK * 4 + (size_t)NBLOCK * (2 * half + 2) * 4 &&
+           cta_scratch_uint4(half) <= (size_t)NBLOCK * (2 * half + 2) * 4;
+}
+static_assert(layout_fits(1) && layout_fits(2) && layout_fits(4) && layout_fits(2048),
+              "the arrays fit in what the limit allows");
 
 // 2^k p for k < POW2 in cached form (y + x, y - x, 2 d x y; Z = 1), passed to
 // the kernels by value as a launch parameter (2304 bytes), so that the call
@@ -76,7 +84,8 @@ struct NoAllocArgs {
 // m - 1.
 __global__ void __launch_bounds__(NBLOCK) noalloc_table_kernel(const NoAllocArgs a, const Pow2Table pow8) {
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= a.half) return;
+    const uint32_t n = groups_of(a.half) * GROUP;
+    if (m >= n) return;
     fe X = words_fe(a.ex), Y = words_fe(a.ey), Z = words_fe(a.ez), T = words_fe(a.et);
     for (uint32_t k = 0; k < POW2; k++)
         if ((m >> k) & 1u) {
@@ -89,7 +98,7 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_table_kernel(const NoAllocArgs
     const fe zi = fe_mulv(Z, fe_invert(fe_mulv(Y, den)));
     const fe v = fe_canon(fe_mulv(den, zi));
     store_fe(a.table + (size_t)m * 2, 1, fe_canon(fe_mulv(fe_sqv(v), const_inv_d())));
-    uint4* const vs = a.table + (size_t)a.half * 2 + (size_t)m * 4;
+    uint4* const vs = a.table + (size_t)n * 2 + (size_t)m * 4;
     store_fe(vs + 0, 1, v);
     store_fe(vs + 2, 1, fe_canon(fe_mulv(fe_mulv(X, Y), zi)));
 }
@@ -113,15 +122,27 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_init_kernel(const NoAllocArgs 
 
 // The production paired kernel with its scratch in the file-scope array; the
 // table is read through L1 as in the single engine.
-__global__ void __launch_bounds__(NBLOCK, 5) noalloc_paired_kernel(const NoAllocArgs a) {
-    __shared__ uint4 stage_s[(NBLOCK / 32) * STAGE_RECORDS * STAGE_WORDS];
+template <bool Narrow>
+__global__ void __launch_bounds__(NBLOCK, 4) noalloc_paired_kernel(const NoAllocArgs a) {
     const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
     const Sink sink{a.bitmap, a.bits, a.hits, a.counter, a.cap, 0, nullptr, 0};
-    const PairTable tab{a.table, a.table + (size_t)a.half * 2};
-    WarpStage st{stage_s + (threadIdx.x / 32) * STAGE_RECORDS * STAGE_WORDS, 0};
-    paired_rounds<true>(a.lanes + lane, a.lanes_n, a.wx, a.wy, a.wdt, tab, a.half, a.rounds,
-                        a.scratch + (size_t)blockIdx.x * a.half * (2 * SCRATCH_ROW) + threadIdx.x, sink, st, lane);
-    stage_flush(sink, tab.vs, st.recs, st.n);
+    const PairTable tab = pair_table_at<const uint4>(a.table, a.half);
+    uint4* const scr = a.scratch + (size_t)blockIdx.x * cta_scratch_uint4(a.half) + threadIdx.x;
+    if constexpr (Narrow) {
+        __shared__ __align__(128) RoundShared sh;
+        MatrixUnit mu;
+        matrix_open(sh);
+        paired_rounds<true>(a.lanes + lane, a.lanes_n, a.wx, a.wy, a.wdt, tab, a.half, a.rounds, scr, sink, sh, mu, lane, true);
+        // a wait that ran out leaves a count beyond any room
+        if (threadIdx.x == 0 && sh.failed) atomicOr(a.counter, 0x80000000u);
+        matrix_close(sh);
+    } else {
+        paired_rounds_full<true>(a.lanes + lane, a.lanes_n, a.wx, a.wy, a.wdt, tab, a.half, a.rounds, scr, sink, lane, true);
+    }
+}
+
+__global__ void __launch_bounds__(NBLOCK) noalloc_groups_kernel(const NoAllocArgs a) {
+    fill_group_table(pair_table_at<const uint4>(a.table, a.half), groups_of(a.half), blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // The array's device address, per device, taken on the first call there.
@@ -182,7 +203,7 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
     NoAllocArgs a;
     std::memset(&a, 0, sizeof a);
     a.table = base;
-    a.lanes = a.table + (size_t)half * 6;
+    a.lanes = a.table + pair_table_uint4(half);
     a.scratch = a.lanes + (size_t)lanes * 4;
     const uint32_t slots = 2 * half + 1;
     // constants computed on the host and passed as launch parameters: the
@@ -216,9 +237,15 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
     // the counter starts at zero on every call
     e = cudaMemsetAsync(d_count, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "memset: %s", cuda_text(e).c_str());
-    noalloc_table_kernel<<<(half + NBLOCK - 1) / NBLOCK, NBLOCK, 0, s>>>(a, pow8);
+    const uint32_t groups = groups_of(half);
+    noalloc_table_kernel<<<(groups * GROUP + NBLOCK - 1) / NBLOCK, NBLOCK, 0, s>>>(a, pow8);
     noalloc_init_kernel<<<lanes / NBLOCK, NBLOCK, 0, s>>>(a, pow2);
-    noalloc_paired_kernel<<<lanes / NBLOCK, NBLOCK, 0, s>>>(a);
+    if (sink_is_narrow(d_bitmap != nullptr, bits, false)) {
+        noalloc_groups_kernel<<<(groups * 48 + NBLOCK - 1) / NBLOCK, NBLOCK, 0, s>>>(a);
+        noalloc_paired_kernel<true><<<lanes / NBLOCK, NBLOCK, 0, s>>>(a);
+    } else {
+        noalloc_paired_kernel<false><<<lanes / NBLOCK, NBLOCK, 0, s>>>(a);
+    }
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "launch: %s", cuda_text(e).c_str());
     return OG_OK;

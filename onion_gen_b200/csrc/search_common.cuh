@@ -9,10 +9,6 @@ namespace og {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-#ifndef OG_LB_THREADS
-#define OG_LB_THREADS 128  // the most threads a block of the search kernels has
-#endif
-
 __device__ __forceinline__ fe load_fe(const uint4* p, size_t qstride) {
     const uint4 a = p[0];
     const uint4 b = p[qstride];
@@ -47,6 +43,7 @@ struct Sink {
     // the prefix bitmap is read from the block's copy in shared memory
     // (og_bitmap_s, staged by the kernel), not through L1
     bool staged = false;
+    uint32_t* failed = nullptr;  // set when a wait of the search kernel ran out
 };
 
 // Prefix bitmaps of at most this many bits (8 KiB) can be staged in shared
@@ -252,23 +249,24 @@ __device__ __forceinline__ void add_cached(fe& X, fe& Y, fe& Z, fe& T, const fe&
 // numerators and 1 -+ d x x2 y y2; the common factors cancel). Its
 // denominator is (1/y2^2 - d x^2) / d, which has no zero because d is not a
 // square, so no centre is exceptional; z is 0 only for the two centres of
-// order four. With one inversion for the round's denominators (Montgomery's
-// trick), the prefix products started from z and e = c / z, a pair costs
-// four multiplications,
+// order four.
 //
-//     P_m = P_(m-1) (q - X),   w = P_(m-1) I  [= z / (q - X)],
-//     I <- I (q - X),          f = e w,
+// The denominators are taken three at a time. With D_i = q_i - X, i = 1..3,
+// and E = D_1 D_2 D_3, the product is a cubic in X whose coefficients are
+// the table's: E = (X^2 + s2) (s1 - X) + e0, one multiplication. With one
+// inversion for the round's E (Montgomery's trick, the prefix products P
+// started from z, and e = c / z):
 //
-// and y(P +- Q) = v w +- s f, of which only what the bitmap reads is
-// computed (low_product below): about a third of a multiplication each.
-// Only P_m is kept between the passes, 32 bytes a pair.
-
-// The table of one half: q per entry (two uint4), then v and s per entry
-// (four), in one array of 6 half uint4.
-struct PairTable {
-    const uint4* q;
-    const uint4* vs;
-};
+//     h = P I [= z / E],  I <- I E,  g_k = X^k h,  f_k = e g_k,  k = 0..2
+//
+// and every key of the group is a sum of the six with constant coefficients,
+//
+//     y(P +- Q_i) = v (q'q'' g_0 - (q' + q'') g_1 + g_2) +- s (the same in f),
+//
+// q' and q'' the other two. So three pairs take nine multiplications, and
+// the six keys are products of lane values with a table of constants: a
+// matrix product, of which only what the bitmap reads is computed, on the
+// tensor cores (keys_of_group).
 
 __device__ __forceinline__ fe const_inv_d() {  // 1/d
     return fe{{0xcdc9f843u, 0x25e0f276u, 0x4279542eu, 0x0b5dd698u, 0xcdb9cf66u, 0x2b162114u, 0x14d5ce43u, 0x40907ed2u}};
@@ -278,167 +276,455 @@ __device__ __forceinline__ fe const_inv_d_plus_1() {  // 1 + 1/d
     return fe{{0xcdc9f844u, 0x25e0f276u, 0x4279542eu, 0x0b5dd698u, 0xcdb9cf66u, 0x2b162114u, 0x14d5ce43u, 0x40907ed2u}};
 }
 
-// What the low limb of a canonical product needs. With T = a b < 2^512 and
-// k = floor(T / p), T mod p = T - k p, and p = -19 (mod 2^32), so its low
-// limb is lo + 19 k with lo = a0 b0 (mod 2^32). T / p is
-// T / 2^255 + 19 T / 2^510 (the next term is below 2^-240), so in units of
-// 2^-31 it is the product's words 7 and 8 plus 38 times its word 15: `acc`
-// holds these from the products of columns 7 and 8 (mod 2^64), the high
-// halves of column 6 and the high half of a7 b7. What is left out: column
-// 6's low halves (below 7), column 5 (below 6) and lower; 38 times the rest
-// of word 15 (below 3.01): the true value is in [acc, acc + 128).
-// About 21 multiply-add slots against 74 for the multiplication.
-struct LowProduct {
-    uint64_t acc;
-    uint32_t lo;
-};
-
-constexpr uint32_t LOW_PRODUCT_ERROR = 128;
-
-__device__ __forceinline__ LowProduct low_product(const fe& a, const fe& b) {
-    uint64_t acc = 0, c6 = 0;
-    uint32_t c8 = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) acc += (uint64_t)a.v[i] * b.v[7 - i];
-#pragma unroll
-    for (int i = 0; i < 7; i++) c6 += __umulhi(a.v[i], b.v[6 - i]);
-#pragma unroll
-    for (int i = 1; i < 8; i++) c8 += a.v[i] * b.v[8 - i];
-    acc += c6 + 38ull * __umulhi(a.v[7], b.v[7]) + ((uint64_t)c8 << 32);
-    return LowProduct{acc, a.v[0] * b.v[0]};
-}
-
-// Whether a key that is the sum (or difference) of two low products may be
-// in the prefix bitmap: its low limb is exact unless the sum's uncertainty
-// (2 LOW_PRODUCT_ERROR above `acc`) reaches the next k, once in 2^23 keys;
-// those count as hits and are decided by the full product.
-__device__ __forceinline__ bool low_may_hit(const Sink& k, uint64_t acc, uint32_t lo) {
-    const uint32_t q = __funnelshift_l((uint32_t)acc, (uint32_t)(acc >> 32), 1);  // acc >> 31
-    const bool unsure = ((uint32_t)acc & 0x7fffffffu) >= 0x80000000u - 2u * LOW_PRODUCT_ERROR;
-    return unsure | prefix_hit(k, lo + 19u * q);
-}
-
-// Candidates that may survive, collected per warp in shared memory: w and f
-// (64 bytes), the candidate's lane and step, and its table entry with the
-// sign (0: the centre, whose y is w). stage_flush computes their keys with
-// 32 lanes at once, tests them exactly and appends the survivors. The search
-// loop itself holds neither the full products nor the record writes, and an
-// index that passes one candidate in a hundred costs it no more than a rare
-// one.
-constexpr uint32_t STAGE_RECORDS = 32;
-constexpr uint32_t STAGE_WORDS = 5;  // uint4 a record
+// Candidates that may survive, collected per warp in shared memory: h, f_0
+// and X (96 bytes), the candidate's lane and step, and its table entry with
+// the sign (0: the centre, whose y is in h's place). stage_flush computes
+// their keys, a lane each, tests them exactly and appends the survivors. The
+// search loop itself holds neither the full products nor the record writes.
+constexpr uint32_t STAGE_RECORDS = 16;
+constexpr uint32_t STAGE_WORDS = 7;  // uint4 a record
 
 struct WarpStage {
     uint4* recs;  // this warp's STAGE_RECORDS records in shared memory
     uint32_t n;   // records held; the same in every lane of the warp
 };
 
-static __device__ __noinline__ void stage_flush(const Sink& k, const uint4* vs, const uint4* recs, uint32_t n) {
+static __device__ __noinline__ void stage_flush(const Sink& k, const PairTable& tab, const uint4* recs, uint32_t n) {
     if (n == 0) return;
     __syncwarp();
     const unsigned me = threadIdx.x & 31u;
     const bool valid = me < n;
     const uint4* r = recs + (valid ? me : 0) * STAGE_WORDS;
-    const fe w = load_fe(r, 1), f = load_fe(r + 2, 1);
-    const uint4 id = r[4];
-    const uint32_t m = id.z & 0x7fffffffu;
-    const uint4* t = vs + (size_t)(m ? m - 1 : 0) * 4;
-    const fe A = fe_mulv(load_fe(t, 1), w), B = fe_mulv(load_fe(t + 2, 1), f);
-    const fe sum = fe_add(A, B), diff = fe_sub(A, B);
-    const fe y = select_fe(m == 0, w, select_fe(id.z >> 31, diff, sum));
+    const fe h = load_fe(r, 1), X = load_fe(r + 4, 1);
+    const uint4 id = r[6];
+    const uint32_t m = id.z & 0x7fffffffu, i = m ? m - 1 : 0, g = i / GROUP * GROUP;
+    // 1 / D_i = (the group's other two D) / E
+    fe others = fe_one();
+    for (uint32_t j = 1; j < GROUP; j++)
+        others = fe_mulv(others, fe_sub(load_fe(tab.q + (size_t)(g + (i - g + j) % GROUP) * 2, 1), X));
+    const uint4* t = tab.vs + (size_t)i * 4;
+    const fe A = fe_mulv(fe_mulv(load_fe(t, 1), others), h);
+    const fe B = fe_mulv(fe_mulv(load_fe(t + 2, 1), others), load_fe(r + 2, 1));
+    const fe y = select_fe(m == 0, h, select_fe(id.z >> 31, fe_sub(A, B), fe_add(A, B)));
     test_emit(k, y, id.x, id.y, valid);
     __syncwarp();
 }
 
-// Adds the candidates of the warp's lanes with `hit` set.
-__device__ __forceinline__ void stage_push(const Sink& k, const uint4* vs, WarpStage& st, bool hit, const fe& w,
-                                           const fe& f, uint32_t lane, uint32_t step, uint32_t entry) {
-    const unsigned mask = __ballot_sync(FULL, hit);
-    if (mask == 0) return;
-    const uint32_t count = (uint32_t)__popc(mask);
-    if (st.n + count > STAGE_RECORDS) {
-        stage_flush(k, vs, st.recs, st.n);
-        st.n = 0;
-    }
-    if (hit) {
-        uint4* r = st.recs + (st.n + (uint32_t)__popc(mask & ((1u << (threadIdx.x & 31u)) - 1u))) * STAGE_WORDS;
-        store_fe(r, 1, w);
-        store_fe(r + 2, 1, f);
-        r[4] = make_uint4(lane, step, entry, 0u);
-    }
-    st.n += count;
+// A lane's group values in shared memory, a row of the matrix product's left
+// operand: g_0, g_1, g_2, f_0, f_1, f_2, whose limbs are its 192 bytes, in
+// twelve 16-byte parts. Part c of row r is at c ROWS + r, so that a warp's
+// stores are contiguous and eight rows of a part are the 128 contiguous bytes
+// the matrix unit reads at once.
+constexpr uint32_t ROWS = 128;
+constexpr uint32_t ROW_PARTS = 12;
+static_assert(OG_LB_THREADS <= ROWS, "a row for every thread of a block");
+
+__device__ __forceinline__ void store_row(uint4* row, uint32_t element, const fe& v) {
+    store_fe(row + element * 2 * ROWS, ROWS, v);
 }
 
-// Rows of a CTA's scratch hold this many threads (the largest block).
-constexpr uint32_t SCRATCH_ROW = OG_LB_THREADS;
+// Adds the candidates of the lanes with `hit` set, from their rows. Every lane
+// of the warp calls it together.
+__device__ __forceinline__ void stage_push(const Sink& k, const PairTable& tab, WarpStage& st, bool hit,
+                                           const uint4* row, const fe& X, uint32_t lane, uint32_t step, uint32_t entry) {
+    for (unsigned mask = __ballot_sync(FULL, hit); mask; mask = __ballot_sync(FULL, hit)) {
+        if (st.n == STAGE_RECORDS) {
+            stage_flush(k, tab, st.recs, st.n);
+            st.n = 0;
+        }
+        const uint32_t at = st.n + (uint32_t)__popc(mask & ((1u << (threadIdx.x & 31u)) - 1u));
+        if (hit && at < STAGE_RECORDS) {
+            uint4* r = st.recs + at * STAGE_WORDS;
+            r[0] = row[0];
+            r[1] = row[ROWS];
+            r[2] = row[6 * ROWS];
+            r[3] = row[7 * ROWS];
+            store_fe(r + 4, 1, X);
+            r[6] = make_uint4(lane, step, entry, 0u);
+            hit = false;
+        }
+        st.n = min(STAGE_RECORDS, st.n + (uint32_t)__popc(mask));
+    }
+}
 
-// One lane's `rounds` paired rounds; see kernels.cuh for the candidate
-// numbering. `centre` points at the lane's affine centre in the lane state
-// (x, then y, 16-byte halves `cstride` apart), which is left on the centre
-// after the last round. `wdt` is d xW yW of the stride W. `scr` is the
-// thread's column of its CTA's scratch: prefix product m, half q at
-// scr + (2 m + q) SCRATCH_ROW. Candidates that may survive go to `st`.
+// Whether a key may be in the prefix bitmap (of at most 24 bits), from its six
+// column sums: with the key T = sum of byte_j rho_j, rho_j the coefficient
+// times 2^(8 j) mod p, the first three sum the bytes against the low 24 bits
+// of rho_j and the others against floor(2^24 rho_j / p), byte by byte. The
+// latter add up to 2^24 T / p less an error below 192 * 255 < 2^16, so
+// k = floor(T / p) is theirs, or one more if bits 16..23 of the sum are all
+// ones; and the key's low limb is that of T + 19 k.
+__device__ __forceinline__ bool columns_may_hit(const Sink& s, const uint32_t* c) {
+    const uint32_t t = c[4] + (c[3] >> 8), u = c[5] + (t >> 8);
+    const uint32_t low = c[0] + (c[1] << 8) + (c[2] << 16) + 19u * (u >> 8);
+    bool hit = prefix_hit(s, low);
+    if ((u & 255u) == 255u) hit |= prefix_hit(s, low + 19u);
+    return hit;
+}
+
+// ---- the matrix product of a group --------------------------------------
+//
+// For the block's 128 lanes, rows (lanes) x 192 bytes times 192 x 48
+// constants (six columns for each of the group's six keys, twelve unused):
+// six tcgen05.mma of kind::i8, unsigned, K = 32, issued by one thread, sums in
+// 48 columns of tensor memory, read back a lane's row by its own thread. It
+// runs while the warps multiply for the next group. The constants come by a
+// bulk copy, 9 KB a group for the whole block. Measured on B200 at half 2048
+// and 757 760 lanes: 52.6 ms a launch, 47.0 with the products left out; by
+// mma.sync a warp, which shares registers and issue slots with the
+// multiplications, 64.2; with the keys' low limbs by multiply-adds, four
+// multiplications and two partial ones a pair, 70.3.
+constexpr uint32_t KEY_COLUMNS = 6;
+constexpr uint32_t COLUMNS = 48;
+constexpr uint32_t TMEM_COLUMNS = 64;  // an allocation is a power of two
+static_assert(GROUP_CONSTANTS == ROW_PARTS * COLUMNS, "the constants of a group are one right operand");
+
+// Shared memory of a block for paired_rounds.
+struct RoundShared {
+    uint4 rows[ROW_PARTS * ROWS];
+    uint4 constants[GROUP_CONSTANTS];  // part c of column n at c COLUMNS + n
+    uint4 stage[(OG_LB_THREADS / 32) * STAGE_RECORDS * STAGE_WORDS];
+    uint64_t product_done, constants_here;  // mbarriers
+    uint32_t tmem;
+    uint32_t failed;  // a wait ran out: the block goes on without products, and the launch has failed
+};
+
+// The block's use of the matrix unit: the phases its two barriers are in.
+struct MatrixUnit {
+    uint32_t product_phase = 0, constants_phase = 0;
+};
+
+__device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// Called by every thread of the block, before the first round and after the
+// last one.
+__device__ __forceinline__ void matrix_open(RoundShared& sh) {
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(shared_addr(&sh.tmem)),
+                     "r"(TMEM_COLUMNS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_addr(&sh.product_done)) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_addr(&sh.constants_here)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        sh.failed = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+
+__device__ __forceinline__ void matrix_close(RoundShared& sh) {
+    // after a failed wait a copy or a product may still be under way: a
+    // millisecond for it to end
+    if (*(volatile uint32_t*)&sh.failed)
+        for (uint32_t i = 0; i < 1000; i++) __nanosleep(1000);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh.tmem), "r"(TMEM_COLUMNS));
+    }
+}
+
+// Waits for the barrier's phase, a bounded number of times (a product takes
+// about a microsecond; the bound is at least tens of milliseconds). If it runs
+// out the block is marked failed, and so is the launch (Sink::failed).
+__device__ __forceinline__ void bounded_wait(RoundShared& sh, const Sink& sink, const uint64_t* bar, uint32_t phase) {
+    constexpr uint32_t LIMIT = 1u << 15;
+    const uint32_t addr = shared_addr(bar);
+    if (*(volatile uint32_t*)&sh.failed) return;
+    for (uint32_t i = 0; i < LIMIT; i++) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(addr), "r"(phase)
+            : "memory");
+        if (done) return;
+    }
+    *(volatile uint32_t*)&sh.failed = 1;
+    if (sink.failed) atomicExch(sink.failed, 1u);
+}
+
+// Fetches group j's constants (one thread; the product that read the last ones
+// is done).
+__device__ __forceinline__ void fetch_constants(RoundShared& sh, const uint4* constants) {
+    const uint32_t bar = shared_addr(&sh.constants_here);
+    constexpr uint32_t bytes = GROUP_CONSTANTS * 16;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     shared_addr(sh.constants)),
+                 "l"(constants), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// Every thread's row is written: starts the product (thread 0 issues it).
+__device__ __forceinline__ void start_product(RoundShared& sh, const Sink& sink, MatrixUnit& mu) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        bounded_wait(sh, sink, &sh.constants_here, mu.constants_phase);
+        if (!sh.failed) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // K-major operands without swizzle: 8 rows of 16 bytes contiguous,
+            // 8-row groups 128 bytes apart (bits 32..45), the 16-byte parts a
+            // part's size apart (bits 16..29), all in units of 16 bytes
+            constexpr uint64_t common = (8ull << 32) | (1ull << 46);
+            uint64_t a = common | ((uint64_t)ROWS << 16) | (shared_addr(sh.rows) >> 4);
+            uint64_t b = common | ((uint64_t)COLUMNS << 16) | (shared_addr(sh.constants) >> 4);
+            // 32-bit sums, unsigned 8-bit operands, N = 48, M = 128
+            constexpr uint32_t idesc = (2u << 4) | ((COLUMNS / 8) << 17) | ((ROWS / 16) << 24);
+#pragma unroll
+            for (uint32_t k = 0; k < ROW_PARTS / 2; k++) {
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\t"
+                    "setp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(sh.tmem),
+                    "l"(a), "l"(b), "r"(idesc), "r"(k)
+                    : "memory");
+                a += 2 * ROWS;
+                b += 2 * COLUMNS;
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             shared_addr(&sh.product_done))
+                         : "memory");
+        }
+    }
+    mu.constants_phase ^= 1;
+}
+
+// Waits for the product.
+__device__ __forceinline__ void finish_product(RoundShared& sh, const Sink& sink, MatrixUnit& mu) {
+    bounded_wait(sh, sink, &sh.product_done, mu.product_phase);
+    mu.product_phase ^= 1;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+
+// Tests the six keys of the group whose first entry is m0 (entries past `half`
+// belong to no key of the round) from the finished product.
+__device__ __forceinline__ void test_group(RoundShared& sh, const Sink& sink, const PairTable& tab, WarpStage& st,
+                                           const fe& X, uint32_t lane, bool active, uint32_t mid, uint32_t m0,
+                                           uint32_t half) {
+    const uint32_t from = sh.tmem + ((threadIdx.x / 32) << 21);  // 32 lanes a warp, in bits 16 and up
+    uint32_t hits = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < GROUP; i++) {
+        uint32_t c[2 * KEY_COLUMNS];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%12];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8, %9, %10, %11}, [%13];\n\t"
+            "tcgen05.wait::ld.sync.aligned;"
+            : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7]), "=r"(c[8]),
+              "=r"(c[9]), "=r"(c[10]), "=r"(c[11])
+            : "r"(from + i * 2 * KEY_COLUMNS), "r"(from + i * 2 * KEY_COLUMNS + 8)
+            : "memory");
+        if (m0 + i <= half)
+            hits |= ((columns_may_hit(sink, c) ? 1u : 0u) | (columns_may_hit(sink, c + KEY_COLUMNS) ? 2u : 0u)) << (2 * i);
+    }
+    if (!active) hits = 0;
+    if (__any_sync(FULL, hits)) {
+        const uint4* row = sh.rows + threadIdx.x;
+#pragma unroll 1
+        for (uint32_t key = 0; key < 2 * GROUP; key++) {
+            const uint32_t m = m0 + key / 2;
+            stage_push(sink, tab, st, (hits >> key) & 1u, row, X, lane, key & 1u ? mid - m : mid + m,
+                       key & 1u ? m | 0x80000000u : m);
+        }
+    }
+}
+
+// What a lane's round keeps for its second pass.
+struct RoundState {
+    fe X, e, I;
+};
+
+// The part of a round between its passes: the inversion, e = c / z and
+// I = 1 / prod E, and the next centre. The stride is added by the complete
+// addition: with k = d x y xW yW, x(P + W) = (x yW + y xW) / (1 + k) and
+// y(P + W) = (y yW + x xW) / (1 - k); 1 - k^2 joins the inversion.
 // OneInversion: one field inversion for the block's lanes (block_invert),
 // else one a lane.
 template <bool OneInversion>
+__device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe& y, const fe& z, const fe& run,
+                                           uint4* centre, size_t cstride, bool active, const FeWords& wx,
+                                           const FeWords& wy, const FeWords& wdt) {
+    const fe k = fe_mulv(fe_mulv(x, y), words_fe(wdt));
+    const fe one_k2 = fe_sub(fe_one(), fe_sqv(k));
+    const fe total = fe_mulv(fe_mulv(run, z), one_k2);
+    const fe U = OneInversion ? block_invert(total) : fe_invert(total);
+    const fe a = fe_mulv(U, one_k2);
+    s.e = fe_mulv(fe_mulv(const_inv_d_plus_1(), x), fe_mulv(a, run));
+    s.I = fe_mulv(fe_sqv(z), a);
+    const fe inv = fe_mulv(run, fe_mulv(z, U));  // 1 / (1 - k^2)
+    const fe nx = fe_mulv(fe_add(fe_mulv(x, words_fe(wy)), fe_mulv(y, words_fe(wx))),
+                          fe_mulv(fe_sub(fe_one(), k), inv));
+    const fe ny = fe_mulv(fe_add(fe_mulv(y, words_fe(wy)), fe_mulv(x, words_fe(wx))),
+                          fe_mulv(fe_add(fe_one(), k), inv));
+    if (active) {
+        store_fe(centre, cstride, nx);
+        store_fe(centre + 2 * cstride, cstride, ny);
+    }
+}
+
+// A block's `rounds` paired rounds, a lane each, against a prefix bitmap of at
+// most 24 bits (sink_is_narrow); see kernels.cuh for the candidate numbering.
+// `centre` points at the lane's affine centre in the lane state (x, then y,
+// 16-byte halves `cstride` apart), which is left on the centre after the last
+// round. `wdt` is d xW yW of the stride W. `scr` is the thread's column of its
+// CTA's scratch: group j's prefix product, then E, half q at
+// scr + (4 j + 2 e + q) SCRATCH_ROW. A thread that is not `active` has no lane:
+// it takes part with another's centre and reports nothing. Every thread of
+// the block calls it together, between matrix_open and matrix_close.
+template <bool OneInversion>
 __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, const FeWords& wx, const FeWords& wy,
                                               const FeWords& wdt, const PairTable& tab, uint32_t half, uint32_t rounds,
-                                              uint4* scr, const Sink& sink, WarpStage& st, uint32_t lane) {
-    const uint32_t slots = 2 * half + 1;
-    const bool approx = sink.bitmap && !sink.sbitmap;
+                                              uint4* scr, const Sink& sink, RoundShared& sh, MatrixUnit& mu,
+                                              uint32_t lane, bool active) {
+    const uint32_t slots = 2 * half + 1, groups = groups_of(half);
+    uint4* const row = sh.rows + threadIdx.x;
+    WarpStage st{sh.stage + threadIdx.x / 32 * STAGE_RECORDS * STAGE_WORDS, 0};
     for (uint32_t r = 0; r < rounds; r++) {
-        fe X, e, I;
+        RoundState s;
+        const uint32_t mid = r * slots + half;
+        if (threadIdx.x == 0 && !sh.failed) fetch_constants(sh, tab.constants + (size_t)(groups - 1) * GROUP_CONSTANTS);
+        {
+            const fe x = load_fe(centre, cstride), y = load_fe(centre + 2 * cstride, cstride);
+            s.X = fe_sqv(x);
+            const fe X2 = fe_sqv(s.X), z = fe_mulv(y, fe_sub(const_inv_d(), s.X));
+            fe run = z;
+#pragma unroll 1
+            for (uint32_t j = 0; j < groups; j++) {
+                const uint4* t = tab.cubic + (size_t)j * 6;
+                uint4* const p = scr + (size_t)j * (4 * SCRATCH_ROW);
+                store_fe(p, SCRATCH_ROW, run);
+                const fe E = fe_add(fe_mulv(fe_add(X2, load_fe(t + 2, 1)), fe_sub(load_fe(t, 1), s.X)),
+                                    load_fe(t + 4, 1));
+                store_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW, E);
+                run = fe_mulv(run, E);
+            }
+            turn_round<OneInversion>(s, x, y, z, run, centre, cstride, active, wx, wy, wdt);
+            // the centre's own key: its low limb is exact with bit 255
+            // folded, unless y is p or more
+            const bool hit = active && ((y.v[7] & 0x7fffffffu) == 0x7fffffffu ||
+                                        prefix_hit(sink, y.v[0] + ((y.v[7] >> 31) ? 19u : 0u)));
+            store_row(row, 0, y);
+            stage_push(sink, tab, st, hit, row, s.X, lane, mid, 0u);
+        }
+#pragma unroll 1
+        for (uint32_t j = groups; j-- > 0;) {
+            const uint4* p = scr + (size_t)j * (4 * SCRATCH_ROW);
+            const fe h = fe_mulv(load_fe(p, SCRATCH_ROW), s.I);
+            s.I = fe_mulv(s.I, load_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW));
+            if (j + 1 < groups) {
+                // the product of the group before, which ran meanwhile
+                finish_product(sh, sink, mu);
+                if (threadIdx.x == 0 && !sh.failed) fetch_constants(sh, tab.constants + (size_t)j * GROUP_CONSTANTS);
+                test_group(sh, sink, tab, st, s.X, lane, active, mid, (j + 1) * GROUP + 1, half);
+            }
+            store_row(row, 0, h);
+            store_row(row, 3, fe_mulv(s.e, h));
+            const fe g1 = fe_mulv(s.X, h);
+            store_row(row, 1, g1);
+            store_row(row, 4, fe_mulv(s.e, g1));
+            const fe g2 = fe_mulv(s.X, g1);
+            store_row(row, 2, g2);
+            store_row(row, 5, fe_mulv(s.e, g2));
+            start_product(sh, sink, mu);
+        }
+        finish_product(sh, sink, mu);
+        test_group(sh, sink, tab, st, s.X, lane, active, mid, 1, half);
+    }
+    stage_flush(sink, tab, st.recs, st.n);
+}
+
+// The same rounds with every key computed in full: for sinks with a suffix
+// bitmap, with a prefix bitmap of more than 24 bits, or with none (every
+// candidate survives). A pair takes six multiplications: per pair the prefix
+// product, w = P I [= z / D], I <- I D, f = e w and y = v w +- s f.
+template <bool OneInversion>
+__device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride, const FeWords& wx, const FeWords& wy,
+                                                   const FeWords& wdt, const PairTable& tab, uint32_t half,
+                                                   uint32_t rounds, uint4* scr, const Sink& sink, uint32_t lane,
+                                                   bool active) {
+    const uint32_t slots = 2 * half + 1;
+    for (uint32_t r = 0; r < rounds; r++) {
+        RoundState s;
         const uint32_t mid = r * slots + half;
         {
             const fe x = load_fe(centre, cstride), y = load_fe(centre + 2 * cstride, cstride);
-            X = fe_sqv(x);
-            const fe z = fe_mulv(y, fe_sub(const_inv_d(), X));
+            s.X = fe_sqv(x);
+            const fe z = fe_mulv(y, fe_sub(const_inv_d(), s.X));
             fe run = z;
 #pragma unroll 1
             for (uint32_t m = 0; m < half; m++) {
                 store_fe(scr + (size_t)m * (2 * SCRATCH_ROW), SCRATCH_ROW, run);
-                run = fe_mulv(run, fe_sub(load_fe(tab.q + (size_t)m * 2, 1), X));
+                run = fe_mulv(run, fe_sub(load_fe(tab.q + (size_t)m * 2, 1), s.X));
             }
-            // the stride by the complete addition: with k = d x y xW yW,
-            // x(P + W) = (x yW + y xW) / (1 + k), y(P + W) = (y yW + x xW) / (1 - k);
-            // 1 - k^2 joins the round's inversion
-            const fe k = fe_mulv(fe_mulv(x, y), words_fe(wdt));
-            const fe E = fe_sub(fe_one(), fe_sqv(k));
-            const fe total = fe_mulv(fe_mulv(run, z), E);  // z^2 E prod(q - X)
-            const fe U = OneInversion ? block_invert(total) : fe_invert(total);
-            const fe a = fe_mulv(U, E);
-            e = fe_mulv(fe_mulv(const_inv_d_plus_1(), x), fe_mulv(a, run));  // c / z
-            I = fe_mulv(fe_sqv(z), a);
-            const fe invE = fe_mulv(run, fe_mulv(z, U));
-            const fe nx = fe_mulv(fe_add(fe_mulv(x, words_fe(wy)), fe_mulv(y, words_fe(wx))),
-                                  fe_mulv(fe_sub(fe_one(), k), invE));
-            const fe ny = fe_mulv(fe_add(fe_mulv(y, words_fe(wy)), fe_mulv(x, words_fe(wx))),
-                                  fe_mulv(fe_add(fe_one(), k), invE));
-            store_fe(centre, cstride, nx);
-            store_fe(centre + 2 * cstride, cstride, ny);
-            // the centre's own key: its low limb is exact with bit 255
-            // folded, unless y is p or more
-            const bool hit = !approx || (y.v[7] & 0x7fffffffu) == 0x7fffffffu ||
-                             prefix_hit(sink, y.v[0] + ((y.v[7] >> 31) ? 19u : 0u));
-            stage_push(sink, tab.vs, st, hit, y, y, lane, mid, 0u);
+            turn_round<OneInversion>(s, x, y, z, run, centre, cstride, active, wx, wy, wdt);
+            test_emit(sink, y, lane, mid, active);
         }
 #pragma unroll 1
         for (uint32_t m = half; m >= 1; m--) {
-            const fe w = fe_mulv(load_fe(scr + (size_t)(m - 1) * (2 * SCRATCH_ROW), SCRATCH_ROW), I);
-            I = fe_mulv(I, fe_sub(load_fe(tab.q + (size_t)(m - 1) * 2, 1), X));
-            const fe f = fe_mulv(e, w);
-            bool plus = true, minus = true;
-            if (approx) {
-                const uint4* t = tab.vs + (size_t)(m - 1) * 4;
-                const LowProduct A = low_product(load_fe(t, 1), w), B = low_product(load_fe(t + 2, 1), f);
-                plus = low_may_hit(sink, A.acc + B.acc, A.lo + B.lo);
-                minus = low_may_hit(sink, A.acc - B.acc - LOW_PRODUCT_ERROR, A.lo - B.lo);
-            }
-            if (__any_sync(FULL, plus | minus)) {
-                stage_push(sink, tab.vs, st, plus, w, f, lane, mid + m, m);
-                stage_push(sink, tab.vs, st, minus, w, f, lane, mid - m, m | 0x80000000u);
-            }
+            const fe w = fe_mulv(load_fe(scr + (size_t)(m - 1) * (2 * SCRATCH_ROW), SCRATCH_ROW), s.I);
+            s.I = fe_mulv(s.I, fe_sub(load_fe(tab.q + (size_t)(m - 1) * 2, 1), s.X));
+            const uint4* t = tab.vs + (size_t)(m - 1) * 4;
+            const fe B = fe_mulv(load_fe(t + 2, 1), fe_mulv(s.e, w)), A = fe_mulv(load_fe(t, 1), w);
+#pragma unroll 1
+            for (uint32_t sign = 0; sign < 2; sign++)
+                test_emit(sink, sign ? fe_sub(A, B) : fe_add(A, B), lane, sign ? mid - m : mid + m, active);
         }
+    }
+}
+
+// Fills the per-group part of a PairTable from its q, v and s, one thread for
+// each (group, key, element) of 8 keys (the last two get zeros) and six
+// elements; the threads of element 0 and key 0 write the cubic. `tab` is the
+// table being written.
+__device__ inline void fill_group_table(const PairTable& tab, uint32_t groups, uint32_t thread) {
+    const uint32_t g = thread / 48, key = thread / 6 % 8, elem = thread % 6;
+    if (g >= groups) return;
+    const uint32_t i = key / 2;  // the key's pair
+    fe q[GROUP];
+    for (uint32_t j = 0; j < GROUP; j++) q[j] = load_fe(tab.q + (size_t)(g * GROUP + j) * 2, 1);
+    if (key == 0 && elem == 0) {
+        const fe s1 = fe_add(fe_add(q[0], q[1]), q[2]), q01 = fe_mulv(q[0], q[1]);
+        const fe s2 = fe_add(q01, fe_mulv(q[2], fe_add(q[0], q[1])));
+        uint4* const t = const_cast<uint4*>(tab.cubic) + (size_t)g * 6;
+        store_fe(t, 1, s1);
+        store_fe(t + 2, 1, s2);
+        store_fe(t + 4, 1, fe_sub(fe_mulv(q01, q[2]), fe_mulv(s1, s2)));
+    }
+    fe c = fe_one();
+    if (key < 2 * GROUP) {
+        const uint4* vs = tab.vs + (size_t)(g * GROUP + i) * 4;
+        const fe zero = fe_sub(fe_one(), fe_one()), qa = q[(i + 1) % GROUP], qb = q[(i + 2) % GROUP];
+        c = load_fe(elem < 3 ? vs : vs + 2, 1);
+        if (elem % 3 == 0) c = fe_mulv(c, fe_mulv(qa, qb));
+        if (elem % 3 == 1) c = fe_sub(zero, fe_mulv(c, fe_add(qa, qb)));
+        if (elem >= 3 && (key & 1)) c = fe_sub(zero, c);
+    }
+    uint32_t* const out = reinterpret_cast<uint32_t*>(const_cast<uint4*>(tab.constants) + (size_t)g * GROUP_CONSTANTS);
+    const fe times256 = fe{{256u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}};
+    for (uint32_t word = 0; word < 8; word++) {
+        uint32_t col[KEY_COLUMNS] = {0, 0, 0, 0, 0, 0};
+        for (uint32_t byte = 0; byte < 4; byte++) {
+            const fe rho = fe_canon(c);
+            const uint32_t frac = rho.v[7] >> 7;  // floor(2^24 rho / p), or one less
+            for (uint32_t n = 0; n < 3; n++) {
+                col[n] |= (rho.v[0] >> (8 * n) & 255u) << (8 * byte);
+                col[3 + n] |= (frac >> (8 * n) & 255u) << (8 * byte);
+            }
+            c = fe_mulv(c, times256);
+        }
+        for (uint32_t n = 0; n < KEY_COLUMNS; n++)
+            out[((elem * 2 + word / 4) * COLUMNS + key * KEY_COLUMNS + n) * 4 + word % 4] =
+                key < 2 * GROUP ? col[n] : 0u;
     }
 }
 
