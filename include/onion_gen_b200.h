@@ -71,32 +71,31 @@ typedef struct og_engine og_engine;
 int og_engine_new(int ordinal, const uint8_t start[128], uint32_t threads, const uint64_t* bitmap,
                   size_t words, uint32_t bits, int retune, og_engine** out, char* err, size_t errlen);
 
-/* Enumeration schemes. */
+/* Enumeration schemes: where a search's candidates lie. Both run on the same
+ * kernel. */
 enum og_scheme {
-    OG_SCHEME_PAIRED = 0, /* y(P +- Q_m) around an affine centre, one inversion per round */
-    OG_SCHEME_CHAIN = 1   /* +8G chain, Z batch-inverted over n steps (src/batch.rs) */
+    OG_SCHEME_PAIRED = 0, /* windows of 2 half + 1 candidates a lane, from 8G past the start on */
+    OG_SCHEME_CHAIN = 1   /* n steps of +8G a lane from the start on (src/batch.rs) */
 };
 
-/* Launch shape of an engine. Zero fields take defaults. */
+/* Launch shape of an engine: what one advance covers. Zero fields take
+ * defaults. How the device tiles an advance's candidates over its threads is
+ * the engine's own choice. */
 typedef struct og_engine_config {
     uint32_t scheme;   /* og_scheme */
-    uint32_t half;     /* paired: table size, a round is 2*half+1 candidates (0: 2048, halved
+    uint32_t half;     /* paired: a lane's round is 2*half+1 candidates (0: 2048, halved
                           down to 256 while one advance would return more than 2^26 expected
                           survivors). chain: n steps (0: 1024) */
-    uint32_t lanes;    /* lanes (independent chains), a multiple of `block`. The paired
-                          kernel runs as many CTAs as are resident and they take the lanes
-                          a block at a time, so its scratch is that of the resident CTAs
-                          whatever the lanes (0: eight blocks per resident CTA, fewer only
-                          if half 256 still passes that survivor budget). The chain kernel is
-                          persistent the same way (0: four blocks per resident CTA) */
+    uint32_t lanes;    /* lanes (independent windows), a multiple of `block` (0, paired: eight
+                          waves of og_engine_resident_lanes, fewer only if half 256 still
+                          passes that survivor budget; chain: four waves) */
     uint32_t rounds;   /* rounds per advance */
-    uint32_t block;    /* threads per CUDA block, a multiple of 32 */
+    uint32_t block;    /* what lanes are rounded up to, a multiple of 32 up to 128 */
     uint32_t dump;     /* 1: ignore the bitmap, every candidate survives (parity runs) */
     uint32_t room;     /* survivor records per advance; 0 sizes it from the bitmaps' occupancy:
                           the expected count plus eight standard deviations */
-    uint32_t lanes_per_thread; /* paired: lanes each thread of the search kernel takes at a time,
-                          1 or 2, one after the other (0: 1); `lanes` is then a multiple of
-                          block x this. Chain: 1 */
+    uint32_t lanes_per_thread; /* paired: 1 or 2 (0: 1); lanes are rounded up to block x this, and
+                          a wave of the default lanes is counted at this many a thread. Chain: 1 */
 } og_engine_config;
 
 /* The same engine with an explicit shape (no tuning). `bitmap` may be NULL
@@ -113,9 +112,9 @@ uint64_t og_engine_batch(const og_engine* e);
 size_t og_engine_room(const og_engine* e);
 /* The shape in use. */
 void og_engine_shape(const og_engine* e, og_engine_config* cfg);
-/* Lanes one wave of the search kernel of `scheme` holds on device `ordinal`:
- * resident blocks per SM x SMs x `block` (0: 128). The paired kernel runs
- * exactly this many threads and they take the lanes a block at a time. */
+/* The lanes that default shapes are counted in waves of, on device `ordinal`:
+ * a fixed number of blocks per SM (five at block 128) x SMs x `block`
+ * (0: 128). */
 int og_engine_resident_lanes(int ordinal, uint32_t scheme, uint32_t block, uint32_t* lanes, char* err,
                              size_t errlen);
 

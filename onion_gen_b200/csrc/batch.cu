@@ -31,7 +31,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstddef>
 #include <cstring>
@@ -61,7 +60,7 @@
 namespace og {
 
 cudaError_t make_pair_table(DevBuf<uint4>& table, uint32_t half, cudaStream_t s);  // engine.cu
-std::array<FeWords, 3> stride_words(const Pt& w);              // engine.cu
+Stride stride_of(const Pt& w);                                     // engine.cu
 std::vector<uint4> pow2_table(const Pt& stride, uint32_t nbits);  // engine.cu
 MatchTables match_tables(const std::vector<FilterSet::DeviceBucket>& buckets, const uint64_t* keys,
                          const uint32_t* owners, const uint32_t* patterns,
@@ -88,7 +87,7 @@ constexpr double NEED_STEPS = 2.0;
 constexpr size_t STAGED_BYTES = (size_t)(1u << STAGED_BITMAP_BITS) / 8u;
 
 struct BatchDesc {
-    FeWords wx, wy, wdt;     // the search's stride for this step: W = L (2 half + 1) 8 G, affine, and d wx wy
+    Stride stride;           // the search's stride for this step: L (2 half + 1) 8 G
     FeWords bx, by, bz, bt;  // centre of window W_done (where new lanes start), extended
     const uint32_t* bitmap;  // prefix bitmap (nullptr: the search has no prefix)
     uint32_t bits;
@@ -209,10 +208,10 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_
                         &a.counters->failed};
         uint4* const scr = a.scratch + blockIdx.x * a.cta_scratch + threadIdx.x;
         if (sink_is_narrow(d.bitmap != nullptr, d.bits, d.sbitmap != nullptr))
-            paired_rounds<false>(a.lanes + slot, a.slots, d.wx, d.wy, d.wdt, a.table, d.half, a.rounds, scr, sink, sh,
+            paired_rounds<false>(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink, sh,
                                  mu, slot, true);
         else
-            paired_rounds_full<false>(a.lanes + slot, a.slots, d.wx, d.wy, d.wdt, a.table, d.half, a.rounds, scr, sink,
+            paired_rounds_full<false>(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink,
                                       slot, true);
     }
     matrix_close(sh);
@@ -398,7 +397,7 @@ struct og_batch {
     std::map<uint64_t, std::unique_ptr<Search>> searches;
     std::vector<uint32_t> free_sidx;
     std::vector<uint32_t> free_blocks;
-    std::map<std::pair<uint32_t, uint32_t>, std::array<FeWords, 3>> strides;  // per (lanes, half)
+    std::map<std::pair<uint32_t, uint32_t>, Stride> strides;  // per (lanes, half)
     uint64_t admitted = 0;
     uint64_t mem_used = 0, mem_budget = 0;
     bool active_changed = true;
@@ -440,11 +439,11 @@ namespace {
                         "%s: %s", #call, cuda_text(_e).c_str());                                 \
     } while (0)
 
-const std::array<FeWords, 3>& stride_for(og_batch* b, uint32_t lanes, uint32_t half) {
+const Stride& stride_for(og_batch* b, uint32_t lanes, uint32_t half) {
     const auto key = std::make_pair(lanes, half);
     auto it = b->strides.find(key);
     if (it != b->strides.end()) return it->second;
-    const std::array<FeWords, 3> w = stride_words(base_mult_u64(8ULL * (2ULL * half + 1) * lanes));
+    const Stride w = stride_of(base_mult_u64(8ULL * (2ULL * half + 1) * lanes));
     return b->strides.emplace(key, w).first->second;
 }
 
@@ -622,11 +621,7 @@ int launch(og_batch* b, bool& launched, char* err, size_t errlen) {
         if (s.done || s.blocks.empty()) continue;
         const uint32_t lanes = (uint32_t)s.blocks.size() * BLOCK;
         if (lanes != s.lanes_stride) {
-            const auto& w = stride_for(b, lanes, s.half);
-            BatchDesc& d = b->h_descs[s.sidx];
-            d.wx = w[0];
-            d.wy = w[1];
-            d.wdt = w[2];
+            b->h_descs[s.sidx].stride = stride_for(b, lanes, s.half);
             s.lanes_stride = lanes;
             b->mark(s.sidx);
         }

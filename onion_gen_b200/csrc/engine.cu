@@ -11,7 +11,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstddef>
@@ -64,11 +63,11 @@ static const F51& inv_curve_d() {
     return v;
 }
 
-// The stride words of the paired round: x, y and d x y of an affine point.
-std::array<FeWords, 3> stride_words(const Pt& w) {
+// A stride of the paired round.
+Stride stride_of(const Pt& w) {
     F51 x, y;
     pt_affine(w, x, y);
-    return {to_words(x), to_words(y), to_words(f_mul(curve_d(), f_mul(x, y)))};
+    return Stride{to_words(x), to_words(y), to_words(f_mul(curve_d(), f_mul(x, y)))};
 }
 
 // The per-entry part of the PairTable of Q_m = 8m G for half `half` (q =
@@ -191,8 +190,9 @@ struct og_engine {
     cudaStream_t stream = nullptr;
     og_engine_config cfg{};
     uint32_t slots = 0;
+    uint64_t batch = 0;  // candidates of an advance
     uint32_t bits = 0;
-    uint32_t grid = 0;  // persistent CTAs of the paired kernel
+    uint32_t grid = 0;  // persistent CTAs of the search kernel
     size_t cap = 0;
     uint64_t launches = 0;
     float last_ms = 0;
@@ -218,7 +218,6 @@ struct og_engine {
     static constexpr int COPY_CHUNKS = 16;
     cudaEvent_t chunk_ev[COPY_CHUNKS] = {};  // a chunk of the records has reached h_recs
     PairedArgs pa{};
-    ChainArgs ca{};
     uint64_t bitmap_hash = 0;  // of the bitmap the engine was created with
     DevBuf<uint32_t> sbitmap;  // suffix bitmap (og_engine_new_filters)
     uint32_t sbits = 0;
@@ -263,42 +262,62 @@ namespace {
                         "%s: %s", #call, cuda_text(_e).c_str());                              \
     } while (0)
 
-// The lanes that shapes are counted in waves of. For the paired scheme these
-// are the blocks an SM held while its kernel had 96 registers a thread (21
-// warps, and at most 11 blocks; 16 and 8 with two lanes per thread): a fixed
-// count, so that a default shape, and with it what one advance covers, does
-// not move with the kernel's resources. The chain kernel's are its resident
-// blocks.
+// The lanes that shapes are counted in waves of: the blocks an SM held while
+// the search kernels had 96 registers a thread (21 warps; at most 11 blocks
+// of the paired scheme's; 16 warps and 8 blocks with two lanes per thread). A
+// fixed count, so that a default shape, and with it what one advance covers,
+// does not move with the kernel's resources.
 int resident_lanes(int device, uint32_t scheme, uint32_t block, uint32_t* out, char* err, size_t errlen,
                    uint32_t lanes_per_thread = 1) {
-    uint32_t blocks = 0;
-    if (scheme == OG_SCHEME_CHAIN) {
-        KernelInfo info{};
-        const cudaError_t e = chain_info((int)block, &info);
-        if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "kernel attributes: %s", cuda_text(e).c_str());
-        blocks = (uint32_t)std::max(0, info.blocks_per_sm);
-    } else if (block <= OG_LB_THREADS) {
-        blocks = lanes_per_thread == 2 ? std::min(8u, 16u / (block / 32)) : std::min(11u, 21u / (block / 32));
+    uint32_t blocks = 1;
+    if (block <= OG_LB_THREADS) {
+        blocks = (lanes_per_thread == 2 ? 16u : 21u) / (block / 32);
+        if (scheme == OG_SCHEME_PAIRED) blocks = std::min(lanes_per_thread == 2 ? 8u : 11u, blocks);
     }
     int sms = 0;
     const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "device attributes: %s", cuda_text(e).c_str());
-    *out = std::max(1u, blocks) * (uint32_t)sms * block * lanes_per_thread;
+    *out = blocks * (uint32_t)sms * block * lanes_per_thread;
     return OG_OK;
 }
 
-// The persistent CTAs a search of `lanes` lanes runs on: as many as are
-// resident, but no more than it has blocks of lanes.
-int search_grid(int device, const og_engine_config& cfg, bool narrow, uint32_t* out, char* err, size_t errlen) {
-    KernelInfo info{};
-    const bool chain = cfg.scheme == OG_SCHEME_CHAIN;
-    cudaError_t e = chain ? chain_info((int)cfg.block, &info) : paired_info(narrow, cfg.lanes_per_thread, &info);
+// How the search kernel covers the `batch` candidates of an advance: on `grid`
+// CTAs, `lanes` lanes of `rounds` windows of 2 half + 1 candidates each. The
+// caller's half and lanes only say how many candidates that is and how they
+// are numbered.
+struct Tile {
+    uint32_t half, lanes, rounds, grid;
+};
+
+// As few rounds a CTA as the scratch allows, all of the same length, and no
+// CTA left with one more than the others. A round's own cost (the prologue, the
+// block's inversion, the next centre) is that of about 20 groups of three pairs
+// when every CTA of an SM pays it at once, and a last wave that some CTAs skip
+// costs nearly a whole one. On B200, ms a launch with 1, 2, 3 and 6 rounds a
+// CTA: 9.7e7 candidates 0.94, 1.10, 1.20, 1.48; 1.9e8 3.50, 3.66, 3.75, 4.05; the
+// callers' shapes (half 256, 333 and 512) ran 1.90 for 1.9e8 at half 256, 2.43
+// for 7.7e7 (now 1.45), and 3.49. 3.1e9 candidates: 9 rounds 51.7, 6 51.6 with
+// half as much scratch again, 10 (the caller's half 2048) 53.0, 20 53.2.
+constexpr uint32_t MIN_GROUPS = 2, MAX_GROUPS = 768;  // the longest: 5.6 GB of scratch
+constexpr uint32_t MAX_TILE_LANES = 1u << 23;  // 0.5 GB of lane state
+
+int plan_tile(int device, uint64_t batch, bool narrow, Tile* out, char* err, size_t errlen) {
+    int blocks = 0, sms = 0;
+    cudaError_t e = paired_blocks_per_sm(narrow, &blocks);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "kernel attributes: %s", cuda_text(e).c_str());
-    int sms = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "device attributes: %s", cuda_text(e).c_str());
-    const uint32_t per_item = chain ? cfg.block : OG_LB_THREADS * cfg.lanes_per_thread;
-    *out = std::min((uint32_t)std::max(1, info.blocks_per_sm) * (uint32_t)sms, (cfg.lanes + per_item - 1) / per_item);
+    const uint32_t ctas = (uint32_t)std::max(1, blocks) * (uint32_t)sms;
+    const uint64_t threads = (uint64_t)ctas * OG_LB_THREADS, longest = 2 * GROUP * MAX_GROUPS + 1;
+    const uint64_t waves = (batch + threads * longest - 1) / (threads * longest);
+    const uint64_t window = (batch + threads * waves - 1) / (threads * waves);
+    out->half = GROUP * std::max(MIN_GROUPS, (uint32_t)((window + 2 * GROUP - 2) / (2 * GROUP)));
+    const uint64_t slots = 2ULL * out->half + 1, windows = (batch + slots - 1) / slots;
+    const uint64_t rounds = (windows + MAX_TILE_LANES - 1) / MAX_TILE_LANES;
+    if (rounds * slots > 0xffffffffULL) return fail(err, errlen, OG_E_ARG, "too many candidates per advance");
+    out->rounds = (uint32_t)rounds;
+    out->lanes = (uint32_t)((windows + rounds - 1) / rounds);
+    out->grid = std::min(ctas, (out->lanes + OG_LB_THREADS - 1) / OG_LB_THREADS);
     return OG_OK;
 }
 
@@ -371,24 +390,15 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
         int rc = resident_lanes(ordinal, cfg.scheme, cfg.block, &resident, err, errlen, lpt);
         if (rc) return rc;
         if (cfg.scheme == OG_SCHEME_PAIRED) {
-            // the persistent kernel takes lanes a block at a time: eight
-            // blocks per resident CTA leave the last ones little tail
-            // (measured +3.5% over two), while the scratch stays that of the
-            // resident CTAs. When one advance would return more than the
-            // survivor budget, a shorter inversion batch comes first (config
-            // 3's 5 % survivors on B200: half 512 at eight waves 19.2 G keys/s,
-            // half 2048 at one wave 16.6), then fewer waves.
+            // eight waves at half 2048: 3.1e9 candidates. When one advance
+            // would return more than the survivor budget, a shorter window
+            // comes first, then fewer waves.
             uint32_t waves = 8;
             const auto expected = [&] { return (double)resident * waves * (2.0 * cfg.half + 1) * occ; };
             while (auto_half && cfg.half > 256 && expected() > SURVIVOR_BUDGET) cfg.half /= 2;
             while (waves > 1 && expected() > SURVIVOR_BUDGET) waves /= 2;
             cfg.lanes = resident * waves;
         } else {
-            // persistent too: four waves of resident blocks (on B200 at
-            // n = 1024: 9.05 G keys/s for the earlier one-lane-per-thread
-            // kernel at two waves; persistent, over two runs, 9.19-9.25 /
-            // 9.31-9.37 / 9.20-9.54 at 2 / 4 / 8 waves, all on the scratch
-            // of one wave)
             cfg.lanes = resident * 4;
         }
     }
@@ -425,18 +435,17 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
 
     const size_t L = cfg.lanes;
     const uint64_t batch = (uint64_t)L * slots * cfg.rounds;
+    e->batch = batch;
+    Tile tile{};
+    {
+        const int rc = plan_tile(ordinal, batch, sink_is_narrow(!cfg.dump && bitmap, bits, suffixed), &tile, err, errlen);
+        if (rc) return rc;
+        e->grid = tile.grid;
+    }
     e->cap = cfg.room ? cfg.room : room_for(batch, cfg.dump != 0, occupancy);
     e->cfg.room = (uint32_t)std::min<size_t>(e->cap, 0xffffffffu);
-    const uint32_t coords = cfg.scheme == OG_SCHEME_CHAIN ? 4 : 2;
-    CU(e->lanes.alloc(L * coords * 2));
-    {
-        // both kernels are persistent: scratch for the resident CTAs only
-        const bool narrow = sink_is_narrow(!cfg.dump && bitmap, bits, suffixed);
-        int rc = search_grid(ordinal, cfg, narrow, &e->grid, err, errlen);
-        if (rc) return rc;
-        const size_t cta = cfg.scheme == OG_SCHEME_CHAIN ? (size_t)4 * CHAIN_ROW * cfg.half : cta_scratch_uint4(cfg.half);
-        CU(e->scratch.alloc((size_t)e->grid * cta));
-    }
+    CU(e->lanes.alloc((size_t)tile.lanes * 4));
+    CU(e->scratch.alloc((size_t)tile.grid * cta_scratch_uint4(tile.half)));
     for (og_engine::Flight& f : e->fl) {
         CU(f.counts.alloc(COUNTS));
         CU(f.hits.alloc(e->cap));
@@ -458,22 +467,15 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     }
     e->start = start_pt;
 
-    // lane start points
-    InitArgs ia{};
-    Pt base, stride;
-    if (cfg.scheme == OG_SCHEME_PAIRED) {
-        base = pt_add(start_pt, base_mult_u64(8ULL * (cfg.half + 1)));  // first centre
-        stride = base_mult_u64(8ULL * slots);
-        ia.affine_out = 1;
-    } else {
-        base = start_pt;
-        stride = base_mult_u64(8ULL * slots);
-        ia.affine_out = 0;
-    }
-    const uint32_t nbits = bits_for(L - 1);
-    std::vector<uint4> pw = pow2_table(stride, nbits);
+    // the lanes' first centres: candidate 0 is the start point (chain) or 8G
+    // past it (paired), and a window's centre its candidate `half`
+    const uint32_t window = 2 * tile.half + 1, offset = cfg.scheme == OG_SCHEME_PAIRED ? 1 : 0;
+    const Pt base = pt_add(start_pt, base_mult_u64(8ULL * (tile.half + offset)));
+    const uint32_t nbits = bits_for(tile.lanes - 1);
+    std::vector<uint4> pw = pow2_table(base_mult_u64(8ULL * window), nbits);
     CU(e->pow2.alloc(pw.size()));
     CU(cudaMemcpyAsync(e->pow2.p, pw.data(), pw.size() * sizeof(uint4), cudaMemcpyHostToDevice, e->stream));
+    InitArgs ia{};
     ia.lanes = e->lanes.p;
     ia.bx = to_words(base.X);
     ia.by = to_words(base.Y);
@@ -481,60 +483,30 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     ia.bt = to_words(base.T);
     ia.pow2 = e->pow2.p;
     ia.nbits = nbits;
-    ia.lanes_n = cfg.lanes;
-    CU(launch_init(ia, 128, e->stream));
-
-    if (cfg.scheme == OG_SCHEME_PAIRED) {
-        CU(make_pair_table(e->table, cfg.half, e->stream));
-        const auto w = stride_words(base_mult_u64(8ULL * slots * L));
-        PairedArgs& a = e->pa;
-        a.table = e->table.p;
-        a.lanes = e->lanes.p;
-        a.scratch = e->scratch.p;
-        a.work = nullptr;  // the flight's counter, set per launch
-        a.lanes_per_thread = lpt;
-        a.bitmap = cfg.dump ? nullptr : e->bitmap.p;
-        a.bits = bits;
-        a.sbitmap = e->sbitmap.p;
-        a.sbits = e->sbits;
-        a.hits = nullptr;     // set per launch to the flight's buffers
-        a.counter = nullptr;
-        a.cap = (uint32_t)std::min<size_t>(e->cap, 0xffffffffu);
-        a.search = 0;
-        a.wx = w[0];
-        a.wy = w[1];
-        a.wdt = w[2];
-        a.lanes_n = cfg.lanes;
-        a.half = cfg.half;
-        a.rounds = cfg.rounds;
-    } else {
-        const Niels step = pt_niels(base_mult_u64(8));
-        ChainArgs& a = e->ca;
-        a.lanes = e->lanes.p;
-        a.scratch = e->scratch.p;
-        a.work = nullptr;  // the flight's counter, set per launch
-        a.slots_n = e->grid * cfg.block;
-        a.bitmap = cfg.dump ? nullptr : e->bitmap.p;
-        a.bits = bits;
-        a.sbitmap = e->sbitmap.p;
-        a.sbits = e->sbits;
-        a.hits = nullptr;     // set per launch to the flight's buffers
-        a.counter = nullptr;
-        a.cap = (uint32_t)std::min<size_t>(e->cap, 0xffffffffu);
-        a.search = 0;
-        a.step_ypx = to_words(step.ypx);
-        a.step_ymx = to_words(step.ymx);
-        a.step_t2d = to_words(step.xy2d);
-        if (L > 1) {
-            const Niels jump = pt_niels(base_mult_u64(8ULL * (L - 1) * slots));
-            a.jump_ypx = to_words(jump.ypx);
-            a.jump_ymx = to_words(jump.ymx);
-            a.jump_t2d = to_words(jump.xy2d);
-        }
-        a.lanes_n = cfg.lanes;
-        a.n = cfg.half;
-        a.rounds = cfg.rounds;
-    }
+    ia.lanes_n = tile.lanes;
+    CU(launch_init(ia, e->stream));
+    CU(make_pair_table(e->table, tile.half, e->stream));
+    PairedArgs& a = e->pa;
+    a.table = e->table.p;
+    a.lanes = e->lanes.p;
+    a.scratch = e->scratch.p;
+    a.work = nullptr;  // the flight's counters and buffers, set per launch
+    a.hits = nullptr;
+    a.counter = nullptr;
+    a.failed = nullptr;
+    a.bitmap = cfg.dump ? nullptr : e->bitmap.p;
+    a.bits = bits;
+    a.sbitmap = e->sbitmap.p;
+    a.sbits = e->sbits;
+    a.cap = (uint32_t)std::min<size_t>(e->cap, 0xffffffffu);
+    a.search = 0;
+    const uint64_t round = (uint64_t)tile.lanes * window;
+    a.between = stride_of(base_mult_u64(8ULL * round));
+    a.last = stride_of(base_mult_u64(8ULL * (batch - (tile.rounds - 1) * round)));
+    a.limit = batch;
+    a.lanes_n = tile.lanes;
+    a.half = tile.half;
+    a.rounds = tile.rounds;
     CU(cudaStreamSynchronize(e->stream));
     *out = e.release();
     return OG_OK;
@@ -620,9 +592,6 @@ int enable_matching(og_engine* e, const og_filters* f, char* err, size_t errlen)
     m.sz = to_words(e->start.Z);
     m.st = to_words(e->start.T);
     m.pow8 = e->pow8.p;
-    m.lanes = e->cfg.lanes;
-    m.slots = e->slots;
-    m.paired = e->cfg.scheme == OG_SCHEME_PAIRED ? 1u : 0u;
     m.out = nullptr;
     m.out_count = nullptr;
     m.out_cap = m.surv_cap;
@@ -631,6 +600,11 @@ int enable_matching(og_engine* e, const og_filters* f, char* err, size_t errlen)
     return OG_OK;
 }
 
+
+// The scalar offset over 8 of candidate 0 of an advance.
+uint64_t first_index(const og_engine* e, uint64_t launch) {
+    return launch * e->batch + (e->cfg.scheme == OG_SCHEME_PAIRED ? 1 : 0);
+}
 
 // One advance onto the engine's stream, into the next free flight: the
 // search kernel, optionally the device match, and the copy of the counters.
@@ -642,18 +616,11 @@ int enqueue_advance(og_engine* e, bool match, char* err, size_t errlen) {
     CU(cudaSetDevice(e->device));
     CU(cudaMemsetAsync(f.counts.p, 0, COUNTS * sizeof(uint32_t), e->stream));
     CU(cudaEventRecord(f.ev0, e->stream));
-    if (e->cfg.scheme == OG_SCHEME_PAIRED) {
-        e->pa.hits = f.hits.p;
-        e->pa.counter = f.counts.p;
-        e->pa.work = f.counts.p + 3;
-        e->pa.failed = f.counts.p + 4;
-        CU(launch_paired(e->pa, (int)e->grid, e->stream));
-    } else {
-        e->ca.hits = f.hits.p;
-        e->ca.counter = f.counts.p;
-        e->ca.work = f.counts.p + 3;
-        CU(launch_chain(e->ca, (int)e->cfg.block, (int)e->grid, e->stream));
-    }
+    e->pa.hits = f.hits.p;
+    e->pa.counter = f.counts.p;
+    e->pa.work = f.counts.p + 3;
+    e->pa.failed = f.counts.p + 4;
+    CU(launch_paired(e->pa, (int)e->grid, e->stream));
     CU(cudaEventRecord(f.ev1, e->stream));
     if (match) {
         MatchArgs& m = e->ma;
@@ -662,7 +629,7 @@ int enqueue_advance(og_engine* e, bool match, char* err, size_t errlen) {
         m.out = f.matches.p;
         m.out_count = f.counts.p + 1;
         m.mismatch = f.counts.p + 2;
-        m.window0 = e->launches * (uint64_t)e->cfg.rounds * e->cfg.lanes;
+        m.first = first_index(e, e->launches);
         int sms = 0;
         CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
         CU(launch_match(m, std::max(sms, 1) * 4, e->stream));
@@ -929,7 +896,7 @@ int og_engine_new(int ordinal, const uint8_t start[128], uint32_t threads, const
 uint32_t og_engine_threads(const og_engine* e) { return e ? e->cfg.lanes : 0; }
 
 uint64_t og_engine_batch(const og_engine* e) {
-    return e ? (uint64_t)e->cfg.lanes * e->slots * e->cfg.rounds : 0;
+    return e ? e->batch : 0;
 }
 
 size_t og_engine_room(const og_engine* e) { return e ? e->cap : 0; }
@@ -951,16 +918,13 @@ int og_engine_collect(og_engine* e, og_survivor* out, size_t cap, size_t* n, cha
     int rc = collect_flight(e, false, &found, &launch, &src, err, errlen);
     if (rc != OG_OK) return rc;
     if (found > cap) return fail(err, errlen, OG_E_CAPACITY, "%u survivors and room for %zu in the caller's buffer", found, cap);
-    const uint64_t L = e->cfg.lanes, slots = e->slots, R = e->cfg.rounds;
-    const bool paired = e->cfg.scheme == OG_SCHEME_PAIRED;
+    const uint64_t first = first_index(e, launch);
     static_assert(sizeof(og_survivor::packed) == sizeof(HitRec::y), "the packed key is the record's eight limbs");
     static_assert(__BYTE_ORDER__ == __ORDER_LITTLE_ENDIAN__, "limbs copied as little-endian bytes");
     rc = copy_records(e, static_cast<const HitRec*>(src), found, [&](size_t lo, size_t hi) {
         for (size_t k = lo; k < hi; k++) {
             const HitRec& h = e->h_recs.p[k];
-            const uint64_t r = h.step / slots, i = h.step % slots;
-            const uint64_t w = (launch * R + r) * L + h.lane;
-            out[k].offset = paired ? 8 * (w * slots + 1 + i) : 8 * (w * slots + i);
+            out[k].offset = 8 * (first + (((uint64_t)h.step << 32) | h.lane));
             std::memcpy(out[k].packed, h.y, sizeof out[k].packed);
         }
     }, err, errlen);

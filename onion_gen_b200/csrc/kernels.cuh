@@ -1,25 +1,22 @@
 // Device kernels of the key search and the host-side launch interface.
 //
-// Two enumeration schemes share one back end (Montgomery batch inversion,
-// canonical packing, prefix-bitmap test, warp-aggregated hit append):
+// A lane holds an affine centre P. One round yields y(P + Q_m) and y(P - Q_m)
+// for the table Q_m = 8m G, m = 1..half, plus y(P) itself, from a formula in
+// which both have the same denominator (search_common.cuh), and moves P to
+// the next centre P + W. Every denominator of the round is inverted with one
+// field inversion (Montgomery's trick): nine multiplications for three pairs.
 //
-//  * paired (the production engine). A lane holds an affine centre P. One
-//    round yields y(P + Q_m) and y(P - Q_m) for the table Q_m = 8m G,
-//    m = 1..half, plus y(P) itself, from a formula in which both have the
-//    same denominator (search_common.cuh), and moves P to the next centre
-//    P + W. Every denominator of the round is inverted with one field
-//    inversion (Montgomery's trick): nine multiplications for three pairs.
-//  * chain (the contract of src/batch.rs): a lane steps its projective point
-//    by +8G (seven multiplications, the addend's Z scaled to one) and
-//    batch-inverts Z over its `n` steps.
-//
-// Candidate numbering. Lane l of L in global round r ("window" w = r L + l):
-//   paired: index i in [0, 2 half] is the key of scalar offset
-//           8 (w (2 half + 1) + 1 + i); i = half is the centre, i = half + m
-//           is P + Q_m, i = half - m is P - Q_m.
-//   chain:  index t in [0, n) is the key of scalar offset 8 (w n + t).
-// Offsets never collide across lanes or rounds, and a run of R rounds covers
-// every candidate index of its range exactly once.
+// Candidate numbering. The kernels number the candidates of a launch from 0:
+// lane l of L in round r covers the window w = r L + l of 2 half + 1
+// candidates, index w (2 half + 1) + i; i = half is the centre, i = half + m is
+// P + Q_m, i = half - m is P - Q_m. An engine's kernel stops at the number of
+// candidates of one advance, whatever half and lanes it runs at, so the
+// tiling is free: both enumeration schemes run on it. With k the index in all
+// advances, the scalar offset is
+//   paired: 8 (k + 1), where lane l's window of user shape (half, lanes) is
+//           k = w (2 half + 1) + i;
+//   chain:  8 k, k = w n + t for step t of lane l (the contract of src/batch.rs).
+// Offsets never collide, and every candidate of a launch is covered once.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -32,8 +29,8 @@ namespace og {
 
 // One bitmap survivor: 48 bytes, three 16-byte stores.
 struct HitRec {
-    uint32_t lane;
-    uint32_t step;  // round-in-launch * slots + candidate index
+    uint32_t lane;  // the lane; or (Sink::limit) the low word of the candidate's index
+    uint32_t step;  // round-in-launch * slots + candidate index; or the index's high word
     uint32_t search;
     uint32_t pad;
     uint32_t y[8];  // canonical y, little-endian limbs (the packed key, sign bit clear)
@@ -54,6 +51,11 @@ static_assert(sizeof(MatchRec) == 48, "MatchRec layout");
 
 struct FeWords {
     uint32_t v[8];
+};
+
+// A stride W between centres: affine x and y, and d x y.
+struct Stride {
+    FeWords x, y, dt;
 };
 
 // Rows of a CTA's scratch hold this many threads (the largest block).
@@ -107,50 +109,24 @@ struct PairedArgs {
     uint32_t search;         // copied into every record
     const uint32_t* sbitmap; // suffix bitmap (nullptr: none); with neither bitmap every candidate survives
     uint32_t sbits;
-    FeWords wx, wy, wdt;     // the round stride W = L (2 half + 1) 8 G, affine, and d wx wy
-    uint32_t lanes_n;        // L, a multiple of the block size times lanes_per_thread
+    Stride between;          // L (2 half + 1) 8 G, after every round but the last
+    Stride last;             // after the last round: to the lane's first centre of the next launch
+    uint64_t limit;          // candidates of a launch: indexes at and above it are none
+    uint32_t lanes_n;        // L
     uint32_t half;
     uint32_t rounds;         // rounds per launch
-    uint32_t lanes_per_thread;  // blocks of lanes a CTA takes at a time, 1 or 2
     uint32_t* failed;        // set to 1 when a wait of the kernel ran out
 };
 
-// Rows of a chain CTA's scratch hold this many threads (the largest block).
-constexpr uint32_t CHAIN_ROW = 128;
-
-struct ChainArgs {
-    uint4* lanes;            // projective points: ({X,Y,Z,T} * 2 + q) * L + lane
-    // per persistent CTA c a region of CHAIN_ROW * 4 n uint4 from c CHAIN_ROW 4 n:
-    // thread j's step t, part w ({num,den}), half q at ((t * 2 + w) * 2 + q) CHAIN_ROW + j
-    uint4* scratch;
-    uint32_t* work;          // blocks of lanes taken so far this launch (starts at 0)
-    uint32_t slots_n;        // persistent CTAs x block
-    const uint32_t* bitmap;
-    uint32_t bits;
-    HitRec* hits;
-    uint32_t* counter;
-    uint32_t cap;
-    uint32_t search;
-    const uint32_t* sbitmap;
-    uint32_t sbits;
-    FeWords step_ypx, step_ymx, step_t2d;  // +8G, Z = 1
-    FeWords jump_ypx, jump_ymx, jump_t2d;  // +8 (L-1) n G, Z = 1 (unused when L = 1)
-    uint32_t lanes_n;
-    uint32_t n;
-    uint32_t rounds;
-};
-
-// Lane start points: lane l starts at base + l * stride, built from the
-// binary expansion of l over `pow2` = { 2^k stride } in cached form with
-// Z = 1 (y+x, y-x, 2dxy). `affine_out` selects the paired layout (x, y)
-// over the chain layout (X, Y, Z, T).
+// Lane start points: lane l starts at base + l * stride, affine, built from
+// the binary expansion of l over `pow2` = { 2^k stride } in cached form with
+// Z = 1 (y+x, y-x, 2dxy).
 struct InitArgs {
-    uint4* lanes;
+    uint4* lanes;            // ({x,y} * 2 + q) * L + lane
     FeWords bx, by, bz, bt;  // base point, extended
     const uint4* pow2;       // (k * 3 + {ypx,ymx,t2d}) * 2 + q
     uint32_t nbits;
     uint32_t lanes_n;
-    uint32_t affine_out;
 };
 
 // Exact-match tables of a literal-prefix filter set in the form the device
@@ -193,40 +169,27 @@ struct MatchArgs {
     uint32_t prefix_count;     // filter index of suffix j is prefix_count + j
     FeWords sx, sy, sz, st;    // the engine's start point, extended
     const uint4* pow8;         // 2^j 8G, j < 64, cached form: (j * 3 + {ypx,ymx,t2d}) * 2 + q
-    uint64_t window0;          // first window of the advance: launch * rounds * lanes
-    uint32_t lanes;
-    uint32_t slots;
-    uint32_t paired;           // offsets 8 (w slots + 1 + i), else 8 (w slots + i)
+    uint64_t first;            // scalar offset over 8 of the advance's candidate 0
     MatchRec* out;
     uint32_t* out_count;
     uint32_t out_cap;
     uint32_t* mismatch;        // survivors whose recomputed key differs from their record
 };
 
-cudaError_t launch_init(const InitArgs& a, int block, cudaStream_t s);
+cudaError_t launch_init(const InitArgs& a, cudaStream_t s);
 cudaError_t launch_match(const MatchArgs& a, int grid, cudaStream_t s);
-// The paired kernel is persistent: `grid` CTAs of OG_LB_THREADS (the resident
-// ones) take the lanes a block at a time (two blocks with two lanes per
-// thread) from `work`, so the scratch covers only the lanes in flight and no
-// SM idles in a tail wave.
+// The search kernel is persistent: `grid` CTAs of OG_LB_THREADS (at most the
+// resident ones) take the lanes a block at a time from `work`, so the scratch
+// covers only the lanes in flight and no SM idles in a tail wave.
 cudaError_t launch_paired(const PairedArgs& a, int grid, cudaStream_t s);
 // Completes a PairTable whose per-entry part is on the device.
 cudaError_t launch_group_table(uint4* table, uint32_t half, cudaStream_t s);
-cudaError_t launch_chain(const ChainArgs& a, int block, int grid, cudaStream_t s);
 
-// Register and shared-memory footprint of the search kernels, for the shape
-// choice.
-struct KernelInfo {
-    int regs;
-    int max_threads;
-    size_t local_bytes;
-    int blocks_per_sm;
-};
-// Resident blocks per SM of a kernel that allocates tensor memory, from its
-// registers, shared memory and tensor memory: the occupancy calculator counts
-// one block per SM for such a kernel.
+// Resident blocks per SM of the search kernel (`narrow`: sink_is_narrow).
+cudaError_t paired_blocks_per_sm(bool narrow, int* blocks);
+// The same of a kernel that allocates tensor memory, from its registers,
+// shared memory and tensor memory: the occupancy calculator counts one block
+// per SM for such a kernel.
 cudaError_t matrix_blocks_per_sm(const void* fn, size_t dynamic_shared, int* blocks);
-cudaError_t paired_info(bool narrow, uint32_t lanes_per_thread, KernelInfo* info);
-cudaError_t chain_info(int block, KernelInfo* info);
 
 }  // namespace og

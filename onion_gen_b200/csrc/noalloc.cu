@@ -17,7 +17,6 @@
 // to the kernels.
 #include <cuda_runtime.h>
 
-#include <array>
 #include <cstring>
 #include <mutex>
 
@@ -27,7 +26,7 @@
 
 namespace og {
 
-std::array<FeWords, 3> stride_words(const Pt& w);  // engine.cu
+Stride stride_of(const Pt& w);  // engine.cu
 
 namespace {
 
@@ -68,7 +67,7 @@ struct NoAllocArgs {
     uint4* scratch;
     FeWords bx, by, bz, bt;  // first centre, extended
     FeWords ex, ey, ez, et;  // 8G, extended (table entry 1)
-    FeWords wx, wy, wdt;     // round stride W, affine, and d wx wy
+    Stride stride;           // between rounds
     const uint32_t* bitmap;
     uint32_t bits;
     HitRec* hits;
@@ -132,12 +131,12 @@ __global__ void __launch_bounds__(NBLOCK, 4) noalloc_paired_kernel(const NoAlloc
         __shared__ __align__(128) RoundShared sh;
         MatrixUnit mu;
         matrix_open(sh);
-        paired_rounds<true>(a.lanes + lane, a.lanes_n, a.wx, a.wy, a.wdt, tab, a.half, a.rounds, scr, sink, sh, mu, lane, true);
+        paired_rounds<true>(a.lanes + lane, a.lanes_n, a.stride, a.stride, tab, a.half, a.rounds, scr, sink, sh, mu, lane, true);
         // a wait that ran out leaves a count beyond any room
         if (threadIdx.x == 0 && sh.failed) atomicOr(a.counter, 0x80000000u);
         matrix_close(sh);
     } else {
-        paired_rounds_full<true>(a.lanes + lane, a.lanes_n, a.wx, a.wy, a.wdt, tab, a.half, a.rounds, scr, sink, lane, true);
+        paired_rounds_full<true>(a.lanes + lane, a.lanes_n, a.stride, a.stride, tab, a.half, a.rounds, scr, sink, lane, true);
     }
 }
 
@@ -218,10 +217,7 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
     a.ey = to_words(eight.Y);
     a.ez = to_words(eight.Z);
     a.et = to_words(eight.T);
-    const auto w = stride_words(base_mult_u64(8ULL * slots * lanes));
-    a.wx = w[0];
-    a.wy = w[1];
-    a.wdt = w[2];
+    a.stride = stride_of(base_mult_u64(8ULL * slots * lanes));
     a.bitmap = d_bitmap;
     a.bits = bits;
     a.hits = reinterpret_cast<HitRec*>(d_hits);

@@ -44,6 +44,13 @@ struct Sink {
     // (og_bitmap_s, staged by the kernel), not through L1
     bool staged = false;
     uint32_t* failed = nullptr;  // set when a wait of the search kernel ran out
+    // With `limit` set, a record holds its candidate's index in the launch
+    // (lane the low word, step the high one) instead of its lane and step, and
+    // candidates at `limit` and above are none: lane l of `lanes` covers in
+    // round r the `slots` candidates from (r lanes + l) slots on.
+    uint64_t limit = 0;
+    uint32_t lanes = 0;
+    uint32_t slots = 0;
 };
 
 // Prefix bitmaps of at most this many bits (8 KiB) can be staged in shared
@@ -100,6 +107,12 @@ __device__ __forceinline__ void test_emit(const Sink& k, const fe& yraw, uint32_
             const uint32_t slot = suffix_slot(y, k.sbits);
             hit |= ((__ldg(k.sbitmap + (slot >> 5)) >> (slot & 31)) & 1u) != 0;
         }
+    }
+    if (k.limit && hit) {
+        const uint64_t index = ((uint64_t)(step / k.slots) * k.lanes + lane) * k.slots + step % k.slots;
+        hit = index < k.limit;
+        lane = (uint32_t)index;
+        step = (uint32_t)(index >> 32);
     }
     const unsigned mask = __ballot_sync(FULL, hit);
     if (mask == 0) return;
@@ -552,9 +565,8 @@ struct RoundState {
 // else one a lane.
 template <bool OneInversion>
 __device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe& y, const fe& z, const fe& run,
-                                           uint4* centre, size_t cstride, bool active, const FeWords& wx,
-                                           const FeWords& wy, const FeWords& wdt) {
-    const fe k = fe_mulv(fe_mulv(x, y), words_fe(wdt));
+                                           uint4* centre, size_t cstride, bool active, const Stride& w) {
+    const fe k = fe_mulv(fe_mulv(x, y), words_fe(w.dt));
     const fe one_k2 = fe_sub(fe_one(), fe_sqv(k));
     const fe total = fe_mulv(fe_mulv(run, z), one_k2);
     const fe U = OneInversion ? block_invert(total) : fe_invert(total);
@@ -562,9 +574,9 @@ __device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe&
     s.e = fe_mulv(fe_mulv(const_inv_d_plus_1(), x), fe_mulv(a, run));
     s.I = fe_mulv(fe_sqv(z), a);
     const fe inv = fe_mulv(run, fe_mulv(z, U));  // 1 / (1 - k^2)
-    const fe nx = fe_mulv(fe_add(fe_mulv(x, words_fe(wy)), fe_mulv(y, words_fe(wx))),
+    const fe nx = fe_mulv(fe_add(fe_mulv(x, words_fe(w.y)), fe_mulv(y, words_fe(w.x))),
                           fe_mulv(fe_sub(fe_one(), k), inv));
-    const fe ny = fe_mulv(fe_add(fe_mulv(y, words_fe(wy)), fe_mulv(x, words_fe(wx))),
+    const fe ny = fe_mulv(fe_add(fe_mulv(y, words_fe(w.y)), fe_mulv(x, words_fe(w.x))),
                           fe_mulv(fe_add(fe_one(), k), inv));
     if (active) {
         store_fe(centre, cstride, nx);
@@ -576,16 +588,16 @@ __device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe&
 // most 24 bits (sink_is_narrow); see kernels.cuh for the candidate numbering.
 // `centre` points at the lane's affine centre in the lane state (x, then y,
 // 16-byte halves `cstride` apart), which is left on the centre after the last
-// round. `wdt` is d xW yW of the stride W. `scr` is the thread's column of its
-// CTA's scratch: group j's prefix product, then E, half q at
+// round: `between` is the stride after every round but the last, `last` the
+// stride after that one. `scr` is the thread's column of its CTA's scratch: group j's prefix product, then E, half q at
 // scr + (4 j + 2 e + q) SCRATCH_ROW. A thread that is not `active` has no lane:
 // it takes part with another's centre and reports nothing. Every thread of
 // the block calls it together, between matrix_open and matrix_close.
 template <bool OneInversion>
-__device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, const FeWords& wx, const FeWords& wy,
-                                              const FeWords& wdt, const PairTable& tab, uint32_t half, uint32_t rounds,
-                                              uint4* scr, const Sink& sink, RoundShared& sh, MatrixUnit& mu,
-                                              uint32_t lane, bool active) {
+__device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, const Stride& between, const Stride& last,
+                                              const PairTable& tab, uint32_t half, uint32_t rounds, uint4* scr,
+                                              const Sink& sink, RoundShared& sh, MatrixUnit& mu, uint32_t lane,
+                                              bool active) {
     const uint32_t slots = 2 * half + 1, groups = groups_of(half);
     uint4* const row = sh.rows + threadIdx.x;
     WarpStage st{sh.stage + threadIdx.x / 32 * STAGE_RECORDS * STAGE_WORDS, 0};
@@ -608,7 +620,7 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
                 store_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW, E);
                 run = fe_mulv(run, E);
             }
-            turn_round<OneInversion>(s, x, y, z, run, centre, cstride, active, wx, wy, wdt);
+            turn_round<OneInversion>(s, x, y, z, run, centre, cstride, active, r + 1 < rounds ? between : last);
             // the centre's own key: its low limb is exact with bit 255
             // folded, unless y is p or more
             const bool hit = active && ((y.v[7] & 0x7fffffffu) == 0x7fffffffu ||
@@ -648,8 +660,8 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
 // candidate survives). A pair takes six multiplications: per pair the prefix
 // product, w = P I [= z / D], I <- I D, f = e w and y = v w +- s f.
 template <bool OneInversion>
-__device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride, const FeWords& wx, const FeWords& wy,
-                                                   const FeWords& wdt, const PairTable& tab, uint32_t half,
+__device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride, const Stride& between,
+                                                   const Stride& last, const PairTable& tab, uint32_t half,
                                                    uint32_t rounds, uint4* scr, const Sink& sink, uint32_t lane,
                                                    bool active) {
     const uint32_t slots = 2 * half + 1;
@@ -666,7 +678,7 @@ __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride
                 store_fe(scr + (size_t)m * (2 * SCRATCH_ROW), SCRATCH_ROW, run);
                 run = fe_mulv(run, fe_sub(load_fe(tab.q + (size_t)m * 2, 1), s.X));
             }
-            turn_round<OneInversion>(s, x, y, z, run, centre, cstride, active, wx, wy, wdt);
+            turn_round<OneInversion>(s, x, y, z, run, centre, cstride, active, r + 1 < rounds ? between : last);
             test_emit(sink, y, lane, mid, active);
         }
 #pragma unroll 1

@@ -10,7 +10,8 @@ import numpy as np
 import pytest
 
 from onion_gen_b200 import _native as N
-from onion_gen_b200 import gpu, workloads
+from onion_gen_b200 import filter as F
+from onion_gen_b200 import gpu, key, workloads
 
 P = 2**255 - 19
 D = -121665 * pow(121666, -1, P) % P
@@ -85,3 +86,49 @@ def test_survivors_of_a_half_set_bitmap(oracle, device, bits, half, lanes, round
     order = np.argsort(offs)
     assert np.array_equal(offs[order], 8 * (1 + want.astype(np.uint64)))
     assert np.array_equal(keys[order], all_keys[want])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scheme,half,lanes,rounds,block", [
+    (N.SCHEME_PAIRED, 37, 416, 3, 32), (N.SCHEME_PAIRED, 2048, 128, 1, 128), (N.SCHEME_CHAIN, 1, 128, 1, 128),
+    (N.SCHEME_CHAIN, 333, 192, 2, 96), (N.SCHEME_CHAIN, 64, 1024, 1, 128)])
+def test_tiled_advances_meet_without_gap(oracle, device, scheme, half, lanes, rounds, block):
+    """However an advance is tiled, two in a row bring the same survivors as
+    the oracle's keys over both ranges: none past the end of an advance, none
+    missing at the seam."""
+    start = oracle.scalar_base_mult(oracle.secret_scalar(workloads.seed(22)))
+    words = np.random.default_rng(half).integers(0, 2**64, size=2**14 // 64, dtype=np.uint64)
+    eng = gpu.Engine(device, start, bitmap=words, bitmap_bits=14,
+                     config=N.EngineConfig(scheme, half, lanes, rounds, block, 0, 0))
+    slots, first = (2 * half + 1, 1) if scheme == N.SCHEME_PAIRED else (half, 0)
+    assert eng.batch() == eng.threads() * rounds * slots
+    got = [eng.advance_raw() for _ in range(2)]
+    n = 2 * eng.batch()
+    all_keys = np.frombuffer(oracle.chain_keys_mt(start, first, n), dtype=np.uint8).reshape(-1, 32)
+    slot = all_keys[:, :4].copy().view(">u4").reshape(-1).astype(np.uint64) >> np.uint64(18)
+    want = np.nonzero((words[slot >> np.uint64(6)] >> (slot & np.uint64(63))) & np.uint64(1))[0]
+    offs, keys = (np.concatenate([g[i] for g in got]) for i in range(2))
+    order = np.argsort(offs)
+    assert np.array_equal(offs[order], 8 * (first + want.astype(np.uint64)))
+    assert np.array_equal(keys[order], all_keys[want])
+
+
+@pytest.mark.gpu
+def test_an_advance_beyond_the_lane_state(device):
+    """4.3e10 candidates, more windows than the lane state holds: every lane
+    runs two rounds. The survivors are as many as the index lets through, inside
+    the range and distinct, and a sample of them re-derives."""
+    seed = workloads.seed(23)
+    fs = F.FilterSet.parse_all(["qqqq"])
+    words, bits = fs.index_words()
+    eng = gpu.Engine(device, key.start_point(seed), bitmap=words, bitmap_bits=bits,
+                     config=N.EngineConfig(N.SCHEME_PAIRED, 2048, 1 << 20, 10, 128, 0, 0))
+    n = eng.batch()
+    offs, keys = eng.advance_raw()
+    mean = n * fs.occupancy()
+    assert abs(len(offs) - mean) < 6 * mean**0.5
+    assert offs.min() >= 8 and offs.max() <= 8 * n and len(np.unique(offs)) == len(offs)
+    order = np.argsort(offs)
+    for i in order[:: len(order) // 100]:
+        key.check_hit(seed, int(offs[i]), bytes(keys[i]))
+    assert offs[order[0]] < 8 * n * 1e-4 and offs[order[-1]] > 8 * n * 0.9999
