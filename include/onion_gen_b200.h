@@ -396,7 +396,7 @@ void og_serve_free(og_serve* s);
  * beyond that the call fails with OG_E_CAPACITY before touching the device.
  * Work is enqueued on `stream` (a cudaStream_t; NULL for the legacy default
  * stream) and the call returns without waiting for it: it enqueues one
- * memset of `*d_count` and three or four kernels, whose constants travel as
+ * memset of `*d_count` and two or three kernels, whose constants travel as
  * launch parameters, and copies nothing from host memory.
  *
  * The first call on a device looks up the array's device address

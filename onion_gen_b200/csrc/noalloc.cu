@@ -17,6 +17,7 @@
 // to the kernels.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -39,19 +40,38 @@ constexpr int MAX_DEVICES = 64;
 static __device__ __align__(256) uint4 og_noalloc_scratch[SCRATCH_BYTES / sizeof(uint4)];
 
 // The limit callers are told, in uint4 units: lanes * (2 half + 3) * 64 +
-// half * 96 bytes. Inside it lie the PairTable, the lane centres (lanes * 4)
-// and the CTAs' scratch: 600 g + lanes * (4 + 6 g) for g = groups_of(half),
-// which is less for every half and at least one block of lanes.
+// half * 96 bytes. The call lays the array out for a tiling of its own.
 size_t need_uint4(uint32_t lanes, uint32_t half) {
     return (size_t)half * 6 + (size_t)lanes * 4 + (size_t)lanes * (2 * (size_t)half + 2) * 4;
 }
-constexpr bool layout_fits(uint32_t half) {
-    return pair_table_uint4(half) + NBLOCK * 4 + cta_scratch_uint4(half) <=
-               half * 6 + NBLOCK * 4 + (size_t)NBLOCK * (2 * half + 2) * 4 &&
-           cta_scratch_uint4(half) <= (size_t)NBLOCK * (2 * half + 2) * 4;
+
+// How the search covers its candidates: `ctas` blocks, a lane a thread, each
+// lane `rounds` windows of 2 half + 1 candidates.
+struct NoAllocTile {
+    uint32_t half, ctas, rounds;
+};
+
+// uint4 the array holds for a tile: the PairTable, the lane centres (four a
+// lane) and the CTAs' scratch.
+size_t tile_uint4(uint32_t half, uint32_t ctas) {
+    return pair_table_uint4(half) + (size_t)ctas * (NBLOCK * 4 + cta_scratch_uint4(half));
 }
-static_assert(layout_fits(1) && layout_fits(2) && layout_fits(4) && layout_fits(2048),
-              "the arrays fit in what the limit allows");
+
+// All `resident` blocks, in one round where the array holds the scratch of
+// windows that long, else in as many as it takes (a round's own cost is that of
+// about 20 groups of three pairs, so the longest windows that fit). Windows of
+// at least two groups.
+NoAllocTile plan_tile(uint64_t candidates, uint32_t resident) {
+    const uint64_t threads = (uint64_t)resident * NBLOCK, window = (candidates + threads - 1) / threads;
+    uint32_t groups = 2;
+    while (2ULL * GROUP * groups + 1 < window && tile_uint4(GROUP * (groups + 1), resident) * sizeof(uint4) <= SCRATCH_BYTES)
+        groups++;
+    NoAllocTile t{GROUP * groups, resident, 1};
+    const uint64_t lane = 2ULL * t.half + 1;
+    t.ctas = (uint32_t)std::min<uint64_t>(resident, (candidates + lane * NBLOCK - 1) / (lane * NBLOCK));
+    t.rounds = (uint32_t)((candidates + lane * NBLOCK * t.ctas - 1) / (lane * NBLOCK * t.ctas));
+    return t;
+}
 
 // 2^k p for k < POW2 in cached form (y + x, y - x, 2 d x y; Z = 1), passed to
 // the kernels by value as a launch parameter (2304 bytes), so that the call
@@ -68,23 +88,25 @@ struct NoAllocArgs {
     FeWords bx, by, bz, bt;  // first centre, extended
     FeWords ex, ey, ez, et;  // 8G, extended (table entry 1)
     Stride stride;           // between rounds
+    uint64_t limit;          // candidates
+    uint32_t out_lanes;      // the caller's shape, in which the records are numbered
+    uint32_t out_slots;
+    uint32_t table_blocks;   // blocks of the first kernel that write the table; the others the lanes
     const uint32_t* bitmap;
     uint32_t bits;
     HitRec* hits;
     uint32_t* counter;
     uint32_t cap;
-    uint32_t lanes_n;
+    uint32_t lanes_n;  // of the tile, as half and rounds
     uint32_t half;
     uint32_t rounds;
 };
 
-// The paired round's table (PairTable) of Q_m = m * 8G, m = 1..half. Entry
-// m - 1 starts from 8G and adds 2^k * 8G (from `pow8`) for every bit k of
-// m - 1.
-__global__ void __launch_bounds__(NBLOCK) noalloc_table_kernel(const NoAllocArgs a, const Pow2Table pow8) {
-    const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n = groups_of(a.half) * GROUP;
-    if (m >= n) return;
+// The per-entry part of the PairTable of Q_m = m * 8G, m = 1.. in whole
+// groups. Entry m - 1 starts from 8G and adds 2^k * 8G (from `pow8`) for every
+// bit k of m - 1.
+__device__ __forceinline__ void table_entry(const NoAllocArgs& a, const Pow2Table& pow8, uint32_t thread) {
+    const uint32_t n = groups_of(a.half) * GROUP, m = min(thread, n - 1);
     fe X = words_fe(a.ex), Y = words_fe(a.ey), Z = words_fe(a.ez), T = words_fe(a.et);
     for (uint32_t k = 0; k < POW2; k++)
         if ((m >> k) & 1u) {
@@ -94,8 +116,9 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_table_kernel(const NoAllocArgs
     // of the affine (x, y): v = 1/y = Z (Z^2 + X^2) i, s = x / (1 + x^2) = X Y Z i and
     // q = v^2 / d, with i = 1 / (Y (Z^2 + X^2))
     const fe den = fe_add(fe_sqv(Z), fe_sqv(X));
-    const fe zi = fe_mulv(Z, fe_invert(fe_mulv(Y, den)));
+    const fe zi = fe_mulv(Z, block_invert(fe_mulv(Y, den)));
     const fe v = fe_canon(fe_mulv(den, zi));
+    if (thread >= n) return;
     store_fe(a.table + (size_t)m * 2, 1, fe_canon(fe_mulv(fe_sqv(v), const_inv_d())));
     uint4* const vs = a.table + (size_t)n * 2 + (size_t)m * 4;
     store_fe(vs + 0, 1, v);
@@ -104,9 +127,7 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_table_kernel(const NoAllocArgs
 
 // Lane l starts on the centre of window l: the first centre plus 2^k times
 // the lane stride (from `pow2`) for every bit k of l.
-__global__ void __launch_bounds__(NBLOCK) noalloc_init_kernel(const NoAllocArgs a, const Pow2Table pow2) {
-    const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lane >= a.lanes_n) return;
+__device__ __forceinline__ void first_centre(const NoAllocArgs& a, const Pow2Table& pow2, uint32_t lane) {
     const size_t L = a.lanes_n;
     fe X = words_fe(a.bx), Y = words_fe(a.by), Z = words_fe(a.bz), T = words_fe(a.bt);
     for (uint32_t k = 0; k < POW2; k++)
@@ -114,9 +135,19 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_init_kernel(const NoAllocArgs 
             const uint4* p = pow2.v + (size_t)k * 6;
             add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
         }
-    const fe zi = fe_invert(Z);
+    const fe zi = block_invert(Z);
     store_fe(a.lanes + 0 * L + lane, L, fe_mulv(X, zi));
     store_fe(a.lanes + 2 * L + lane, L, fe_mulv(Y, zi));
+}
+
+// The table's entries on the first blocks, the lanes' first centres on the
+// others: neither needs the other.
+__global__ void __launch_bounds__(NBLOCK) noalloc_start_kernel(const NoAllocArgs a, const Pow2Table pow8,
+                                                               const Pow2Table pow2) {
+    if (blockIdx.x < a.table_blocks)
+        table_entry(a, pow8, blockIdx.x * NBLOCK + threadIdx.x);
+    else
+        first_centre(a, pow2, (blockIdx.x - a.table_blocks) * NBLOCK + threadIdx.x);
 }
 
 // The production paired kernel with its scratch in the file-scope array; the
@@ -124,7 +155,9 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_init_kernel(const NoAllocArgs 
 template <bool Narrow>
 __global__ void __launch_bounds__(NBLOCK, 4) noalloc_paired_kernel(const NoAllocArgs a) {
     const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    const Sink sink{a.bitmap, a.bits, a.hits, a.counter, a.cap, 0, nullptr, 0};
+    const Sink sink{a.bitmap, a.bits,  a.hits,    a.counter, a.cap,           0,           nullptr,
+                    0,        false,   nullptr,   a.limit,   a.lanes_n,       2 * a.half + 1, a.out_lanes,
+                    a.out_slots};
     const PairTable tab = pair_table_at<const uint4>(a.table, a.half);
     uint4* const scr = a.scratch + (size_t)blockIdx.x * cta_scratch_uint4(a.half) + threadIdx.x;
     if constexpr (Narrow) {
@@ -148,15 +181,35 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_groups_kernel(const NoAllocArg
 std::mutex g_mu;
 uint4* g_addr[MAX_DEVICES];
 
-// 2^k * p for k < POW2 in cached form.
+// 2^k * p for k < POW2 in cached form, with one inversion.
 void pow2_into(Pt p, uint4* out) {
+    Pt pts[POW2];
+    F51 prefix[POW2], run = f_one();
     for (uint32_t k = 0; k < POW2; k++) {
-        const Niels c = pt_niels(p);
-        put_fe(out + k * 6 + 0, 1, c.ypx);
-        put_fe(out + k * 6 + 2, 1, c.ymx);
-        put_fe(out + k * 6 + 4, 1, c.xy2d);
+        pts[k] = p;
+        prefix[k] = run;
+        run = f_mul(run, p.Z);
         p = pt_dbl(p);
     }
+    F51 inv = f_inv(run);
+    for (uint32_t k = POW2; k-- > 0;) {
+        const F51 zi = f_mul(inv, prefix[k]);
+        inv = f_mul(inv, pts[k].Z);
+        const F51 x = f_mul(pts[k].X, zi), y = f_mul(pts[k].Y, zi);
+        put_fe(out + k * 6 + 0, 1, f_add(y, x));
+        put_fe(out + k * 6 + 2, 1, f_sub(y, x));
+        put_fe(out + k * 6 + 4, 1, f_mul(f_mul(x, y), curve_2d()));
+    }
+}
+
+// 2^k * 8G, the same in every call.
+const Pow2Table& eight_powers() {
+    static const Pow2Table table = [] {
+        Pow2Table t;
+        pow2_into(base_mult_u64(8), t.v);
+        return t;
+    }();
+    return table;
 }
 
 }  // namespace
@@ -199,15 +252,28 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
         base = g_addr[ordinal];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const bool narrow = sink_is_narrow(d_bitmap != nullptr, bits, false);
+    const uint32_t slots = 2 * half + 1;
+    const uint64_t candidates = (uint64_t)lanes * rounds * slots;
+    int per_sm = 0, sms = 0;
+    e = narrow ? matrix_blocks_per_sm((const void*)noalloc_paired_kernel<true>, 0, &per_sm)
+               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, noalloc_paired_kernel<false>, NBLOCK, 0);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ordinal);
+    if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "device attributes: %s", cuda_text(e).c_str());
+    const NoAllocTile tile = plan_tile(candidates, (uint32_t)(std::max(1, per_sm) * sms));
+    const uint32_t window = 2 * tile.half + 1;
+    if ((uint64_t)tile.rounds * window > 0xffffffffULL) return fail(err, errlen, OG_E_ARG, "too many rounds");
     NoAllocArgs a;
     std::memset(&a, 0, sizeof a);
+    a.lanes_n = tile.ctas * NBLOCK;
+    a.half = tile.half;
+    a.rounds = tile.rounds;
     a.table = base;
-    a.lanes = a.table + pair_table_uint4(half);
-    a.scratch = a.lanes + (size_t)lanes * 4;
-    const uint32_t slots = 2 * half + 1;
+    a.lanes = a.table + pair_table_uint4(tile.half);
+    a.scratch = a.lanes + (size_t)a.lanes_n * 4;
     // constants computed on the host and passed as launch parameters: the
     // first centre, 8G, the round stride
-    const Pt first = pt_add(A, base_mult_u64(8ULL * (half + 1)));
+    const Pt first = pt_add(A, base_mult_u64(8ULL * (tile.half + 1)));
     a.bx = to_words(first.X);
     a.by = to_words(first.Y);
     a.bz = to_words(first.Z);
@@ -217,30 +283,29 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
     a.ey = to_words(eight.Y);
     a.ez = to_words(eight.Z);
     a.et = to_words(eight.T);
-    a.stride = stride_of(base_mult_u64(8ULL * slots * lanes));
+    a.stride = stride_of(base_mult_u64(8ULL * window * a.lanes_n));
+    a.limit = candidates;
+    a.out_lanes = lanes;
+    a.out_slots = slots;
     a.bitmap = d_bitmap;
     a.bits = bits;
     a.hits = reinterpret_cast<HitRec*>(d_hits);
     a.counter = d_count;
     a.cap = cap;
-    a.lanes_n = lanes;
-    a.half = half;
-    a.rounds = rounds;
+    const uint32_t groups = groups_of(tile.half);
+    a.table_blocks = (groups * GROUP + NBLOCK - 1) / NBLOCK;
     // the two power-of-two tables travel as launch parameters
-    Pow2Table pow2, pow8;
-    pow2_into(base_mult_u64(8ULL * slots), pow2.v);
-    pow2_into(eight, pow8.v);
+    Pow2Table pow2;
+    pow2_into(base_mult_u64(8ULL * window), pow2.v);
     // the counter starts at zero on every call
     e = cudaMemsetAsync(d_count, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "memset: %s", cuda_text(e).c_str());
-    const uint32_t groups = groups_of(half);
-    noalloc_table_kernel<<<(groups * GROUP + NBLOCK - 1) / NBLOCK, NBLOCK, 0, s>>>(a, pow8);
-    noalloc_init_kernel<<<lanes / NBLOCK, NBLOCK, 0, s>>>(a, pow2);
-    if (sink_is_narrow(d_bitmap != nullptr, bits, false)) {
+    noalloc_start_kernel<<<a.table_blocks + tile.ctas, NBLOCK, 0, s>>>(a, eight_powers(), pow2);
+    if (narrow) {
         noalloc_groups_kernel<<<(groups * 48 + NBLOCK - 1) / NBLOCK, NBLOCK, 0, s>>>(a);
-        noalloc_paired_kernel<true><<<lanes / NBLOCK, NBLOCK, 0, s>>>(a);
+        noalloc_paired_kernel<true><<<tile.ctas, NBLOCK, 0, s>>>(a);
     } else {
-        noalloc_paired_kernel<false><<<lanes / NBLOCK, NBLOCK, 0, s>>>(a);
+        noalloc_paired_kernel<false><<<tile.ctas, NBLOCK, 0, s>>>(a);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "launch: %s", cuda_text(e).c_str());

@@ -51,6 +51,10 @@ struct Sink {
     uint64_t limit = 0;
     uint32_t lanes = 0;
     uint32_t slots = 0;
+    // the caller's lanes and slots, when its records are to hold the lane and
+    // step that the index has among those instead
+    uint32_t out_lanes = 0;
+    uint32_t out_slots = 0;
 };
 
 // Prefix bitmaps of at most this many bits (8 KiB) can be staged in shared
@@ -113,6 +117,11 @@ __device__ __forceinline__ void test_emit(const Sink& k, const fe& yraw, uint32_
         hit = index < k.limit;
         lane = (uint32_t)index;
         step = (uint32_t)(index >> 32);
+        if (k.out_slots) {
+            const uint64_t window = index / k.out_slots;
+            lane = (uint32_t)(window % k.out_lanes);
+            step = (uint32_t)(window / k.out_lanes * k.out_slots + index % k.out_slots);
+        }
     }
     const unsigned mask = __ballot_sync(FULL, hit);
     if (mask == 0) return;

@@ -132,3 +132,33 @@ def test_an_advance_beyond_the_lane_state(device):
     for i in order[:: len(order) // 100]:
         key.check_hit(seed, int(offs[i]), bytes(keys[i]))
     assert offs[order[0]] < 8 * n * 1e-4 and offs[order[-1]] > 8 * n * 0.9999
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("half,lanes,rounds", [(1, 128, 1), (56, 8960, 40), (200, 2432, 31), (2048, 128, 3)])
+def test_search_without_allocation_in_several_rounds(device, half, lanes, rounds):
+    """The search in the fixed array finds what an engine of the shape does,
+    numbered in the caller's lanes and steps, whether its tiling takes one round
+    or many."""
+    import torch
+
+    start = key.start_point(workloads.seed(24))
+    words, bits = F.FilterSet.parse_all(["ab", "q7x", "mm"]).index_words()
+    slots = 2 * half + 1
+    n = lanes * rounds * slots
+    cap = n // 64 + 4096
+    bitmap = torch.from_numpy(words.view(np.int64)).cuda()
+    hits, count = (torch.zeros(k, dtype=torch.int32, device="cuda") for k in (cap * 12, 1))
+    err = N.errbuf()
+    N.check(N.lib.og_search_noalloc(device.ordinal, start, lanes, half, rounds, bitmap.data_ptr(), bits, hits.data_ptr(),
+                                    cap, count.data_ptr(), torch.cuda.current_stream().cuda_stream, err, 512), err)
+    recs = hits[: int(count.item()) * 12].cpu().numpy().reshape(-1, 12)
+    lane, step = recs[:, 0].astype(np.int64), recs[:, 1].astype(np.int64)
+    assert lane.size == 0 or (lane.max() < lanes and step.max() < rounds * slots)
+    got = 8 * ((step // slots * lanes + lane) * slots + 1 + step % slots)
+    eng = gpu.Engine(device, start, bitmap=words, bitmap_bits=bits,
+                     config=N.EngineConfig(N.SCHEME_PAIRED, half, lanes, rounds, 128, 0, 0))
+    want, keys = eng.advance_raw()
+    a, b = np.argsort(got), np.argsort(want)
+    assert np.array_equal(got[a], want[b].astype(np.int64)) and len(got) > n // 1000
+    assert np.array_equal(np.ascontiguousarray(recs[a, 4:]).view(np.uint8), keys[b])
