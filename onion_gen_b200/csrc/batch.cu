@@ -196,19 +196,19 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_
         // the block's search decides this, the same for every thread; the
         // barrier at the loop's top has retired every read of the old map
         const bool staged = d.bitmap && d.bits <= STAGED_BITMAP_BITS;
+        extern __shared__ uint32_t og_bitmap_s[];
         if (staged && staged_s != sb.sidx) {
-            extern __shared__ uint32_t og_bitmap_s[];
             const uint32_t words = (1u << d.bits) / 32u;
             for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) og_bitmap_s[i] = d.bitmap[i];
             __syncthreads();
             if (threadIdx.x == 0) staged_s = sb.sidx;
         }
         const uint32_t slot = item * BLOCK + threadIdx.x;
-        const Sink sink{d.bitmap, d.bits, a.surv, &a.counters->surv, a.surv_cap, sb.sidx, d.sbitmap, d.sbits, staged,
+        const Sink sink{staged ? og_bitmap_s : d.bitmap, d.bits, a.surv, &a.counters->surv, a.surv_cap, sb.sidx, d.sbitmap, d.sbits,
                         &a.counters->failed};
         uint4* const scr = a.scratch + blockIdx.x * a.cta_scratch + threadIdx.x;
-        if (sink_is_narrow(d.bitmap != nullptr, d.bits, d.sbitmap != nullptr))
-            paired_rounds<false>(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink, sh,
+        if (sink_kind(d.bitmap ? d.bits : 0, d.sbitmap ? d.sbits : 0) == SINK_PREFIX)
+            paired_rounds<false, false>(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink, sh,
                                  mu, slot, true);
         else
             paired_rounds_full<false>(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink,
@@ -227,10 +227,7 @@ __global__ void __launch_bounds__(256) batch_exact_kernel(const BatchArgs a) {
         const BatchDesc& d = a.descs[r.search];
         uint32_t owner = (d.match.nbuckets || d.match.npatterns) ? exact_owner(d.match, r.y) : NONE;
         if (owner == NONE && d.sbitmap) {
-            fe y;
-#pragma unroll
-            for (int q = 0; q < 8; q++) y.v[q] = r.y[q];
-            const uint32_t slot = suffix_slot(y, d.sbits);
+            const uint32_t slot = suffix_slot(r.y[6], r.y[7], d.sbits);
             if ((__ldg(d.sbitmap + (slot >> 5)) >> (slot & 31)) & 1u) {
                 // lane l of the search at round r of this step covers window
                 // W_done + r L + l; its candidate i has scalar offset

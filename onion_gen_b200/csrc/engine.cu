@@ -301,9 +301,9 @@ struct Tile {
 constexpr uint32_t MIN_GROUPS = 2, MAX_GROUPS = 768;  // the longest: 5.6 GB of scratch
 constexpr uint32_t MAX_TILE_LANES = 1u << 23;  // 0.5 GB of lane state
 
-int plan_tile(int device, uint64_t batch, bool narrow, Tile* out, char* err, size_t errlen) {
+int plan_tile(int device, uint64_t batch, SinkKind kind, Tile* out, char* err, size_t errlen) {
     int blocks = 0, sms = 0;
-    cudaError_t e = paired_blocks_per_sm(narrow, &blocks);
+    cudaError_t e = paired_blocks_per_sm(kind, &blocks);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "kernel attributes: %s", cuda_text(e).c_str());
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "device attributes: %s", cuda_text(e).c_str());
@@ -438,7 +438,7 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     e->batch = batch;
     Tile tile{};
     {
-        const int rc = plan_tile(ordinal, batch, sink_is_narrow(!cfg.dump && bitmap, bits, suffixed), &tile, err, errlen);
+        const int rc = plan_tile(ordinal, batch, sink_kind(!cfg.dump && bitmap ? bits : 0, suffixed ? f->suffixes.bits() : 0), &tile, err, errlen);
         if (rc) return rc;
         e->grid = tile.grid;
     }

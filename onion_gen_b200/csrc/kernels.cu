@@ -41,19 +41,18 @@ __global__ void __launch_bounds__(OG_LB_THREADS) init_kernel(const InitArgs a) {
 // next block of lanes until none is left; its scratch belongs to the CTA, not
 // the lanes. On B200 at half 2048, 757 760 lanes and one 6-symbol prefix a
 // launch takes 52.6 ms (5.9e10 keys/s); ten multiplications a pair took 147.
-// Narrow: a prefix bitmap of at most 24 bits (sink_is_narrow).
-template <bool Narrow>
+template <SinkKind Kind>
 __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) paired_kernel(const PairedArgs a) {
     __shared__ uint32_t item_s;
     const size_t L = a.lanes_n;
     const uint32_t nitems = (a.lanes_n + OG_LB_THREADS - 1) / OG_LB_THREADS;
     const Sink sink{a.bitmap, a.bits,   a.hits,  a.counter, a.cap,     a.search,          a.sbitmap,
-                    a.sbits,  false,    a.failed, a.limit,  a.lanes_n, 2 * a.half + 1};
+                    a.sbits,  a.failed, a.limit, a.lanes_n, 2 * a.half + 1};
     const PairTable tab = pair_table_at(a.table, a.half);
     uint4* const scr = a.scratch + (size_t)blockIdx.x * cta_scratch_uint4(a.half) + threadIdx.x;
     MatrixUnit mu;
     RoundShared* sh = nullptr;
-    if constexpr (Narrow) {
+    if constexpr (Kind != SINK_FULL) {
         __shared__ __align__(128) RoundShared shared;
         sh = &shared;
         matrix_open(*sh);
@@ -67,12 +66,13 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) paired_kernel
         const uint32_t lane = item * OG_LB_THREADS + threadIdx.x;
         const bool active = lane < a.lanes_n;
         uint4* const centre = a.lanes + (active ? lane : 0);
-        if constexpr (Narrow)
-            paired_rounds<true>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, *sh, mu, lane, active);
+        if constexpr (Kind != SINK_FULL)
+            paired_rounds<true, Kind == SINK_SUFFIX>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, *sh,
+                                                     mu, lane, active);
         else
             paired_rounds_full<true>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, lane, active);
     }
-    if constexpr (Narrow) matrix_close(*sh);
+    if constexpr (Kind != SINK_FULL) matrix_close(*sh);
 }
 
 // The per-group part of a PairTable whose q, v and s are in place.
@@ -99,10 +99,7 @@ __global__ void __launch_bounds__(128) match_kernel(const MatchArgs a) {
         const HitRec r = a.surv[i];
         uint32_t owner = (a.t.nbuckets || a.t.npatterns) ? exact_owner(a.t, r.y) : 0xffffffffu;
         if (owner == 0xffffffffu && a.sbitmap) {
-            fe y;
-#pragma unroll
-            for (int q = 0; q < 8; q++) y.v[q] = r.y[q];
-            const uint32_t slot = suffix_slot(y, a.sbits);
+            const uint32_t slot = suffix_slot(r.y[6], r.y[7], a.sbits);
             if ((__ldg(a.sbitmap + (slot >> 5)) >> (slot & 31)) & 1u) owner = suffix_owner(a, r);
         }
         if (owner != 0xffffffffu) {
@@ -132,15 +129,18 @@ cudaError_t launch_init(const InitArgs& a, cudaStream_t s) {
 
 cudaError_t launch_paired(const PairedArgs& a, int grid, cudaStream_t s) {
     if (grid <= 0) return cudaErrorInvalidValue;
-    if (sink_is_narrow(a.bitmap != nullptr, a.bits, a.sbitmap != nullptr))
-        paired_kernel<true><<<grid, OG_LB_THREADS, 0, s>>>(a);
+    const SinkKind kind = sink_kind(a.bitmap ? a.bits : 0, a.sbitmap ? a.sbits : 0);
+    if (kind == SINK_PREFIX)
+        paired_kernel<SINK_PREFIX><<<grid, OG_LB_THREADS, 0, s>>>(a);
+    else if (kind == SINK_SUFFIX)
+        paired_kernel<SINK_SUFFIX><<<grid, OG_LB_THREADS, 0, s>>>(a);
     else
-        paired_kernel<false><<<grid, OG_LB_THREADS, 0, s>>>(a);
+        paired_kernel<SINK_FULL><<<grid, OG_LB_THREADS, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_group_table(uint4* table, uint32_t half, cudaStream_t s) {
-    group_table_kernel<<<(groups_of(half) * 48 + 127) / 128, 128, 0, s>>>(table, half);
+    group_table_kernel<<<(groups_of(half) * 36 + 127) / 128, 128, 0, s>>>(table, half);
     return cudaGetLastError();
 }
 
@@ -160,9 +160,10 @@ cudaError_t matrix_blocks_per_sm(const void* fn, size_t smem, int* blocks) {
     return cudaSuccess;
 }
 
-cudaError_t paired_blocks_per_sm(bool narrow, int* blocks) {
-    if (narrow) return matrix_blocks_per_sm((const void*)paired_kernel<true>, 0, blocks);
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, paired_kernel<false>, OG_LB_THREADS, 0);
+cudaError_t paired_blocks_per_sm(SinkKind kind, int* blocks) {
+    if (kind == SINK_PREFIX) return matrix_blocks_per_sm((const void*)paired_kernel<SINK_PREFIX>, 0, blocks);
+    if (kind == SINK_SUFFIX) return matrix_blocks_per_sm((const void*)paired_kernel<SINK_SUFFIX>, 0, blocks);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, paired_kernel<SINK_FULL>, OG_LB_THREADS, 0);
 }
 
 }  // namespace og

@@ -91,9 +91,13 @@ __host__ __device__ constexpr size_t cta_scratch_uint4(uint32_t half) {
     return (size_t)groups_of(half) * GROUP * 2 * SCRATCH_ROW;
 }
 
-// Whether paired_rounds can serve a sink.
-__host__ __device__ inline bool sink_is_narrow(bool prefix_bitmap, uint32_t bits, bool suffix_bitmap) {
-    return prefix_bitmap && bits <= 24 && !suffix_bitmap;
+// How a sink's keys are tested: by paired_rounds, whose matrix product gives a
+// key's low 24 bits and its bits from 232 on, or in full. A width of 0 stands
+// for no bitmap.
+enum SinkKind { SINK_PREFIX, SINK_SUFFIX, SINK_FULL };
+__host__ __device__ inline SinkKind sink_kind(uint32_t prefix_bits, uint32_t suffix_bits) {
+    if (prefix_bits > 24 || suffix_bits > 23 || (!prefix_bits && !suffix_bits)) return SINK_FULL;
+    return suffix_bits ? SINK_SUFFIX : SINK_PREFIX;
 }
 
 struct PairedArgs {
@@ -185,8 +189,8 @@ cudaError_t launch_paired(const PairedArgs& a, int grid, cudaStream_t s);
 // Completes a PairTable whose per-entry part is on the device.
 cudaError_t launch_group_table(uint4* table, uint32_t half, cudaStream_t s);
 
-// Resident blocks per SM of the search kernel (`narrow`: sink_is_narrow).
-cudaError_t paired_blocks_per_sm(bool narrow, int* blocks);
+// Resident blocks per SM of the search kernel.
+cudaError_t paired_blocks_per_sm(SinkKind kind, int* blocks);
 // The same of a kernel that allocates tensor memory, from its registers,
 // shared memory and tensor memory: the occupancy calculator counts one block
 // per SM for such a kernel.

@@ -156,7 +156,7 @@ template <bool Narrow>
 __global__ void __launch_bounds__(NBLOCK, 4) noalloc_paired_kernel(const NoAllocArgs a) {
     const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
     const Sink sink{a.bitmap, a.bits,  a.hits,    a.counter, a.cap,           0,           nullptr,
-                    0,        false,   nullptr,   a.limit,   a.lanes_n,       2 * a.half + 1, a.out_lanes,
+                    0,        nullptr, a.limit,   a.lanes_n,       2 * a.half + 1, a.out_lanes,
                     a.out_slots};
     const PairTable tab = pair_table_at<const uint4>(a.table, a.half);
     uint4* const scr = a.scratch + (size_t)blockIdx.x * cta_scratch_uint4(a.half) + threadIdx.x;
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(NBLOCK, 4) noalloc_paired_kernel(const NoAlloc
         __shared__ __align__(128) RoundShared sh;
         MatrixUnit mu;
         matrix_open(sh);
-        paired_rounds<true>(a.lanes + lane, a.lanes_n, a.stride, a.stride, tab, a.half, a.rounds, scr, sink, sh, mu, lane, true);
+        paired_rounds<true, false>(a.lanes + lane, a.lanes_n, a.stride, a.stride, tab, a.half, a.rounds, scr, sink, sh, mu, lane, true);
         // a wait that ran out leaves a count beyond any room
         if (threadIdx.x == 0 && sh.failed) atomicOr(a.counter, 0x80000000u);
         matrix_close(sh);
@@ -252,7 +252,7 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
         base = g_addr[ordinal];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool narrow = sink_is_narrow(d_bitmap != nullptr, bits, false);
+    const bool narrow = sink_kind(d_bitmap ? bits : 0, 0) == SINK_PREFIX;
     const uint32_t slots = 2 * half + 1;
     const uint64_t candidates = (uint64_t)lanes * rounds * slots;
     int per_sm = 0, sms = 0;
@@ -302,7 +302,7 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "memset: %s", cuda_text(e).c_str());
     noalloc_start_kernel<<<a.table_blocks + tile.ctas, NBLOCK, 0, s>>>(a, eight_powers(), pow2);
     if (narrow) {
-        noalloc_groups_kernel<<<(groups * 48 + NBLOCK - 1) / NBLOCK, NBLOCK, 0, s>>>(a);
+        noalloc_groups_kernel<<<(groups * 36 + NBLOCK - 1) / NBLOCK, NBLOCK, 0, s>>>(a);
         noalloc_paired_kernel<true><<<tile.ctas, NBLOCK, 0, s>>>(a);
     } else {
         noalloc_paired_kernel<false><<<tile.ctas, NBLOCK, 0, s>>>(a);

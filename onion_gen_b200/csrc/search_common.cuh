@@ -32,7 +32,7 @@ __device__ __forceinline__ fe words_fe(const FeWords& w) {
 
 // Where survivors go: the bitmaps, the record buffer and its counter.
 struct Sink {
-    const uint32_t* bitmap;
+    const uint32_t* bitmap;  // prefix bitmap in global or in the block's shared memory, or nullptr
     uint32_t bits;
     HitRec* hits;
     uint32_t* counter;
@@ -40,9 +40,6 @@ struct Sink {
     uint32_t search;
     const uint32_t* sbitmap;  // suffix bitmap, or nullptr
     uint32_t sbits;
-    // the prefix bitmap is read from the block's copy in shared memory
-    // (og_bitmap_s, staged by the kernel), not through L1
-    bool staged = false;
     uint32_t* failed = nullptr;  // set when a wait of the search kernel ran out
     // With `limit` set, a record holds its candidate's index in the launch
     // (lane the low word, step the high one) instead of its lane and step, and
@@ -58,31 +55,36 @@ struct Sink {
 };
 
 // Prefix bitmaps of at most this many bits (8 KiB) can be staged in shared
-// memory by a kernel that sets Sink::staged.
+// memory.
 constexpr uint32_t STAGED_BITMAP_BITS = 16;
 
-// Slot of a canonical key in the suffix bitmap: base32 bits
+// Slot of a canonical key, from its limbs 6 and 7, in the suffix bitmap: base32 bits
 // [255 - sbits, 255) of the packed key, i.e. bits 1..sbits of its last eight
 // bytes read big-endian (BitmapIndex::slot with offset 255 - sbits,
 // src/filter.rs:2536-2549). The sign bit (bit 7 of byte 31) is clear in the
 // packed key and the bitmap holds both of its values.
-__device__ __forceinline__ uint32_t suffix_slot(const fe& y, uint32_t sbits) {
-    const uint32_t lo = __byte_perm(y.v[7], 0, 0x0123), hi = __byte_perm(y.v[6], 0, 0x0123);
+__device__ __forceinline__ uint32_t suffix_slot(uint32_t y6, uint32_t y7, uint32_t sbits) {
+    const uint32_t lo = __byte_perm(y7, 0, 0x0123), hi = __byte_perm(y6, 0, 0x0123);
     const uint32_t w = (lo >> 1) | (hi << 31);
     return sbits >= 32 ? w : w & ((1u << sbits) - 1u);
 }
 
-// Whether the slot of a key whose canonical low limb is `y0` is set in the
-// sink's prefix bitmap: bytes 0..3 of the key, big-endian, are the top of the
-// slot.
+// Slot in the prefix bitmap of a key whose canonical low limb is `y0`: bytes
+// 0..3 of the key, big-endian, are the top of the slot.
+__device__ __forceinline__ uint32_t prefix_slot(const Sink& k, uint32_t y0) {
+    return __byte_perm(y0, 0, 0x0123) >> (32 - k.bits);  // bits is 8..32
+}
+
 __device__ __forceinline__ bool prefix_hit(const Sink& k, uint32_t y0) {
-    const uint32_t head = __byte_perm(y0, 0, 0x0123);
-    const uint32_t slot = k.bits >= 32 ? head : head >> (32 - k.bits);
-    if (k.staged) {
-        extern __shared__ uint32_t og_bitmap_s[];
-        return (og_bitmap_s[slot >> 5] >> (slot & 31)) & 1u;
-    }
-    return (__ldg(k.bitmap + (slot >> 5)) >> (slot & 31)) & 1u;
+    const uint32_t slot = prefix_slot(k, y0);
+    return (k.bitmap[slot >> 5] >> (slot & 31)) & 1u;
+}
+
+// Whether the slot of a key with the limbs 6 and 7 is set in the sink's suffix
+// bitmap.
+__device__ __forceinline__ bool suffix_hit(const Sink& k, uint32_t y6, uint32_t y7) {
+    const uint32_t slot = suffix_slot(y6, y7, k.sbits);
+    return (__ldg(k.sbitmap + (slot >> 5)) >> (slot & 31)) & 1u;
 }
 
 // Tests a candidate's slots in the prefix bitmap and in the suffix bitmap
@@ -107,10 +109,7 @@ __device__ __forceinline__ void test_emit(const Sink& k, const fe& yraw, uint32_
     if (k.bitmap || k.sbitmap) {
         hit = false;
         if (k.bitmap && valid) hit = prefix_hit(k, y.v[0]);
-        if (k.sbitmap && valid) {
-            const uint32_t slot = suffix_slot(y, k.sbits);
-            hit |= ((__ldg(k.sbitmap + (slot >> 5)) >> (slot & 31)) & 1u) != 0;
-        }
+        if (k.sbitmap && valid) hit |= suffix_hit(k, y.v[6], y.v[7]);
     }
     if (k.limit && hit) {
         const uint64_t index = ((uint64_t)(step / k.slots) * k.lanes + lane) * k.slots + step % k.slots;
@@ -303,7 +302,7 @@ __device__ __forceinline__ fe const_inv_d_plus_1() {  // 1 + 1/d
 // the sign (0: the centre, whose y is in h's place). stage_flush computes
 // their keys, a lane each, tests them exactly and appends the survivors. The
 // search loop itself holds neither the full products nor the record writes.
-constexpr uint32_t STAGE_RECORDS = 16;
+constexpr uint32_t STAGE_RECORDS = 24;
 constexpr uint32_t STAGE_WORDS = 7;  // uint4 a record
 
 struct WarpStage {
@@ -369,26 +368,10 @@ __device__ __forceinline__ void stage_push(const Sink& k, const PairTable& tab, 
     }
 }
 
-// Whether a key may be in the prefix bitmap (of at most 24 bits), from its six
-// column sums: with the key T = sum of byte_j rho_j, rho_j the coefficient
-// times 2^(8 j) mod p, the first three sum the bytes against the low 24 bits
-// of rho_j and the others against floor(2^24 rho_j / p), byte by byte. The
-// latter add up to 2^24 T / p less an error below 192 * 255 < 2^16, so
-// k = floor(T / p) is theirs, or one more if bits 16..23 of the sum are all
-// ones; and the key's low limb is that of T + 19 k.
-__device__ __forceinline__ bool columns_may_hit(const Sink& s, const uint32_t* c) {
-    const uint32_t t = c[4] + (c[3] >> 8), u = c[5] + (t >> 8);
-    const uint32_t low = c[0] + (c[1] << 8) + (c[2] << 16) + 19u * (u >> 8);
-    bool hit = prefix_hit(s, low);
-    if ((u & 255u) == 255u) hit |= prefix_hit(s, low + 19u);
-    return hit;
-}
-
 // ---- the matrix product of a group --------------------------------------
 //
 // For the block's 128 lanes, rows (lanes) x 192 bytes times 192 x 48
-// constants (six columns for each of the group's six keys, twelve unused):
-// six tcgen05.mma of kind::i8, unsigned, K = 32, issued by one thread, sums in
+// constants (eight columns for each of the group's six keys): six tcgen05.mma of kind::i8, unsigned, K = 32, issued by one thread, sums in
 // 48 columns of tensor memory, read back a lane's row by its own thread. It
 // runs while the warps multiply for the next group. The constants come by a
 // bulk copy, 9 KB a group for the whole block. Measured on B200 at half 2048
@@ -396,7 +379,7 @@ __device__ __forceinline__ bool columns_may_hit(const Sink& s, const uint32_t* c
 // mma.sync a warp, which shares registers and issue slots with the
 // multiplications, 64.2; with the keys' low limbs by multiply-adds, four
 // multiplications and two partial ones a pair, 70.3.
-constexpr uint32_t KEY_COLUMNS = 6;
+constexpr uint32_t KEY_COLUMNS = 8;
 constexpr uint32_t COLUMNS = 48;
 constexpr uint32_t TMEM_COLUMNS = 64;  // an allocation is a power of two
 static_assert(GROUP_CONSTANTS == ROW_PARTS * COLUMNS, "the constants of a group are one right operand");
@@ -529,35 +512,67 @@ __device__ __forceinline__ void finish_product(RoundShared& sh, const Sink& sink
 }
 
 // Tests the six keys of the group whose first entry is m0 (entries past `half`
-// belong to no key of the round) from the finished product.
+// belong to no key of the round) from the finished product: whether each may be
+// in the sink's bitmaps. With the key T = sum of byte_j rho_j, rho_j the
+// coefficient times 2^(8 j) mod p, a key's first three columns sum the bytes
+// against the low 24 bits of rho_j and the others against
+// floor(2^40 rho_j / p), byte by byte. The latter add up to K = 2^40 T / p less
+// an error below 192 * 255 < 2^16. So k = floor(T / p) is K >> 40, unless bits
+// 16..39 of K are all ones (such a key counts as a hit), and the key's low limb
+// is that of T + 19 k; and K's bits 16..39, or those plus one, are the key's
+// bits 231..254 (2^255 T / p modulo 2^255 exceeds the key by less than 19). The
+// bitmap's words are loaded for all keys before the first is looked at, and no
+// key takes a branch: with a branch a key a launch of 3.1e9 candidates took
+// 59 ms, so 52.
+template <bool Suffixes>
 __device__ __forceinline__ void test_group(RoundShared& sh, const Sink& sink, const PairTable& tab, WarpStage& st,
                                            const fe& X, uint32_t lane, bool active, uint32_t mid, uint32_t m0,
                                            uint32_t half) {
+    constexpr int KEYS = 2 * GROUP;
     const uint32_t from = sh.tmem + ((threadIdx.x / 32) << 21);  // 32 lanes a warp, in bits 16 and up
-    uint32_t hits = 0;
+    uint32_t slot[KEYS], top[KEYS], hits = 0;
 #pragma unroll
-    for (uint32_t i = 0; i < GROUP; i++) {
+    for (int i = 0; i < (int)GROUP; i++) {
         uint32_t c[2 * KEY_COLUMNS];
         asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%12];\n\t"
-            "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8, %9, %10, %11}, [%13];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+            "%15}, [%16];\n\t"
             "tcgen05.wait::ld.sync.aligned;"
             : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7]), "=r"(c[8]),
-              "=r"(c[9]), "=r"(c[10]), "=r"(c[11])
-            : "r"(from + i * 2 * KEY_COLUMNS), "r"(from + i * 2 * KEY_COLUMNS + 8)
+              "=r"(c[9]), "=r"(c[10]), "=r"(c[11]), "=r"(c[12]), "=r"(c[13]), "=r"(c[14]), "=r"(c[15])
+            : "r"(from + i * 2 * KEY_COLUMNS)
             : "memory");
-        if (m0 + i <= half)
-            hits |= ((columns_may_hit(sink, c) ? 1u : 0u) | (columns_may_hit(sink, c + KEY_COLUMNS) ? 2u : 0u)) << (2 * i);
-    }
-    if (!active) hits = 0;
-    if (__any_sync(FULL, hits)) {
-        const uint4* row = sh.rows + threadIdx.x;
-#pragma unroll 1
-        for (uint32_t key = 0; key < 2 * GROUP; key++) {
-            const uint32_t m = m0 + key / 2;
-            stage_push(sink, tab, st, (hits >> key) & 1u, row, X, lane, key & 1u ? mid - m : mid + m,
-                       key & 1u ? m | 0x80000000u : m);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const uint32_t* k = c + j * KEY_COLUMNS;
+            const uint32_t t0 = k[4] + (k[3] >> 8), t1 = k[5] + (t0 >> 8), t2 = k[6] + (t1 >> 8), t3 = k[7] + (t2 >> 8);
+            const uint32_t low = k[0] + (k[1] << 8) + (k[2] << 16) + 19u * (t3 >> 8);
+            slot[2 * i + j] = prefix_slot(sink, low);
+            hits |= (t1 & t2 & t3 & 255u) == 255u ? 1u << (2 * i + j) : 0u;
+            // the top limb down to bit 231
+            if (Suffixes) top[2 * i + j] = (t3 & 255u) << 23 | (t2 & 255u) << 15 | (t1 & 255u) << 7;
         }
+    }
+    if (!Suffixes || sink.bitmap) {
+        uint32_t word[KEYS];
+#pragma unroll
+        for (int k = 0; k < KEYS; k++) word[k] = sink.bitmap[slot[k] >> 5];
+#pragma unroll
+        for (int k = 0; k < KEYS; k++) hits |= (word[k] >> (slot[k] & 31) & 1u) << k;
+    }
+    if (Suffixes) {
+#pragma unroll
+        for (int k = 0; k < KEYS; k++)
+            hits |= suffix_hit(sink, 0u, top[k]) | suffix_hit(sink, 0u, (top[k] + 128u) & 0x7fffffffu) ? 1u << k : 0u;
+    }
+    const uint32_t entries = min(GROUP, half - m0 + 1);
+    hits &= active ? (1u << (2 * entries)) - 1u : 0u;
+    const uint4* row = sh.rows + threadIdx.x;
+#pragma unroll 1
+    for (uint32_t keys = __reduce_or_sync(FULL, hits); keys; keys &= keys - 1) {
+        const uint32_t key = __ffs(keys) - 1, m = m0 + key / 2;
+        stage_push(sink, tab, st, (hits >> key) & 1u, row, X, lane, key & 1u ? mid - m : mid + m,
+                   key & 1u ? m | 0x80000000u : m);
     }
 }
 
@@ -593,8 +608,8 @@ __device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe&
     }
 }
 
-// A block's `rounds` paired rounds, a lane each, against a prefix bitmap of at
-// most 24 bits (sink_is_narrow); see kernels.cuh for the candidate numbering.
+// A block's `rounds` paired rounds, a lane each, against bitmaps of at most 24
+// and 23 bits (sink_is_narrow); see kernels.cuh for the candidate numbering.
 // `centre` points at the lane's affine centre in the lane state (x, then y,
 // 16-byte halves `cstride` apart), which is left on the centre after the last
 // round: `between` is the stride after every round but the last, `last` the
@@ -602,7 +617,7 @@ __device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe&
 // scr + (4 j + 2 e + q) SCRATCH_ROW. A thread that is not `active` has no lane:
 // it takes part with another's centre and reports nothing. Every thread of
 // the block calls it together, between matrix_open and matrix_close.
-template <bool OneInversion>
+template <bool OneInversion, bool Suffixes>
 __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, const Stride& between, const Stride& last,
                                               const PairTable& tab, uint32_t half, uint32_t rounds, uint4* scr,
                                               const Sink& sink, RoundShared& sh, MatrixUnit& mu, uint32_t lane,
@@ -631,9 +646,12 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
             }
             turn_round<OneInversion>(s, x, y, z, run, centre, cstride, active, r + 1 < rounds ? between : last);
             // the centre's own key: its low limb is exact with bit 255
-            // folded, unless y is p or more
-            const bool hit = active && ((y.v[7] & 0x7fffffffu) == 0x7fffffffu ||
-                                        prefix_hit(sink, y.v[0] + ((y.v[7] >> 31) ? 19u : 0u)));
+            // folded, unless y is p or more, and its high limbs unless the
+            // fold carries that far
+            bool hit = (y.v[7] & 0x7fffffffu) == 0x7fffffffu || (Suffixes && y.v[1] == 0xffffffffu);
+            if (!Suffixes || sink.bitmap) hit |= prefix_hit(sink, y.v[0] + ((y.v[7] >> 31) ? 19u : 0u));
+            if (Suffixes) hit |= suffix_hit(sink, y.v[6], y.v[7] & 0x7fffffffu);
+            hit &= active;
             store_row(row, 0, y);
             stage_push(sink, tab, st, hit, row, s.X, lane, mid, 0u);
         }
@@ -646,7 +664,7 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
                 // the product of the group before, which ran meanwhile
                 finish_product(sh, sink, mu);
                 if (threadIdx.x == 0 && !sh.failed) fetch_constants(sh, tab.constants + (size_t)j * GROUP_CONSTANTS);
-                test_group(sh, sink, tab, st, s.X, lane, active, mid, (j + 1) * GROUP + 1, half);
+                test_group<Suffixes>(sh, sink, tab, st, s.X, lane, active, mid, (j + 1) * GROUP + 1, half);
             }
             store_row(row, 0, h);
             store_row(row, 3, fe_mulv(s.e, h));
@@ -659,14 +677,13 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
             start_product(sh, sink, mu);
         }
         finish_product(sh, sink, mu);
-        test_group(sh, sink, tab, st, s.X, lane, active, mid, 1, half);
+        test_group<Suffixes>(sh, sink, tab, st, s.X, lane, active, mid, 1, half);
     }
     stage_flush(sink, tab, st.recs, st.n);
 }
 
-// The same rounds with every key computed in full: for sinks with a suffix
-// bitmap, with a prefix bitmap of more than 24 bits, or with none (every
-// candidate survives). A pair takes six multiplications: per pair the prefix
+// The same rounds with every key computed in full: for sinks with wider bitmaps
+// than paired_rounds reads, or with none (every candidate survives). A pair takes six multiplications: per pair the prefix
 // product, w = P I [= z / D], I <- I D, f = e w and y = v w +- s f.
 template <bool OneInversion>
 __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride, const Stride& between,
@@ -704,11 +721,10 @@ __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride
 }
 
 // Fills the per-group part of a PairTable from its q, v and s, one thread for
-// each (group, key, element) of 8 keys (the last two get zeros) and six
-// elements; the threads of element 0 and key 0 write the cubic. `tab` is the
-// table being written.
+// each (group, key, element) of six keys and six elements; the threads of
+// element 0 and key 0 write the cubic. `tab` is the table being written.
 __device__ inline void fill_group_table(const PairTable& tab, uint32_t groups, uint32_t thread) {
-    const uint32_t g = thread / 48, key = thread / 6 % 8, elem = thread % 6;
+    const uint32_t g = thread / 36, key = thread / 6 % 6, elem = thread % 6;
     if (g >= groups) return;
     const uint32_t i = key / 2;  // the key's pair
     fe q[GROUP];
@@ -721,31 +737,26 @@ __device__ inline void fill_group_table(const PairTable& tab, uint32_t groups, u
         store_fe(t + 2, 1, s2);
         store_fe(t + 4, 1, fe_sub(fe_mulv(q01, q[2]), fe_mulv(s1, s2)));
     }
-    fe c = fe_one();
-    if (key < 2 * GROUP) {
-        const uint4* vs = tab.vs + (size_t)(g * GROUP + i) * 4;
-        const fe zero = fe_sub(fe_one(), fe_one()), qa = q[(i + 1) % GROUP], qb = q[(i + 2) % GROUP];
-        c = load_fe(elem < 3 ? vs : vs + 2, 1);
-        if (elem % 3 == 0) c = fe_mulv(c, fe_mulv(qa, qb));
-        if (elem % 3 == 1) c = fe_sub(zero, fe_mulv(c, fe_add(qa, qb)));
-        if (elem >= 3 && (key & 1)) c = fe_sub(zero, c);
-    }
+    const uint4* vs = tab.vs + (size_t)(g * GROUP + i) * 4;
+    const fe zero = fe_sub(fe_one(), fe_one()), qa = q[(i + 1) % GROUP], qb = q[(i + 2) % GROUP];
+    fe c = load_fe(elem < 3 ? vs : vs + 2, 1);
+    if (elem % 3 == 0) c = fe_mulv(c, fe_mulv(qa, qb));
+    if (elem % 3 == 1) c = fe_sub(zero, fe_mulv(c, fe_add(qa, qb)));
+    if (elem >= 3 && (key & 1)) c = fe_sub(zero, c);
     uint32_t* const out = reinterpret_cast<uint32_t*>(const_cast<uint4*>(tab.constants) + (size_t)g * GROUP_CONSTANTS);
     const fe times256 = fe{{256u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}};
     for (uint32_t word = 0; word < 8; word++) {
-        uint32_t col[KEY_COLUMNS] = {0, 0, 0, 0, 0, 0};
+        uint32_t col[KEY_COLUMNS] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (uint32_t byte = 0; byte < 4; byte++) {
             const fe rho = fe_canon(c);
-            const uint32_t frac = rho.v[7] >> 7;  // floor(2^24 rho / p), or one less
-            for (uint32_t n = 0; n < 3; n++) {
-                col[n] |= (rho.v[0] >> (8 * n) & 255u) << (8 * byte);
-                col[3 + n] |= (frac >> (8 * n) & 255u) << (8 * byte);
-            }
+            // floor(2^40 rho / p), or one less
+            const uint64_t frac = (((uint64_t)rho.v[7] << 32) | rho.v[6]) >> 23;
+            for (uint32_t n = 0; n < 3; n++) col[n] |= (rho.v[0] >> (8 * n) & 255u) << (8 * byte);
+            for (uint32_t n = 0; n < 5; n++) col[3 + n] |= (uint32_t)(frac >> (8 * n) & 255u) << (8 * byte);
             c = fe_mulv(c, times256);
         }
         for (uint32_t n = 0; n < KEY_COLUMNS; n++)
-            out[((elem * 2 + word / 4) * COLUMNS + key * KEY_COLUMNS + n) * 4 + word % 4] =
-                key < 2 * GROUP ? col[n] : 0u;
+            out[((elem * 2 + word / 4) * COLUMNS + key * KEY_COLUMNS + n) * 4 + word % 4] = col[n];
     }
 }
 

@@ -162,3 +162,30 @@ def test_search_without_allocation_in_several_rounds(device, half, lanes, rounds
     a, b = np.argsort(got), np.argsort(want)
     assert np.array_equal(got[a], want[b].astype(np.int64)) and len(got) > n // 1000
     assert np.array_equal(np.ascontiguousarray(recs[a, 4:]).view(np.uint8), keys[b])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prefixes,suffixes,length", [([], 40, 8), (["ab", "q7x"], 16, 9), (["m"], 3, 11)])
+def test_survivors_of_suffix_and_prefix_bitmaps(oracle, device, prefixes, suffixes, length):
+    """The survivors of a filter engine are the candidates whose slot is set in
+    either bitmap, over two advances."""
+    fs = F.FilterSet.parse_all(prefixes + workloads.suffix_filters(suffixes, length))
+    start = oracle.scalar_base_mult(oracle.secret_scalar(workloads.seed(25)))
+    eng = gpu.Engine(device, start, filters=fs, config=N.EngineConfig(N.SCHEME_PAIRED, 100, 3712, 2, 128, 0, 0))
+    n = 2 * eng.batch()
+    keys = np.frombuffer(oracle.chain_keys_mt(start, 1, n), dtype=np.uint8).reshape(-1, 32)
+    hit = np.zeros(n, dtype=bool)
+    tail = keys[:, 24:].copy().view(">u8").reshape(-1).astype(np.uint64) >> np.uint64(1)
+    words, bits = fs.suffix_index_words()
+    slot = tail & np.uint64(2**bits - 1)
+    hit |= (words[slot >> np.uint64(6)] >> (slot & np.uint64(63)) & np.uint64(1)).astype(bool)
+    if prefixes:
+        words, bits = fs.index_words()
+        slot = keys[:, :4].copy().view(">u4").reshape(-1).astype(np.uint64) >> np.uint64(32 - bits)
+        hit |= (words[slot >> np.uint64(6)] >> (slot & np.uint64(63)) & np.uint64(1)).astype(bool)
+    want = np.nonzero(hit)[0]
+    got = [eng.advance_raw() for _ in range(2)]
+    offs, found = (np.concatenate([g[i] for g in got]) for i in range(2))
+    order = np.argsort(offs)
+    assert len(want) > 200 and np.array_equal(offs[order], 8 * (1 + want.astype(np.uint64)))
+    assert np.array_equal(found[order], keys[want])
