@@ -208,10 +208,10 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_
                         &a.counters->failed};
         uint4* const scr = a.scratch + blockIdx.x * a.cta_scratch + threadIdx.x;
         if (sink_kind(d.bitmap ? d.bits : 0, d.sbitmap ? d.sbits : 0) == SINK_PREFIX)
-            paired_rounds<false, false>(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink, sh,
+            paired_rounds<false>(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink, sh,
                                  mu, slot, true);
         else
-            paired_rounds_full<false>(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink,
+            paired_rounds_full(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink,
                                       slot, true);
     }
     matrix_close(sh);

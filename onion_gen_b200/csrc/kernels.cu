@@ -67,10 +67,10 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) paired_kernel
         const bool active = lane < a.lanes_n;
         uint4* const centre = a.lanes + (active ? lane : 0);
         if constexpr (Kind != SINK_FULL)
-            paired_rounds<true, Kind == SINK_SUFFIX>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, *sh,
-                                                     mu, lane, active);
+            paired_rounds<Kind == SINK_SUFFIX>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, *sh, mu,
+                                               lane, active);
         else
-            paired_rounds_full<true>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, lane, active);
+            paired_rounds_full(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, lane, active);
     }
     if constexpr (Kind != SINK_FULL) matrix_close(*sh);
 }

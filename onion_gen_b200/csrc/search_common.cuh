@@ -585,15 +585,12 @@ struct RoundState {
 // I = 1 / prod E, and the next centre. The stride is added by the complete
 // addition: with k = d x y xW yW, x(P + W) = (x yW + y xW) / (1 + k) and
 // y(P + W) = (y yW + x xW) / (1 - k); 1 - k^2 joins the inversion.
-// OneInversion: one field inversion for the block's lanes (block_invert),
-// else one a lane.
-template <bool OneInversion>
 __device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe& y, const fe& z, const fe& run,
                                            uint4* centre, size_t cstride, bool active, const Stride& w) {
     const fe k = fe_mulv(fe_mulv(x, y), words_fe(w.dt));
     const fe one_k2 = fe_sub(fe_one(), fe_sqv(k));
     const fe total = fe_mulv(fe_mulv(run, z), one_k2);
-    const fe U = OneInversion ? block_invert(total) : fe_invert(total);
+    const fe U = block_invert(total);
     const fe a = fe_mulv(U, one_k2);
     s.e = fe_mulv(fe_mulv(const_inv_d_plus_1(), x), fe_mulv(a, run));
     s.I = fe_mulv(fe_sqv(z), a);
@@ -617,7 +614,7 @@ __device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe&
 // scr + (4 j + 2 e + q) SCRATCH_ROW. A thread that is not `active` has no lane:
 // it takes part with another's centre and reports nothing. Every thread of
 // the block calls it together, between matrix_open and matrix_close.
-template <bool OneInversion, bool Suffixes>
+template <bool Suffixes>
 __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, const Stride& between, const Stride& last,
                                               const PairTable& tab, uint32_t half, uint32_t rounds, uint4* scr,
                                               const Sink& sink, RoundShared& sh, MatrixUnit& mu, uint32_t lane,
@@ -644,7 +641,7 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
                 store_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW, E);
                 run = fe_mulv(run, E);
             }
-            turn_round<OneInversion>(s, x, y, z, run, centre, cstride, active, r + 1 < rounds ? between : last);
+            turn_round(s, x, y, z, run, centre, cstride, active, r + 1 < rounds ? between : last);
             // the centre's own key: its low limb is exact with bit 255
             // folded, unless y is p or more, and its high limbs unless the
             // fold carries that far
@@ -685,7 +682,6 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
 // The same rounds with every key computed in full: for sinks with wider bitmaps
 // than paired_rounds reads, or with none (every candidate survives). A pair takes six multiplications: per pair the prefix
 // product, w = P I [= z / D], I <- I D, f = e w and y = v w +- s f.
-template <bool OneInversion>
 __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride, const Stride& between,
                                                    const Stride& last, const PairTable& tab, uint32_t half,
                                                    uint32_t rounds, uint4* scr, const Sink& sink, uint32_t lane,
@@ -704,7 +700,7 @@ __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride
                 store_fe(scr + (size_t)m * (2 * SCRATCH_ROW), SCRATCH_ROW, run);
                 run = fe_mulv(run, fe_sub(load_fe(tab.q + (size_t)m * 2, 1), s.X));
             }
-            turn_round<OneInversion>(s, x, y, z, run, centre, cstride, active, r + 1 < rounds ? between : last);
+            turn_round(s, x, y, z, run, centre, cstride, active, r + 1 < rounds ? between : last);
             test_emit(sink, y, lane, mid, active);
         }
 #pragma unroll 1
