@@ -5,12 +5,13 @@
 // Candidate windows. A search runs at its own inversion batch `half`; its
 // window w is the round centred on scalar offset 8 (w (2 half + 1) + half + 1),
 // whose 2 half + 1 candidates are offsets 8 (w (2 half + 1) + 1 + i),
-// i in [0, 2 half]. A search holding L lanes for a step of R rounds processes
-// windows [W, W + R L) — lane l takes W + r L + l in round r — and ends the
-// step with lane l centred on window W + R L + l. So after every step lane l
-// sits on window W_done + l whatever L was: a search that grows only
-// initialises its new lanes, one that shrinks drops its highest lanes, and
-// the windows it has processed are always exactly [0, W_done).
+// i in [0, 2 half]. A search holding L lanes of the pool for a step of R rounds
+// processes windows [W, W + R L): the windows it has processed are always
+// exactly [0, W_done). That is a run of R L (2 half + 1) consecutive offsets,
+// which the device tiles as it suits it: into items of 128 threads, a longer
+// window each, as many over all searches as make the CTAs a few rounds of equal
+// length (retile). A thread's centre moves on by the whole run each step, so
+// items are set up again only when the search's share of the pool changes.
 //
 // Results. A search is done when it holds `quota` verified hits; because its
 // windows are processed in increasing order, these are its first `quota`
@@ -71,7 +72,11 @@ namespace {
 constexpr uint32_t BLOCK = 128;
 constexpr uint32_t NONE = 0xffffffffu;
 constexpr int MAX_BUCKETS = MAX_MATCH_BUCKETS;
-constexpr uint32_t POW2_BITS = 24;  // lanes of one search stay below 2^24
+// Longest windows of an item, in groups of three pairs, unless max_half asks
+// for longer: 1.9 GB of scratch.
+constexpr uint32_t ITEM_GROUPS = 256;
+// At most this many items a CTA; a longer step runs its items in several rounds.
+constexpr uint32_t CTA_ITEMS = 8;
 constexpr uint32_t MAX_HALF = 2048;
 constexpr int FLIGHTS = 2;
 // A filter set whose bitmap lets more than this fraction of candidates
@@ -87,8 +92,12 @@ constexpr double NEED_STEPS = 2.0;
 constexpr size_t STAGED_BYTES = (size_t)(1u << STAGED_BITMAP_BITS) / 8u;
 
 struct BatchDesc {
-    Stride stride;           // the search's stride for this step: L (2 half + 1) 8 G
-    FeWords bx, by, bz, bt;  // centre of window W_done (where new lanes start), extended
+    Stride between, last;    // a thread's strides between its rounds and to the next step
+    FeWords bx, by, bz, bt;  // first centre of the search's lane 0 (where its items start), extended
+    uint64_t limit;          // candidates of a step
+    uint32_t item_half;      // the items' windows are 2 item_half + 1 candidates
+    uint32_t item_lanes;     // threads of its items
+    uint32_t rounds;         // windows a thread takes in a step
     const uint32_t* bitmap;  // prefix bitmap (nullptr: the search has no prefix)
     uint32_t bits;
     uint32_t half;           // the search's inversion batch: a round is 2 half + 1 candidates
@@ -99,26 +108,25 @@ struct BatchDesc {
     const uint32_t* suffixes; // the suffix patterns (SuffixTables layout)
     uint32_t nsuffix;
     uint32_t quota;           // exact hits after which the device skips the search's blocks (0: never)
-    const uint4* pow2;        // 2^k (2 half + 1) 8 G, k < POW2_BITS, cached: new lanes' start points
     FeWords sx, sy, sz, st;   // the search's start point s B, extended
 };
 
-// Where a search stands in a step: the windows done before it and the
-// lanes it runs (a survivor's offset is decoded from them on the device).
+// Where a search stands in a step: the windows done before it (a survivor's
+// offset is decoded from them on the device).
 struct SearchPos {
     uint64_t windows;
-    uint32_t lanes;
-    uint32_t pad;
 };
 
-struct SlotBlock {
-    uint32_t sidx;   // descriptor index, NONE when the block is idle
-    uint32_t lane0;  // lane index (within its search) of the block's first slot
+struct Item {
+    uint32_t sidx;   // descriptor index
+    uint32_t lane0;  // the search's lane of the item's first thread
+    uint32_t place;  // where its centres are: lanes [128 place, 128 place + 128)
+    uint32_t fresh;  // 1: its centres are to be set up first
 };
 
 struct Counters {
     uint32_t work;        // next work item of the persistent kernel
-    uint32_t init_count;  // slot blocks in the init list
+    uint32_t items;       // items of the step
     uint32_t surv;        // bitmap survivors written
     uint32_t hits;        // exact hits written
     uint32_t mismatch;    // suffix survivors whose recomputed key differed
@@ -128,58 +136,55 @@ struct Counters {
 
 struct BatchArgs {
     const BatchDesc* descs;
-    const SlotBlock* blocks;
-    const uint32_t* init_list;
+    const Item* items;
     Counters* counters;  // the flight's
-    uint32_t nblocks;
-    uint4* lanes;    // ({x,y} * 2 + q) * slots + slot
-    // per persistent CTA, cta_scratch uint4 (cta_scratch_uint4 of the largest half)
-    uint4* scratch;
+    uint4* lanes;    // ({x,y} * 2 + q) * slots + place * 128 + thread
+    uint4* scratch;  // cta_scratch uint4 a CTA (cta_scratch_uint4 of the longest window)
     size_t cta_scratch;
     size_t slots;
-    PairTable table;  // of Q_m, m = 1..max half; a search of half h reads the first h
-    uint32_t rounds;
+    PairTable table;  // of Q_m, m = 1..the longest half; a shorter window reads the first
     HitRec* surv;  // the flight's
     uint32_t surv_cap;
     HitRec* hits;  // the flight's
     uint32_t hit_cap;
     const SearchPos* pos;  // per descriptor
-    const uint4* pow8;     // 2^j 8G, j < 64, for the suffix key recomputation
+    const uint4* pow8;     // 2^j 8G, j < 64, for first centres and the suffix key recomputation
     uint32_t* found;       // per descriptor: exact hits counted on the device so far
     uint32_t* mism;        // per descriptor: suffix survivors whose recomputed key differed
 };
 
+// First centres of the step's fresh items: lane l of a search starts l windows
+// past its first centre.
 __global__ void __launch_bounds__(BLOCK) batch_init_kernel(const BatchArgs a) {
-    if (blockIdx.x >= a.counters->init_count) return;
-    const uint32_t b = a.init_list[blockIdx.x];
-    const SlotBlock sb = a.blocks[b];
-    const BatchDesc& d = a.descs[sb.sidx];
-    const uint32_t lane = sb.lane0 + threadIdx.x;
-    const size_t slot = (size_t)b * BLOCK + threadIdx.x;
-    fe X = words_fe(d.bx), Y = words_fe(d.by), Z = words_fe(d.bz), T = words_fe(d.bt);
-    for (uint32_t k = 0; k < POW2_BITS; k++) {
-        if ((lane >> k) & 1u) {
-            const uint4* p = d.pow2 + (size_t)k * 6;
-            add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
+    for (uint32_t i = blockIdx.x; i < a.counters->items; i += gridDim.x) {
+        const Item item = a.items[i];
+        if (!item.fresh) continue;
+        const BatchDesc& d = a.descs[item.sidx];
+        const uint64_t k = (uint64_t)(item.lane0 + threadIdx.x) * (2 * d.item_half + 1);
+        const size_t slot = (size_t)item.place * BLOCK + threadIdx.x;
+        fe X = words_fe(d.bx), Y = words_fe(d.by), Z = words_fe(d.bz), T = words_fe(d.bt);
+        for (uint32_t j = 0; k >> j; j++) {
+            if ((k >> j) & 1u) {
+                const uint4* p = a.pow8 + (size_t)j * 6;
+                add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
+            }
         }
+        const fe zi = block_invert(Z);
+        store_fe(a.lanes + 0 * a.slots + slot, a.slots, fe_mulv(X, zi));
+        store_fe(a.lanes + 2 * a.slots + slot, a.slots, fe_mulv(Y, zi));
     }
-    const fe zi = fe_invert(Z);
-    store_fe(a.lanes + 0 * a.slots + slot, a.slots, fe_mulv(X, zi));
-    store_fe(a.lanes + 2 * a.slots + slot, a.slots, fe_mulv(Y, zi));
 }
 
-// Persistent: one CTA per resident slot, each pulling slot blocks until the
-// pool is exhausted. Every block of lanes belongs to one search, whose
-// descriptor gives its half, stride and bitmap. A block of a search whose
-// exact hits have reached its quota (counted by the previous steps' exact
-// kernels) is skipped: its lanes stay where they are. A prefix bitmap of up
-// to 16 bits is staged in shared memory, again only when the CTA's next
-// block belongs to another search (config 4 on B200: 19.52-19.55 s against
-// 19.67-19.82 s, the searches' small bitmaps no longer competing with the
-// table Q_m for L1).
+// Persistent: each CTA pulls the step's items until none is left. Every item
+// belongs to one search, whose descriptor gives its windows, strides and
+// bitmap. An item of a search whose exact hits have reached its quota (counted
+// by the previous steps' exact kernels) is skipped: its threads stay where they
+// are. A prefix bitmap of up to 16 bits is staged in shared memory, again only
+// when the CTA's next item belongs to another search.
 __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_kernel(const BatchArgs a) {
     __shared__ __align__(128) RoundShared sh;
     __shared__ uint32_t item_s, staged_s;  // staged_s: the search whose bitmap is in og_bitmap_s
+    extern __shared__ uint32_t og_bitmap_s[];
     if (threadIdx.x == 0) staged_s = NONE;
     MatrixUnit mu;
     matrix_open(sh);
@@ -187,32 +192,30 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_
         __syncthreads();
         if (threadIdx.x == 0) item_s = atomicAdd(&a.counters->work, 1u);
         __syncthreads();
-        const uint32_t item = item_s;
-        if (item >= a.nblocks) break;
-        const SlotBlock sb = a.blocks[item];
-        if (sb.sidx == NONE) continue;
-        const BatchDesc& d = a.descs[sb.sidx];
-        if (d.quota && a.found[sb.sidx] >= d.quota) continue;
-        // the block's search decides this, the same for every thread; the
+        if (item_s >= a.counters->items) break;
+        const Item item = a.items[item_s];
+        const BatchDesc& d = a.descs[item.sidx];
+        if (d.quota && a.found[item.sidx] >= d.quota) continue;
+        // the item's search decides this, the same for every thread; the
         // barrier at the loop's top has retired every read of the old map
         const bool staged = d.bitmap && d.bits <= STAGED_BITMAP_BITS;
-        extern __shared__ uint32_t og_bitmap_s[];
-        if (staged && staged_s != sb.sidx) {
+        if (staged && staged_s != item.sidx) {
             const uint32_t words = (1u << d.bits) / 32u;
             for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) og_bitmap_s[i] = d.bitmap[i];
             __syncthreads();
-            if (threadIdx.x == 0) staged_s = sb.sidx;
+            if (threadIdx.x == 0) staged_s = item.sidx;
         }
-        const uint32_t slot = item * BLOCK + threadIdx.x;
-        const Sink sink{staged ? og_bitmap_s : d.bitmap, d.bits, a.surv, &a.counters->surv, a.surv_cap, sb.sidx, d.sbitmap, d.sbits,
-                        &a.counters->failed};
+        const Sink sink{staged ? og_bitmap_s : d.bitmap, d.bits,   a.surv,  &a.counters->surv, a.surv_cap, item.sidx,
+                        d.sbitmap,                       d.sbits,  &a.counters->failed, d.limit, d.item_lanes,
+                        2 * d.item_half + 1};
         uint4* const scr = a.scratch + blockIdx.x * a.cta_scratch + threadIdx.x;
+        uint4* const centre = a.lanes + (size_t)item.place * BLOCK + threadIdx.x;
+        const uint32_t lane = item.lane0 + threadIdx.x;
         if (sink_kind(d.bitmap ? d.bits : 0, d.sbitmap ? d.sbits : 0) == SINK_PREFIX)
-            paired_rounds<false>(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink, sh,
-                                 mu, slot, true);
+            paired_rounds<false>(centre, a.slots, d.between, d.last, a.table, d.item_half, d.rounds, scr, sink, sh, mu,
+                                 lane, true);
         else
-            paired_rounds_full(a.lanes + slot, a.slots, d.stride, d.stride, a.table, d.half, a.rounds, scr, sink,
-                                      slot, true);
+            paired_rounds_full(centre, a.slots, d.between, d.last, a.table, d.item_half, d.rounds, scr, sink, lane, true);
     }
     matrix_close(sh);
 }
@@ -229,14 +232,9 @@ __global__ void __launch_bounds__(256) batch_exact_kernel(const BatchArgs a) {
         if (owner == NONE && d.sbitmap) {
             const uint32_t slot = suffix_slot(r.y[6], r.y[7], d.sbits);
             if ((__ldg(d.sbitmap + (slot >> 5)) >> (slot & 31)) & 1u) {
-                // lane l of the search at round r of this step covers window
-                // W_done + r L + l; its candidate i has scalar offset
-                // 8 (w (2 half + 1) + 1 + i)
-                const SearchPos p = a.pos[r.search];
-                const uint32_t slots = 2 * d.half + 1;
-                const uint64_t lane = a.blocks[r.lane / BLOCK].lane0 + r.lane % BLOCK;
-                const uint64_t w = p.windows + (uint64_t)(r.step / slots) * p.lanes + lane;
-                const uint64_t k = w * slots + 1 + r.step % slots;
+                // the record holds its candidate's index in the step, whose
+                // candidate 0 has scalar offset 8 (W_done (2 half + 1) + 1)
+                const uint64_t k = a.pos[r.search].windows * (2 * d.half + 1) + 1 + (((uint64_t)r.step << 32) | r.lane);
                 const SuffixTables t{d.suffixes, d.nsuffix, a.pow8};
                 bool bad = false;
                 const uint32_t j = suffix_match(t, d.sx, d.sy, d.sz, d.st, k, r.y, bad);
@@ -319,9 +317,11 @@ struct Search {
     uint64_t table_bytes = 0;
     uint64_t windows = 0;            // windows of the steps launched so far
     uint64_t windows_collected = 0;  // windows of the steps collected: processed
-    std::vector<uint32_t> blocks;    // slot blocks held, in lane order
+    std::vector<uint32_t> blocks;    // blocks of the pool held: its share of a step
     uint32_t lanes_last = 0;         // lanes held in the last step launched
-    uint32_t lanes_stride = 0;       // lane count the descriptor's stride is for
+    uint32_t lanes_tiled = 0;        // lanes its items were set up for
+    std::vector<uint32_t> places;    // its items' places, in lane order
+    bool fresh = false;              // its items are to be set up in the next step
     std::vector<og_batch_hit> hits;  // verified, in offset order
     bool done = false;
     uint32_t status = OG_OK;         // OG_E_VERIFY when a device hit did not re-derive
@@ -346,8 +346,8 @@ struct Flight {
     DevBuf<HitRec> surv, hits;
     HostBuf<Counters> h_counters;
     HostBuf<BatchDesc> h_descs;   // descriptors uploaded at this launch
-    HostBuf<SlotBlock> h_blocks;  // the block table this step ran (decodes its records)
-    HostBuf<uint32_t> h_init;     // init list, then its length at [nblocks]
+    HostBuf<Item> h_items;        // the items this step runs
+    HostBuf<uint32_t> h_count;    // and their number
     HostBuf<SearchPos> h_pos;
     BatchArgs args{};
     cudaGraph_t graph = nullptr;
@@ -378,14 +378,11 @@ struct og_batch {
     og_batch_config cfg{};
     uint32_t slots = 0, nblocks = 0, grid = 0;
     DevBuf<uint4> lanes, scratch, table, pow8;
-    std::map<uint32_t, DevBuf<uint4>> pow2;  // per half
     DevBuf<BatchDesc> descs;
     DevBuf<SearchPos> pos;
-    DevBuf<SlotBlock> blocks;
-    DevBuf<uint32_t> init_list;
+    DevBuf<Item> items;
     DevBuf<uint32_t> found, mism;
     std::vector<BatchDesc> h_descs;     // the descriptors as the host has them
-    std::vector<SlotBlock> h_blocks;    // the block table as the host has it
     HostBuf<HitRec> h_hits;
     HostBuf<uint32_t> h_mism;
     Flight flights[FLIGHTS];
@@ -394,7 +391,10 @@ struct og_batch {
     std::map<uint64_t, std::unique_ptr<Search>> searches;
     std::vector<uint32_t> free_sidx;
     std::vector<uint32_t> free_blocks;
-    std::map<std::pair<uint32_t, uint32_t>, Stride> strides;  // per (lanes, half)
+    std::vector<uint32_t> free_places;
+    uint32_t places = 0;      // items the lane state holds
+    uint32_t item_half = 0;   // the longest windows of an item
+    std::map<uint64_t, Stride> strides;  // per candidates
     uint64_t admitted = 0;
     uint64_t mem_used = 0, mem_budget = 0;
     bool active_changed = true;
@@ -436,23 +436,24 @@ namespace {
                         "%s: %s", #call, cuda_text(_e).c_str());                                 \
     } while (0)
 
-const Stride& stride_for(og_batch* b, uint32_t lanes, uint32_t half) {
-    const auto key = std::make_pair(lanes, half);
-    auto it = b->strides.find(key);
+// The stride over that many candidates. The cache is dropped when it has grown
+// past what a run of steps uses.
+Stride stride_for(og_batch* b, uint64_t candidates) {
+    auto it = b->strides.find(candidates);
     if (it != b->strides.end()) return it->second;
-    const Stride w = stride_of(base_mult_u64(8ULL * (2ULL * half + 1) * lanes));
-    return b->strides.emplace(key, w).first->second;
-}
-
-// Window W's centre for search s: s * B + 8 (W (2 half + 1) + half + 1) B.
-Pt window_centre(const Search& s, uint64_t w) {
-    const uint64_t k = 8ULL * (w * (2ULL * s.half + 1) + s.half + 1);
-    return pt_add(s.start, base_mult_u64(k));
+    if (b->strides.size() >= 4096) b->strides.clear();
+    return b->strides.emplace(candidates, stride_of(base_mult_u64(8ULL * candidates))).first->second;
 }
 
 void release_blocks(og_batch* b, Search& s) {
     for (uint32_t blk : s.blocks) b->free_blocks.push_back(blk);
     s.blocks.clear();
+}
+
+void release_items(og_batch* b, Search& s) {
+    for (uint32_t p : s.places) b->free_places.push_back(p);
+    s.places.clear();
+    s.lanes_tiled = 0;
 }
 
 // A search ends: done with its quota, or failed with `status`. Its lanes go
@@ -461,6 +462,7 @@ void finish(og_batch* b, Search& s, uint32_t status) {
     s.done = true;
     s.status = status;
     release_blocks(b, s);
+    release_items(b, s);
     b->active_changed = true;
 }
 
@@ -472,10 +474,9 @@ void finish(og_batch* b, Search& s, uint32_t status) {
 // smaller: short searches get all they can use and finish within a few
 // steps, long ones split the rest equally, and when there are more searches
 // than blocks the longest wait. Blocks nobody needs are spread evenly.
-// Searches well above their share drop their highest blocks; those below
-// take free blocks, whose lanes are queued for initialisation. Which lanes
-// a search holds never changes its results.
-void rebalance(og_batch* b, std::vector<uint32_t>& init) {
+// Searches well above their share drop blocks; those below take free ones.
+// How many a search holds never changes its results.
+void rebalance(og_batch* b) {
     std::vector<Search*> running;
     for (auto& kv : b->searches)
         if (!kv.second->done) running.push_back(kv.second.get());
@@ -538,33 +539,119 @@ void rebalance(og_batch* b, std::vector<uint32_t>& init) {
     }
     for (size_t i = 0; i < running.size(); i++) {
         Search& s = *running[i];
-        const size_t had = s.blocks.size();
         while (s.blocks.size() < target[i] && !b->free_blocks.empty()) {
             s.blocks.push_back(b->free_blocks.back());
             b->free_blocks.pop_back();
         }
-        if (s.blocks.size() > had) {
-            // the new lanes start on windows W_done + lane, W_done counting
-            // the steps already launched
-            const Pt c = window_centre(s, s.windows);
-            BatchDesc& d = b->h_descs[s.sidx];
-            d.bx = to_words(c.X);
-            d.by = to_words(c.Y);
-            d.bz = to_words(c.Z);
-            d.bt = to_words(c.T);
-            b->mark(s.sidx);
-            for (size_t j = had; j < s.blocks.size(); j++) init.push_back(s.blocks[j]);
-        }
     }
-    for (uint32_t i = 0; i < b->nblocks; i++) b->h_blocks[i] = SlotBlock{NONE, 0};
-    for (Search* s : running)
-        for (size_t j = 0; j < s->blocks.size(); j++) b->h_blocks[s->blocks[j]] = SlotBlock{s->sidx, (uint32_t)(j * BLOCK)};
+}
+
+// Candidates of a search's step.
+uint64_t step_candidates(const og_batch* b, const Search& s) {
+    return (uint64_t)b->cfg.rounds * s.blocks.size() * BLOCK * (2ULL * s.half + 1);
+}
+
+// Time of `items` items with windows of `groups` groups, in items a CTA: an SM
+// takes four at a time, and for a rest of one, two or three 2.7, 2.9 or 3.3
+// quarters of that (fewer warps keep its pipes less busy); an item's own cost is
+// that of about 20 groups (the prologue, the inversion, the next centre).
+double items_cost(uint64_t items, uint32_t sms, double groups) {
+    static constexpr double REST[4] = {0.0, 2.7, 2.9, 3.3};
+    const uint64_t per_sm = (items + sms - 1) / sms;
+    return ((double)(per_sm / 4 * 4) + REST[per_sm % 4]) * (20.0 + groups);
+}
+
+// Cuts the steps of the searches whose share has changed into items of 128
+// threads. The window is the one that costs least over all searches, each of
+// which takes whole items of it (and shortens its own to use them up). On B200,
+// ms a step with windows of the search's half, an item a block of the pool, and
+// so: half 64, 189440 lanes, 32 searches 0.87 and 0.57; half 256, 94720 lanes, 16
+// searches 1.30 and 1.01; half 256, 189440 lanes, 300 searches 2.11 and 2.06.
+void retile(og_batch* b) {
+    std::vector<Search*> running;
+    std::vector<uint64_t> size;
+    uint64_t total = 0;
+    for (auto& kv : b->searches) {
+        Search& s = *kv.second;
+        if (s.done || s.blocks.empty()) {
+            release_items(b, s);
+            continue;
+        }
+        running.push_back(&s);
+        size.push_back(step_candidates(b, s));
+        total += size.back();
+    }
+    if (!total) return;
+    const uint64_t longest = 2ULL * b->item_half + 1, shortest = 2 * GROUP * 2 + 1;
+    const uint64_t threads = (uint64_t)b->grid * BLOCK;
+    // rounds of every item, so that there are no more than CTA_ITEMS a CTA
+    const uint64_t rounds = (total + threads * CTA_ITEMS * longest - 1) / (threads * CTA_ITEMS * longest);
+    const uint32_t sms = b->grid / b->cfg.grid;
+    uint64_t window = longest, items = 0;
+    double least = INFINITY;
+    const uint64_t step = running.size() <= 256 ? 48 : 12;  // how finely windows are tried: a few hundred sums
+    for (uint64_t w = longest;; w = std::max(shortest, w - w / step - 1)) {
+        uint64_t n = 0;
+        for (uint64_t c : size) n += (c + w * BLOCK * rounds - 1) / (w * BLOCK * rounds);
+        if (n > (uint64_t)CTA_ITEMS * b->grid + running.size()) break;
+        const double cost = items_cost(n, sms, (double)w / (2 * GROUP));
+        if (cost < least) {
+            least = cost;
+            window = w;
+            items = n;
+        }
+        if (w == shortest) break;
+    }
+    const auto items_of = [&](const Search& s) {
+        const uint64_t per = window * BLOCK * rounds;
+        return (step_candidates(b, s) + per - 1) / per;
+    };
+    const auto tile = [&](Search& s) {
+        const uint64_t n = step_candidates(b, s);
+        uint64_t items = items_of(s);
+        const uint64_t w = (n + items * BLOCK * rounds - 1) / (items * BLOCK * rounds);  // at most `window`
+        const uint64_t half = GROUP * std::max<uint64_t>(1, (w + 2 * GROUP - 2) / (2 * GROUP));
+        const uint64_t lane = (2 * half + 1) * rounds;
+        items = (n + lane * BLOCK - 1) / (lane * BLOCK);
+        const uint64_t round = items * BLOCK * (2 * half + 1), used = (n + round - 1) / round;
+        if (items > b->free_places.size()) return false;
+        for (uint64_t j = 0; j < items; j++) {
+            s.places.push_back(b->free_places.back());
+            b->free_places.pop_back();
+        }
+        s.lanes_tiled = (uint32_t)s.blocks.size() * BLOCK;
+        s.fresh = true;
+        BatchDesc& d = b->h_descs[s.sidx];
+        d.between = stride_for(b, round);
+        d.last = stride_for(b, n - (used - 1) * round);
+        d.limit = n;
+        d.item_half = (uint32_t)half;
+        d.item_lanes = (uint32_t)(items * BLOCK);
+        d.rounds = (uint32_t)used;
+        return true;
+    };
+    // searches whose share is as it was keep their items, unless the step
+    // would then have more than a sixteenth over the best, or the places do not
+    // suffice
+    bool fits = true;
+    uint64_t have = 0;
+    for (Search* s : running) {
+        if (s->lanes_tiled != s->blocks.size() * BLOCK) {
+            release_items(b, *s);
+            if (!(fits = tile(*s))) break;
+        }
+        have += s->places.size();
+    }
+    if (!fits || have > items + items / 16) {
+        for (Search* s : running) release_items(b, *s);
+        for (Search* s : running) tile(*s);
+    }
 }
 
 int enqueue_step(og_batch* b, const BatchArgs& a, char* err, size_t errlen) {
-    CU(cudaMemsetAsync(a.counters, 0, offsetof(Counters, init_count), b->stream));
+    CU(cudaMemsetAsync(a.counters, 0, offsetof(Counters, items), b->stream));
     CU(cudaMemsetAsync(&a.counters->surv, 0, 4 * sizeof(uint32_t), b->stream));  // surv, hits, mismatch, failed
-    batch_init_kernel<<<b->nblocks, BLOCK, 0, b->stream>>>(a);
+    batch_init_kernel<<<b->grid, BLOCK, 0, b->stream>>>(a);
     CU(cudaGetLastError());
     batch_search_kernel<<<b->grid, BLOCK, STAGED_BYTES, b->stream>>>(a);
     CU(cudaGetLastError());
@@ -607,21 +694,30 @@ int launch(og_batch* b, bool& launched, char* err, size_t errlen) {
     launched = false;
     Flight& f = b->flights[b->launched % FLIGHTS];
     if (f.pending) return fail(err, errlen, OG_E_STATE, "no free step buffers");
-    std::vector<uint32_t> init;
     if (b->active_changed) {
-        rebalance(b, init);
+        rebalance(b);
+        retile(b);
         b->active_changed = false;
     }
     f.plan.clear();
+    uint32_t items = 0;
     for (auto& kv : b->searches) {
         Search& s = *kv.second;
         if (s.done || s.blocks.empty()) continue;
         const uint32_t lanes = (uint32_t)s.blocks.size() * BLOCK;
-        if (lanes != s.lanes_stride) {
-            b->h_descs[s.sidx].stride = stride_for(b, lanes, s.half);
-            s.lanes_stride = lanes;
+        if (s.fresh) {
+            // its items start past the windows of the steps already launched
+            BatchDesc& d = b->h_descs[s.sidx];
+            const Pt c = pt_add(s.start, base_mult_u64(8ULL * (s.windows * (2ULL * s.half + 1) + d.item_half + 1)));
+            d.bx = to_words(c.X);
+            d.by = to_words(c.Y);
+            d.bz = to_words(c.Z);
+            d.bt = to_words(c.T);
             b->mark(s.sidx);
         }
+        for (size_t j = 0; j < s.places.size(); j++)
+            f.h_items.p[items++] = Item{s.sidx, (uint32_t)(j * BLOCK), s.places[j], s.fresh ? 1u : 0u};
+        s.fresh = false;
         f.plan.push_back(Planned{s.id, s.admit_order, s.sidx, s.half, lanes, b->h_descs[s.sidx].quota != 0, s.windows});
     }
     if (f.plan.empty()) return OG_OK;
@@ -632,23 +728,19 @@ int launch(og_batch* b, bool& launched, char* err, size_t errlen) {
         b->dirty_lo = NONE;
         b->dirty_hi = 0;
     }
-    std::memcpy(f.h_blocks.p, b->h_blocks.data(), b->nblocks * sizeof(SlotBlock));
-    CU(cudaMemcpyAsync(b->blocks.p, f.h_blocks.p, b->nblocks * sizeof(SlotBlock), cudaMemcpyHostToDevice, b->stream));
+    f.h_count.p[0] = items;
+    CU(cudaMemcpyAsync(b->items.p, f.h_items.p, items * sizeof(Item), cudaMemcpyHostToDevice, b->stream));
+    CU(cudaMemcpyAsync(&f.counters.p->items, f.h_count.p, 4, cudaMemcpyHostToDevice, b->stream));
     if (b->suffix_searches) {
         // where each search stands, for the device's offset decode of its
         // suffix survivors
         uint32_t top = 0;
         for (const Planned& p : f.plan) {
-            f.h_pos.p[p.sidx] = SearchPos{p.windows0, p.lanes, 0};
+            f.h_pos.p[p.sidx] = SearchPos{p.windows0};
             top = std::max(top, p.sidx + 1);
         }
         CU(cudaMemcpyAsync(b->pos.p, f.h_pos.p, top * sizeof(SearchPos), cudaMemcpyHostToDevice, b->stream));
     }
-    for (size_t i = 0; i < init.size(); i++) f.h_init.p[i] = init[i];
-    if (!init.empty())
-        CU(cudaMemcpyAsync(b->init_list.p, f.h_init.p, init.size() * 4, cudaMemcpyHostToDevice, b->stream));
-    f.h_init.p[b->nblocks] = (uint32_t)init.size();
-    CU(cudaMemcpyAsync(&f.counters.p->init_count, &f.h_init.p[b->nblocks], 4, cudaMemcpyHostToDevice, b->stream));
     CU(cudaEventRecord(f.ev0, b->stream));
     if (f.exec) {
         CU(cudaGraphLaunch(f.exec, b->stream));
@@ -670,7 +762,7 @@ int launch(og_batch* b, bool& launched, char* err, size_t errlen) {
 }
 
 // Waits for the oldest step in flight and takes its results: decodes every
-// exact hit's offset from the step's own plan and block table, and verifies
+// exact hit's offset from the step's own plan, and verifies
 // each search's hits in offset order up to its quota.
 int collect(og_batch* b, og_batch_hit* out, size_t cap, size_t* n, char* err, size_t errlen) {
     Flight& f = b->flights[b->collected % FLIGHTS];
@@ -702,18 +794,12 @@ int collect(og_batch* b, og_batch_hit* out, size_t cap, size_t* n, char* err, si
     for (size_t i = 0; i < f.plan.size(); i++) by_sidx[f.plan[i].sidx] = i;
     std::vector<std::vector<og_batch_hit>> found(f.plan.size());
     for (const HitRec& h : recs) {
-        const SlotBlock sb = f.h_blocks.p[h.lane / BLOCK];
-        if (sb.sidx != h.search) continue;
-        auto it = by_sidx.find(sb.sidx);
+        auto it = by_sidx.find(h.search);
         if (it == by_sidx.end()) continue;
         const Planned& p = f.plan[it->second];
-        const uint64_t slots_per_window = 2ULL * p.half + 1;
-        const uint64_t lane = sb.lane0 + h.lane % BLOCK;
-        const uint64_t r = h.step / slots_per_window, i = h.step % slots_per_window;
-        const uint64_t w = p.windows0 + r * p.lanes + lane;
         og_batch_hit o{};
         o.search_id = p.id;
-        o.offset = 8 * (w * slots_per_window + 1 + i);
+        o.offset = 8 * (p.windows0 * (2ULL * p.half + 1) + 1 + (((uint64_t)h.step << 32) | h.lane));
         for (int k = 0; k < 8; k++)
             for (int j = 0; j < 4; j++) o.packed[4 * k + j] = (uint8_t)(h.y[k] >> (8 * j));
         o.filter = h.pad;
@@ -843,6 +929,7 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
     // with the staged bitmap a block's shared memory passes 48 KB
     CU(cudaFuncSetAttribute(batch_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STAGED_BYTES));
     CU(matrix_blocks_per_sm((const void*)batch_search_kernel, STAGED_BYTES, &per_sm));
+
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ordinal));
     const uint32_t fit = (uint32_t)std::max(1, per_sm);
     cfg.grid = cfg.grid == 0 ? fit : std::min(cfg.grid, fit);
@@ -877,23 +964,18 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
         int no = 0;
         CU(cudaMemPoolSetAttribute(b->pool, cudaMemPoolReuseAllowInternalDependencies, &no));
     }
-    const size_t S = cfg.slots;
+    b->item_half = GROUP * std::max(groups_of(cfg.max_half), ITEM_GROUPS);
+    // a full step's items: CTA_ITEMS a CTA and, as every search rounds to whole
+    // items, one more for each of at most nblocks searches; twice that, as the
+    // items of a search stay while its share does
+    b->places = 2 * (CTA_ITEMS * b->grid + b->nblocks);
+    const size_t S = (size_t)b->places * BLOCK;
     CU(b->lanes.alloc(S * 4));
-    // the scratch of the persistent CTAs, not of every slot: a CTA uses it for
-    // one block of slots at a time. Each CTA's is one region whose rows hold
-    // its BLOCK threads, so a CTA's accesses stay within a few pages (config
-    // 4's long searches at half 2048 on B200: 2.08e10 against 2.05e10 keys/s
-    // with rows across the whole grid)
-    const size_t cta_scratch = cta_scratch_uint4(cfg.max_half);
+    // the scratch of the persistent CTAs: a CTA uses it for one item at a time
+    const size_t cta_scratch = cta_scratch_uint4(b->item_half);
     CU(b->scratch.alloc((size_t)b->grid * cta_scratch));
-    CU(make_pair_table(b->table, cfg.max_half, b->stream));
+    CU(make_pair_table(b->table, b->item_half, b->stream));
     CU(cudaStreamSynchronize(b->stream));
-    for (uint32_t h = cfg.half; h <= cfg.max_half; h *= 2) {
-        std::vector<uint4> pw = pow2_table(base_mult_u64(8ULL * (2ULL * h + 1)), POW2_BITS);
-        DevBuf<uint4>& d = b->pow2[h];
-        CU(d.alloc(pw.size()));
-        CU(cudaMemcpy(d.p, pw.data(), pw.size() * sizeof(uint4), cudaMemcpyHostToDevice));
-    }
     b->h_descs.assign(cfg.max_searches, BatchDesc{});
     CU(b->descs.alloc(cfg.max_searches));
     CU(b->pos.alloc(cfg.max_searches));
@@ -905,14 +987,12 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
     std::vector<uint4> p8 = pow2_table(base_mult_u64(8), 64);
     CU(b->pow8.alloc(p8.size()));
     CU(cudaMemcpy(b->pow8.p, p8.data(), p8.size() * sizeof(uint4), cudaMemcpyHostToDevice));
-    CU(b->blocks.alloc(b->nblocks));
-    CU(b->init_list.alloc(b->nblocks));
+    CU(b->items.alloc(b->places));
     CU(b->h_hits.alloc(std::min<uint64_t>(cfg.max_hits, 1u << 16)));
-    b->h_blocks.assign(b->nblocks, SlotBlock{NONE, 0});
+    for (uint32_t i = 0; i < b->places; i++) b->free_places.push_back(b->places - 1 - i);
     for (uint32_t i = 0; i < b->nblocks; i++) b->free_blocks.push_back(b->nblocks - 1 - i);
     for (uint32_t i = 0; i < cfg.max_searches; i++) b->free_sidx.push_back(cfg.max_searches - 1 - i);
     CU(cudaMemcpy(b->descs.p, b->h_descs.data(), cfg.max_searches * sizeof(BatchDesc), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(b->blocks.p, b->h_blocks.data(), b->nblocks * sizeof(SlotBlock), cudaMemcpyHostToDevice));
 
     for (int fi = 0; fi < FLIGHTS; fi++) {
         Flight& f = b->flights[fi];
@@ -922,24 +1002,21 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
         CU(f.hits.alloc(cfg.max_hits));
         CU(f.h_counters.alloc(1));
         CU(f.h_descs.alloc(cfg.max_searches));
-        CU(f.h_blocks.alloc(b->nblocks));
-        CU(f.h_init.alloc(b->nblocks + 1));
+        CU(f.h_items.alloc(b->places));
+        CU(f.h_count.alloc(1));
         CU(f.h_pos.alloc(cfg.max_searches));
         std::memset(f.h_pos.p, 0, cfg.max_searches * sizeof(SearchPos));
         CU(cudaEventCreate(&f.ev0));
         CU(cudaEventCreate(&f.ev1));
         BatchArgs& a = f.args;
         a.descs = b->descs.p;
-        a.blocks = b->blocks.p;
-        a.init_list = b->init_list.p;
+        a.items = b->items.p;
         a.counters = f.counters.p;
-        a.nblocks = b->nblocks;
         a.lanes = b->lanes.p;
         a.scratch = b->scratch.p;
         a.cta_scratch = cta_scratch;
         a.slots = S;
-        a.table = pair_table_at<const uint4>(b->table.p, cfg.max_half);
-        a.rounds = cfg.rounds;
+        a.table = pair_table_at<const uint4>(b->table.p, b->item_half);
         a.surv = f.surv.p;
         a.surv_cap = (uint32_t)surv_cap;
         a.hits = f.hits.p;
@@ -1035,9 +1112,6 @@ int og_batch_admit(og_batch* b, uint64_t search_id, const uint8_t seed[32], cons
                     (unsigned long long)s->table_bytes, (unsigned long long)b->mem_used, (unsigned long long)b->mem_budget);
     s->half = choose_half(b, *s);
     s->prob = (double)s->quota / expected_work(*s);
-    const auto pw = b->pow2.find(s->half);
-    if (pw == b->pow2.end() || !pw->second.p)
-        return fail(err, errlen, OG_E_STATE, "no lane-start table for half %u", s->half);
     CU(cudaSetDevice(b->device));
     // the tables come from the batch's pool on the upload stream, so that
     // nothing here waits for a step in flight
@@ -1083,7 +1157,6 @@ int og_batch_admit(og_batch* b, uint64_t search_id, const uint8_t seed[32], cons
     // the device may skip a search once it counts its quota, unless some of
     // its hits still need the host's confirmation
     d.quota = s->long_filters ? 0 : quota;
-    d.pow2 = pw->second.p;
     d.sx = to_words(s->start.X);
     d.sy = to_words(s->start.Y);
     d.sz = to_words(s->start.Z);
@@ -1156,6 +1229,7 @@ int og_batch_retire(og_batch* b, uint64_t search_id) {
     Search& s = *it->second;
     cudaSetDevice(b->device);
     release_blocks(b, s);
+    release_items(b, s);
     b->free_sidx.push_back(s.sidx);
     b->mem_used -= s.table_bytes;
     if (s.has_suffixes) b->suffix_searches--;
@@ -1202,6 +1276,7 @@ int og_batch_tune(int ordinal, uint32_t searches, float max_step_ms, og_batch_co
     // with the staged bitmap a block's shared memory passes 48 KB
     CU(cudaFuncSetAttribute(batch_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STAGED_BYTES));
     CU(matrix_blocks_per_sm((const void*)batch_search_kernel, STAGED_BYTES, &per_sm));
+
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ordinal));
     const uint32_t fit = (uint32_t)std::max(1, per_sm);
     // a mix that never finishes: each search one ten-symbol prefix (50 bits)

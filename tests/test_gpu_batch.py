@@ -355,3 +355,25 @@ def test_an_id_admitted_again_while_a_step_is_in_flight(device):
     b.close()
     alone, _ = run_batch(device, [(5, ["cd"], 3)])
     assert got == alone[5]
+
+
+@pytest.mark.parametrize("half,slots,rounds,searches", [(5, 256, 40, 3), (64, 20480, 1, 7), (300, 1280, 3, 2),
+                                                        (256, 94720, 40, 2)])
+def test_items_cover_a_step_whatever_the_pool(device, half, slots, rounds, searches):
+    """A step's candidates are cut into items of the device's own windows; the
+    hits of every search are the run driver's, in pools that leave an item a
+    fraction of a block and in ones whose items take several rounds."""
+    filters = [["ab%s" % c, "q7"] for c in "cdefghi"] if rounds < 100 else [["abcde"], ["zzzzz", "qqqqq"]]
+    b = B.Batch(device, half=half, slots=slots, rounds=rounds)
+    for i in range(searches):
+        b.admit(i, workloads.seed(40 + i), filters[i], 12)
+    for _ in range(100000):
+        if not b.running():
+            break
+        b.step()
+    for i in range(searches):
+        want, _, _ = run.device_search(device, workloads.seed(40 + i), filters[i], 12,
+                                     config=N.EngineConfig(N.SCHEME_PAIRED, 256, 8192, 1, 128, 0, 0))
+        got = b.results(i)
+        assert [(h.offset, h.public_key, h.filter) for h in got] == [(h.offset, h.public_key, h.filter) for h in want]
+    b.close()
