@@ -320,13 +320,12 @@ static __device__ __noinline__ void stage_flush(const Sink& k, const PairTable& 
     const uint4 id = r[6];
     const uint32_t m = id.z & 0x7fffffffu, i = m ? m - 1 : 0, g = i / GROUP * GROUP;
     // 1 / D_i = (the group's other two D) / E
-    fe others = fe_one();
-    for (uint32_t j = 1; j < GROUP; j++)
-        others = fe_mulv(others, fe_sub(load_fe(tab.q + (size_t)(g + (i - g + j) % GROUP) * 2, 1), X));
+    const fe others = fe_mulv(fe_sub(load_fe(tab.q + (size_t)(g + (i - g + 1) % GROUP) * 2, 1), X),
+                              fe_sub(load_fe(tab.q + (size_t)(g + (i - g + 2) % GROUP) * 2, 1), X));
     const uint4* t = tab.vs + (size_t)i * 4;
-    const fe A = fe_mulv(fe_mulv(load_fe(t, 1), others), h);
-    const fe B = fe_mulv(fe_mulv(load_fe(t + 2, 1), others), load_fe(r + 2, 1));
-    const fe y = select_fe(m == 0, h, select_fe(id.z >> 31, fe_sub(A, B), fe_add(A, B)));
+    const fe A = fe_mulv(load_fe(t, 1), h), B = fe_mulv(load_fe(t + 2, 1), load_fe(r + 2, 1));
+    const fe key = fe_mulv(select_fe(id.z >> 31, fe_sub(A, B), fe_add(A, B)), others);
+    const fe y = select_fe(m == 0, h, key);
     test_emit(k, y, id.x, id.y, valid);
     __syncwarp();
 }
