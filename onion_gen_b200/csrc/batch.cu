@@ -681,9 +681,8 @@ double expected_work(const Search& s) {
 // The search's inversion batch: the batch's half, doubled (up to max_half)
 // while the search's expected work covers LONG_STEPS steps of the whole pool
 // at the doubled half. Results do not depend on it.
-uint32_t choose_half(const og_batch* b, const Search& s) {
+uint32_t choose_half(const og_batch* b, double work) {
     uint32_t h = b->cfg.half;
-    const double work = expected_work(s);
     while (2 * h <= b->cfg.max_half && work >= LONG_STEPS * (2.0 * (2 * h) + 1) * b->slots * b->cfg.rounds) h *= 2;
     return h;
 }
@@ -1110,8 +1109,9 @@ int og_batch_admit(og_batch* b, uint64_t search_id, const uint8_t seed[32], cons
     if (b->mem_used + s->table_bytes > b->mem_budget)
         return fail(err, errlen, OG_E_NOMEM, "its tables (%llu bytes) do not fit the remaining budget (%llu of %llu used)",
                     (unsigned long long)s->table_bytes, (unsigned long long)b->mem_used, (unsigned long long)b->mem_budget);
-    s->half = choose_half(b, *s);
-    s->prob = (double)s->quota / expected_work(*s);
+    const double work = expected_work(*s);
+    s->half = choose_half(b, work);
+    s->prob = (double)s->quota / work;
     CU(cudaSetDevice(b->device));
     // the tables come from the batch's pool on the upload stream, so that
     // nothing here waits for a step in flight

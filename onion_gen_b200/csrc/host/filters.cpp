@@ -74,6 +74,39 @@ bool PrefixFilter::matches_address(const std::string& address) const {
     return true;
 }
 
+// A literal prefix: its canonical text, and its first min(len, 49) symbols as
+// bytes plus a mask for the partly significant last byte (src/filter.rs:649-685).
+static bool parse_literal(const char* s, size_t n, PrefixFilter& out, std::string& err) {
+    out.sets.clear();
+    if (n > ADDRESS_SYMBOLS) {
+        err = "a filter of " + std::to_string(n) + " symbols is longer than an address (56)";
+        return false;
+    }
+    out.text.resize(n);
+    std::memset(out.bytes, 0, sizeof out.bytes);
+    const size_t sym = std::min(n, KEY_ONLY_SYMBOLS);
+    for (size_t i = 0; i < n; i++) {
+        const int v = base32_value(s[i]);
+        if (v < 0) {
+            err = std::string("invalid character '") + s[i] + "' at position " + std::to_string(i) +
+                  ": the base32 alphabet is a-z and 2-7";
+            return false;
+        }
+        out.text[i] = BASE32_ALPHABET[v];
+        if (i < sym) {  // five bits from bit 5 i on: 245 bits at most, so byte 5 i / 8 + 1 is within the 32
+            const unsigned w = (unsigned)v << (11 - 5 * i % 8);
+            out.bytes[5 * i / 8] |= (uint8_t)(w >> 8);
+            out.bytes[5 * i / 8 + 1] |= (uint8_t)w;
+        }
+    }
+    const size_t bits = sym * 5;
+    out.nbytes = (bits + 7) / 8;
+    const unsigned rem = bits % 8;
+    out.mask = rem == 0 ? 0xff : (uint8_t)(0xff << (8 - rem));
+    out.bytes[out.nbytes - 1] &= out.mask;
+    return true;
+}
+
 bool parse_prefix(const std::string& raw, PrefixFilter& out, std::string& err) {
     std::string s = trim(raw);
     const size_t colon = s.find(':');
@@ -113,39 +146,7 @@ bool parse_prefix(const std::string& raw, PrefixFilter& out, std::string& err) {
         std::memset(out.bytes, 0, sizeof out.bytes);
         return true;
     }
-    out.sets.clear();
-    if (s.size() > ADDRESS_SYMBOLS) {
-        err = "a filter of " + std::to_string(s.size()) + " symbols is longer than an address (56)";
-        return false;
-    }
-    std::string canon;
-    for (size_t i = 0; i < s.size(); i++) {
-        const int v = base32_value(s[i]);
-        if (v < 0) {
-            err = std::string("invalid character '") + s[i] + "' at position " + std::to_string(i) +
-                  ": the base32 alphabet is a-z and 2-7";
-            return false;
-        }
-        canon.push_back(BASE32_ALPHABET[v]);
-    }
-    out.text = canon;
-    // decode the first min(len, 49) symbols into bytes plus a mask for the
-    // partly significant last byte (src/filter.rs:649-685)
-    const size_t sym = std::min(canon.size(), KEY_ONLY_SYMBOLS);
-    const size_t bits = sym * 5;
-    std::memset(out.bytes, 0, sizeof out.bytes);
-    for (size_t i = 0; i < sym; i++) {
-        const unsigned v = (unsigned)base32_value(canon[i]);
-        for (unsigned k = 0; k < 5; k++) {
-            const size_t b = i * 5 + k;
-            if ((v >> (4 - k)) & 1) out.bytes[b / 8] |= (uint8_t)(0x80 >> (b % 8));
-        }
-    }
-    out.nbytes = (bits + 7) / 8;
-    const unsigned rem = bits % 8;
-    out.mask = rem == 0 ? 0xff : (uint8_t)(0xff << (8 - rem));
-    out.bytes[out.nbytes - 1] &= out.mask;
-    return true;
+    return parse_literal(s.data(), s.size(), out, err);
 }
 
 bool parse_filter_lines(const char* text, std::vector<PrefixFilter>& prefixes, std::vector<SuffixPattern>& suffixes,
@@ -154,13 +155,23 @@ bool parse_filter_lines(const char* text, std::vector<PrefixFilter>& prefixes, s
     size_t line = 0;
     while (*p) {
         const char* e = std::strchr(p, '\n');
-        const std::string s = e ? std::string(p, (size_t)(e - p)) : std::string(p);
         line++;
-        const std::string t = trim(s);
+        // most lines are bare literals: no copies for those
+        size_t n = e ? (size_t)(e - p) : std::strlen(p), valid = 0;
+        while (valid < n && base32_value(p[valid]) >= 0) valid++;
+        PrefixFilter literal;
+        std::string unused;
+        if (n && valid == n && parse_literal(p, n, literal, unused)) {
+            prefixes.push_back(std::move(literal));
+            if (!e) break;
+            p = e + 1;
+            continue;
+        }
+        const std::string t = trim(e ? std::string(p, (size_t)(e - p)) : std::string(p));
         if (!t.empty()) {
-            std::string why;
+            std::string why, form;
             const size_t colon = t.find(':');
-            std::string form = colon == std::string::npos ? "" : trim(t.substr(0, colon));
+            if (colon != std::string::npos) form = trim(t.substr(0, colon));
             for (char& ch : form) ch = (char)std::tolower((unsigned char)ch);
             if (form == "suffix") {
                 SuffixPattern sp;
@@ -168,14 +179,14 @@ bool parse_filter_lines(const char* text, std::vector<PrefixFilter>& prefixes, s
                     err = "line " + std::to_string(line) + ": " + why;
                     return false;
                 }
-                suffixes.push_back(sp);
+                suffixes.push_back(std::move(sp));
             } else {
                 PrefixFilter f;
                 if (!parse_prefix(t, f, why)) {
                     err = "line " + std::to_string(line) + ": " + why;
                     return false;
                 }
-                prefixes.push_back(f);
+                prefixes.push_back(std::move(f));
             }
         }
         if (!e) break;
@@ -228,16 +239,27 @@ double bitmap_occupancy(const std::vector<uint64_t>& words, uint32_t bits) {
 }
 
 bool FilterSet::build(std::vector<PrefixFilter> filters, uint32_t bits, std::string& err) {
-    std::sort(filters.begin(), filters.end(),
-              [](const PrefixFilter& a, const PrefixFilter& b) { return a.text < b.text; });
+    // in text order, by the first eight characters and where to find the rest:
+    // a filter is a hundred bytes to move
+    std::vector<std::pair<uint64_t, uint32_t>> order(filters.size());
+    for (size_t i = 0; i < filters.size(); i++) {
+        uint64_t head = 0;
+        for (size_t k = 0; k < 8; k++) head = head << 8 | (k < filters[i].text.size() ? (uint8_t)filters[i].text[k] : 0u);
+        order[i] = {head, (uint32_t)i};
+    }
+    std::sort(order.begin(), order.end(), [&](const auto& a, const auto& b) {
+        return a.first != b.first ? a.first < b.first : filters[a.second].text < filters[b.second].text;
+    });
     filters_.clear();
+    filters_.reserve(filters.size());
     long last_literal = -1;
-    for (PrefixFilter& f : filters) {
+    for (const auto& at : order) {
+        PrefixFilter& f = filters[at.second];
         if (f.is_pattern()) {
             // patterns: exact duplicates only
             bool dup = false;
             for (const PrefixFilter& g : filters_) dup |= g.is_pattern() && g.text == f.text;
-            if (!dup) filters_.push_back(f);
+            if (!dup) filters_.push_back(std::move(f));
             continue;
         }
         // a literal prefix absorbs the literals it starts (src/filter.rs:1326-1339)
@@ -246,7 +268,7 @@ bool FilterSet::build(std::vector<PrefixFilter> filters, uint32_t bits, std::str
             if (f.text.compare(0, prev.size(), prev) == 0) continue;
         }
         last_literal = (long)filters_.size();
-        filters_.push_back(f);
+        filters_.push_back(std::move(f));
     }
     if (filters_.empty()) {
         err = "no filters";
@@ -301,17 +323,13 @@ bool FilterSet::build(std::vector<PrefixFilter> filters, uint32_t bits, std::str
         it->owners.push_back((uint32_t)i);
     }
     for (Bucket& b : buckets_) {
-        std::vector<size_t> order(b.keys.size());
-        for (size_t k = 0; k < order.size(); k++) order[k] = k;
-        std::sort(order.begin(), order.end(), [&](size_t x, size_t y) { return b.keys[x] < b.keys[y]; });
-        std::vector<uint64_t> keys(order.size());
-        std::vector<uint32_t> owners(order.size());
-        for (size_t k = 0; k < order.size(); k++) {
-            keys[k] = b.keys[order[k]];
-            owners[k] = b.owners[order[k]];
+        std::vector<std::pair<uint64_t, uint32_t>> sorted(b.keys.size());
+        for (size_t k = 0; k < sorted.size(); k++) sorted[k] = {b.keys[k], b.owners[k]};
+        std::sort(sorted.begin(), sorted.end());
+        for (size_t k = 0; k < sorted.size(); k++) {
+            b.keys[k] = sorted[k].first;
+            b.owners[k] = sorted[k].second;
         }
-        b.keys.swap(keys);
-        b.owners.swap(owners);
     }
     return true;
 }
@@ -387,9 +405,9 @@ double FilterSet::match_probability() const {
         if (f.is_pattern()) {
             p.push_back(anchored_probability(f.sets.data(), f.sets.size(), 0));
         } else {
-            std::vector<uint32_t> sets(f.text.size());
+            uint32_t sets[ADDRESS_SYMBOLS];
             for (size_t i = 0; i < f.text.size(); i++) sets[i] = 1u << base32_value(f.text[i]);
-            p.push_back(anchored_probability(sets.data(), sets.size(), 0));
+            p.push_back(anchored_probability(sets, f.text.size(), 0));
         }
     }
     return either_of(p);
