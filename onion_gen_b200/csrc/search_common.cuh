@@ -567,11 +567,14 @@ __device__ __forceinline__ void test_group(RoundShared& sh, const Sink& sink, co
     const uint32_t entries = min(GROUP, half - m0 + 1);
     hits &= active ? (1u << (2 * entries)) - 1u : 0u;
     const uint4* row = sh.rows + threadIdx.x;
-#pragma unroll 1
-    for (uint32_t keys = __reduce_or_sync(FULL, hits); keys; keys &= keys - 1) {
-        const uint32_t key = __ffs(keys) - 1, m = m0 + key / 2;
-        stage_push(sink, tab, st, (hits >> key) & 1u, row, X, lane, key & 1u ? mid - m : mid + m,
-                   key & 1u ? m | 0x80000000u : m);
+    // Each lane pushes a hit of its own at a time, whichever keys they are: at
+    // 5 % of candidates surviving that is two pushes a group where one per key
+    // was five (22.0 ms for 7.8e8 candidates, now 20.3; 1.9e8 at 0.95 % 4.17,
+    // now 3.98), and the shorter loop gave 2 % at any density.
+    while (__any_sync(FULL, hits != 0)) {
+        const uint32_t key = __ffs(hits) - 1, m = m0 + key / 2;
+        stage_push(sink, tab, st, hits != 0, row, X, lane, key & 1u ? mid - m : mid + m, key & 1u ? m | 0x80000000u : m);
+        hits &= hits - 1;
     }
 }
 
