@@ -654,16 +654,25 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
             store_row(row, 0, y);
             stage_push(sink, tab, st, hit, row, s.X, lane, mid, 0u);
         }
+        // A group's P and E are read a group ahead, under the five
+        // multiplications of the one before: 50.3 -> 49.7 ms for 3.1e9
+        // candidates (prefetch hints instead, to L1 or L2: 51.0).
+        const uint4* p = scr + (size_t)(groups - 1) * (4 * SCRATCH_ROW);
+        fe P = load_fe(p, SCRATCH_ROW), E = load_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW);
 #pragma unroll 1
         for (uint32_t j = groups; j-- > 0;) {
-            const uint4* p = scr + (size_t)j * (4 * SCRATCH_ROW);
-            const fe h = fe_mulv(load_fe(p, SCRATCH_ROW), s.I);
-            s.I = fe_mulv(s.I, load_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW));
+            const fe h = fe_mulv(P, s.I);
+            s.I = fe_mulv(s.I, E);
             if (j + 1 < groups) {
                 // the product of the group before, which ran meanwhile
                 finish_product(sh, sink, mu);
                 if (threadIdx.x == 0 && !sh.failed) fetch_constants(sh, tab.constants + (size_t)j * GROUP_CONSTANTS);
                 test_group<Suffixes>(sh, sink, tab, st, s.X, lane, active, mid, (j + 1) * GROUP + 1, half);
+            }
+            if (j > 0) {
+                p = scr + (size_t)(j - 1) * (4 * SCRATCH_ROW);
+                P = load_fe(p, SCRATCH_ROW);
+                E = load_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW);
             }
             store_row(row, 0, h);
             store_row(row, 3, fe_mulv(s.e, h));
