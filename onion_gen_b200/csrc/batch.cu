@@ -62,7 +62,7 @@ namespace og {
 
 cudaError_t make_pair_table(DevBuf<uint4>& table, uint32_t half, cudaStream_t s);  // engine.cu
 Stride stride_of(const Pt& w);                                     // engine.cu
-std::vector<uint4> pow2_table(const Pt& stride, uint32_t nbits);  // engine.cu
+const std::vector<uint4>& multiples_8g();                          // engine.cu
 MatchTables match_tables(const std::vector<FilterSet::DeviceBucket>& buckets, const uint64_t* keys,
                          const uint32_t* owners, const uint32_t* patterns,
                          uint32_t npatterns);                      // engine.cu
@@ -148,7 +148,7 @@ struct BatchArgs {
     HitRec* hits;  // the flight's
     uint32_t hit_cap;
     const SearchPos* pos;  // per descriptor
-    const uint4* pow8;     // 2^j 8G, j < 64, for first centres and the suffix key recomputation
+    const uint4* mul8;     // multiples of 8G, for first centres and the suffix key recomputation
     uint32_t* found;       // per descriptor: exact hits counted on the device so far
     uint32_t* mism;        // per descriptor: suffix survivors whose recomputed key differed
 };
@@ -163,12 +163,7 @@ __global__ void __launch_bounds__(BLOCK) batch_init_kernel(const BatchArgs a) {
         const uint64_t k = (uint64_t)(item.lane0 + threadIdx.x) * (2 * d.item_half + 1);
         const size_t slot = (size_t)item.place * BLOCK + threadIdx.x;
         fe X = words_fe(d.bx), Y = words_fe(d.by), Z = words_fe(d.bz), T = words_fe(d.bt);
-        for (uint32_t j = 0; k >> j; j++) {
-            if ((k >> j) & 1u) {
-                const uint4* p = a.pow8 + (size_t)j * 6;
-                add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
-            }
-        }
+        add_multiple_8g(X, Y, Z, T, a.mul8, k);
         const fe zi = block_invert(Z);
         store_fe(a.lanes + 0 * a.slots + slot, a.slots, fe_mulv(X, zi));
         store_fe(a.lanes + 2 * a.slots + slot, a.slots, fe_mulv(Y, zi));
@@ -235,7 +230,7 @@ __global__ void __launch_bounds__(256) batch_exact_kernel(const BatchArgs a) {
                 // the record holds its candidate's index in the step, whose
                 // candidate 0 has scalar offset 8 (W_done (2 half + 1) + 1)
                 const uint64_t k = a.pos[r.search].windows * (2 * d.half + 1) + 1 + (((uint64_t)r.step << 32) | r.lane);
-                const SuffixTables t{d.suffixes, d.nsuffix, a.pow8};
+                const SuffixTables t{d.suffixes, d.nsuffix, a.mul8};
                 bool bad = false;
                 const uint32_t j = suffix_match(t, d.sx, d.sy, d.sz, d.st, k, r.y, bad);
                 if (bad) {
@@ -377,7 +372,7 @@ struct og_batch {
     cudaMemPool_t pool = nullptr;
     og_batch_config cfg{};
     uint32_t slots = 0, nblocks = 0, grid = 0;
-    DevBuf<uint4> lanes, scratch, table, pow8;
+    DevBuf<uint4> lanes, scratch, table, mul8;
     DevBuf<BatchDesc> descs;
     DevBuf<SearchPos> pos;
     DevBuf<Item> items;
@@ -983,9 +978,9 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
     CU(b->h_mism.alloc(cfg.max_searches));
     CU(cudaMemset(b->found.p, 0, cfg.max_searches * 4));
     CU(cudaMemset(b->mism.p, 0, cfg.max_searches * 4));
-    std::vector<uint4> p8 = pow2_table(base_mult_u64(8), 64);
-    CU(b->pow8.alloc(p8.size()));
-    CU(cudaMemcpy(b->pow8.p, p8.data(), p8.size() * sizeof(uint4), cudaMemcpyHostToDevice));
+    const std::vector<uint4>& m8 = multiples_8g();
+    CU(b->mul8.alloc(m8.size()));
+    CU(cudaMemcpy(b->mul8.p, m8.data(), m8.size() * sizeof(uint4), cudaMemcpyHostToDevice));
     CU(b->items.alloc(b->places));
     CU(b->h_hits.alloc(std::min<uint64_t>(cfg.max_hits, 1u << 16)));
     for (uint32_t i = 0; i < b->places; i++) b->free_places.push_back(b->places - 1 - i);
@@ -1021,7 +1016,7 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
         a.hits = f.hits.p;
         a.hit_cap = cfg.max_hits;
         a.pos = b->pos.p;
-        a.pow8 = b->pow8.p;
+        a.mul8 = b->mul8.p;
         a.found = b->found.p;
         a.mism = b->mism.p;
         if (cfg.graph != 2) {

@@ -70,18 +70,17 @@ Stride stride_of(const Pt& w) {
     return Stride{to_words(x), to_words(y), to_words(f_mul(curve_d(), f_mul(x, y)))};
 }
 
-// The per-entry part of the PairTable of Q_m = 8m G for half `half` (q =
-// 1/(d y^2) of every entry, then v = 1/y and s = x/(1 + x^2) of every entry;
-// whole groups, so up to two entries past `half`), in the device layout; the
-// same for every search, so built once per half. y and 1 + x^2 are never 0
+// The per-entry part of a PairTable for Q_m = 8m G, m = 1..n, n a power of two
+// (q = 1/(d y^2) of every entry, then v = 1/y and s = x/(1 + x^2) of every
+// entry), in the device layout. The same for every search and half, so built
+// once per power of two and kept: 96 bytes an entry. y and 1 + x^2 are never 0
 // for a point of odd order.
-static const std::vector<uint4>& pair_entries(uint32_t half) {
+static const std::vector<uint4>& pair_entries(uint32_t n) {
     static std::mutex mu;
     static std::map<uint32_t, std::unique_ptr<std::vector<uint4>>> cache;
     std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(half);
+    auto it = cache.find(n);
     if (it != cache.end()) return *it->second;
-    const uint32_t n = groups_of(half) * GROUP;
     std::vector<Pt> pts(n);
     const Pt eight = base_mult_u64(8);
     Pt p = eight;
@@ -111,7 +110,7 @@ static const std::vector<uint4>& pair_entries(uint32_t half) {
         put_fe(vs + 2, 1, f_mul(xs[m], f_mul(ys[m], i)));
     }
     auto& ref = *tab;
-    cache[half] = std::move(tab);
+    cache[n] = std::move(tab);
     return ref;
 }
 
@@ -120,8 +119,14 @@ static const std::vector<uint4>& pair_entries(uint32_t half) {
 cudaError_t make_pair_table(DevBuf<uint4>& table, uint32_t half, cudaStream_t s) {
     cudaError_t e = table.alloc(pair_table_uint4(half));
     if (e != cudaSuccess) return e;
-    const std::vector<uint4>& tab = pair_entries(half);
-    e = cudaMemcpyAsync(table.p, tab.data(), tab.size() * sizeof(uint4), cudaMemcpyHostToDevice, s);
+    // whole groups, so up to two entries past `half`
+    const size_t n = (size_t)groups_of(half) * GROUP;
+    uint32_t built = 256;
+    while (built < n) built *= 2;
+    const std::vector<uint4>& tab = pair_entries(built);
+    e = cudaMemcpyAsync(table.p, tab.data(), n * 2 * sizeof(uint4), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(table.p + n * 2, tab.data() + (size_t)built * 2, n * 4 * sizeof(uint4), cudaMemcpyHostToDevice, s);
     return e == cudaSuccess ? launch_group_table(table.p, half, s) : e;
 }
 
@@ -138,6 +143,32 @@ std::vector<uint4> pow2_table(const Pt& stride, uint32_t nbits) {
         p = pt_dbl(p);
     }
     return out;
+}
+
+// The table of add_multiple_8g, the same for every search: built once.
+const std::vector<uint4>& multiples_8g() {
+    static const std::vector<uint4> table = [] {
+        std::vector<Pt> pts;
+        Pt base = base_mult_u64(8);
+        for (uint32_t w = 0; w < MULTIPLES_8G / 16; w++) {
+            Pt p = pt_identity();
+            for (uint32_t d = 0; d < 16; d++) {
+                pts.push_back(p);
+                p = pt_add(p, base);
+            }
+            base = p;  // 16 times the digit's weight
+        }
+        std::vector<F51> xs, ys;
+        batch_affine(pts, xs, ys);
+        std::vector<uint4> out(pts.size() * 6);
+        for (size_t i = 0; i < pts.size(); i++) {
+            put_fe(out.data() + i * 6 + 0, 1, f_add(ys[i], xs[i]));
+            put_fe(out.data() + i * 6 + 2, 1, f_sub(ys[i], xs[i]));
+            put_fe(out.data() + i * 6 + 4, 1, f_mul(f_mul(xs[i], ys[i]), curve_2d()));
+        }
+        return out;
+    }();
+    return table;
 }
 
 uint32_t bits_for(uint64_t v) {
@@ -230,7 +261,7 @@ struct og_engine {
     DevBuf<uint64_t> mkeys;
     DevBuf<uint32_t> mowners, mpatterns;
     DevBuf<uint32_t> suffixes;
-    DevBuf<uint4> pow8;
+    DevBuf<uint4> mul8;
     MatchArgs ma{};
 
     ~og_engine() {
@@ -558,13 +589,12 @@ int enable_matching(og_engine* e, const og_filters* f, char* err, size_t errlen)
         CU(e->mpatterns.alloc(pats.size()));
         CU(cudaMemcpyAsync(e->mpatterns.p, pats.data(), pats.size() * 4, cudaMemcpyHostToDevice, e->stream));
     }
-    std::vector<uint4> pw;
     if (!sfx.empty()) {
         CU(e->suffixes.alloc(sfx.size()));
         CU(cudaMemcpyAsync(e->suffixes.p, sfx.data(), sfx.size() * 4, cudaMemcpyHostToDevice, e->stream));
-        pw = pow2_table(base_mult_u64(8), 64);
-        CU(e->pow8.alloc(pw.size()));
-        CU(cudaMemcpyAsync(e->pow8.p, pw.data(), pw.size() * sizeof(uint4), cudaMemcpyHostToDevice, e->stream));
+        const std::vector<uint4>& m8 = multiples_8g();
+        CU(e->mul8.alloc(m8.size()));
+        CU(cudaMemcpyAsync(e->mul8.p, m8.data(), m8.size() * sizeof(uint4), cudaMemcpyHostToDevice, e->stream));
     }
     for (og_engine::Flight& fl : e->fl) CU(fl.matches.alloc(e->cap));
     CU(cudaStreamSynchronize(e->stream));
@@ -591,7 +621,7 @@ int enable_matching(og_engine* e, const og_filters* f, char* err, size_t errlen)
     m.sy = to_words(e->start.Y);
     m.sz = to_words(e->start.Z);
     m.st = to_words(e->start.T);
-    m.pow8 = e->pow8.p;
+    m.mul8 = e->mul8.p;
     m.out = nullptr;
     m.out_count = nullptr;
     m.out_cap = m.surv_cap;

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(128) group_table_kernel(uint4* table, uint32_t
 // survivor's scalar offset over 8 decoded from its record.
 __device__ __noinline__ uint32_t suffix_owner(const MatchArgs& a, const HitRec& r) {
     const uint64_t k = a.first + (((uint64_t)r.step << 32) | r.lane);
-    const SuffixTables t{a.suffixes, a.nsuffix, a.pow8};
+    const SuffixTables t{a.suffixes, a.nsuffix, a.mul8};
     bool bad = false;
     const uint32_t j = suffix_match(t, a.sx, a.sy, a.sz, a.st, k, r.y, bad);
     if (bad) atomicAdd(a.mismatch, 1u);

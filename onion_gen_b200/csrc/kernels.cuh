@@ -49,6 +49,9 @@ struct MatchRec {
 };
 static_assert(sizeof(MatchRec) == 48, "MatchRec layout");
 
+// Entries of the table of multiples of 8G (add_multiple_8g): 16 digits of four bits.
+constexpr uint32_t MULTIPLES_8G = 16 * 16;
+
 struct FeWords {
     uint32_t v[8];
 };
@@ -172,7 +175,7 @@ struct MatchArgs {
     uint32_t nsuffix;
     uint32_t prefix_count;     // filter index of suffix j is prefix_count + j
     FeWords sx, sy, sz, st;    // the engine's start point, extended
-    const uint4* pow8;         // 2^j 8G, j < 64, cached form: (j * 3 + {ypx,ymx,t2d}) * 2 + q
+    const uint4* mul8;         // multiples of 8G (add_multiple_8g)
     uint64_t first;            // scalar offset over 8 of the advance's candidate 0
     MatchRec* out;
     uint32_t* out_count;

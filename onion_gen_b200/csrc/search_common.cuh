@@ -256,6 +256,19 @@ __device__ __forceinline__ void add_cached(fe& X, fe& Y, fe& Z, fe& T, const fe&
     T = fe_mulv(x3, y3);
 }
 
+// Adds k 8G from a table of d 16^w 8G (w < 16, d < 16; 0 is the identity) in
+// cached form, (((w * 16 + d) * 3 + {ypx,ymx,t2d}) * 2 + q). Four bits an
+// addition: the lanes' k differ in every digit, so a warp would take all the
+// additions of a table of powers of two, a chain of 3 500 clocks for each bit of
+// the longest k. The table, 24 KB, stays in L1.
+__device__ __forceinline__ void add_multiple_8g(fe& X, fe& Y, fe& Z, fe& T, const uint4* table, uint64_t k) {
+#pragma unroll 1
+    for (; k; k >>= 4, table += 16 * 6) {
+        const uint4* p = table + (k & 15u) * 6;
+        add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
+    }
+}
+
 // ---- the paired round ---------------------------------------------------
 //
 // For a centre P = (x, y) and a table point Q = (x2, y2) of odd order, the

@@ -8,29 +8,23 @@
 
 namespace og {
 
-// The suffixes of one filter set, and the table of 2^j 8G (j < 64, cached
-// form, (j * 3 + {ypx,ymx,t2d}) * 2 + q) the key recomputation walks.
+// The suffixes of one filter set, and the table of multiples of 8G the key
+// recomputation walks (add_multiple_8g).
 struct SuffixTables {
     const uint32_t* suffixes;  // per suffix MAX_SUFFIX_SYMBOLS + 1 words: its length, then a set per position
     uint32_t nsuffix;
-    const uint4* pow8;
+    const uint4* mul8;
 };
 
 // Index of the first suffix the key at scalar offset 8 k from `start`
-// matches, or 0xffffffff. The key is start + k 8G over the binary expansion
-// of k, made affine; its y must equal the survivor's canonical `yrec` (a
+// matches, or 0xffffffff. The key is start + k 8G, made affine; its y must equal the survivor's canonical `yrec` (a
 // mismatch sets `mismatch` and never matches; the caller counts it). The
 // sign bit is the parity of the canonical x.
 __device__ __forceinline__ uint32_t suffix_match(const SuffixTables& t, const FeWords& sx, const FeWords& sy,
                                                  const FeWords& sz, const FeWords& st, uint64_t k,
                                                  const uint32_t yrec[8], bool& mismatch) {
     fe X = words_fe(sx), Y = words_fe(sy), Z = words_fe(sz), T = words_fe(st);
-#pragma unroll 1
-    for (uint32_t j = 0; j < 64; j++)
-        if ((k >> j) & 1) {
-            const uint4* p = t.pow8 + (size_t)j * 6;
-            add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
-        }
+    add_multiple_8g(X, Y, Z, T, t.mul8, k);
     const fe zi = fe_invert(Z);
     const fe x = fe_canon(fe_mulv(X, zi)), y = fe_canon(fe_mulv(Y, zi));
     bool same = true;
