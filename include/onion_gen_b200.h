@@ -379,7 +379,7 @@ void og_serve_free(og_serve* s);
  * reserve all device memory up front — og_search_noalloc runs one paired
  * search over a fixed range without calling cudaMalloc, cudaFree or any
  * allocating library routine. The caller passes the inputs and outputs in
- * device memory it owns; lane state, the Montgomery scratch and the tables
+ * device memory it owns; lane state, the rounds' products and the tables
  * live in one file-scope device array of OG_NOALLOC_SCRATCH_BYTES, which
  * every GPU that loads this library holds until the process exits.
  *

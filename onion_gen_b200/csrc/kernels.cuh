@@ -95,11 +95,13 @@ __host__ __device__ constexpr size_t cta_scratch_uint4(uint32_t half) {
 }
 
 // How a sink's keys are tested: by paired_rounds, whose matrix product gives a
-// key's low 24 bits and its bits from 232 on, or in full. A width of 0 stands
-// for no bitmap.
+// key's low 24 bits and its bits from 231 on, or in full. A suffix bitmap of 24
+// bits reads one bit more, and paired_rounds looks both of its values up: twice
+// the possible survivors to compute, but 9.7e7 candidates against 40 eight-symbol
+// suffixes (0.24 % of them survive) took 3.45 ms in full and take 2.43. A width of 0 stands for no bitmap.
 enum SinkKind { SINK_PREFIX, SINK_SUFFIX, SINK_FULL };
 __host__ __device__ inline SinkKind sink_kind(uint32_t prefix_bits, uint32_t suffix_bits) {
-    if (prefix_bits > 24 || suffix_bits > 23 || (!prefix_bits && !suffix_bits)) return SINK_FULL;
+    if (prefix_bits > 24 || suffix_bits > 24 || (!prefix_bits && !suffix_bits)) return SINK_FULL;
     return suffix_bits ? SINK_SUFFIX : SINK_PREFIX;
 }
 

@@ -6,7 +6,7 @@
 // processes that reserve all device memory up front. This entry point lets
 // them run the search: they pass the inputs (start point, bitmap) and the
 // outputs (survivor records and their counter) in device memory they own,
-// and everything else — lane state, the Montgomery scratch and the tables —
+// and everything else — lane state, the rounds' products and the tables —
 // lives in one file-scope device array, `og_noalloc_scratch`, sized
 // OG_NOALLOC_SCRATCH_BYTES. Every GPU that loads the library holds that array
 // until the process exits.

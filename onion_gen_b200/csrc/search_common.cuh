@@ -576,6 +576,14 @@ __device__ __forceinline__ void test_group(RoundShared& sh, const Sink& sink, co
 #pragma unroll
         for (int k = 0; k < KEYS; k++)
             hits |= suffix_hit(sink, 0u, top[k]) | suffix_hit(sink, 0u, (top[k] + 128u) & 0x7fffffffu) ? 1u << k : 0u;
+        // a 24-bit slot's bit 23 is the key's bit 224, which the sums do not give
+        if (sink.sbits > 23) {
+#pragma unroll
+            for (int k = 0; k < KEYS; k++)
+                hits |= suffix_hit(sink, 0u, top[k] | 1u) | suffix_hit(sink, 0u, ((top[k] + 128u) & 0x7fffffffu) | 1u)
+                            ? 1u << k
+                            : 0u;
+        }
     }
     const uint32_t entries = min(GROUP, half - m0 + 1);
     hits &= active ? (1u << (2 * entries)) - 1u : 0u;
