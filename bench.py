@@ -75,12 +75,12 @@ BATCH_STEP_CAP_MS = 8.0
 CPU_HALF = 4096  # PairEngine::new(8192) (src/run.rs:601, src/batch.rs:32)
 # DRAM bytes per candidate of paired_kernel, from the ncu capture of the
 # small case (bench.py --case small: half 256, 757,760 lanes, one launch of
-# 388,730,880 candidates; dram__bytes_read.sum + dram__bytes_write.sum =
-# 24.96 + 25.03 GB), scaled to a launch of the plain line by its candidates:
-# the traffic is the Montgomery scratch, 64 B written and 64 B read per
-# candidate, whatever the shape, so it grows in proportion.
-TRAFFIC_PER_CANDIDATE = 128.6
-ALGORITHMIC_BYTES_PER_CANDIDATE = 128
+# 388,730,880 candidates; dram__bytes.sum.per_second 1.195 TB/s over 6.987 ms),
+# scaled to a launch of the plain line by its candidates: the traffic is a
+# running product and a group's denominator, 32 bytes each, written and read
+# back once for three pairs, so it grows in proportion.
+TRAFFIC_PER_CANDIDATE = 21.5
+ALGORITHMIC_BYTES_PER_CANDIDATE = 128 / 6
 
 
 def parse():
@@ -545,7 +545,7 @@ def config3_leg(dev, peak, steps=2):
     wall = time.perf_counter() - t0
     eng.close()
     n = batch * total
-    w = pp_per_candidate(shape.half)
+    w = PP_PER_CANDIDATE
     rate = n / (kernel_ms * 1e-3)
     log(f"config 3 leg: {rate:.4e} keys/s device, {n / wall:.4e} end to end, {matches} matches")
     return {
@@ -567,32 +567,19 @@ def config3_leg(dev, peak, steps=2):
     }
 
 
-BLOCK_LANES = 128  # lanes a block of the search kernels, which share one inversion
-
-
-def block_inversion_pp():
-    """Partial products a lane spends on its share of the block's one
-    inversion: 16 multiplications of its own (two five-step warp scans, the
-    other three warps' totals, the last three products) and 1/128 of thread
-    0's (three multiplications for the block's product and the inversion,
-    254 squarings of 36 products and 11 multiplications)."""
-    return 16 * 64 + (14 * 64 + 254 * 36) / BLOCK_LANES
-
-
-def pp_per_candidate(half):
-    """Partial products per candidate of the paired round: 10 + 10 half
-    multiplications of 64 and the lane's share of the block's inversion,
-    over 2 half + 1 keys."""
-    return ((10 + 10 * half) * 64 + block_inversion_pp()) / (2 * half + 1)
+# Partial products per candidate of the search kernel: nine multiplications of
+# 64 for a group of three pairs, six candidates. Both schemes run on it. What a
+# round adds (the centre, its powers, the step to the next centre, the block's
+# inversion) is not counted: 30 or so multiplications for thousands of
+# candidates.
+PP_PER_CANDIDATE = 9 * 64 / 6
 
 
 def small_case(args):
     """Three advances of one round each: the case the ncu summaries under
-    profiles/ are captured on. Half 256 (or --half) keeps the scratch of the
-    persistent CTAs near 3.8 GB; the lanes are eight blocks per resident CTA
-    (SMs x 5 x 128 x 8), as in production. The kernel is the production one,
-    and its DRAM bytes per candidate do not depend on the shape (64 B written
-    and read back per candidate)."""
+    profiles/ are captured on. Half 256 (or --half) with the default lanes is an
+    eighth of the production advance's candidates; the kernel is the production
+    one, and its DRAM bytes per candidate do not depend on the shape."""
     from onion_gen_b200 import _native as N
     from onion_gen_b200 import filter as F
     from onion_gen_b200 import gpu, key, workloads
@@ -603,7 +590,7 @@ def small_case(args):
     fs = F.FilterSet.parse_all([workloads.config2_prefix()])
     words, bits = fs.index_words()
     start = key.start_point(workloads.seed(0))
-    # eight blocks of lanes per resident CTA (lanes 0: the engine's default waves)
+    # lanes 0: the engine's default waves
     eng = gpu.Engine(dev, start, bitmap=words, bitmap_bits=bits,
                      config=N.EngineConfig(0, half, 0, 1, 128, 0, 0, lpt))
     lanes = eng.threads()
@@ -616,8 +603,7 @@ def small_case(args):
 
 def chain_small_case(args):
     """Three advances of the chain scheme on config 2's search at its default
-    shape (n = 1024, four waves of lanes): the case the chain kernel's ncu
-    summary is captured on."""
+    shape (n = 1024, four waves of lanes)."""
     from onion_gen_b200 import _native as N
     from onion_gen_b200 import filter as F
     from onion_gen_b200 import gpu, key, workloads
@@ -673,14 +659,6 @@ def config3_small_case(args):
               f"kernel {ms:.3f} ms, {eng.batch() / ms * 1e3:.4e} keys/s")
 
 
-def chain_pp_per_candidate(n):
-    """Partial products per candidate of the chain scheme (the config-1
-    contract, src/batch.rs:78-122): 7 multiplications for the +8G step, 4 for
-    Montgomery's trick and y / Z, and the lane's share of the block's
-    inversion per n steps."""
-    return (11 * 64 * n + block_inversion_pp()) / n
-
-
 def chain_leg(dev, peak):
     """The chain scheme (the device restatement of BatchEngine, which config 1
     pins bit for bit) on config 2's search at its default shape (n = 1024,
@@ -702,11 +680,11 @@ def chain_leg(dev, peak):
         ms += eng.last_kernel_ms()
     rate = 3 * eng.batch() / (ms * 1e-3)
     eng.close()
-    w = chain_pp_per_candidate(shape.half)
+    w = PP_PER_CANDIDATE
     log(f"chain leg: {rate:.4e} keys/s at n = {shape.half}, {shape.lanes} lanes")
     return {
-        "workload": "chain scheme on config 2's search (seed LE32(0), its 16-bit index), n = %d steps per lane "
-        "between inversions, %d lanes" % (shape.half, shape.lanes),
+        "workload": "chain scheme on config 2's search (seed LE32(0), its 16-bit index), n = %d steps per lane, "
+        "%d lanes" % (shape.half, shape.lanes),
         "keys_per_s": rate,
         "per_candidate": w,
         "roofline_frac": rate * w / peak,
@@ -767,8 +745,7 @@ def batch_small_case(args):
     """Three steps of the batched engine with the first 16 config-4 searches
     admitted (two of them long), at the batched leg's shape except for the
     largest inversion batch: half 256, long searches at up to 512 (the leg
-    uses 2048; 512 keeps the scratch near 6 GB for a multi-pass capture), two
-    waves of slots, two steps in flight. The case the batched kernels' ncu
+    uses 2048), two waves of slots, two steps in flight. The case the batched kernels' ncu
     summaries are captured on."""
     from onion_gen_b200 import batch as B
     from onion_gen_b200 import gpu, workloads
@@ -878,7 +855,7 @@ def main():
     mulpp = C.c_double()
     err = N.errbuf()
     N.check(N.lib.og_measure_int_peak(dev.ordinal, C.byref(imad), C.byref(mulpp), err, 512), err)
-    w = pp_per_candidate(shape.half)
+    w = PP_PER_CANDIDATE
     hbm_peak = None
     try:
         hbm_peak = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["hbm_gbs"]
@@ -896,8 +873,7 @@ def main():
     # is `advances` advances with the D2H of their survivors and the host's
     # checks. The clock stops when the last step's hits are verified; the
     # engine's free comes after every result is delivered and is reported
-    # beside it (freeing 25 GB of scratch usually takes 0.02 s, but some
-    # runs saw 0.2-0.8 s inside cudaFree).
+    # beside it.
     eng.close()  # the plain line's engine is done; the e2e run makes its own
     e2e = None
     if not args.no_e2e:
@@ -979,7 +955,7 @@ def main():
                 "frac": achieved / peak,
                 "traffic": TRAFFIC_PER_CANDIDATE * batch,
                 "traffic_unit": "DRAM bytes per launch (ncu dram__bytes_read.sum + dram__bytes_write.sum on the "
-                "small case, 128.6 B a candidate, scaled to this launch's candidates)",
+                "small case, 21.5 B a candidate, scaled to this launch's candidates)",
                 "per_candidate": w,
                 "peak_source": "measured: og_measure_int_peak mad.lo.u32 issue rate / 2 (lo+hi per product)",
                 "peak_theoretical": theoretical,
@@ -992,7 +968,7 @@ def main():
                     "peak": hbm_peak,
                     "unit": "GB/s",
                     "frac": value / world * ALGORITHMIC_BYTES_PER_CANDIDATE / 1e9 / hbm_peak if hbm_peak else None,
-                    "note": "the Montgomery scratch: not the bound",
+                    "note": "the round's stored products: not the bound",
                 },
             },
             "clocks": clock_summary,
