@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) paired_kernel
         const bool active = lane < a.lanes_n;
         uint4* const centre = a.lanes + (active ? lane : 0);
         if constexpr (Kind != SINK_FULL)
-            paired_rounds<Kind == SINK_SUFFIX>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, *sh, mu,
+            paired_rounds<Kind == SINK_SUFFIX, true>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, *sh, mu,
                                                lane, active);
         else
             paired_rounds_full(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, lane, active);

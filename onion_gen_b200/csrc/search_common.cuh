@@ -629,15 +629,21 @@ __device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe&
 }
 
 // A block's `rounds` paired rounds, a lane each, against bitmaps of at most 24
-// and 23 bits (sink_is_narrow); see kernels.cuh for the candidate numbering.
-// `centre` points at the lane's affine centre in the lane state (x, then y,
-// 16-byte halves `cstride` apart), which is left on the centre after the last
-// round: `between` is the stride after every round but the last, `last` the
-// stride after that one. `scr` is the thread's column of its CTA's scratch: group j's prefix product, then E, half q at
-// scr + (4 j + 2 e + q) SCRATCH_ROW. A thread that is not `active` has no lane:
-// it takes part with another's centre and reports nothing. Every thread of
-// the block calls it together, between matrix_open and matrix_close.
-template <bool Suffixes>
+// bits (sink_kind); see kernels.cuh for the candidate numbering. `centre` points
+// at the lane's affine centre in the lane state (x, then y, 16-byte halves
+// `cstride` apart), which is left on the centre after the last round: `between`
+// is the stride after every round but the last, `last` the stride after that
+// one. `scr` is the thread's column of its CTA's scratch: group j's prefix
+// product, then E, half q at scr + (4 j + 2 e + q) SCRATCH_ROW. With Ahead, a
+// group's two are read a group ahead, under the five multiplications of the one
+// before, at the cost of 16 registers: the engine's kernel 50.3 -> 49.8 ms for
+// 3.1e9 candidates (prefetch hints to L1 or L2 instead: 51.0); the batched one,
+// with less to spare, ran some mixes 1 % faster and others 3.34 -> 3.57 ms a
+// step, and the no-allocation one 1.68 -> 1.72 ms a call, so they go without. A
+// thread that is not `active` has no lane: it takes part with another's centre
+// and reports nothing. Every thread of the block calls it together, between
+// matrix_open and matrix_close.
+template <bool Suffixes, bool Ahead>
 __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, const Stride& between, const Stride& last,
                                               const PairTable& tab, uint32_t half, uint32_t rounds, uint4* scr,
                                               const Sink& sink, RoundShared& sh, MatrixUnit& mu, uint32_t lane,
@@ -675,13 +681,16 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
             store_row(row, 0, y);
             stage_push(sink, tab, st, hit, row, s.X, lane, mid, 0u);
         }
-        // A group's P and E are read a group ahead, under the five
-        // multiplications of the one before: 50.3 -> 49.7 ms for 3.1e9
-        // candidates (prefetch hints instead, to L1 or L2: 51.0).
-        const uint4* p = scr + (size_t)(groups - 1) * (4 * SCRATCH_ROW);
-        fe P = load_fe(p, SCRATCH_ROW), E = load_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW);
+        fe P, E;
+        const auto load_group = [&](uint32_t j) {
+            const uint4* p = scr + (size_t)j * (4 * SCRATCH_ROW);
+            P = load_fe(p, SCRATCH_ROW);
+            E = load_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW);
+        };
+        if (Ahead) load_group(groups - 1);
 #pragma unroll 1
         for (uint32_t j = groups; j-- > 0;) {
+            if (!Ahead) load_group(j);
             const fe h = fe_mulv(P, s.I);
             s.I = fe_mulv(s.I, E);
             if (j + 1 < groups) {
@@ -690,11 +699,7 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
                 if (threadIdx.x == 0 && !sh.failed) fetch_constants(sh, tab.constants + (size_t)j * GROUP_CONSTANTS);
                 test_group<Suffixes>(sh, sink, tab, st, s.X, lane, active, mid, (j + 1) * GROUP + 1, half);
             }
-            if (j > 0) {
-                p = scr + (size_t)(j - 1) * (4 * SCRATCH_ROW);
-                P = load_fe(p, SCRATCH_ROW);
-                E = load_fe(p + 2 * SCRATCH_ROW, SCRATCH_ROW);
-            }
+            if (Ahead && j > 0) load_group(j - 1);
             store_row(row, 0, h);
             store_row(row, 3, fe_mulv(s.e, h));
             const fe g1 = fe_mulv(s.X, h);
