@@ -300,7 +300,7 @@ __device__ __forceinline__ void add_multiple_8g(fe& X, fe& Y, fe& Z, fe& T, cons
 // q' and q'' the other two. So three pairs take nine multiplications, and
 // the six keys are products of lane values with a table of constants: a
 // matrix product, of which only what the bitmap reads is computed, on the
-// tensor cores (keys_of_group).
+// tensor cores (test_group).
 
 __device__ __forceinline__ fe const_inv_d() {  // 1/d
     return fe{{0xcdc9f843u, 0x25e0f276u, 0x4279542eu, 0x0b5dd698u, 0xcdb9cf66u, 0x2b162114u, 0x14d5ce43u, 0x40907ed2u}};
