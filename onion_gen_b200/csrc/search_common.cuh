@@ -416,6 +416,7 @@ __device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_
 // Called by every thread of the block, before the first round and after the
 // last one.
 __device__ __forceinline__ void matrix_open(RoundShared& sh) {
+    __syncwarp();  // the allocation takes the whole warp, and some of its lanes may come from a branch
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(shared_addr(&sh.tmem)),
                      "r"(TMEM_COLUMNS)
@@ -543,6 +544,9 @@ __device__ __forceinline__ void test_group(RoundShared& sh, const Sink& sink, co
     constexpr int KEYS = 2 * GROUP;
     const uint32_t from = sh.tmem + ((threadIdx.x / 32) << 21);  // 32 lanes a warp, in bits 16 and up
     uint32_t slot[KEYS], top[KEYS], hits = 0;
+    // the loads take the whole warp, whose lanes left the wait one by one; thread
+    // 0 has fetched and issued besides
+    __syncwarp();
 #pragma unroll
     for (int i = 0; i < (int)GROUP; i++) {
         uint32_t c[2 * KEY_COLUMNS];
