@@ -207,10 +207,10 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_
         uint4* const centre = a.lanes + (size_t)item.place * BLOCK + threadIdx.x;
         const uint32_t lane = item.lane0 + threadIdx.x;
         if (sink_kind(d.bitmap ? d.bits : 0, d.sbitmap ? d.sbits : 0) == SINK_PREFIX)
-            paired_rounds<false, false>(centre, a.slots, d.between, d.last, a.table, d.item_half, d.rounds, scr, sink, sh, mu,
+            paired_rounds<false, false, false>(centre, a.slots, d.between, d.last, a.table, d.item_half, d.rounds, scr, sink, sh, mu,
                                  lane, true);
         else
-            paired_rounds_full(centre, a.slots, d.between, d.last, a.table, d.item_half, d.rounds, scr, sink, lane, true);
+            paired_rounds_full<false>(centre, a.slots, d.between, d.last, a.table, d.item_half, d.rounds, scr, sink, lane, true);
     }
     matrix_close(sh);
 }

@@ -171,6 +171,15 @@ const std::vector<uint4>& multiples_8g() {
     return table;
 }
 
+// Whether p plus a multiple of 8G can have order four: l p has it then, l the
+// prime order of G.
+static bool may_meet_order_four(const Pt& p) {
+    static const uint8_t l[32] = {0xed, 0xd3, 0xf5, 0x5c, 0x1a, 0x63, 0x12, 0x58, 0xd6, 0x9c, 0xf7,
+                                  0xa2, 0xde, 0xf9, 0xde, 0x14, 0,    0,    0,    0,    0,    0,
+                                  0,    0,    0,    0,    0,    0,    0,    0,    0,    0x10};
+    return f_is_zero(point_mult(p, l).Y);
+}
+
 uint32_t bits_for(uint64_t v) {
     uint32_t b = 0;
     while (b < 64 && (v >> b) != 0) b++;
@@ -224,6 +233,7 @@ struct og_engine {
     uint64_t batch = 0;  // candidates of an advance
     uint32_t bits = 0;
     uint32_t grid = 0;  // persistent CTAs of the search kernel
+    SinkKind kind = SINK_FULL;
     size_t cap = 0;
     uint64_t launches = 0;
     float last_ms = 0;
@@ -469,7 +479,8 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     e->batch = batch;
     Tile tile{};
     {
-        const int rc = plan_tile(ordinal, batch, sink_kind(!cfg.dump && bitmap ? bits : 0, suffixed ? f->suffixes.bits() : 0), &tile, err, errlen);
+        if (!may_meet_order_four(start_pt)) e->kind = sink_kind(!cfg.dump && bitmap ? bits : 0, suffixed ? f->suffixes.bits() : 0);
+        const int rc = plan_tile(ordinal, batch, e->kind, &tile, err, errlen);
         if (rc) return rc;
         e->grid = tile.grid;
     }
@@ -650,7 +661,7 @@ int enqueue_advance(og_engine* e, bool match, char* err, size_t errlen) {
     e->pa.counter = f.counts.p;
     e->pa.work = f.counts.p + 3;
     e->pa.failed = f.counts.p + 4;
-    CU(launch_paired(e->pa, (int)e->grid, e->stream));
+    CU(launch_paired(e->pa, e->kind, (int)e->grid, e->stream));
     CU(cudaEventRecord(f.ev1, e->stream));
     if (match) {
         MatchArgs& m = e->ma;

@@ -144,6 +144,8 @@ __device__ __forceinline__ fe fe_canon(const fe& a) {
     return r;
 }
 
+__device__ __forceinline__ fe fe_zero() { return fe{{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}}; }
+
 __device__ __forceinline__ fe fe_one() {
     fe r;
 #pragma unroll

@@ -67,10 +67,10 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) paired_kernel
         const bool active = lane < a.lanes_n;
         uint4* const centre = a.lanes + (active ? lane : 0);
         if constexpr (Kind != SINK_FULL)
-            paired_rounds<Kind == SINK_SUFFIX, true>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, *sh, mu,
-                                               lane, active);
+            paired_rounds<Kind == SINK_SUFFIX, true, false>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink,
+                                                      *sh, mu, lane, active);
         else
-            paired_rounds_full(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, lane, active);
+            paired_rounds_full<true>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, lane, active);
     }
     if constexpr (Kind != SINK_FULL) matrix_close(*sh);
 }
@@ -127,9 +127,8 @@ cudaError_t launch_init(const InitArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_paired(const PairedArgs& a, int grid, cudaStream_t s) {
+cudaError_t launch_paired(const PairedArgs& a, SinkKind kind, int grid, cudaStream_t s) {
     if (grid <= 0) return cudaErrorInvalidValue;
-    const SinkKind kind = sink_kind(a.bitmap ? a.bits : 0, a.sbitmap ? a.sbits : 0);
     if (kind == SINK_PREFIX)
         paired_kernel<SINK_PREFIX><<<grid, OG_LB_THREADS, 0, s>>>(a);
     else if (kind == SINK_SUFFIX)

@@ -190,7 +190,8 @@ cudaError_t launch_match(const MatchArgs& a, int grid, cudaStream_t s);
 // The search kernel is persistent: `grid` CTAs of OG_LB_THREADS (at most the
 // resident ones) take the lanes a block at a time from `work`, so the scratch
 // covers only the lanes in flight and no SM idles in a tail wave.
-cudaError_t launch_paired(const PairedArgs& a, int grid, cudaStream_t s);
+// `kind` is that of its bitmaps, or SINK_FULL, which takes any bitmaps and any start.
+cudaError_t launch_paired(const PairedArgs& a, SinkKind kind, int grid, cudaStream_t s);
 // Completes a PairTable whose per-entry part is on the device.
 cudaError_t launch_group_table(uint4* table, uint32_t half, cudaStream_t s);
 

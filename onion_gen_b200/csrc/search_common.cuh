@@ -282,8 +282,13 @@ __device__ __forceinline__ void add_multiple_8g(fe& X, fe& Y, fe& Z, fe& T, cons
 // (substitute y^2 = (1 + x^2) / (1 - d x^2) into the addition formula's
 // numerators and 1 -+ d x x2 y y2; the common factors cancel). Its
 // denominator is (1/y2^2 - d x^2) / d, which has no zero because d is not a
-// square, so no centre is exceptional; z is 0 only for the two centres of
-// order four.
+// square. Only z can be 0, for the two centres of order four, (+-sqrt(-1), 0):
+// no s B + 8 k G is one, but a caller's start point may lead to them, and the 0
+// would take the whole block's inversion with it. With AnyStart, such a lane's
+// round runs with 1 for z (then e = c), and its g_k are set to 0 where they are
+// stored. The batch's starts are multiples of the base point, and the engine tells
+// by its start which rounds to run (may_meet_order_four), because the test costs
+// them 1 to 2 %: the default advance 53.2 -> 54.5 ms.
 //
 // The denominators are taken three at a time. With D_i = q_i - X, i = 1..3,
 // and E = D_1 D_2 D_3, the product is a cubic in X whose coefficients are
@@ -603,6 +608,12 @@ __device__ __forceinline__ void test_group(RoundShared& sh, const Sink& sink, co
     }
 }
 
+// Whether a centre has order four: its y is 0 modulo p.
+__device__ __forceinline__ bool order_four(const fe& y) {
+    const fe v = fe_canon(y);
+    return (v.v[0] | v.v[1] | v.v[2] | v.v[3] | v.v[4] | v.v[5] | v.v[6] | v.v[7]) == 0;
+}
+
 // What a lane's round keeps for its second pass.
 struct RoundState {
     fe X, e, I;
@@ -647,7 +658,7 @@ __device__ __forceinline__ void turn_round(RoundState& s, const fe& x, const fe&
 // thread that is not `active` has no lane: it takes part with another's centre
 // and reports nothing. Every thread of the block calls it together, between
 // matrix_open and matrix_close.
-template <bool Suffixes, bool Ahead>
+template <bool Suffixes, bool Ahead, bool AnyStart>
 __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, const Stride& between, const Stride& last,
                                               const PairTable& tab, uint32_t half, uint32_t rounds, uint4* scr,
                                               const Sink& sink, RoundShared& sh, MatrixUnit& mu, uint32_t lane,
@@ -658,11 +669,13 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
     for (uint32_t r = 0; r < rounds; r++) {
         RoundState s;
         const uint32_t mid = r * slots + half;
+        bool four;
         if (threadIdx.x == 0 && !sh.failed) fetch_constants(sh, tab.constants + (size_t)(groups - 1) * GROUP_CONSTANTS);
         {
             const fe x = load_fe(centre, cstride), y = load_fe(centre + 2 * cstride, cstride);
             s.X = fe_sqv(x);
-            const fe X2 = fe_sqv(s.X), z = fe_mulv(y, fe_sub(const_inv_d(), s.X));
+            four = AnyStart && order_four(y);
+            const fe X2 = fe_sqv(s.X), z = select_fe(four, fe_one(), fe_mulv(y, fe_sub(const_inv_d(), s.X)));
             fe run = z;
 #pragma unroll 1
             for (uint32_t j = 0; j < groups; j++) {
@@ -712,6 +725,9 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
             const fe g2 = fe_mulv(s.X, g1);
             store_row(row, 2, g2);
             store_row(row, 5, fe_mulv(s.e, g2));
+            if (AnyStart && four) {
+                for (uint32_t k = 0; k < 3; k++) store_row(row, k, fe_zero());
+            }
             start_product(sh, sink, mu);
         }
         finish_product(sh, sink, mu);
@@ -723,6 +739,7 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
 // The same rounds with every key computed in full: for sinks with wider bitmaps
 // than paired_rounds reads, or with none (every candidate survives). A pair takes six multiplications: per pair the prefix
 // product, w = P I [= z / D], I <- I D, f = e w and y = v w +- s f.
+template <bool AnyStart>
 __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride, const Stride& between,
                                                    const Stride& last, const PairTable& tab, uint32_t half,
                                                    uint32_t rounds, uint4* scr, const Sink& sink, uint32_t lane,
@@ -731,10 +748,12 @@ __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride
     for (uint32_t r = 0; r < rounds; r++) {
         RoundState s;
         const uint32_t mid = r * slots + half;
+        bool four;
         {
             const fe x = load_fe(centre, cstride), y = load_fe(centre + 2 * cstride, cstride);
             s.X = fe_sqv(x);
-            const fe z = fe_mulv(y, fe_sub(const_inv_d(), s.X));
+            four = AnyStart && order_four(y);
+            const fe z = select_fe(four, fe_one(), fe_mulv(y, fe_sub(const_inv_d(), s.X)));
             fe run = z;
 #pragma unroll 1
             for (uint32_t m = 0; m < half; m++) {
@@ -749,7 +768,9 @@ __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride
             const fe w = fe_mulv(load_fe(scr + (size_t)(m - 1) * (2 * SCRATCH_ROW), SCRATCH_ROW), s.I);
             s.I = fe_mulv(s.I, fe_sub(load_fe(tab.q + (size_t)(m - 1) * 2, 1), s.X));
             const uint4* t = tab.vs + (size_t)(m - 1) * 4;
-            const fe B = fe_mulv(load_fe(t + 2, 1), fe_mulv(s.e, w)), A = fe_mulv(load_fe(t, 1), w);
+            const fe B = fe_mulv(load_fe(t + 2, 1), fe_mulv(s.e, w));
+            fe A = fe_mulv(load_fe(t, 1), w);
+            if (AnyStart && four) A = fe_zero();
 #pragma unroll 1
             for (uint32_t sign = 0; sign < 2; sign++)
                 test_emit(sink, sign ? fe_sub(A, B) : fe_add(A, B), lane, sign ? mid - m : mid + m, active);
@@ -775,7 +796,7 @@ __device__ inline void fill_group_table(const PairTable& tab, uint32_t groups, u
         store_fe(t + 4, 1, fe_sub(fe_mulv(q01, q[2]), fe_mulv(s1, s2)));
     }
     const uint4* vs = tab.vs + (size_t)(g * GROUP + i) * 4;
-    const fe zero = fe_sub(fe_one(), fe_one()), qa = q[(i + 1) % GROUP], qb = q[(i + 2) % GROUP];
+    const fe zero = fe_zero(), qa = q[(i + 1) % GROUP], qb = q[(i + 2) % GROUP];
     fe c = load_fe(elem < 3 ? vs : vs + 2, 1);
     if (elem % 3 == 0) c = fe_mulv(c, fe_mulv(qa, qb));
     if (elem % 3 == 1) c = fe_sub(zero, fe_mulv(c, fe_add(qa, qb)));
