@@ -388,7 +388,9 @@ void og_serve_free(og_serve* s);
  * of the same shape, and writes each bitmap survivor (every candidate when
  * `d_bitmap` is NULL) to `d_hits` (room `cap`) and their number to
  * `*d_count` (zeroed by the call; a count above `cap` means records were
- * dropped). A record's offset is 8 (w (2 half + 1) + 1 + i) with
+ * dropped). With the bit OG_NOALLOC_FAILED of it set, a wait of the search
+ * kernel ran out (OG_E_TIMEOUT of the other entry points) and the records are
+ * not to be used, however large `cap` is. A record's offset is 8 (w (2 half + 1) + 1 + i) with
  * w = (step / (2 half + 1)) * lanes + lane and i = step % (2 half + 1).
  *
  * Limits: lanes a multiple of 128, half <= 2048, and
@@ -404,6 +406,7 @@ void og_serve_free(og_serve* s);
  * Every call shares the one array: calls whose work overlaps on the GPU
  * (different streams or host threads without ordering) race. */
 #define OG_NOALLOC_SCRATCH_BYTES (64u * 1024u * 1024u)
+#define OG_NOALLOC_FAILED 0x80000000u
 
 typedef struct og_hit_record {
     uint32_t lane;

@@ -25,6 +25,7 @@ STATUS = {
     9: "OG_E_TIMEOUT",
     10: "OG_E_VERIFY",
 }
+NOALLOC_FAILED = 0x80000000  # OG_NOALLOC_FAILED
 SCHEME_PAIRED = 0
 SCHEME_CHAIN = 1
 

@@ -165,8 +165,7 @@ __global__ void __launch_bounds__(NBLOCK, 4) noalloc_paired_kernel(const NoAlloc
         MatrixUnit mu;
         matrix_open(sh);
         paired_rounds<false, false, true>(a.lanes + lane, a.lanes_n, a.stride, a.stride, tab, a.half, a.rounds, scr, sink, sh, mu, lane, true);
-        // a wait that ran out leaves a count beyond any room
-        if (threadIdx.x == 0 && sh.failed) atomicOr(a.counter, 0x80000000u);
+        if (threadIdx.x == 0 && sh.failed) atomicOr(a.counter, OG_NOALLOC_FAILED);
         matrix_close(sh);
     } else {
         paired_rounds_full<true>(a.lanes + lane, a.lanes_n, a.stride, a.stride, tab, a.half, a.rounds, scr, sink, lane, true);

@@ -65,6 +65,18 @@ def resident_lanes(device, scheme=None, block=128):
     return n.value
 
 
+def noalloc_records(count, room):
+    """Records og_search_noalloc left in a buffer of ``room``, from its counter
+    as read back (a 32-bit word, signed or not). Raises when a wait of the
+    kernel ran out or records were dropped."""
+    count = int(count) & 0xFFFFFFFF
+    if count & N.NOALLOC_FAILED:
+        raise OgError(9, "a wait of the search kernel ran out; its records are not to be used")
+    if count > room:
+        raise OgError(5, f"{count} survivors and room for {room}")
+    return count
+
+
 def _words(bitmap):
     if bitmap is None:
         return None, 0
