@@ -80,7 +80,12 @@ enum og_scheme {
 
 /* Launch shape of an engine: what one advance covers. Zero fields take
  * defaults. How the device tiles an advance's candidates over its threads is
- * the engine's own choice. */
+ * the engine's own choice. Device memory: up to 3.7 GB of scratch for an advance
+ * of 3.5e8 candidates or more (5.6 GB with a bitmap over 24 bits, or in a dump),
+ * in proportion below; but no more than the larger of a 64th of the memory free
+ * at creation and 64 bytes per candidate of one wave of lanes at `half`. Then the
+ * record buffers: 48 bytes a record of room, on the device twice (four times with
+ * the device match) and pinned on the host once; and the lanes, up to 0.5 GB. */
 typedef struct og_engine_config {
     uint32_t scheme;   /* og_scheme */
     uint32_t half;     /* paired: a lane's round is 2*half+1 candidates (0: 2048, halved
@@ -214,11 +219,16 @@ void og_engine_free(og_engine* e);
 typedef struct og_batch og_batch;
 
 typedef struct og_batch_config {
-    uint32_t half;          /* table size of every search; a round is 2*half+1 keys (0: 256) */
-    uint32_t slots;         /* lanes in the shared pool, a multiple of 128 (0: two waves of resident blocks) */
+    uint32_t half;          /* a round of a lane is 2*half+1 keys (0: 256) */
+    uint32_t slots;         /* lanes in the shared pool, a multiple of 128 (0: two waves of five blocks
+                               of 128 an SM). With half, max_half and rounds it sets how many candidates
+                               a step has, and with that the batch's device memory: scratch of up to
+                               1.9 GB at a step of 6e7 candidates and more (5.0 GB at max_half 2048), in
+                               proportion below, and within the bound of og_engine_config; 0.1 GB of
+                               lanes; and two record buffers a step in flight */
     uint32_t rounds;        /* rounds per step (0: 1) */
     uint32_t max_searches;  /* searches admitted at once (0: 4096) */
-    uint32_t max_hits;      /* exact hits one step may return (0: 65536) */
+    uint32_t max_hits;      /* exact hits one step may return (0: as many as survivors have room) */
     uint32_t graph;         /* 0 or 1: replay each step as a captured CUDA graph; 2: plain launches */
     uint32_t grid;          /* persistent CTAs per SM (0: as many as fit) */
     uint64_t memory_budget; /* device bytes for per-search tables (0: half of the free memory after the pool) */

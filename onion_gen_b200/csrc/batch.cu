@@ -62,6 +62,7 @@ namespace og {
 
 cudaError_t make_pair_table(DevBuf<uint4>& table, uint32_t half, cudaStream_t s);  // engine.cu
 Stride stride_of(const Pt& w);                                     // engine.cu
+cudaError_t scratch_limit(size_t own, size_t* limit);              // engine.cu
 const std::vector<uint4>& multiples_8g();                          // engine.cu
 MatchTables match_tables(const std::vector<FilterSet::DeviceBucket>& buckets, const uint64_t* keys,
                          const uint32_t* owners, const uint32_t* patterns,
@@ -72,8 +73,8 @@ namespace {
 constexpr uint32_t BLOCK = 128;
 constexpr uint32_t NONE = 0xffffffffu;
 constexpr int MAX_BUCKETS = MAX_MATCH_BUCKETS;
-// Longest windows of an item, in groups of three pairs, unless max_half asks
-// for longer: 1.9 GB of scratch.
+// Longest windows of an item, in groups of three pairs, unless max_half asks for
+// longer: 1.9 GB of scratch. A small pool's are shorter (item_groups).
 constexpr uint32_t ITEM_GROUPS = 256;
 // At most this many items a CTA; a longer step runs its items in several rounds.
 constexpr uint32_t CTA_ITEMS = 8;
@@ -139,7 +140,7 @@ struct BatchArgs {
     const Item* items;
     Counters* counters;  // the flight's
     uint4* lanes;    // ({x,y} * 2 + q) * slots + place * 128 + thread
-    uint4* scratch;  // cta_scratch uint4 a CTA (cta_scratch_uint4 of the longest window)
+    uint4* scratch;  // cta_scratch uint4 a CTA (cta_scratch_uint4 of the longest window, in full)
     size_t cta_scratch;
     size_t slots;
     PairTable table;  // of Q_m, m = 1..the longest half; a shorter window reads the first
@@ -556,6 +557,17 @@ double items_cost(uint64_t items, uint32_t sms, double groups) {
     return ((double)(per_sm / 4 * 4) + REST[per_sm % 4]) * (20.0 + groups);
 }
 
+// Groups of the longest window an item may have where a step has at most
+// `candidates`: twice what spreads them over the `ctas` CTAs (items_cost asks for
+// longer ones only where an item has less than one group), and no more than
+// `limit` bytes of scratch hold, at least the two groups that retile goes down to.
+uint32_t item_groups(uint64_t candidates, uint32_t ctas, uint32_t max_half, size_t limit) {
+    const uint64_t threads = (uint64_t)ctas * BLOCK;
+    const uint64_t spread = (candidates + threads * 2 * GROUP - 1) / (threads * 2 * GROUP);
+    const uint64_t held = limit / (ctas * cta_scratch_uint4(GROUP, SINK_FULL) * sizeof(uint4));
+    return (uint32_t)std::max<uint64_t>(2, std::min({(uint64_t)std::max(groups_of(max_half), ITEM_GROUPS), 2 * spread, held}));
+}
+
 // Cuts the steps of the searches whose share has changed into items of 128
 // threads. The window is the one that costs least over all searches, each of
 // which takes whole items of it (and shortens its own to use them up). On B200,
@@ -958,15 +970,20 @@ int og_batch_new(int ordinal, const og_batch_config* cfgp, og_batch** out, char*
         int no = 0;
         CU(cudaMemPoolSetAttribute(b->pool, cudaMemPoolReuseAllowInternalDependencies, &no));
     }
-    b->item_half = GROUP * std::max(groups_of(cfg.max_half), ITEM_GROUPS);
-    // a full step's items: CTA_ITEMS a CTA and, as every search rounds to whole
-    // items, one more for each of at most nblocks searches; twice that, as the
-    // items of a search stay while its share does
-    b->places = 2 * (CTA_ITEMS * b->grid + b->nblocks);
+    // 64 bytes a candidate of five blocks an SM at max_half: what a pool without
+    // items of its own would hold
+    size_t limit = 0;
+    CU(scratch_limit((size_t)5 * sms * BLOCK * (2 * (size_t)cfg.max_half + 2) * 64, &limit));
+    b->item_half = GROUP * item_groups(per_step, b->grid, cfg.max_half, limit);
+    // a full step's items: CTA_ITEMS a CTA, or as many as the shortest windows make,
+    // and, as every search rounds to whole items, one more for each of at most
+    // nblocks searches; twice that, as the items of a search stay while its share does
+    const uint64_t shortest = (per_step + BLOCK * (2 * GROUP * 2 + 1) - 1) / (BLOCK * (2 * GROUP * 2 + 1));
+    b->places = 2 * ((uint32_t)std::min<uint64_t>(CTA_ITEMS * b->grid, shortest) + b->nblocks);
     const size_t S = (size_t)b->places * BLOCK;
     CU(b->lanes.alloc(S * 4));
     // the scratch of the persistent CTAs: a CTA uses it for one item at a time
-    const size_t cta_scratch = cta_scratch_uint4(b->item_half);
+    const size_t cta_scratch = cta_scratch_uint4(b->item_half, SINK_FULL);
     CU(b->scratch.alloc((size_t)b->grid * cta_scratch));
     CU(make_pair_table(b->table, b->item_half, b->stream));
     CU(cudaStreamSynchronize(b->stream));

@@ -171,6 +171,15 @@ const std::vector<uint4>& multiples_8g() {
     return table;
 }
 
+// Scratch that a search whose callers' windows would take `own` bytes may hold: those,
+// or a 64th of what is free now, when that is more (2.8 GB of an empty B200).
+cudaError_t scratch_limit(size_t own, size_t* limit) {
+    size_t free_bytes = 0, total = 0;
+    const cudaError_t e = cudaMemGetInfo(&free_bytes, &total);
+    *limit = std::max(own, free_bytes / 64);
+    return e;
+}
+
 // Whether p plus a multiple of 8G can have order four: l p has it then, l the
 // prime order of G.
 static bool may_meet_order_four(const Pt& p) {
@@ -339,27 +348,44 @@ struct Tile {
 // callers' shapes (half 256, 333 and 512) ran 1.90 for 1.9e8 at half 256, 2.43
 // for 7.7e7 (now 1.45), and 3.49. 3.1e9 candidates: 9 rounds 51.7, 6 51.6 with
 // half as much scratch again, 10 (the caller's half 2048) 53.0, 20 53.2.
-constexpr uint32_t MIN_GROUPS = 2, MAX_GROUPS = 768;  // the longest: 5.6 GB of scratch
+//
+// `own` is the scratch that the callers' windows would take on the resident lanes.
+// Windows that take more are cut where scratch_limit says: a search of a small half
+// may run beside many others.
+constexpr uint32_t MIN_GROUPS = 2, MAX_GROUPS = 768;  // the longest: 3.7 GB of scratch, in full 5.6 GB
 constexpr uint32_t MAX_TILE_LANES = 1u << 23;  // 0.5 GB of lane state
 
-int plan_tile(int device, uint64_t batch, SinkKind kind, Tile* out, char* err, size_t errlen) {
+int plan_tile(int device, uint64_t batch, SinkKind kind, size_t own, Tile* out, char* err, size_t errlen) {
     int blocks = 0, sms = 0;
     cudaError_t e = paired_blocks_per_sm(kind, &blocks);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "kernel attributes: %s", cuda_text(e).c_str());
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "device attributes: %s", cuda_text(e).c_str());
     const uint32_t ctas = (uint32_t)std::max(1, blocks) * (uint32_t)sms;
-    const uint64_t threads = (uint64_t)ctas * OG_LB_THREADS, longest = 2 * GROUP * MAX_GROUPS + 1;
-    const uint64_t waves = (batch + threads * longest - 1) / (threads * longest);
-    const uint64_t window = (batch + threads * waves - 1) / (threads * waves);
-    out->half = GROUP * std::max(MIN_GROUPS, (uint32_t)((window + 2 * GROUP - 2) / (2 * GROUP)));
-    const uint64_t slots = 2ULL * out->half + 1, windows = (batch + slots - 1) / slots;
-    const uint64_t rounds = (windows + MAX_TILE_LANES - 1) / MAX_TILE_LANES;
-    if (rounds * slots > 0xffffffffULL) return fail(err, errlen, OG_E_ARG, "too many candidates per advance");
-    out->rounds = (uint32_t)rounds;
-    out->lanes = (uint32_t)((windows + rounds - 1) / rounds);
-    out->grid = std::min(ctas, (out->lanes + OG_LB_THREADS - 1) / OG_LB_THREADS);
-    return OG_OK;
+    const uint64_t threads = (uint64_t)ctas * OG_LB_THREADS;
+    uint64_t most_groups = MAX_GROUPS, most_lanes = MAX_TILE_LANES;
+    for (;;) {
+        const uint64_t longest = 2 * GROUP * most_groups + 1;
+        const uint64_t waves = (batch + threads * longest - 1) / (threads * longest);
+        const uint64_t window = (batch + threads * waves - 1) / (threads * waves);
+        out->half = GROUP * std::max(MIN_GROUPS, (uint32_t)((window + 2 * GROUP - 2) / (2 * GROUP)));
+        const uint64_t slots = 2ULL * out->half + 1, windows = (batch + slots - 1) / slots;
+        uint64_t rounds = (windows + most_lanes - 1) / most_lanes;
+        if (rounds * slots > 0xffffffffULL) rounds = (windows + MAX_TILE_LANES - 1) / MAX_TILE_LANES;
+        if (rounds * slots > 0xffffffffULL) return fail(err, errlen, OG_E_ARG, "too many candidates per advance");
+        out->rounds = (uint32_t)rounds;
+        out->lanes = (uint32_t)((windows + rounds - 1) / rounds);
+        out->grid = std::min(ctas, (out->lanes + OG_LB_THREADS - 1) / OG_LB_THREADS);
+        const size_t scratch = out->grid * cta_scratch_uint4(out->half, kind) * sizeof(uint4);
+        if (scratch <= own || most_groups < MAX_GROUPS) return OG_OK;
+        size_t limit = 0;
+        e = scratch_limit(own, &limit);
+        if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "free memory: %s", cuda_text(e).c_str());
+        if (scratch <= limit) return OG_OK;
+        most_groups = std::max<uint64_t>(MIN_GROUPS, limit / (ctas * cta_scratch_uint4(GROUP, kind) * sizeof(uint4)));
+        if (most_groups >= MAX_GROUPS) return OG_OK;
+        most_lanes = std::min<uint64_t>(MAX_TILE_LANES, std::max<uint64_t>(threads, limit / (4 * sizeof(uint4))));
+    }
 }
 
 // Records one advance may produce: every candidate in dump mode; else what
@@ -480,14 +506,20 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     Tile tile{};
     {
         if (!may_meet_order_four(start_pt)) e->kind = sink_kind(!cfg.dump && bitmap ? bits : 0, suffixed ? f->suffixes.bits() : 0);
-        const int rc = plan_tile(ordinal, batch, e->kind, &tile, err, errlen);
+        uint32_t resident = 0;
+        int rc = resident_lanes(ordinal, cfg.scheme, cfg.block, &resident, err, errlen, lpt);
+        if (rc) return rc;
+        // a prefix product and its denominator, 64 bytes, per lane and candidate
+        const size_t own = cfg.scheme == OG_SCHEME_CHAIN ? (size_t)std::min(resident, cfg.lanes) * cfg.half * 64
+                                                         : (size_t)resident * (2 * (size_t)cfg.half + 2) * 64;
+        rc = plan_tile(ordinal, batch, e->kind, own, &tile, err, errlen);
         if (rc) return rc;
         e->grid = tile.grid;
     }
     e->cap = cfg.room ? cfg.room : room_for(batch, cfg.dump != 0, occupancy);
     e->cfg.room = (uint32_t)std::min<size_t>(e->cap, 0xffffffffu);
     CU(e->lanes.alloc((size_t)tile.lanes * 4));
-    CU(e->scratch.alloc((size_t)tile.grid * cta_scratch_uint4(tile.half)));
+    CU(e->scratch.alloc((size_t)tile.grid * cta_scratch_uint4(tile.half, e->kind)));
     for (og_engine::Flight& f : e->fl) {
         CU(f.counts.alloc(COUNTS));
         CU(f.hits.alloc(e->cap));

@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) paired_kernel
     const Sink sink{a.bitmap, a.bits,   a.hits,  a.counter, a.cap,     a.search,          a.sbitmap,
                     a.sbits,  a.failed, a.limit, a.lanes_n, 2 * a.half + 1};
     const PairTable tab = pair_table_at(a.table, a.half);
-    uint4* const scr = a.scratch + (size_t)blockIdx.x * cta_scratch_uint4(a.half) + threadIdx.x;
+    uint4* const scr = a.scratch + (size_t)blockIdx.x * cta_scratch_uint4(a.half, Kind) + threadIdx.x;
     MatrixUnit mu;
     RoundShared* sh = nullptr;
     if constexpr (Kind != SINK_FULL) {

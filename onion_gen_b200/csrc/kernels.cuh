@@ -88,12 +88,6 @@ __host__ __device__ PairTable pair_table_at(T* base, uint32_t half) {
     const size_t g = groups_of(half);
     return PairTable{base, base + g * GROUP * 2, base + g * GROUP * 6, base + g * (GROUP * 6 + 6)};
 }
-// uint4 of a CTA's scratch: per group a prefix product and E, per thread; or
-// per pair a prefix product (paired_rounds_full).
-__host__ __device__ constexpr size_t cta_scratch_uint4(uint32_t half) {
-    return (size_t)groups_of(half) * GROUP * 2 * SCRATCH_ROW;
-}
-
 // How a sink's keys are tested: by paired_rounds, whose matrix product gives a
 // key's low 24 bits and its bits from 231 on, or in full. A suffix bitmap of 24
 // bits reads one bit more, and paired_rounds looks both of its values up: twice
@@ -105,10 +99,16 @@ __host__ __device__ inline SinkKind sink_kind(uint32_t prefix_bits, uint32_t suf
     return suffix_bits ? SINK_SUFFIX : SINK_PREFIX;
 }
 
+// uint4 of a CTA's scratch: paired_rounds keeps a prefix product and E per group and
+// thread, paired_rounds_full a prefix product per pair.
+__host__ __device__ constexpr size_t cta_scratch_uint4(uint32_t half, SinkKind kind) {
+    return (size_t)groups_of(half) * (kind == SINK_FULL ? 2 * GROUP : 4) * SCRATCH_ROW;
+}
+
 struct PairedArgs {
     const uint4* table;      // PairTable of Q_m, m = 1..half (pair_table_at)
     uint4* lanes;            // affine centres: ({x,y} * 2 + q) * L + lane
-    uint4* scratch;          // cta_scratch_uint4(half) per CTA
+    uint4* scratch;          // cta_scratch_uint4(half, kind) per CTA
     uint32_t* work;          // next block of lanes to take, zero at launch
     const uint32_t* bitmap;  // prefix bitmap as 32-bit words (nullptr: none)
     uint32_t bits;

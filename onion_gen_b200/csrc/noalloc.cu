@@ -53,18 +53,20 @@ struct NoAllocTile {
 
 // uint4 the array holds for a tile: the PairTable, the lane centres (four a
 // lane) and the CTAs' scratch.
-size_t tile_uint4(uint32_t half, uint32_t ctas) {
-    return pair_table_uint4(half) + (size_t)ctas * (NBLOCK * 4 + cta_scratch_uint4(half));
+size_t tile_uint4(uint32_t half, uint32_t ctas, SinkKind kind) {
+    return pair_table_uint4(half) + (size_t)ctas * (NBLOCK * 4 + cta_scratch_uint4(half, kind));
 }
 
 // All `resident` blocks, in one round where the array holds the scratch of
 // windows that long, else in as many as it takes (a round's own cost is that of
-// about 20 groups of three pairs, so the longest windows that fit). Windows of
-// at least two groups.
-NoAllocTile plan_tile(uint64_t candidates, uint32_t resident) {
+// about 20 groups of three pairs, so the longest windows that fit: on 592 CTAs 12
+// groups; while room was kept to compute every key in full, 8, and 4.05e7 candidates
+// took 1.77 ms for 1.60). Windows of at least two groups.
+NoAllocTile plan_tile(uint64_t candidates, uint32_t resident, SinkKind kind) {
     const uint64_t threads = (uint64_t)resident * NBLOCK, window = (candidates + threads - 1) / threads;
     uint32_t groups = 2;
-    while (2ULL * GROUP * groups + 1 < window && tile_uint4(GROUP * (groups + 1), resident) * sizeof(uint4) <= SCRATCH_BYTES)
+    while (2ULL * GROUP * groups + 1 < window &&
+           tile_uint4(GROUP * (groups + 1), resident, kind) * sizeof(uint4) <= SCRATCH_BYTES)
         groups++;
     NoAllocTile t{GROUP * groups, resident, 1};
     const uint64_t lane = 2ULL * t.half + 1;
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(NBLOCK, 4) noalloc_paired_kernel(const NoAlloc
                     0,        nullptr, a.limit,   a.lanes_n,       2 * a.half + 1, a.out_lanes,
                     a.out_slots};
     const PairTable tab = pair_table_at<const uint4>(a.table, a.half);
-    uint4* const scr = a.scratch + (size_t)blockIdx.x * cta_scratch_uint4(a.half) + threadIdx.x;
+    uint4* const scr = a.scratch + (size_t)blockIdx.x * cta_scratch_uint4(a.half, Narrow ? SINK_PREFIX : SINK_FULL) + threadIdx.x;
     if constexpr (Narrow) {
         __shared__ __align__(128) RoundShared sh;
         MatrixUnit mu;
@@ -251,7 +253,8 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
         base = g_addr[ordinal];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool narrow = sink_kind(d_bitmap ? bits : 0, 0) == SINK_PREFIX;
+    const SinkKind kind = sink_kind(d_bitmap ? bits : 0, 0);
+    const bool narrow = kind == SINK_PREFIX;
     const uint32_t slots = 2 * half + 1;
     const uint64_t candidates = (uint64_t)lanes * rounds * slots;
     int per_sm = 0, sms = 0;
@@ -259,7 +262,7 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, noalloc_paired_kernel<false>, NBLOCK, 0);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ordinal);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "device attributes: %s", cuda_text(e).c_str());
-    const NoAllocTile tile = plan_tile(candidates, (uint32_t)(std::max(1, per_sm) * sms));
+    const NoAllocTile tile = plan_tile(candidates, (uint32_t)(std::max(1, per_sm) * sms), kind);
     const uint32_t window = 2 * tile.half + 1;
     if ((uint64_t)tile.rounds * window > 0xffffffffULL) return fail(err, errlen, OG_E_ARG, "too many rounds");
     NoAllocArgs a;
