@@ -57,10 +57,11 @@ static void batch_affine(const std::vector<Pt>& pts, std::vector<F51>& xs, std::
     }
 }
 
-// 1/d and d of the curve, for the paired round's table and strides.
-static const F51& inv_curve_d() {
-    static const F51 v = f_inv(curve_d());
-    return v;
+// An affine point in cached form (y + x, y - x, 2 d x y), device layout.
+static void put_cached(uint4* d, const F51& x, const F51& y) {
+    put_fe(d + 0, 1, f_add(y, x));
+    put_fe(d + 2, 1, f_sub(y, x));
+    put_fe(d + 4, 1, f_mul(f_mul(x, y), curve_2d()));
 }
 
 // A stride of the paired round.
@@ -70,79 +71,30 @@ Stride stride_of(const Pt& w) {
     return Stride{to_words(x), to_words(y), to_words(f_mul(curve_d(), f_mul(x, y)))};
 }
 
-// The per-entry part of a PairTable for Q_m = 8m G, m = 1..n, n a power of two
-// (q = 1/(d y^2) of every entry, then v = 1/y and s = x/(1 + x^2) of every
-// entry), in the device layout. The same for every search and half, so built
-// once per power of two and kept: 96 bytes an entry. y and 1 + x^2 are never 0
-// for a point of odd order.
-static const std::vector<uint4>& pair_entries(uint32_t n) {
-    static std::mutex mu;
-    static std::map<uint32_t, std::unique_ptr<std::vector<uint4>>> cache;
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(n);
-    if (it != cache.end()) return *it->second;
-    std::vector<Pt> pts(n);
-    const Pt eight = base_mult_u64(8);
-    Pt p = eight;
-    for (uint32_t m = 0; m < n; m++) {
-        pts[m] = p;
-        p = pt_add(p, eight);
+// The Pow2Table of p, with one inversion.
+Pow2Table pow2_table(Pt p) {
+    std::vector<Pt> pts(POW2);
+    for (Pt& at : pts) {
+        at = p;
+        p = pt_dbl(p);
     }
     std::vector<F51> xs, ys;
     batch_affine(pts, xs, ys);
-    // 1 / (y (1 + x^2)) of all entries with one inversion
-    std::vector<F51> prefix(n), den(n);
-    F51 run = f_one();
-    for (uint32_t m = 0; m < n; m++) {
-        den[m] = f_add(f_one(), f_sq(xs[m]));
-        prefix[m] = run;
-        run = f_mul(run, f_mul(ys[m], den[m]));
-    }
-    F51 inv = f_inv(run);
-    auto tab = std::make_unique<std::vector<uint4>>((size_t)n * 6);
-    for (uint32_t m = n; m-- > 0;) {
-        const F51 i = f_mul(inv, prefix[m]);
-        inv = f_mul(inv, f_mul(ys[m], den[m]));
-        const F51 v = f_mul(den[m], i);
-        put_fe(tab->data() + (size_t)m * 2, 1, f_mul(f_sq(v), inv_curve_d()));
-        uint4* const vs = tab->data() + (size_t)n * 2 + (size_t)m * 4;
-        put_fe(vs + 0, 1, v);
-        put_fe(vs + 2, 1, f_mul(xs[m], f_mul(ys[m], i)));
-    }
-    auto& ref = *tab;
-    cache[n] = std::move(tab);
-    return ref;
+    Pow2Table t;
+    for (uint32_t k = 0; k < POW2; k++) put_cached(t.v + k * 6, xs[k], ys[k]);
+    return t;
 }
 
-// A device PairTable for half `half`, its entries copied and its groups
-// computed on `s`.
+// That of 8G, the same in every search.
+const Pow2Table& powers_of_8g() {
+    static const Pow2Table table = pow2_table(base_mult_u64(8));
+    return table;
+}
+
+// A device PairTable for half `half`, computed on `s`.
 cudaError_t make_pair_table(DevBuf<uint4>& table, uint32_t half, cudaStream_t s) {
-    cudaError_t e = table.alloc(pair_table_uint4(half));
-    if (e != cudaSuccess) return e;
-    // whole groups, so up to two entries past `half`
-    const size_t n = (size_t)groups_of(half) * GROUP;
-    uint32_t built = 256;
-    while (built < n) built *= 2;
-    const std::vector<uint4>& tab = pair_entries(built);
-    e = cudaMemcpyAsync(table.p, tab.data(), n * 2 * sizeof(uint4), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(table.p + n * 2, tab.data() + (size_t)built * 2, n * 4 * sizeof(uint4), cudaMemcpyHostToDevice, s);
-    return e == cudaSuccess ? launch_group_table(table.p, half, s) : e;
-}
-
-// 2^k * stride for k < nbits in cached form (y+x, y-x, 2dxy), device layout.
-std::vector<uint4> pow2_table(const Pt& stride, uint32_t nbits) {
-    std::vector<uint4> out((size_t)std::max<uint32_t>(nbits, 1) * 6);
-    Pt p = stride;
-    for (uint32_t k = 0; k < nbits; k++) {
-        const Niels c = pt_niels(p);
-        uint4* d = out.data() + (size_t)k * 6;
-        put_fe(d + 0, 1, c.ypx);
-        put_fe(d + 2, 1, c.ymx);
-        put_fe(d + 4, 1, c.xy2d);
-        p = pt_dbl(p);
-    }
-    return out;
+    const cudaError_t e = table.alloc(pair_table_uint4(half));
+    return e == cudaSuccess ? launch_pair_table(table.p, half, powers_of_8g(), s) : e;
 }
 
 // The table of add_multiple_8g, the same for every search: built once.
@@ -161,11 +113,7 @@ const std::vector<uint4>& multiples_8g() {
         std::vector<F51> xs, ys;
         batch_affine(pts, xs, ys);
         std::vector<uint4> out(pts.size() * 6);
-        for (size_t i = 0; i < pts.size(); i++) {
-            put_fe(out.data() + i * 6 + 0, 1, f_add(ys[i], xs[i]));
-            put_fe(out.data() + i * 6 + 2, 1, f_sub(ys[i], xs[i]));
-            put_fe(out.data() + i * 6 + 4, 1, f_mul(f_mul(xs[i], ys[i]), curve_2d()));
-        }
+        for (size_t i = 0; i < pts.size(); i++) put_cached(out.data() + i * 6, xs[i], ys[i]);
         return out;
     }();
     return table;
@@ -187,12 +135,6 @@ static bool may_meet_order_four(const Pt& p) {
                                   0xa2, 0xde, 0xf9, 0xde, 0x14, 0,    0,    0,    0,    0,    0,
                                   0,    0,    0,    0,    0,    0,    0,    0,    0,    0x10};
     return f_is_zero(point_mult(p, l).Y);
-}
-
-uint32_t bits_for(uint64_t v) {
-    uint32_t b = 0;
-    while (b < 64 && (v >> b) != 0) b++;
-    return b;
 }
 
 static_assert(FilterSet::PATTERN_ROW == PATTERN_WORDS, "pattern rows: host and device layouts agree");
@@ -247,7 +189,7 @@ struct og_engine {
     uint64_t launches = 0;
     float last_ms = 0;
     bool overflowed = false;
-    DevBuf<uint4> lanes, scratch, table, pow2;
+    DevBuf<uint4> lanes, scratch, table;
     DevBuf<uint32_t> bitmap;
     // Two advances can be in flight (og_engine_launch / og_engine_collect):
     // each has its own record buffers and counters, so the host can read one
@@ -545,20 +487,15 @@ int build_engine(int ordinal, const uint8_t start[128], og_engine_config cfg, co
     // past it (paired), and a window's centre its candidate `half`
     const uint32_t window = 2 * tile.half + 1, offset = cfg.scheme == OG_SCHEME_PAIRED ? 1 : 0;
     const Pt base = pt_add(start_pt, base_mult_u64(8ULL * (tile.half + offset)));
-    const uint32_t nbits = bits_for(tile.lanes - 1);
-    std::vector<uint4> pw = pow2_table(base_mult_u64(8ULL * window), nbits);
-    CU(e->pow2.alloc(pw.size()));
-    CU(cudaMemcpyAsync(e->pow2.p, pw.data(), pw.size() * sizeof(uint4), cudaMemcpyHostToDevice, e->stream));
+    static_assert(MAX_TILE_LANES <= 1u << POW2, "a lane's number has POW2 bits");
     InitArgs ia{};
     ia.lanes = e->lanes.p;
     ia.bx = to_words(base.X);
     ia.by = to_words(base.Y);
     ia.bz = to_words(base.Z);
     ia.bt = to_words(base.T);
-    ia.pow2 = e->pow2.p;
-    ia.nbits = nbits;
     ia.lanes_n = tile.lanes;
-    CU(launch_init(ia, e->stream));
+    CU(launch_init(ia, pow2_table(base_mult_u64(8ULL * window)), e->stream));
     CU(make_pair_table(e->table, tile.half, e->stream));
     PairedArgs& a = e->pa;
     a.table = e->table.p;

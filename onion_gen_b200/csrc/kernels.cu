@@ -19,22 +19,9 @@ namespace og {
 
 namespace {
 
-__global__ void __launch_bounds__(OG_LB_THREADS) init_kernel(const InitArgs a) {
-    const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t L = a.lanes_n;
-    fe X = words_fe(a.bx), Y = words_fe(a.by), Z = words_fe(a.bz), T = words_fe(a.bt);
-    for (uint32_t k = 0; k < a.nbits; k++) {
-        if ((lane >> k) & 1u) {
-            const uint4* p = a.pow2 + (size_t)k * 6;
-            const fe ypx = load_fe(p + 0, 1), ymx = load_fe(p + 2, 1), t2d = load_fe(p + 4, 1);
-            add_cached(X, Y, Z, T, ypx, ymx, t2d);
-        }
-    }
-    const fe zi = block_invert(Z);  // Z is never 0
-    if (lane < a.lanes_n) {
-        store_fe(a.lanes + 0 * L + lane, L, fe_mulv(X, zi));
-        store_fe(a.lanes + 2 * L + lane, L, fe_mulv(Y, zi));
-    }
+__global__ void __launch_bounds__(OG_LB_THREADS) init_kernel(const InitArgs a, const Pow2Table stride) {
+    first_centre(words_fe(a.bx), words_fe(a.by), words_fe(a.bz), words_fe(a.bt), stride,
+                 blockIdx.x * blockDim.x + threadIdx.x, a.lanes, a.lanes_n);
 }
 
 // The search, bound by the multiply-add pipe. Persistent: each CTA takes the
@@ -73,6 +60,12 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) paired_kernel
             paired_rounds_full<true>(centre, L, a.between, a.last, tab, a.half, a.rounds, scr, sink, lane, active);
     }
     if constexpr (Kind != SINK_FULL) matrix_close(*sh);
+}
+
+// The per-entry part of a PairTable.
+__global__ void __launch_bounds__(OG_LB_THREADS) pair_entry_kernel(uint4* table, uint32_t half, const Pow2Table eight) {
+    fill_pair_entry(pair_table_at<const uint4>(table, half), groups_of(half) * GROUP, eight,
+                    blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // The per-group part of a PairTable whose q, v and s are in place.
@@ -122,8 +115,8 @@ cudaError_t launch_match(const MatchArgs& a, int grid, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_init(const InitArgs& a, cudaStream_t s) {
-    init_kernel<<<(a.lanes_n + OG_LB_THREADS - 1) / OG_LB_THREADS, OG_LB_THREADS, 0, s>>>(a);
+cudaError_t launch_init(const InitArgs& a, const Pow2Table& stride, cudaStream_t s) {
+    init_kernel<<<(a.lanes_n + OG_LB_THREADS - 1) / OG_LB_THREADS, OG_LB_THREADS, 0, s>>>(a, stride);
     return cudaGetLastError();
 }
 
@@ -138,7 +131,8 @@ cudaError_t launch_paired(const PairedArgs& a, SinkKind kind, int grid, cudaStre
     return cudaGetLastError();
 }
 
-cudaError_t launch_group_table(uint4* table, uint32_t half, cudaStream_t s) {
+cudaError_t launch_pair_table(uint4* table, uint32_t half, const Pow2Table& eight, cudaStream_t s) {
+    pair_entry_kernel<<<(groups_of(half) * GROUP + OG_LB_THREADS - 1) / OG_LB_THREADS, OG_LB_THREADS, 0, s>>>(table, half, eight);
     group_table_kernel<<<(groups_of(half) * 36 + 127) / 128, 128, 0, s>>>(table, half);
     return cudaGetLastError();
 }

@@ -56,6 +56,14 @@ struct FeWords {
     uint32_t v[8];
 };
 
+// 2^k p for k < POW2 in cached form (y + x, y - x, 2 d x y; Z = 1), passed to
+// kernels by value as a launch parameter (2304 bytes), so that nothing is copied
+// from host memory for it.
+constexpr uint32_t POW2 = 24;
+struct Pow2Table {
+    uint4 v[POW2 * 6];  // (k * 3 + {ypx,ymx,t2d}) * 2 + q
+};
+
 // A stride W between centres: affine x and y, and d x y.
 struct Stride {
     FeWords x, y, dt;
@@ -128,13 +136,10 @@ struct PairedArgs {
 };
 
 // Lane start points: lane l starts at base + l * stride, affine, built from
-// the binary expansion of l over `pow2` = { 2^k stride } in cached form with
-// Z = 1 (y+x, y-x, 2dxy).
+// the binary expansion of l over the Pow2Table of the stride.
 struct InitArgs {
     uint4* lanes;            // ({x,y} * 2 + q) * L + lane
     FeWords bx, by, bz, bt;  // base point, extended
-    const uint4* pow2;       // (k * 3 + {ypx,ymx,t2d}) * 2 + q
-    uint32_t nbits;
     uint32_t lanes_n;
 };
 
@@ -185,15 +190,15 @@ struct MatchArgs {
     uint32_t* mismatch;        // survivors whose recomputed key differs from their record
 };
 
-cudaError_t launch_init(const InitArgs& a, cudaStream_t s);
+cudaError_t launch_init(const InitArgs& a, const Pow2Table& stride, cudaStream_t s);
 cudaError_t launch_match(const MatchArgs& a, int grid, cudaStream_t s);
 // The search kernel is persistent: `grid` CTAs of OG_LB_THREADS (at most the
 // resident ones) take the lanes a block at a time from `work`, so the scratch
 // covers only the lanes in flight and no SM idles in a tail wave.
 // `kind` is that of its bitmaps, or SINK_FULL, which takes any bitmaps and any start.
 cudaError_t launch_paired(const PairedArgs& a, SinkKind kind, int grid, cudaStream_t s);
-// Completes a PairTable whose per-entry part is on the device.
-cudaError_t launch_group_table(uint4* table, uint32_t half, cudaStream_t s);
+// Writes a PairTable of `half` from the Pow2Table of 8G.
+cudaError_t launch_pair_table(uint4* table, uint32_t half, const Pow2Table& eight, cudaStream_t s);
 
 // Resident blocks per SM of the search kernel.
 cudaError_t paired_blocks_per_sm(SinkKind kind, int* blocks);

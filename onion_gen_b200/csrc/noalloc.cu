@@ -27,14 +27,15 @@
 
 namespace og {
 
-Stride stride_of(const Pt& w);  // engine.cu
+Stride stride_of(const Pt& w);    // engine.cu
+Pow2Table pow2_table(Pt p);       // engine.cu
+const Pow2Table& powers_of_8g();  // engine.cu
 
 namespace {
 
 constexpr size_t SCRATCH_BYTES = OG_NOALLOC_SCRATCH_BYTES;
 constexpr uint32_t NBLOCK = 128;
 static_assert(NBLOCK == SCRATCH_ROW, "a row of a CTA's scratch holds its threads");
-constexpr uint32_t POW2 = 24;
 constexpr int MAX_DEVICES = 64;
 
 static __device__ __align__(256) uint4 og_noalloc_scratch[SCRATCH_BYTES / sizeof(uint4)];
@@ -75,20 +76,11 @@ NoAllocTile plan_tile(uint64_t candidates, uint32_t resident, SinkKind kind) {
     return t;
 }
 
-// 2^k p for k < POW2 in cached form (y + x, y - x, 2 d x y; Z = 1), passed to
-// the kernels by value as a launch parameter (2304 bytes), so that the call
-// copies nothing from host memory: a host-to-device copy from pageable
-// memory would wait for the work already queued on the caller's stream.
-struct Pow2Table {
-    uint4 v[POW2 * 6];
-};
-
 struct NoAllocArgs {
     uint4* table;
     uint4* lanes;
     uint4* scratch;
     FeWords bx, by, bz, bt;  // first centre, extended
-    FeWords ex, ey, ez, et;  // 8G, extended (table entry 1)
     Stride stride;           // between rounds
     uint64_t limit;          // candidates
     uint32_t out_lanes;      // the caller's shape, in which the records are numbered
@@ -104,52 +96,18 @@ struct NoAllocArgs {
     uint32_t rounds;
 };
 
-// The per-entry part of the PairTable of Q_m = m * 8G, m = 1.. in whole
-// groups. Entry m - 1 starts from 8G and adds 2^k * 8G (from `pow8`) for every
-// bit k of m - 1.
-__device__ __forceinline__ void table_entry(const NoAllocArgs& a, const Pow2Table& pow8, uint32_t thread) {
-    const uint32_t n = groups_of(a.half) * GROUP, m = min(thread, n - 1);
-    fe X = words_fe(a.ex), Y = words_fe(a.ey), Z = words_fe(a.ez), T = words_fe(a.et);
-    for (uint32_t k = 0; k < POW2; k++)
-        if ((m >> k) & 1u) {
-            const uint4* p = pow8.v + (size_t)k * 6;
-            add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
-        }
-    // of the affine (x, y): v = 1/y = Z (Z^2 + X^2) i, s = x / (1 + x^2) = X Y Z i and
-    // q = v^2 / d, with i = 1 / (Y (Z^2 + X^2))
-    const fe den = fe_add(fe_sqv(Z), fe_sqv(X));
-    const fe zi = fe_mulv(Z, block_invert(fe_mulv(Y, den)));
-    const fe v = fe_canon(fe_mulv(den, zi));
-    if (thread >= n) return;
-    store_fe(a.table + (size_t)m * 2, 1, fe_canon(fe_mulv(fe_sqv(v), const_inv_d())));
-    uint4* const vs = a.table + (size_t)n * 2 + (size_t)m * 4;
-    store_fe(vs + 0, 1, v);
-    store_fe(vs + 2, 1, fe_canon(fe_mulv(fe_mulv(X, Y), zi)));
-}
-
-// Lane l starts on the centre of window l: the first centre plus 2^k times
-// the lane stride (from `pow2`) for every bit k of l.
-__device__ __forceinline__ void first_centre(const NoAllocArgs& a, const Pow2Table& pow2, uint32_t lane) {
-    const size_t L = a.lanes_n;
-    fe X = words_fe(a.bx), Y = words_fe(a.by), Z = words_fe(a.bz), T = words_fe(a.bt);
-    for (uint32_t k = 0; k < POW2; k++)
-        if ((lane >> k) & 1u) {
-            const uint4* p = pow2.v + (size_t)k * 6;
-            add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
-        }
-    const fe zi = block_invert(Z);
-    store_fe(a.lanes + 0 * L + lane, L, fe_mulv(X, zi));
-    store_fe(a.lanes + 2 * L + lane, L, fe_mulv(Y, zi));
-}
-
 // The table's entries on the first blocks, the lanes' first centres on the
-// others: neither needs the other.
-__global__ void __launch_bounds__(NBLOCK) noalloc_start_kernel(const NoAllocArgs a, const Pow2Table pow8,
-                                                               const Pow2Table pow2) {
+// others: neither needs the other. The power tables travel as launch parameters: a
+// copy from pageable host memory would wait for the work already queued on the
+// caller's stream.
+__global__ void __launch_bounds__(NBLOCK) noalloc_start_kernel(const NoAllocArgs a, const Pow2Table eight,
+                                                               const Pow2Table stride) {
     if (blockIdx.x < a.table_blocks)
-        table_entry(a, pow8, blockIdx.x * NBLOCK + threadIdx.x);
+        fill_pair_entry(pair_table_at<const uint4>(a.table, a.half), groups_of(a.half) * GROUP, eight,
+                        blockIdx.x * NBLOCK + threadIdx.x);
     else
-        first_centre(a, pow2, (blockIdx.x - a.table_blocks) * NBLOCK + threadIdx.x);
+        first_centre(words_fe(a.bx), words_fe(a.by), words_fe(a.bz), words_fe(a.bt), stride,
+                     (blockIdx.x - a.table_blocks) * NBLOCK + threadIdx.x, a.lanes, a.lanes_n);
 }
 
 // The production paired kernel with its scratch in the file-scope array; the
@@ -181,37 +139,6 @@ __global__ void __launch_bounds__(NBLOCK) noalloc_groups_kernel(const NoAllocArg
 // The array's device address, per device, taken on the first call there.
 std::mutex g_mu;
 uint4* g_addr[MAX_DEVICES];
-
-// 2^k * p for k < POW2 in cached form, with one inversion.
-void pow2_into(Pt p, uint4* out) {
-    Pt pts[POW2];
-    F51 prefix[POW2], run = f_one();
-    for (uint32_t k = 0; k < POW2; k++) {
-        pts[k] = p;
-        prefix[k] = run;
-        run = f_mul(run, p.Z);
-        p = pt_dbl(p);
-    }
-    F51 inv = f_inv(run);
-    for (uint32_t k = POW2; k-- > 0;) {
-        const F51 zi = f_mul(inv, prefix[k]);
-        inv = f_mul(inv, pts[k].Z);
-        const F51 x = f_mul(pts[k].X, zi), y = f_mul(pts[k].Y, zi);
-        put_fe(out + k * 6 + 0, 1, f_add(y, x));
-        put_fe(out + k * 6 + 2, 1, f_sub(y, x));
-        put_fe(out + k * 6 + 4, 1, f_mul(f_mul(x, y), curve_2d()));
-    }
-}
-
-// 2^k * 8G, the same in every call.
-const Pow2Table& eight_powers() {
-    static const Pow2Table table = [] {
-        Pow2Table t;
-        pow2_into(base_mult_u64(8), t.v);
-        return t;
-    }();
-    return table;
-}
 
 }  // namespace
 }  // namespace og
@@ -274,17 +201,12 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
     a.lanes = a.table + pair_table_uint4(tile.half);
     a.scratch = a.lanes + (size_t)a.lanes_n * 4;
     // constants computed on the host and passed as launch parameters: the
-    // first centre, 8G, the round stride
+    // first centre and the round stride
     const Pt first = pt_add(A, base_mult_u64(8ULL * (tile.half + 1)));
     a.bx = to_words(first.X);
     a.by = to_words(first.Y);
     a.bz = to_words(first.Z);
     a.bt = to_words(first.T);
-    const Pt eight = base_mult_u64(8);
-    a.ex = to_words(eight.X);
-    a.ey = to_words(eight.Y);
-    a.ez = to_words(eight.Z);
-    a.et = to_words(eight.T);
     a.stride = stride_of(base_mult_u64(8ULL * window * a.lanes_n));
     a.limit = candidates;
     a.out_lanes = lanes;
@@ -296,13 +218,11 @@ extern "C" int og_search_noalloc(int ordinal, const uint8_t start[128], uint32_t
     a.cap = cap;
     const uint32_t groups = groups_of(tile.half);
     a.table_blocks = (groups * GROUP + NBLOCK - 1) / NBLOCK;
-    // the two power-of-two tables travel as launch parameters
-    Pow2Table pow2;
-    pow2_into(base_mult_u64(8ULL * window), pow2.v);
     // the counter starts at zero on every call
     e = cudaMemsetAsync(d_count, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return fail(err, errlen, OG_E_DEVICE, "memset: %s", cuda_text(e).c_str());
-    noalloc_start_kernel<<<a.table_blocks + tile.ctas, NBLOCK, 0, s>>>(a, eight_powers(), pow2);
+    noalloc_start_kernel<<<a.table_blocks + tile.ctas, NBLOCK, 0, s>>>(
+        a, powers_of_8g(), pow2_table(base_mult_u64(8ULL * window)));
     if (narrow) {
         noalloc_groups_kernel<<<(groups * 36 + NBLOCK - 1) / NBLOCK, NBLOCK, 0, s>>>(a);
         noalloc_paired_kernel<true><<<tile.ctas, NBLOCK, 0, s>>>(a);

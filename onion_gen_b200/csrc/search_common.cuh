@@ -778,6 +778,45 @@ __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride
     }
 }
 
+// p (extended) plus k times the point of a Pow2Table, k < 2^POW2.
+__device__ __forceinline__ void add_multiple(fe& X, fe& Y, fe& Z, fe& T, const Pow2Table& table, uint32_t k) {
+    for (const uint4* p = table.v; k; k >>= 1, p += 6)
+        if (k & 1u) add_cached(X, Y, Z, T, load_fe(p + 0, 1), load_fe(p + 2, 1), load_fe(p + 4, 1));
+}
+
+// Entry m of the per-entry part of a PairTable of `n` entries, Q_m+1 = 8 (m + 1) G
+// from the Pow2Table of 8G, m the thread's number. Every thread of the block calls
+// it; those past the table write nothing.
+__device__ __forceinline__ void fill_pair_entry(const PairTable& tab, uint32_t n, const Pow2Table& eight, uint32_t thread) {
+    const uint32_t m = min(thread, n - 1);
+    fe X = fe_zero(), Y = fe_one(), Z = fe_one(), T = fe_zero();
+    add_multiple(X, Y, Z, T, eight, m + 1);
+    // of the affine (x, y): v = 1/y = Z (Z^2 + X^2) i, s = x / (1 + x^2) = X Y Z i and
+    // q = v^2 / d, with i = 1 / (Y (Z^2 + X^2)); y and 1 + x^2 are never 0 for a point
+    // of odd order
+    const fe den = fe_add(fe_sqv(Z), fe_sqv(X));
+    const fe zi = fe_mulv(Z, block_invert(fe_mulv(Y, den)));
+    const fe v = fe_canon(fe_mulv(den, zi));
+    if (thread >= n) return;
+    store_fe(const_cast<uint4*>(tab.q) + (size_t)m * 2, 1, fe_canon(fe_mulv(fe_sqv(v), const_inv_d())));
+    uint4* const vs = const_cast<uint4*>(tab.vs) + (size_t)m * 4;
+    store_fe(vs + 0, 1, v);
+    store_fe(vs + 2, 1, fe_canon(fe_mulv(fe_mulv(X, Y), zi)));
+}
+
+// The affine centre of lane `lane`: a base point (extended) plus that many times
+// the point of a Pow2Table. Every thread of the block calls it.
+__device__ __forceinline__ void first_centre(fe X, fe Y, fe Z, fe T, const Pow2Table& stride, uint32_t lane,
+                                             uint4* lanes, uint32_t lanes_n) {
+    const size_t L = lanes_n;
+    add_multiple(X, Y, Z, T, stride, lane);
+    const fe zi = block_invert(Z);  // Z is never 0
+    if (lane < lanes_n) {
+        store_fe(lanes + 0 * L + lane, L, fe_mulv(X, zi));
+        store_fe(lanes + 2 * L + lane, L, fe_mulv(Y, zi));
+    }
+}
+
 // Fills the per-group part of a PairTable from its q, v and s, one thread for
 // each (group, key, element) of six keys and six elements; the threads of
 // element 0 and key 0 write the cubic. `tab` is the table being written.
