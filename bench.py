@@ -98,8 +98,6 @@ def parse():
                    "suffix-small: three advances of a forty-suffix search with the device match; "
                    "chain-small: three advances of the chain scheme at its default shape; "
                    "config3-small: three advances of config 3's 10,000-prefix search at its default shape")
-    p.add_argument("--lanes-per-thread", type=int, default=1,
-                   help="lanes each thread of the paired search kernel carries in --case small (1 or 2)")
     p.add_argument("--half", type=int, default=0,
                    help=f"inversion batch half-width (default {HALF} for the plain line, 256 for --case small, "
                    f"{SHORT_HALF} for the batch's profiling case)")
@@ -349,7 +347,7 @@ def batched_leg(dev, shape, cap, kernel_rate):
                    "candidates_per_advance": tuned.lanes * (2 * tuned.half + 1) * tuned.rounds}
     plain_tuned, arm_tuned = plain_arm(dev, searches, None, True)
     log(f"batched leg: plain engine (tuned shape {tuned_shape}) {len(searches)} searches in {arm_tuned['wall_s']:.2f} s")
-    # the same loop with a short round (half 256, two waves of resident
+    # the same loop with a short round (half 256, two waves of
     # blocks: 9.7e7 candidates an advance), which overshoots a small quota
     # less, and the exact match on the device, as the batch has it
     short = N.EngineConfig(N.SCHEME_PAIRED, SHORT_HALF, 2 * gpu.resident_lanes(dev), 1, 128, 0, 0)
@@ -485,8 +483,8 @@ def serving_leg(dev, shape, n, cap_s):
         "p99_censored": c99,
         "ttf_note": "percentiles over all submitted requests; a request unfinished at the cap counts with its "
         "elapsed time (cap end - arrival), a lower bound, and a percentile that lands on one is marked censored. "
-        "The mix's expected work (2.4e13 candidates, 20 minutes of one GPU) is about 30 times what arrives per "
-        "second of capacity, so its longest requests cannot finish within the cap",
+        "The mix's expected work (2.4e13 candidates) takes one GPU about seven minutes and arrives over 40 s, so its "
+        "longest requests cannot finish within the cap",
         "keys_per_s": st.candidates / elapsed,
         "device_busy": st.device_ms / 1e3 / elapsed,
         "steps": int(st.steps),
@@ -586,18 +584,17 @@ def small_case(args):
 
     dev = gpu.look()[0]
     half = args.half or 256
-    lpt = args.lanes_per_thread
     fs = F.FilterSet.parse_all([workloads.config2_prefix()])
     words, bits = fs.index_words()
     start = key.start_point(workloads.seed(0))
     # lanes 0: the engine's default waves
     eng = gpu.Engine(dev, start, bitmap=words, bitmap_bits=bits,
-                     config=N.EngineConfig(0, half, 0, 1, 128, 0, 0, lpt))
+                     config=N.EngineConfig(0, half, 0, 1, 128, 0, 0))
     lanes = eng.threads()
     for i in range(3):
         o, _ = eng.advance_raw()
         ms = eng.last_kernel_ms()
-        print(f"advance {i}: half {half}, {lanes} lanes ({lpt} a thread), {len(o)} survivors, kernel {ms:.3f} ms, "
+        print(f"advance {i}: half {half}, {lanes} lanes, {len(o)} survivors, kernel {ms:.3f} ms, "
               f"{eng.batch() / ms * 1e3:.4e} keys/s")
 
 
@@ -622,7 +619,7 @@ def chain_small_case(args):
 
 def suffix_small_case(args):
     """Three advances of a suffix search (og_engine_new_filters, forty
-    eight-symbol suffixes, half 256, one resident wave): the case the suffix
+    eight-symbol suffixes, half 256, one wave of lanes): the case the suffix
     match kernel's ncu summary is captured on."""
     from onion_gen_b200 import _native as N
     from onion_gen_b200 import filter as F
@@ -650,7 +647,7 @@ def config3_small_case(args):
     fs = F.FilterSet.parse_all(workloads.config3_prefixes())
     words, bits = fs.index_words()
     eng = gpu.Engine(dev, key.start_point(workloads.seed(0)), bitmap=words, bitmap_bits=bits,
-                     config=N.EngineConfig(N.SCHEME_PAIRED, args.half, 0, 1, 128, 0, 0, args.lanes_per_thread))
+                     config=N.EngineConfig(N.SCHEME_PAIRED, args.half, 0, 1, 128, 0, 0))
     shape = eng.shape()
     for i in range(3):
         o, _ = eng.advance_raw()

@@ -855,24 +855,22 @@ int og_engine_new(int ordinal, const uint8_t start[128], uint32_t threads, const
         if (build_engine(ordinal, start, cfg, bitmap, words, bits, out, err, errlen) == OG_OK) return OG_OK;
         // the remembered shape no longer builds: measure again
     }
-    // Timed walk over lanes per thread, inversion batch and lanes in flight
-    // (waves of the resident CTAs); the fastest is kept and recorded
-    // (src/gpu/mod.rs:383-411; the reference's OpenCL tuner walks two
-    // dimensions the same way, src/gpu/opencl.rs:207-271).
+    // Timed walk over how many candidates an advance covers, as half and waves of
+    // lanes say it; the fastest is kept and recorded (src/gpu/mod.rs:383-411; the
+    // reference's OpenCL tuner walks two dimensions the same way,
+    // src/gpu/opencl.rs:207-271).
     og_engine* best = nullptr;
     double best_rate = -1;
     int last = OG_E_DEVICE;
-    for (uint32_t lpt : {1u, 2u})
+    uint32_t resident = 0;
+    if (const int rc = resident_lanes(ordinal, OG_SCHEME_PAIRED, 128, &resident, err, errlen)) return rc;
     for (uint32_t half : {512u, 1024u, 2048u}) {
-        uint32_t resident = 0;
-        if (resident_lanes(ordinal, OG_SCHEME_PAIRED, 128, &resident, err, errlen, lpt) != OG_OK) continue;
         for (uint32_t mult : {2u, 4u, 8u}) {
             og_engine_config c{};
             c.scheme = OG_SCHEME_PAIRED;
             c.half = half;
             c.lanes = resident * mult;
             c.block = 128;
-            c.lanes_per_thread = lpt;
             og_engine* e = nullptr;
             last = build_engine(ordinal, start, c, bitmap, words, bits, &e, err, errlen);
             if (last != OG_OK) continue;
