@@ -140,6 +140,11 @@ int og_engine_advance(og_engine* e, og_survivor* out, size_t cap, size_t* n, cha
 int og_engine_launch(og_engine* e, char* err, size_t errlen);
 int og_engine_collect(og_engine* e, og_survivor* out, size_t cap, size_t* n, char* err, size_t errlen);
 
+/* For tests of the failure path: the next advance collected counts as one whose
+ * kernel's wait ran out (OG_E_TIMEOUT; the engine is then closed). The fault is
+ * made on the host; nothing on the device changes. */
+int og_engine_plant_timeout(og_engine* e);
+
 /* Device time of the last collected advance's search kernel, milliseconds
  * (CUDA events on the engine's stream). */
 float og_engine_last_kernel_ms(const og_engine* e);
@@ -323,6 +328,9 @@ void og_batch_memory(const og_batch* b, uint64_t* used, uint64_t* budget);
  * that it verifies as one that did not re-derive. The fault is made on the
  * host; nothing on the device changes. */
 int og_batch_plant_mismatch(og_batch* b, uint64_t search_id);
+/* The same for a wait of the search kernel: the next step collected counts as one
+ * whose wait ran out (OG_E_TIMEOUT; the batch is then closed). */
+int og_batch_plant_timeout(og_batch* b);
 void og_batch_free(og_batch* b);
 
 /* ---- serving: a request loop over the batched engine -------------------

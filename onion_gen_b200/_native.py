@@ -181,6 +181,8 @@ def _load():
     sig("og_batch_last_step_launches", U32, [P])
     sig("og_batch_memory", None, [P, C.POINTER(U64), C.POINTER(U64)])
     sig("og_batch_plant_mismatch", I, [P, U64])
+    sig("og_batch_plant_timeout", I, [P])
+    sig("og_engine_plant_timeout", I, [P])
     sig("og_batch_free", None, [P])
     sig("og_serve_new", I, [I, C.POINTER(ServeConfig), C.POINTER(P), B, SZ])
     sig("og_serve_submit", I, [P, U64, B, B, U32, B, SZ])

@@ -400,6 +400,7 @@ struct og_batch {
     uint64_t last_candidates = 0;
     uint32_t last_launches = 0;
     uint32_t dirty_lo = NONE, dirty_hi = 0;
+    bool planted_timeout = false;  // the next step collected counts as one whose wait ran out (tests)
     std::set<uint64_t> planted;  // searches whose next hit is treated as not re-deriving (tests)
 
     ~og_batch() {
@@ -778,7 +779,7 @@ int collect(og_batch* b, og_batch_hit* out, size_t cap, size_t* n, char* err, si
     cudaEventElapsedTime(&b->last_ms, f.ev0, f.ev1);
     b->last_launches = 3;
     const Counters c = *f.h_counters.p;
-    if (c.failed) return fail(err, errlen, OG_E_TIMEOUT, "a wait of the search kernel ran out");
+    if (c.failed || b->planted_timeout) return fail(err, errlen, OG_E_TIMEOUT, "a wait of the search kernel ran out");
     if (c.surv > f.args.surv_cap || c.hits > f.args.hit_cap)
         return fail(err, errlen, OG_E_OVERFLOW, "a step produced %u survivors (room %u) and %u hits (room %u)", c.surv,
                     f.args.surv_cap, c.hits, f.args.hit_cap);
@@ -1365,6 +1366,12 @@ int og_batch_plant_mismatch(og_batch* b, uint64_t search_id) {
     if (!b) return OG_E_ARG;
     if (!b->searches.count(search_id)) return OG_E_STATE;
     b->planted.insert(search_id);
+    return OG_OK;
+}
+
+int og_batch_plant_timeout(og_batch* b) {
+    if (!b) return OG_E_ARG;
+    b->planted_timeout = true;
     return OG_OK;
 }
 

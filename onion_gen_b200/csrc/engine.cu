@@ -189,6 +189,7 @@ struct og_engine {
     uint64_t launches = 0;
     float last_ms = 0;
     bool overflowed = false;
+    bool planted = false;  // the next advance collected counts as one whose wait ran out (tests)
     DevBuf<uint4> lanes, scratch, table;
     DevBuf<uint32_t> bitmap;
     // Two advances can be in flight (og_engine_launch / og_engine_collect):
@@ -674,7 +675,7 @@ int collect_flight(og_engine* e, bool match, uint32_t* count, uint64_t* launch, 
     CU(cudaEventSynchronize(f.done));
     cudaEventElapsedTime(&e->last_ms, f.ev0, f.ev1);
     *launch = f.launch;
-    if (f.h_counts.p[4]) {
+    if (f.h_counts.p[4] || e->planted) {
         e->overflowed = true;
         return fail(err, errlen, OG_E_TIMEOUT, "a wait of the search kernel ran out; the engine is closed");
     }
@@ -1026,6 +1027,12 @@ int og_engine_advance_matches(og_engine* e, og_match* out, size_t cap, size_t* n
     const int rc = og_engine_launch_matches(e, err, errlen);
     if (rc != OG_OK) return rc;
     return og_engine_collect_matches(e, out, cap, n, err, errlen);
+}
+
+int og_engine_plant_timeout(og_engine* e) {
+    if (!e) return OG_E_ARG;
+    e->planted = true;
+    return OG_OK;
 }
 
 void og_engine_free(og_engine* e) { delete e; }
