@@ -207,6 +207,9 @@ __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) batch_search_
         uint4* const scr = a.scratch + blockIdx.x * a.cta_scratch + threadIdx.x;
         uint4* const centre = a.lanes + (size_t)item.place * BLOCK + threadIdx.x;
         const uint32_t lane = item.lane0 + threadIdx.x;
+        // Suffix searches run in full here, 9.7e7 candidates of 16 of them 3.6 ms a step
+        // (5.9 by the addition formula; the engine's kernel for suffixes alone 1.9): the
+        // loop for suffix bitmaps would be a third copy of the round in this kernel.
         if (sink_kind(d.bitmap ? d.bits : 0, d.sbitmap ? d.sbits : 0) == SINK_PREFIX)
             paired_rounds<false, false, false>(centre, a.slots, d.between, d.last, a.table, d.item_half, d.rounds, scr, sink, sh, mu,
                                  lane, true);
@@ -550,8 +553,13 @@ uint64_t step_candidates(const og_batch* b, const Search& s) {
 
 // Time of `items` items with windows of `groups` groups, in items a CTA: an SM
 // takes four at a time, and for a rest of one, two or three 2.7, 2.9 or 3.3
-// quarters of that (fewer warps keep its pipes less busy); an item's own cost is
-// that of about 20 groups (the prologue, the inversion, the next centre).
+// quarters of that (fewer warps keep its pipes less busy); an item's own cost counts
+// as 20 groups (the prologue, the inversion, the next centre). It is about 10 since
+// the inversion takes a third of what it did, but with 10 here 13 of 14 pools ran
+// within 0.7 % of this and one 36 % slower (half 64, 94720 lanes, 40 searches, three
+// CTAs an SM: 0.31 and 0.42 ms a step). Four at a time holds for the CTAs that fit;
+// for fewer (og_batch_config.grid) it is only a guess: 4.9e7 candidates of 16 searches
+// 1.99, 1.21 and 0.96 ms at one, two and four.
 double items_cost(uint64_t items, uint32_t sms, double groups) {
     static constexpr double REST[4] = {0.0, 2.7, 2.9, 3.3};
     const uint64_t per_sm = (items + sms - 1) / sms;

@@ -284,13 +284,14 @@ struct Tile {
 
 // As few rounds a CTA as the scratch allows, all of the same length, and no
 // CTA left with one more than the others. A round's own cost (the prologue, the
-// block's inversion, the next centre) is that of about 20 groups of three pairs
+// block's inversion, the next centre) is that of about 10 groups of three pairs
 // when every CTA of an SM pays it at once, and a last wave that some CTAs skip
-// costs nearly a whole one. On B200, ms a launch with 1, 2, 3 and 6 rounds a
-// CTA: 9.7e7 candidates 0.94, 1.10, 1.20, 1.48; 1.9e8 3.50, 3.66, 3.75, 4.05; the
-// callers' shapes (half 256, 333 and 512) ran 1.90 for 1.9e8 at half 256, 2.43
-// for 7.7e7 (now 1.45), and 3.49. 3.1e9 candidates: 9 rounds 51.7, 6 51.6 with
-// half as much scratch again, 10 (the caller's half 2048) 53.0, 20 53.2.
+// costs nearly a whole one. On B200, ms a launch with 1, 2, 3, 6 and 12 rounds a
+// CTA: 4.9e7 candidates 0.91, 0.99, 1.07, 1.24, 1.63; 9.7e7 1.73, 1.83, 1.83, 2.05,
+// 2.50; 1.9e8 3.38, 3.48, 3.37, 3.64, 4.09. Longer launches care less: 3.9e8 6.77 with
+// two, the fewest that the scratch holds, 6.47, 6.93 and 7.05; 3.1e9 49.9 with nine
+// to twelve. In the callers' windows, when this came in, half 256 took 1.90 for
+// 9.7e7, half 333 2.43 for 7.7e7 (1.40 so).
 //
 // `own` is the scratch that the callers' windows would take on the resident lanes.
 // Windows that take more are cut where scratch_limit says: a search of a small half

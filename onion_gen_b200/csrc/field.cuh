@@ -162,7 +162,9 @@ __device__ __forceinline__ fe fe_one() {
 // are decided by the low words alone and gathered in a matrix (u v; q r), which
 // then goes onto (f, g), exactly divisible by 2^30, and onto (d, e) from (0, 1),
 // divisible after adding a multiple of p, so that d x = f (mod p) throughout.
-// Numbers are nine signed limbs of 30 bits, p = 2^15 2^240 - 19 with two of them.
+// Numbers are nine signed limbs of 30 bits, the layout of libsecp256k1's 32-bit
+// modular inversion, of which the names of the matrix and the sums are too; p =
+// 2^15 2^240 - 19 has two of them.
 // |d| and |e| grow by at most p / 2 in thirty steps, below 13 p. One thread's
 // latency is what counts (block_invert): on B200 29 000 clocks (35 000 with the
 // steps' zeros counted instead of taken one by one), the power x^(p - 2) by 254

@@ -9,8 +9,10 @@
 
 // Register budget of the search kernels: at most OG_LB_THREADS threads per
 // block and at least OG_LB_MIN_BLOCKS resident blocks per SM. 128 x 4 gives
-// them 128 registers (16 warps per SM); the paired kernel ran 52.6 ms a launch
-// of 3.1e9 candidates so, 54.3 at 96 registers (20 warps), 56.0 at 168.
+// them 128 registers (16 warps per SM); the paired kernel runs 49.9 ms a launch
+// of 3.1e9 candidates so, 51.9 at 96 registers (20 warps) and 51.9 at 168 (12);
+// 9.7e7 candidates 1.74, 1.86 and 1.75. ptxas reports 244 bytes of spill stores
+// and 120 of loads at 128.
 #ifndef OG_LB_MIN_BLOCKS
 #define OG_LB_MIN_BLOCKS 4
 #endif
@@ -27,7 +29,7 @@ __global__ void __launch_bounds__(OG_LB_THREADS) init_kernel(const InitArgs a, c
 // The search, bound by the multiply-add pipe. Persistent: each CTA takes the
 // next block of lanes until none is left; its scratch belongs to the CTA, not
 // the lanes. On B200 at half 2048, 757 760 lanes and one 6-symbol prefix a
-// launch takes 52.6 ms (5.9e10 keys/s); ten multiplications a pair took 147.
+// launch takes 49.9 ms (6.2e10 keys/s); ten multiplications a pair took 147.
 template <SinkKind Kind>
 __global__ void __launch_bounds__(OG_LB_THREADS, OG_LB_MIN_BLOCKS) paired_kernel(const PairedArgs a) {
     __shared__ uint32_t item_s;

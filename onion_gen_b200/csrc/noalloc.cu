@@ -60,7 +60,7 @@ size_t tile_uint4(uint32_t half, uint32_t ctas, SinkKind kind) {
 
 // All `resident` blocks, in one round where the array holds the scratch of
 // windows that long, else in as many as it takes (a round's own cost is that of
-// about 20 groups of three pairs, so the longest windows that fit: on 592 CTAs 12
+// about 10 groups of three pairs, so the longest windows that fit: on 592 CTAs 12
 // groups; while room was kept to compute every key in full, 8, and 4.05e7 candidates
 // took 1.77 ms for 1.60). Windows of at least two groups.
 NoAllocTile plan_tile(uint64_t candidates, uint32_t resident, SinkKind kind) {

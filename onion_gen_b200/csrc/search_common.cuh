@@ -388,12 +388,12 @@ __device__ __forceinline__ void stage_push(const Sink& k, const PairTable& tab, 
 // ---- the matrix product of a group --------------------------------------
 //
 // For the block's 128 lanes, rows (lanes) x 192 bytes times 192 x 48
-// constants (eight columns for each of the group's six keys): six tcgen05.mma of kind::i8, unsigned, K = 32, issued by one thread, sums in
-// 48 columns of tensor memory, read back a lane's row by its own thread. It
+// constants (eight columns for each of the group's six keys): six tcgen05.mma of
+// kind::i8, unsigned, K = 32, issued by one thread, sums in 48 columns of tensor memory, read back a lane's row by its own thread. It
 // runs while the warps multiply for the next group. The constants come by a
-// bulk copy, 9 KB a group for the whole block. Measured on B200 at half 2048
-// and 757 760 lanes: 52.6 ms a launch, 47.0 with the products left out; by
-// mma.sync a warp, which shares registers and issue slots with the
+// bulk copy, 9 KB a group for the whole block. Measured on B200 at 3.1e9
+// candidates a launch when it came in: 52.6 ms (49.9 now), 47.0 with the products
+// left out; by mma.sync a warp, which shares registers and issue slots with the
 // multiplications, 64.2; with the keys' low limbs by multiply-adds, four
 // multiplications and two partial ones a pair, 70.3.
 constexpr uint32_t KEY_COLUMNS = 8;
@@ -737,8 +737,10 @@ __device__ __forceinline__ void paired_rounds(uint4* centre, size_t cstride, con
 }
 
 // The same rounds with every key computed in full: for sinks with wider bitmaps
-// than paired_rounds reads, or with none (every candidate survives). A pair takes six multiplications: per pair the prefix
-// product, w = P I [= z / D], I <- I D, f = e w and y = v w +- s f.
+// than paired_rounds reads, or with none (every candidate survives), and for any
+// start. A pair takes six multiplications: per pair the prefix product, w = P I
+// [= z / D], I <- I D, f = e w and y = v w +- s f. 3.9e8 candidates against a
+// bitmap of 25 bits 13.4 ms, of 24 bits by paired_rounds 6.9.
 template <bool AnyStart>
 __device__ __forceinline__ void paired_rounds_full(uint4* centre, size_t cstride, const Stride& between,
                                                    const Stride& last, const PairTable& tab, uint32_t half,

@@ -55,9 +55,9 @@ def look():
 
 
 def resident_lanes(device, scheme=None, block=128):
-    """Lanes one wave of the search kernel holds on ``device``: resident
-    blocks per SM x SMs x ``block``. The paired kernel runs exactly this
-    many threads; its lanes are taken a block at a time."""
+    """The lanes that default shapes are counted in waves of on ``device``: a
+    fixed number of blocks per SM (five of 128) x SMs x ``block``. How many
+    threads the search kernel runs is its own choice."""
     n = C.c_uint32()
     err = N.errbuf()
     scheme = N.SCHEME_PAIRED if scheme is None else scheme
